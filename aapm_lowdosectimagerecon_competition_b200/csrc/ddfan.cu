@@ -238,14 +238,8 @@ void boundaries(int n, const float* c, std::vector<double>& out) {
 // creation precedes every launch on a plan and never runs under capture.
 int dd_prepare_device(int dev) {
   cudaError_t e = cudaSuccess;
-#define DDFAN_DD_ALLOW(ZLv, NZv)                                                                  \
-  if (e == cudaSuccess)                                                                           \
-    e = dd_allow_dyn(k_fwd_dd<ZLv, DdFwdCG<ZLv>::v, NZv>, DdFwdTile<ZLv, DdFwdCG<ZLv>::v, NZv>::DYN);
-  DDFAN_DD_ALLOW(8, 4) DDFAN_DD_ALLOW(8, 2) DDFAN_DD_ALLOW(8, 1)
-  DDFAN_DD_ALLOW(4, 4) DDFAN_DD_ALLOW(4, 2) DDFAN_DD_ALLOW(4, 1)
-  DDFAN_DD_ALLOW(2, 4) DDFAN_DD_ALLOW(2, 2) DDFAN_DD_ALLOW(2, 1)
-  DDFAN_DD_ALLOW(1, 4) DDFAN_DD_ALLOW(1, 2) DDFAN_DD_ALLOW(1, 1)
-#undef DDFAN_DD_ALLOW
+  if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd<8>, DdFwdTile<8>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd<4>, DdFwdTile<4>::DYN);
   if (e != cudaSuccess)
     return set_err(DDFAN_ERR_CUDA, "forward kernel attributes on device %d: %s", dev, cudaGetErrorString(e));
   return DDFAN_OK;
@@ -658,57 +652,63 @@ int launch_publish_masked(const float* x, int Zi, const float* x0, int Z, const 
   return check_launch("k_publish_masked");
 }
 
-template <int ZL>
-static void fwd_dd_go(const DdFwdArgs& a, int nzt, cudaStream_t st) {
-  constexpr int CG = DdFwdCG<ZL>::v;
-  constexpr int kMaxRows = DDFAN_DD_FWD_ROWS_X ? (1 << 30) : 65535;  // grid x / y limit
-  const auto go = [&](auto nz) {
-    constexpr int NZ = decltype(nz)::value;
-    using T = DdFwdTile<ZL, CG, NZ>;
-    for (int r0 = 0; r0 < a.PN; r0 += kMaxRows) {
-      DdFwdArgs b = a;
-      b.row0 = r0;
-      const int rows = std::min(a.PN - r0, kMaxRows), cblk = (a.U + T::CW - 1) / T::CW;
-      const dim3 grid(DDFAN_DD_FWD_ROWS_X ? rows : cblk, DDFAN_DD_FWD_ROWS_X ? cblk : rows, (nzt + NZ - 1) / NZ);
-      k_fwd_dd<ZL, CG, NZ><<<grid, T::NT, T::DYN, st>>>(b);
-    }
-  };
-  switch (dd_nz(nzt, a.nzc)) {
-    case 4: go(std::integral_constant<int, 4>()); break;
-    case 2: go(std::integral_constant<int, 2>()); break;
-    default: go(std::integral_constant<int, 1>()); break;
+// Lanes per group (vectors per z-tile) of the direct kernels for nvb vectors
+// of slices: at most a warp's 32, and of the splits into z-tiles the one that
+// leaves the fewest lanes idle -- 32 / zl groups fill a warp only when zl
+// divides it well, and the last tile may be short.  Every extra tile decodes
+// the walks again (a third of a walk's own cost at 4 lanes), hence the 10 %.
+int dd_lanes(int nvb) {
+  int best = 1;
+  double bc = 1e300;
+  for (int nt = (nvb + 31) / 32; nt <= std::max(1, (nvb + 3) / 4); ++nt) {
+    const int zl = (nvb + nt - 1) / nt;
+    const double c = (double)nt / (32 / zl) * (1.0 + 0.1 * (nt - 1));
+    if (c < bc - 1e-9) { bc = c; best = zl; }
   }
+  return best;
 }
 
 DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc,
                            const float* cvd, const int* order, int PN, float* out, int orow, int ostride, int zlo,
                            int zhi, const DdResidual* res) {
   DdFwdArgs a{};
-  a.img = reinterpret_cast<const float4*>(img); a.P4 = p.P4;
+  const int Zs = 4 * p.P4;  // slices of an image pixel
+  a.sv = Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(img) & 31) == 0 ? 8 : 4;
+  a.img = img; a.ZP = Zs / a.sv;
   a.vg = vg; a.fc = fc; a.cvd = cvd; a.order = order;
   a.out = out; a.orow = orow; a.ostride = ostride;
-  a.PN = PN; a.U = p.U; a.Z = p.Z; a.XN = p.XN; a.YN = p.YN; a.dx = (float)p.dx;
-  a.zlo = zlo; a.zhi = zhi < 0 ? p.Z : zhi; a.row0 = 0; a.nzc = p.NZ;
+  a.PN = PN; a.U = p.U; a.XN = p.XN; a.YN = p.YN; a.dx = (float)p.dx;
+  a.zlo = std::max(0, zlo); a.zhi = zhi < 0 ? p.Z : std::min(zhi, p.Z);
+  a.vb0 = a.zlo / a.sv;
+  a.nvb = a.zhi > a.zlo ? (a.zhi + a.sv - 1) / a.sv - a.vb0 : 0;
+  a.zl = dd_lanes(std::max(a.nvb, 1));
+  a.nzt = (a.nvb + a.zl - 1) / a.zl;
+  // a launch of fewer warps than the SMs hold (24 each) splits every ray's
+  // lines over 2, 4 or 8 of them
+  const int cww = 32 / a.zl * DDFAN_DD_FWD_CG;
+  const long long warps = (long long)PN * ((p.U + cww - 1) / cww) * a.nzt;
+  a.nseg = 1;
+  while (a.nseg < 8 && warps * a.nseg < 148 * 24) a.nseg *= 2;
   if (res) {
     a.y = res->y; a.yview = res->yview; a.rowsum = res->rowsum; a.wgt = res->wgt; a.ystride = res->ystride;
   }
-  ztile_range(p, zlo, zhi, &a.zt0, &a.nzt);
   return a;
+}
+
+int dd_fwd_cblocks(const DdFwdArgs& a) {
+  const int cw = 32 / a.zl * DDFAN_DD_FWD_CG * (8 / a.nseg);
+  return (a.U + cw - 1) / cw;
 }
 
 int launch_fwd_dd(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc, const float* cvd,
                   const int* order, int PN, float* out, int orow, int ostride, int zlo, int zhi,
                   const DdResidual* res, cudaStream_t st) {
   const DdFwdArgs a = make_fwd_dd_args(p, img, vg, fc, cvd, order, PN, out, orow, ostride, zlo, zhi, res);
-  const int nzt = a.nzt;
-  if (nzt == 0 || PN < 1) return DDFAN_OK;
+  if (a.nvb == 0 || PN < 1) return DDFAN_OK;
   ProfScope ps(KIND_FWD, st);
-  switch (p.ZL) {
-    case 8: fwd_dd_go<8>(a, nzt, st); break;
-    case 4: fwd_dd_go<4>(a, nzt, st); break;
-    case 2: fwd_dd_go<2>(a, nzt, st); break;
-    default: fwd_dd_go<1>(a, nzt, st); break;
-  }
+  const dim3 grid(PN, dd_fwd_cblocks(a), a.nzt);
+  if (a.sv == 8) k_fwd_dd<8><<<grid, DdFwdTile<8>::NT, DdFwdTile<8>::DYN, st>>>(a);
+  else k_fwd_dd<4><<<grid, DdFwdTile<4>::NT, DdFwdTile<4>::DYN, st>>>(a);
   return check_launch("k_fwd_dd");
 }
 

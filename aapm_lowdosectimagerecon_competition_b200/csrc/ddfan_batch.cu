@@ -37,27 +37,10 @@ namespace {
 enum BatchKind { BK_FWD = 0, BK_ADJ_X = 1, BK_ADJ_Y = 2, BK_REF = 3 };
 
 struct BatchLaunch {
-  int kind, ZL, NZ;
+  int kind, ZL, NZ;  // forward: slices per thread, 0
   size_t items_off, nitems;
   int group;  // the solver group whose chain the launch belongs to
 };
-
-int fwd_cw(int ZL, int NZ) {
-  switch (ZL * 8 + NZ) {
-    case 8 * 8 + 4: return DdFwdTile<8, DdFwdCG<8>::v, 4>::CW;
-    case 8 * 8 + 2: return DdFwdTile<8, DdFwdCG<8>::v, 2>::CW;
-    case 8 * 8 + 1: return DdFwdTile<8, DdFwdCG<8>::v, 1>::CW;
-    case 4 * 8 + 4: return DdFwdTile<4, DdFwdCG<4>::v, 4>::CW;
-    case 4 * 8 + 2: return DdFwdTile<4, DdFwdCG<4>::v, 2>::CW;
-    case 4 * 8 + 1: return DdFwdTile<4, DdFwdCG<4>::v, 1>::CW;
-    case 2 * 8 + 4: return DdFwdTile<2, DdFwdCG<2>::v, 4>::CW;
-    case 2 * 8 + 2: return DdFwdTile<2, DdFwdCG<2>::v, 2>::CW;
-    case 2 * 8 + 1: return DdFwdTile<2, DdFwdCG<2>::v, 1>::CW;
-    case 1 * 8 + 4: return DdFwdTile<1, DdFwdCG<1>::v, 4>::CW;
-    case 1 * 8 + 2: return DdFwdTile<1, DdFwdCG<1>::v, 2>::CW;
-    default: return DdFwdTile<1, DdFwdCG<1>::v, 1>::CW;
-  }
-}
 
 // (lines per tile, voxels per line per tile) of the direct exact adjoint and
 // of the REF backprojector
@@ -68,11 +51,6 @@ void adj_tile(int ZL, int* LT, int* KT) {
     case 2: *LT = DdBackTile<2>::LT; *KT = DdBackTile<2>::KT; break;
     default: *LT = DdBackTile<1>::LT; *KT = DdBackTile<1>::KT; break;
   }
-}
-
-template <int ZL, int NZ>
-void go_fwd(const DdFwdArgs* a, const int4* it, unsigned n, cudaStream_t st) {
-  k_fwd_dd_batch<ZL, DdFwdCG<ZL>::v, NZ><<<n, 256, DdFwdTile<ZL, DdFwdCG<ZL>::v, NZ>::DYN, st>>>(a, it);
 }
 
 template <int ZL, int NZ>
@@ -96,14 +74,8 @@ void go_ref(const DdRefArgs* a, const int4* it, unsigned n, cudaStream_t st) {
 // (at every batch creation: the attribute belongs to the context)
 int batch_prepare_device(int dev) {
   cudaError_t e = cudaSuccess;
-#define DDFAN_DD_ALLOW(ZLv, NZv)                                                                        \
-  if (e == cudaSuccess)                                                                                 \
-    e = dd_allow_dyn(k_fwd_dd_batch<ZLv, DdFwdCG<ZLv>::v, NZv>, DdFwdTile<ZLv, DdFwdCG<ZLv>::v, NZv>::DYN);
-  DDFAN_DD_ALLOW(8, 4) DDFAN_DD_ALLOW(8, 2) DDFAN_DD_ALLOW(8, 1)
-  DDFAN_DD_ALLOW(4, 4) DDFAN_DD_ALLOW(4, 2) DDFAN_DD_ALLOW(4, 1)
-  DDFAN_DD_ALLOW(2, 4) DDFAN_DD_ALLOW(2, 2) DDFAN_DD_ALLOW(2, 1)
-  DDFAN_DD_ALLOW(1, 4) DDFAN_DD_ALLOW(1, 2) DDFAN_DD_ALLOW(1, 1)
-#undef DDFAN_DD_ALLOW
+  if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd_batch<8>, DdFwdTile<8>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd_batch<4>, DdFwdTile<4>::DYN);
   if (e != cudaSuccess)
     return set_err(DDFAN_ERR_CUDA, "batched forward kernel attributes on device %d: %s", dev, cudaGetErrorString(e));
   return DDFAN_OK;
@@ -171,20 +143,8 @@ static int batch_launch(Batch& b, const BatchLaunch& L, cudaStream_t st) {
     const unsigned n = (unsigned)L.nitems;
     if (L.kind == BK_FWD) {
       ProfScope ps(KIND_FWD, st);
-      do {
-        DDFAN_BATCH_ZL_NZ(8, 4, (go_fwd<8, 4>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(8, 2, (go_fwd<8, 2>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(8, 1, (go_fwd<8, 1>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 4, (go_fwd<4, 4>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 2, (go_fwd<4, 2>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 1, (go_fwd<4, 1>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 4, (go_fwd<2, 4>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 2, (go_fwd<2, 2>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 1, (go_fwd<2, 1>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 4, (go_fwd<1, 4>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 2, (go_fwd<1, 2>(b.d_fargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 1, (go_fwd<1, 1>(b.d_fargs, it, n, st)))
-      } while (0);
+      if (L.ZL == 8) k_fwd_dd_batch<8><<<n, DdFwdTile<8>::NT, DdFwdTile<8>::DYN, st>>>(b.d_fargs, it);
+      else k_fwd_dd_batch<4><<<n, DdFwdTile<4>::NT, DdFwdTile<4>::DYN, st>>>(b.d_fargs, it);
     } else if (L.kind == BK_ADJ_X || L.kind == BK_ADJ_Y) {
       const bool xm = L.kind == BK_ADJ_X;
       ProfScope ps(xm ? KIND_BACK_A : KIND_BACK_B, st);
@@ -323,24 +283,17 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
       r.y = s.d_y; r.yview = s.d_yview + o; r.rowsum = s.d_rows + (size_t)o * s.U; r.wgt = adj ? cvd : nullptr;
       r.ystride = s.Zi;
       const DdFwdArgs fa = make_fwd_dd_args(p, s.d_x, vg, fc, cvd, s.d_order + o, c, s.d_ax, s.U + 1, s.Zi, 0, s.Zi, &r);
-      if (fa.nzt < 1) continue;
-      const int fnz = dd_nz(fa.nzt, fa.nzc);
+      if (fa.nvb < 1) continue;
       const int fi = (int)fargs.size();
       fargs.push_back(fa);
-      const int cw = fwd_cw(p.ZL, fnz), ncb = (s.U + cw - 1) / cw, nzg = (fa.nzt + fnz - 1) / fnz;
-      // z-tile groups outermost and the rest in the single-solve grid's
-      // order: the CTAs in flight share one group's slices, whose image part
+      const int ncb = dd_fwd_cblocks(fa);
+      // z-tiles outermost and the rest in the single-solve grid's
+      // order: the CTAs in flight share one tile's slices, whose image part
       // then stays in L2
-      auto& fl = fwd[{p.ZL, fnz}];
-      for (int zg = 0; zg < nzg; ++zg) {
-        if (DDFAN_DD_FWD_ROWS_X) {
-          for (int cb = 0; cb < ncb; ++cb)
-            for (int row = 0; row < c; ++row) fl.push_back(make_int4(fi, row, cb, zg));
-        } else {
-          for (int row = 0; row < c; ++row)
-            for (int cb = 0; cb < ncb; ++cb) fl.push_back(make_int4(fi, row, cb, zg));
-        }
-      }
+      auto& fl = fwd[{fa.sv, 0}];
+      for (int zt = 0; zt < fa.nzt; ++zt)
+        for (int cb = 0; cb < ncb; ++cb)
+          for (int row = 0; row < c; ++row) fl.push_back(make_int4(fi, row, cb, zt));
       BackEpi e{};
       e.out = s.d_x; e.xin = s.d_x; e.colsum = s.d_cols + (size_t)k * s.XN * s.YN;
       e.nonneg = s.nonneg; e.mask = p.has_mask ? p.d_mask : nullptr; e.zlo = 0; e.zhi = s.Zi;

@@ -29,10 +29,10 @@
 namespace ddfan {
 
 // Resident CTAs per SM the register allocation is sized for (256 threads:
-// 2 -> up to 128 registers, which the 4-z-tile accumulators need without
-// spilling).  Build-time knobs for tuning sweeps, like the tile shapes below.
+// 2 -> up to 128 registers, which the backprojectors' 4-z-tile accumulators
+// need without spilling; 3 -> 80 for the forward).  Build-time knobs for tuning sweeps, like the tile shapes below.
 #ifndef DDFAN_DD_FWD_MIN_CTAS
-#define DDFAN_DD_FWD_MIN_CTAS 2
+#define DDFAN_DD_FWD_MIN_CTAS 3
 #endif
 #ifndef DDFAN_DD_BACK_MIN_CTAS
 #define DDFAN_DD_BACK_MIN_CTAS 2
@@ -166,21 +166,81 @@ __device__ __forceinline__ void walk_nz(float (&acc)[NZ][4], float4 (&cur)[NZ], 
   }
 }
 
+// ============================================================ vectors of slices
+
+// The slices a thread owns, loaded at once: 8 (32 bytes, one 256-bit load --
+// half the load instructions and address arithmetic of two 128-bit ones), 4
+// (16 bytes) or 1.  8 and 4 are kept as pairs for fma.rn.f32x2.
+using u64 = unsigned long long;
+
+template <int SV> struct Vec {
+  static constexpr int Q = SV / 2;
+  u64 q[Q];
+};
+template <> struct Vec<1> {
+  float f;
+};
+
+__device__ __forceinline__ void vload(Vec<8>& v, const char* p) {
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+      : "=l"(v.q[0]), "=l"(v.q[1]), "=l"(v.q[2]), "=l"(v.q[3])
+      : "l"(p));
+}
+__device__ __forceinline__ void vload(Vec<4>& v, const char* p) {
+  asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(v.q[0]), "=l"(v.q[1]) : "l"(p));
+}
+__device__ __forceinline__ void vload(Vec<1>& v, const char* p) { v.f = __ldg(reinterpret_cast<const float*>(p)); }
+
+constexpr unsigned DD_INNER = 0x80000000u;  // the walk has an interior value (offsets stay below 2^31 vectors)
+
+// w in both halves of a 64-bit word
+__device__ __forceinline__ u64 dup2(float w) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(w));
+  return r;
+}
+__device__ __forceinline__ float lo2(u64 w) { return __uint_as_float((unsigned)w); }
+__device__ __forceinline__ float hi2(u64 w) { return __uint_as_float((unsigned)(w >> 32)); }
+
+// a += w v (w in both halves of ww)
+template <int SV>
+__device__ __forceinline__ void vfma(Vec<SV>& a, u64 ww, const Vec<SV>& v) {
+#pragma unroll
+  for (int i = 0; i < Vec<SV>::Q; ++i) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a.q[i]) : "l"(ww), "l"(v.q[i]));
+}
+__device__ __forceinline__ void vfma(Vec<1>& a, u64 ww, const Vec<1>& v) { a.f = fmaf(lo2(ww), v.f, a.f); }
+
+template <int SV>
+__device__ __forceinline__ void vzero(Vec<SV>& a) {
+#pragma unroll
+  for (int i = 0; i < Vec<SV>::Q; ++i) a.q[i] = 0ull;
+}
+__device__ __forceinline__ void vzero(Vec<1>& a) { a.f = 0.f; }
+
+template <int SV>
+__device__ __forceinline__ float vget(const Vec<SV>& a, int s) {
+  return (s & 1) ? hi2(a.q[s >> 1]) : lo2(a.q[s >> 1]);
+}
+__device__ __forceinline__ float vget(const Vec<1>& a, int) { return a.f; }
+
 // ============================================================ forward projector
 
 struct DdFwdArgs {
-  const float4* img;   // masked image [YN][XN][P4]
-  int P4;
+  const float* img;    // masked image [YN][XN][ZP vectors of SV slices]
+  int ZP;
   const ViewGeom* vg;
   const double2* fc;   // [PN][U+1] boundary lines
   const float* cvd;    // [PN][U] 1 / |dir.axis|
   const int* order;    // CTA row -> view, x-major first (null = identity)
   float* out;          // [slot][orow][ostride]
   int orow, ostride;
-  int PN, U, Z, XN, YN;
+  int PN, U, XN, YN;
   float dx;
-  int zlo, zhi, zt0, nzt, row0;
-  int nzc;             // most z-tiles per thread (launch shape; the kernel reads NZ)
+  int zlo, zhi;        // slices written
+  int sv;              // slices per thread (the kernel's SV)
+  int zl;              // lanes of a channel group: vectors of a z-tile
+  int vb0, nvb, nzt;   // first vector and vectors of [zlo, zhi); z-tiles of zl vectors
+  int nseg;            // line segments a warp's lines are split into (1, 2, 4 or 8)
   // fused OS-SART residual (AAPM_script/OSSART_AAPM.m:86-88); y null = plain projection
   const float* y;      // measured [views][U][ystride]
   const int* yview;    // slot -> measured view
@@ -189,233 +249,261 @@ struct DdFwdArgs {
   int ystride;
 };
 
-// Lines of a forward chunk unrolled together, geometry elements (line,
-// channel) a warp prepares per chunk, and z-tiles per thread.
-#ifndef DDFAN_DD_FWD_UNROLL
-#define DDFAN_DD_FWD_UNROLL 1
-#endif
-#ifndef DDFAN_DD_FWD_GEOM
-#define DDFAN_DD_FWD_GEOM 256
-#endif
-// Ray sums: 0 = one running FP32 sum per ray; 1 = a sum per chunk of
-// lines in registers, added to the totals, also in registers; 2 = chunk sums
-// in registers, totals in dynamic shared memory (one slot per thread and
-// value, so a chunk's sum is added with one load and one store per value).
-// Chunk sums keep a 512-line ray's rounding at the level of ~CC terms; in
-// registers they spill two channels per thread, in shared memory they cost
-// the registers nothing.
-#ifndef DDFAN_DD_FWD_PART
-#define DDFAN_DD_FWD_PART 2
-#endif
-// geometry chunks per ray-sum chunk (DDFAN_DD_FWD_PART == 2)
-#ifndef DDFAN_DD_FWD_FLUSH
-#define DDFAN_DD_FWD_FLUSH 1
-#endif
-// most z-tiles per thread (1, 2 or 4; fewer when a call has fewer)
-#ifndef DDFAN_DD_NZ
-#define DDFAN_DD_NZ 4
-#endif
-
-// channels per thread of the direct forward projector for a z-lane count:
-// two share the boundary value between them and the per-line decode
-// (c3 subset: 2.16 -> 1.90 ms with one running sum per ray; with chunk sums
-// the extra registers spill and the gain is gone)
+// channels per thread of the forward projector (at most 3: s_m's layout)
 #ifndef DDFAN_DD_FWD_CG
 #define DDFAN_DD_FWD_CG 2
 #endif
-template <int ZL> struct DdFwdCG { static constexpr int v = ZL >= 4 ? DDFAN_DD_FWD_CG : (ZL == 2 ? 2 : 1); };
 
-// z-tiles per thread of the direct kernels: each decoded footprint serves
-// 4 slices per z-tile, so more z-tiles per thread means fewer instructions
-// per slice (the measured lever: 1 -> 4 took a 96-view c3 subset's forward
-// from 3.5 to 2.6 ms); at most the call's z-tiles
-// (at most cap, the plan's tuned value)
-inline int dd_nz(int nzt, int cap) { return nzt >= 4 && cap >= 4 ? 4 : (nzt >= 2 && cap >= 2 ? 2 : 1); }
-
-template <int ZL, int CG, int NZ>
+template <int SV>
 struct DdFwdTile {
   static constexpr int NT = 256, NW = NT / 32;
-  static constexpr int GW = 32 / ZL;                  // channel groups per warp
-  static constexpr int CWW = GW * CG;                 // channels per warp
-  static constexpr int CW = NW * CWW;                 // channels per CTA
-  static constexpr int CC = DDFAN_DD_FWD_GEOM / CWW;  // lines per geometry chunk
-  static constexpr int UNROLL = DDFAN_DD_FWD_UNROLL;
-  // dynamic shared memory of the ray totals (DDFAN_DD_FWD_PART == 2)
-  static constexpr int DYN = DDFAN_DD_FWD_PART == 2 ? CG * NZ * 4 * NT * (int)sizeof(float) : 0;
+  static constexpr int CG = DDFAN_DD_FWD_CG;
+  static constexpr int REC = 128;      // (line, channel) walks a warp decodes at a time
+  static constexpr int FLUSH = 32;     // lines per FP32 partial sum
+  // dynamic shared memory of the ray totals
+  static constexpr int DYN = CG * SV * NT * (int)sizeof(float);
 };
 
-// CTA = one view x CW channels x NZ z-tiles of 4*ZL slices; a thread owns CG
-// consecutive channels x 4 slices in each of its NZ z-tiles and walks their
-// footprints along each line, carrying the value at the boundary two channels
-// share.  Every warp prepares the geometry of its own CWW channels (per chunk
-// of CC lines: each channel's two cell indices and walk weights over
-// 1 / footprint length, MultiSlicesProjGPU.cu:166-170) and synchronises with
-// itself only, so warps interleave FP64 geometry with other warps' gathers.
-template <int ZL, int CG, int NZ>
-__device__ __forceinline__ void fwd_dd_body(const DdFwdArgs& a, int row, int cblk, int zgrp) {
-  using T = DdFwdTile<ZL, CG, NZ>;
-  constexpr int NW = T::NW, CWW = T::CWW, CW = T::CW, CC = T::CC;
-  __shared__ double2 s_fc[NW][CWW + 1];
-  __shared__ float4 s_w[NW][CC][CWW];  // (w0, wm, we) / length; k0 | k1 << 16 as int bits
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const int zl = lane % ZL, gw = lane / ZL;
-  if (row >= a.PN) return;  // uniform per CTA
-  const int slot = a.order ? a.order[row] : row;
-  const int p = slot;
-  const int wc0 = cblk * CW + w * CWW;  // the warp's first channel
-  if (wc0 >= a.U) return;  // uniform per warp; no CTA-wide barrier follows
-  // z-tiles zt0 + zgrp * NZ + z of the call's nzt; block zb = zt * ZL + zl
-  const int zt_first = a.zt0 + zgrp * NZ;
-  int zbk[NZ], zoff[NZ];
-  bool zok[NZ];
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) {
-    zbk[z] = (zt_first + z) * ZL + zl;
-    zok[z] = zgrp * NZ + z < a.nzt && zbk[z] < a.P4;
-    zoff[z] = zok[z] ? z * ZL : 0;  // a tile past the image reads the first one again (dropped)
+// Lines on which a boundary ray c(ii) = ii F + C can lie above 0 and below N,
+// as [pl, ph) and [ql, qh) within [0, nl], rounded outwards.
+__device__ __forceinline__ void dd_line_range(double F, double C, double N, int nl, int& pl, int& ph, int& ql, int& qh) {
+  pl = ql = 0;
+  ph = qh = nl;
+  if (!isfinite(F) || !isfinite(C)) return;
+  if (F == 0.0) {
+    if (!(C > 0.0)) pl = nl, ph = 0;
+    if (!(C < N)) ql = nl, qh = 0;
+    return;
   }
+  const double r = 1.0 / F, top = (double)nl;
+  const double z0 = fmin(fmax(-C * r, -2.0), top + 2.0), zN = fmin(fmax((N - C) * r, -2.0), top + 2.0);
+  const int a0 = (int)floor(z0), aN = (int)floor(zN);
+  if (F > 0.0) {
+    pl = min(max(a0 - 1, 0), nl);
+    qh = min(max(aN + 2, 0), nl);
+  } else {
+    ph = min(max(a0 + 2, 0), nl);
+    ql = min(max(aN - 1, 0), nl);
+  }
+}
+
+// What bounds it (c3 subset, 96 views x 736 channels x 512^2 x 128): the loads'
+// latency, and behind it the L1 pipe -- 1.30 ms, of which 1.0 ms remain when
+// every load hits L1; 14.2 GB cross from L2 (every view reads the image once:
+// 12.9 GB) at 11 TB/s, half of what L2 gives a 64 MB working set.  24 warps an
+// SM at 80 registers and 2 channels a thread beat 16 warps at 128 with 3
+// channels (1.34 ms) or 2 (1.41).  Before: 1.90 ms (4 z-tiles of 4 slices a
+// thread, no lines skipped).
+//
+// Warp = one view x (32 / zl) groups of CG consecutive channels x zl vectors
+// of SV slices; CTA = 8 warps, on consecutive channels (and, when nseg > 1, on
+// nseg segments of the lines, added up in shared memory at the end).  A
+// thread walks its channels' footprints along each line: the value at the
+// boundary two channels share is loaded once, so a line costs CG + 1 loads
+// plus one for every footprint with an interior value, all issued before the
+// first is used.  Every warp decodes its own walks (REC at a time, FP64
+// boundary lines: each channel's two cell offsets and walk weights over
+// 1 / footprint length, MultiSlicesProjGPU.cu:166-170) and synchronises with
+// itself only.  Lines on which none of the warp's footprints meet the image
+// are skipped (their weights are zero): a third of all (channel, line) pairs
+// at the c2 geometry, whose detector covers more than the image.
+template <int SV>
+__device__ __forceinline__ void fwd_dd_body(const DdFwdArgs& a, int row, int cblk, int ztile) {
+  using T = DdFwdTile<SV>;
+  constexpr int NW = T::NW, CG = T::CG, REC = T::REC, VB = SV * 4;
+  static_assert(CG >= 1 && CG <= 3, "s_m holds a start and three interior offsets");
+  __shared__ float4 s_w[NW][REC];         // (w0, wm, we) / length, end offset (bits) of walk (line, j, group)
+  __shared__ uint4 s_m[NW][REC / CG];     // (line, group): start offset, then each channel's interior one
+  extern __shared__ float s_tot[];          // [CG * SV][NT]: this thread's totals at tid
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int ZL = a.zl, GW = 32 / ZL, CWW = GW * CG, CC = REC / CWW;
+  const int g = lane / ZL, zi = lane - g * ZL;
+  const int nseg = a.nseg, wch = w / nseg, seg = w - wch * nseg;
+  const int wc0 = (cblk * (NW / nseg) + wch) * CWW;  // the warp's first channel
+  const int p = a.order ? a.order[row] : row;
+  const bool active = g < GW && ztile * ZL + zi < a.nvb && wc0 + g * CG < a.U;
+  const int vb = a.vb0 + ztile * ZL + zi;
   const bool xm = a.vg[p].xmajor != 0;
   const int nl = xm ? a.XN : a.YN, N = xm ? a.YN : a.XN;
-  for (int b = lane; b <= CWW; b += 32) s_fc[w][b] = a.fc[(size_t)p * (a.U + 1) + min(wc0 + b, a.U)];
-  const bool active = (wc0 + gw * CG < a.U) && zok[0];
-  // x-major views integrate along x columns (line = x, k = y), the others along y rows
-  const size_t P4 = (size_t)a.P4;
-  const size_t kstride = (xm ? (size_t)a.XN : 1) * P4;
-  const size_t lstride = (xm ? 1 : (size_t)a.XN) * P4;
-  const float4* img = a.img + (active ? zbk[0] : 0);
-  float acc[CG][NZ][4];
-  float4 vm[NZ];  // first interior values (kept between walks; see walk_nz)
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) vm[z] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int j = 0; j < CG; ++j)
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) acc[j][z][0] = acc[j][z][1] = acc[j][z][2] = acc[j][z][3] = 0.f;
   const double Nd = (double)N;
-  const float dx = a.dx;
-#if DDFAN_DD_FWD_PART == 2
-  extern __shared__ float s_tot[];  // [CG * NZ * 4][NT]: this thread's totals at tid
+  const double2* fcp = a.fc + (size_t)p * (a.U + 1);
+  // x-major views integrate along x columns (line = x, k = y), the others along y rows
+  const unsigned ks = (unsigned)(xm ? a.XN : 1) * (unsigned)a.ZP;  // vectors from k to k + 1
+  const size_t lstride = (size_t)(xm ? 1 : a.XN) * a.ZP * VB;
+  const char* img0 = reinterpret_cast<const char*>(a.img) + (size_t)(a.vb0 + ztile * ZL) * VB;  // the z-tile's first vector
+  const char* img = img0 + (size_t)(active ? zi : 0) * VB;
   float* tot = s_tot + tid;
 #pragma unroll
-  for (int e = 0; e < CG * NZ * 4; ++e) tot[e * T::NT] = 0.f;
-#endif
-  __syncwarp();
-  for (int ii0 = 0; ii0 < nl; ii0 += CC) {
-    for (int e = lane; e < CC * CWW; e += 32) {
-      const int col = e / CWW, j = e - col * CWW;
+  for (int e = 0; e < CG * SV; ++e) tot[e * T::NT] = 0.f;
+  Vec<SV> acc[CG];
+#pragma unroll
+  for (int j = 0; j < CG; ++j) vzero(acc[j]);
+  // the lines that any of the warp's footprints meet
+  int lo = 0, hi = 0;
+  if (wc0 < a.U) {
+    int pl = nl, ph = 0, ql = nl, qh = 0;
+    for (int b = lane; b <= CWW; b += 32) {
+      const double2 f = __ldg(fcp + min(wc0 + b, a.U));
+      int b0, b1, b2, b3;
+      dd_line_range(f.x, f.y, Nd, nl, b0, b1, b2, b3);
+      pl = min(pl, b0);
+      ph = max(ph, b1);
+      ql = min(ql, b2);
+      qh = max(qh, b3);
+    }
+    pl = __reduce_min_sync(0xffffffffu, pl);
+    ph = __reduce_max_sync(0xffffffffu, ph);
+    ql = __reduce_min_sync(0xffffffffu, ql);
+    qh = __reduce_max_sync(0xffffffffu, qh);
+    lo = max(pl, ql);
+    hi = max(lo, min(ph, qh));
+  }
+  if (nseg > 1) {
+    const int n = hi - lo, l0 = lo;
+    lo = l0 + n * seg / nseg;
+    hi = l0 + n * (seg + 1) / nseg;
+  }
+  const float dx = a.dx;
+  const float icww = 1.f / (float)CWW;
+  int since = 0;
+  for (int ii0 = lo; ii0 < hi; ii0 += CC) {
+    const int ncol = min(CC, hi - ii0);
+    bool wide = false;
+#pragma unroll 1
+    for (int e = lane; e < ncol * CWW; e += 32) {
+      const int col = (int)(((float)e + 0.5f) * icww), r = e - col * CWW;
+      const int gg = r / CG, j = r - gg * CG;
+      const int u = wc0 + gg * CG + j;
       const double di = (double)(ii0 + col);
-      const double2 fa = s_fc[w][j], fb = s_fc[w][j + 1];
+      const double2 fa = __ldg(fcp + min(u, a.U)), fb = __ldg(fcp + min(u + 1, a.U));
       const double c0 = fma(di, fa.x, fa.y), c1 = fma(di, fb.x, fb.y);
       const double cc0 = fmin(fmax(c0, 0.0), Nd), cc1 = fmin(fmax(c1, 0.0), Nd);
       const int k0 = min((int)cc0, N - 1), k1 = min((int)cc1, N - 1);
       const float f0 = (float)(cc0 - (double)k0), f1 = (float)(cc1 - (double)k1);
-      const float inv = wc0 + j < a.U ? __frcp_rn((float)(c1 - c0) * dx) : 0.f;
+      const float inv = u < a.U ? __frcp_rn((float)(c1 - c0) * dx) : 0.f;
       const float3 wt = walk3(k0, f0, k1, f1, inv);
-      s_w[w][col][j] = make_float4(wt.x, wt.y, wt.z, __int_as_float(pack_k(k0, k1)));
+      const int n = k1 > k0 ? k1 - k0 : k0 - k1;
+      wide |= n > 2;
+      const unsigned oe = (unsigned)k1 * ks;
+      s_w[w][(col * GW + gg) * CG + j] = make_float4(wt.x, wt.y, wt.z, __uint_as_float(oe));
+      unsigned* m = reinterpret_cast<unsigned*>(&s_m[w][col * GW + gg]);
+      m[1 + j] = n >= 2 ? DD_INNER | (unsigned)(k1 > k0 ? k0 + 1 : k0 - 1) * ks : 0u;
+      if (j == 0) m[0] = (unsigned)k0 * ks;
     }
+    wide = __any_sync(0xffffffffu, wide);
     __syncwarp();
     if (active) {
-      const int ncol = min(CC, nl - ii0);
-#if DDFAN_DD_FWD_PART == 1
-      float part[CG][NZ][4];
+      // the start and end values of a line's walks are all loaded before the
+      // first is used; a walk's interior value (one in six at the c2 geometry)
+      // is loaded and added behind a branch.  Loading it ahead under a
+      // predicate, or always, cost more in register moves and L1 wavefronts
+      // than the wait (1.42 and 1.47 ms against 1.30 per c3 subset).
+      const char* lp = img + (size_t)ii0 * lstride;
+      const float4* pw = &s_w[w][g * CG];
+      const uint4* pm = &s_m[w][g];
+#pragma unroll 1
+      for (int col = 0; col < ncol; ++col, lp += lstride, pw += GW * CG, pm += GW) {
+        Vec<SV> S, E[CG];
+        float4 wt[CG];
+        const uint4 m = *pm;
+        const unsigned om[3] = {m.y, m.z, m.w};
+        vload(S, lp + (size_t)m.x * VB);
 #pragma unroll
-      for (int j = 0; j < CG; ++j)
-#pragma unroll
-        for (int z = 0; z < NZ; ++z) part[j][z][0] = part[j][z][1] = part[j][z][2] = part[j][z][3] = 0.f;
-#else
-      float (&part)[CG][NZ][4] = acc;
-#endif
-#pragma unroll(T::UNROLL)
-      for (int col = 0; col < ncol; ++col) {
-        const float4* line = img + (size_t)(ii0 + col) * lstride;
-        float4 cur[NZ];
-        {
-          const float4* p0 = line + (size_t)(__float_as_int(s_w[w][col][gw * CG].w) & 0xffff) * kstride;
-#pragma unroll
-          for (int z = 0; z < NZ; ++z) cur[z] = __ldg(p0 + zoff[z]);
+        for (int j = 0; j < CG; ++j) {
+          wt[j] = pw[j];
+          vload(E[j], lp + (size_t)__float_as_uint(wt[j].w) * VB);
         }
 #pragma unroll
         for (int j = 0; j < CG; ++j) {
-          const float4 wt = s_w[w][col][gw * CG + j];
-          const int pk = __float_as_int(wt.w);
-          walk_nz<NZ>(part[j], cur, vm, line, kstride, zoff, pk & 0xffff, pk >> 16, N - 1, wt);
+          vfma(acc[j], dup2(wt[j].x), j ? E[j - 1] : S);
+          vfma(acc[j], dup2(wt[j].z), E[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < CG; ++j) {
+          if ((int)om[j] < 0) {
+            Vec<SV> v;
+            vload(v, lp + (size_t)(om[j] & ~DD_INNER) * VB);
+            vfma(acc[j], dup2(wt[j].y), v);
+          }
         }
       }
-#if DDFAN_DD_FWD_PART == 1
+      if (wide) {
+        // interior values past the first (footprints over more than two cells)
+        lp = img + (size_t)ii0 * lstride;
+#pragma unroll 1
+        for (int col = 0; col < ncol; ++col, lp += lstride) {
 #pragma unroll
-      for (int j = 0; j < CG; ++j)
-#pragma unroll
-        for (int z = 0; z < NZ; ++z)
-#pragma unroll
-          for (int s = 0; s < 4; ++s) acc[j][z][s] += part[j][z][s];
-#elif DDFAN_DD_FWD_PART == 2
-      if ((ii0 / CC) % DDFAN_DD_FWD_FLUSH == DDFAN_DD_FWD_FLUSH - 1 || ii0 + CC >= nl) {
-#pragma unroll
-        for (int j = 0; j < CG; ++j)
-#pragma unroll
-          for (int z = 0; z < NZ; ++z)
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-              float* t = tot + ((j * NZ + z) * 4 + s) * T::NT;
-              *t += acc[j][z][s];
-              acc[j][z][s] = 0.f;
+          for (int j = 0; j < CG; ++j) {
+            const unsigned* m = reinterpret_cast<const unsigned*>(&s_m[w][col * GW + g]);
+            if (!(m[1 + j] & DD_INNER)) continue;
+            const float4 wt = s_w[w][(col * GW + g) * CG + j];
+            const unsigned o0 = j ? __float_as_uint(s_w[w][(col * GW + g) * CG + j - 1].w) : m[0];
+            const unsigned om = m[1 + j] & ~DD_INNER, oe = __float_as_uint(wt.w), st = om - o0;  // one step (mod 2^32)
+            for (unsigned q = om + st; q != oe; q += st) {
+              Vec<SV> v;
+              vload(v, lp + (size_t)q * VB);
+              vfma(acc[j], dup2(wt.y), v);
             }
+          }
+        }
       }
-#endif
+      since += ncol;
+      if (since >= T::FLUSH || ii0 + CC >= hi) {
+        since = 0;
+#pragma unroll
+        for (int j = 0; j < CG; ++j) {
+#pragma unroll
+          for (int s = 0; s < SV; ++s) tot[(j * SV + s) * T::NT] += vget(acc[j], s);
+          vzero(acc[j]);
+        }
+      }
     }
     __syncwarp();
   }
+  if (nseg > 1) {
+    __syncthreads();
+    if (seg != 0) return;
+  }
   if (!active) return;
-#if DDFAN_DD_FWD_PART == 2
-#pragma unroll
-  for (int j = 0; j < CG; ++j)
-#pragma unroll
-    for (int z = 0; z < NZ; ++z)
-#pragma unroll
-      for (int s = 0; s < 4; ++s) acc[j][z][s] = tot[((j * NZ + z) * 4 + s) * T::NT];
-#endif
 #pragma unroll
   for (int j = 0; j < CG; ++j) {
-    const int u = wc0 + gw * CG + j;
+    const int u = wc0 + g * CG + j;
     if (u >= a.U) break;
-    const size_t e = (size_t)slot * a.U + u;
+    const size_t e = (size_t)p * a.U + u;
     const float cv = __ldg(a.cvd + e) * dx;
-    float* o = a.out + ((size_t)slot * a.orow + u) * a.ostride;
+    float* o = a.out + ((size_t)p * a.orow + u) * a.ostride;
     float rs = 0.f, wt = 1.f;
     const float* yv = nullptr;
     if (a.y) {
       rs = __ldg(a.rowsum + e);
       if (a.wgt) wt = __ldg(a.wgt + e);
-      yv = a.y + ((size_t)__ldg(a.yview + slot) * a.U + u) * a.ystride;
+      yv = a.y + ((size_t)__ldg(a.yview + p) * a.U + u) * a.ystride;
     }
+    float val[SV];
 #pragma unroll
-    for (int z = 0; z < NZ; ++z) {
-      if (!zok[z]) continue;
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const int zs = zbk[z] * 4 + s;
-        if (zs < a.zlo || zs >= a.zhi) continue;
-        float val = acc[j][z][s] * cv;
-        if (yv) {
-          // (y - A x) / rowSum where rowSum != 0, else A x (AAPM_script/OSSART_AAPM.m:88)
-          val = rs != 0.f ? __fdiv_rn(__fsub_rn(__ldg(yv + zs), val), rs) : val;
-          val *= wt;
-        }
-        o[zs] = val;
+    for (int s = 0; s < SV; ++s) {
+      float t = tot[(j * SV + s) * T::NT];
+      for (int q = 1; q < nseg; ++q) t += tot[(j * SV + s) * T::NT + 32 * q];
+      val[s] = t * cv;
+      const int zs = vb * SV + s;
+      if (yv && zs >= a.zlo && zs < a.zhi) {
+        // (y - A x) / rowSum where rowSum != 0, else A x (AAPM_script/OSSART_AAPM.m:88)
+        val[s] = rs != 0.f ? __fdiv_rn(__fsub_rn(__ldg(yv + zs), val[s]), rs) : val[s];
+        val[s] *= wt;
       }
+    }
+    float* oz = o + vb * SV;
+    if (SV >= 4 && (a.ostride & 3) == 0 && vb * SV >= a.zlo && vb * SV + SV <= a.zhi &&
+        (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) {
+#pragma unroll
+      for (int s = 0; s + 4 <= SV; s += 4) *reinterpret_cast<float4*>(oz + s) = make_float4(val[s], val[s + 1], val[s + 2], val[s + 3]);
+    } else {
+#pragma unroll
+      for (int s = 0; s < SV; ++s)
+        if (vb * SV + s >= a.zlo && vb * SV + s < a.zhi) oz[s] = val[s];
     }
   }
 }
-
-// Grid order of the forward: with DDFAN_DD_FWD_ROWS_X the view rows run
-// along grid x (dispatched first), so the CTAs in flight are every view of a
-// few channel blocks -- rays at one distance from the centre, which miss the
-// disk inside it -- instead of every channel block of a few views.  On a c3
-// subset this cut the DRAM reads of the image from 2.05 to 1.33 GB per launch
-// (L2 hits 74 -> 82 %) and the launch from 2.36 to 2.15 ms.
-#ifndef DDFAN_DD_FWD_ROWS_X
-#define DDFAN_DD_FWD_ROWS_X 1
-#endif
 
 // Allows a forward kernel its dynamic shared memory on the current device
 // (above the 48 KB default with the static arrays).  Host-side, once per
@@ -425,31 +513,35 @@ inline cudaError_t dd_allow_dyn(K kernel, int bytes) {
   return bytes > 0 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
 }
 
-// One CTA per (view row, channel block, z-tile group) of one call.
-template <int ZL, int CG, int NZ>
-__global__ void __launch_bounds__(256, (DdMinCtas<NZ, DDFAN_DD_FWD_MIN_CTAS>::v)) k_fwd_dd(const __grid_constant__ DdFwdArgs a) {
-#if DDFAN_DD_FWD_ROWS_X
-  fwd_dd_body<ZL, CG, NZ>(a, a.row0 + (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z);
-#else
-  fwd_dd_body<ZL, CG, NZ>(a, a.row0 + (int)blockIdx.y, (int)blockIdx.x, (int)blockIdx.z);
-#endif
+// One CTA per (view row, channel block, z-tile) of one call.  View rows run
+// along grid x (dispatched first): the CTAs in flight are then every view of
+// a few channel blocks -- rays at one distance from the centre, which miss the
+// disk inside it -- instead of every channel block of a few views.  On a c3
+// subset this cut the DRAM reads of the image from 2.05 to 1.33 GB per launch.
+template <int SV>
+__global__ void __launch_bounds__(256, DDFAN_DD_FWD_MIN_CTAS) k_fwd_dd(const __grid_constant__ DdFwdArgs a) {
+  fwd_dd_body<SV>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z);
 }
 
 // One launch over a work list of many calls (batched reconstructions): CTA
-// b takes item {call, view row, channel block, z-tile group} = items[b].
-template <int ZL, int CG, int NZ>
-__global__ void __launch_bounds__(256, (DdMinCtas<NZ, DDFAN_DD_FWD_MIN_CTAS>::v)) k_fwd_dd_batch(const DdFwdArgs* __restrict__ args,
-                                                                              const int4* __restrict__ items) {
+// b takes item {call, view row, channel block, z-tile} = items[b].
+template <int SV>
+__global__ void __launch_bounds__(256, DDFAN_DD_FWD_MIN_CTAS) k_fwd_dd_batch(const DdFwdArgs* __restrict__ args,
+                                                                             const int4* __restrict__ items) {
   const int4 it = items[blockIdx.x];
-#if DDFAN_DD_BATCH_ARGS_COPY
-  const DdFwdArgs a = args[it.x];  // a local copy: its fields stay in registers
-#else
-  const DdFwdArgs& a = args[it.x];  // read in place (read-only, cached)
-#endif
-  fwd_dd_body<ZL, CG, NZ>(a, it.y, it.z, it.w);
+  fwd_dd_body<SV>(args[it.x], it.y, it.z, it.w);
 }
 
 // ============================================================ exact adjoint
+
+// most z-tiles per thread (1, 2 or 4; fewer when a call has fewer)
+#ifndef DDFAN_DD_NZ
+#define DDFAN_DD_NZ 4
+#endif
+
+// z-tiles per thread of the backprojectors: each decoded footprint serves
+// 4 slices per z-tile; at most the call's z-tiles (at most cap, the plan's tuned value)
+inline int dd_nz(int nzt, int cap) { return nzt >= 4 && cap >= 4 ? 4 : (nzt >= 2 && cap >= 2 ? 2 : 1); }
 
 struct DdAdjArgs {
   const float4* w;      // weighted residual [slot][U+1][P4], r_u / |dir_u.axis|, channel U = 0

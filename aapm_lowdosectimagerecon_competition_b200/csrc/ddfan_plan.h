@@ -146,7 +146,11 @@ struct DdResidual {
 int launch_fwd_dd(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc, const float* cvd,
                   const int* order, int PN, float* out, int orow, int ostride, int zlo, int zhi,
                   const DdResidual* res, cudaStream_t st);
-// The arguments launch_fwd_dd would launch with (nzt: z-tiles of [zlo, zhi)).
+// Lanes per group of the direct kernels for nvb vectors of slices.
+int dd_lanes(int nvb);
+// Channel blocks (grid y) of a forward launch.
+int dd_fwd_cblocks(const DdFwdArgs& a);
+// The arguments launch_fwd_dd would launch with (nvb: vectors of [zlo, zhi)).
 DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc,
                            const float* cvd, const int* order, int PN, float* out, int orow, int ostride, int zlo,
                            int zhi, const DdResidual* res);

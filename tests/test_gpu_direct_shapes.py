@@ -1,0 +1,55 @@
+"""The direct-mode kernels at the edges of their launch shapes, against the
+FP64 oracle: slice counts that fill, leave over or split the vectors and
+z-tiles (1 to 260 slices), channel counts around a warp's and a CTA's, footprints
+of no cell to many cells, rays that all cross or mostly miss the image, and
+launches small and large enough to split and not to split a ray's lines.
+The bound is the direct mode's (2e-6 relative L2: FP32 products of FP64
+weights rounded to FP32, summed in short chunks)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# (XN, YN, slices, views, channels, off-centre, masked)
+CASES = [
+    (40, 40, 1, 24, 72, False, False),     # one slice, few warps: lines split
+    (33, 27, 3, 17, 41, True, True),       # ragged, off centre
+    (24, 24, 8, 30, 48, False, False),     # one 8-slice vector
+    (24, 30, 12, 30, 48, False, True),     # three 4-slice vectors
+    (30, 24, 40, 12, 49, True, False),     # five vectors: idle lanes in a warp
+    (20, 20, 88, 12, 31, False, False),    # eleven vectors: two z-tiles
+    (16, 18, 260, 9, 33, False, True),     # more vectors than a warp has lanes
+    (64, 64, 16, 20, 12, False, False),    # 5 pixels a channel: wide footprints
+    (12, 12, 16, 20, 240, False, False),   # 20 channels a pixel: narrow footprints, wide voxels
+    (48, 40, 24, 700, 64, False, True),    # enough warps that lines are not split
+    (3, 5, 9, 7, 2, False, False),         # fewer pixels and channels than any tile
+]
+
+
+@pytest.mark.parametrize("XN,YN,Z,PN,U,off,masked", CASES)
+@pytest.mark.parametrize("sat", ["direct", "hilo"])
+def test_direct_shapes_match_oracle(XN, YN, Z, PN, U, off, masked, sat):
+    import torch
+    from aapm_lowdosectimagerecon_competition_b200 import configs, dd2, device
+    from oracle import oracle as O
+    assert torch.cuda.is_available()
+    s = configs.scaled(configs.c2(SLN=Z), XN=XN, DNU=U, PN=PN)
+    x0, y0, xds, yds = dd2.fan_geometry(s.sid, s.sdd, U, s.detCellWidth, s.detCntIdx)
+    cx, cy = (np.float32(2.5 * s.dx), np.float32(-1.5 * s.dx)) if off else (np.float32(0), np.float32(0))
+    rng = np.random.default_rng(XN + 7 * Z + PN)
+    vol = (rng.random((YN, XN, Z)) * 0.04).astype(np.float32)
+    prj = (rng.random((PN, U, Z)) - 0.3).astype(np.float32)
+    mask = (rng.random((YN, XN)) < 0.9).astype(np.uint8) if masked else None
+    a = s.angles()
+    h = np.repeat(a[:, None], Z, 1)
+    plan = device.Plan(x0, y0, U, xds, yds, s.detCntIdx, XN, YN, Z, PN, s.dx, mask=mask, imgXCenter=cx, imgYCenter=cy, sat=sat)
+    angs = torch.from_numpy(a).cuda()
+    rel = lambda g, e: float(np.linalg.norm((g - e).ravel()) / max(np.linalg.norm(e.ravel()), 1e-30))
+    got = plan.proj(angs, torch.from_numpy(vol).cuda()).cpu().numpy()
+    exp = O.proj(x0, y0, U, xds, yds, cx, cy, h, PN, XN, YN, Z, vol, s.dx, mask)
+    assert rel(got, exp) < 2e-6
+    for back, mode in (("adj", O.ADJ), ("ref", O.REF)):
+        gb = plan.back(angs, torch.from_numpy(prj).cuda(), mode=back).cpu().numpy()
+        eb = O.back(x0, y0, U, xds, yds, s.detCntIdx, cx, cy, h, PN, XN, YN, Z, prj, s.dx, mask, mode=mode)
+        assert rel(gb, eb) < 2e-6, back
+    plan.close()
