@@ -108,7 +108,7 @@ int plan_nz(int ZB) {
   }
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto it = g_tuned_nz.find(ZB);
-  return it == g_tuned_nz.end() ? DDFAN_DD_NZ : it->second;
+  return it == g_tuned_nz.end() ? 4 : it->second;
 }
 
 int plan_zl(int ZB, int zl_force) {
@@ -196,7 +196,7 @@ void plan_free(Plan* P) {
   cudaSetDevice(P->device);
   if (P->alloc_stream) {
     if (P->last_use) cudaStreamWaitEvent(P->alloc_stream, P->last_use, 0);
-    void* ptrs[] = {P->d_bx, P->d_by, P->d_xd, P->d_yd, P->d_mask, P->d_tb, P->d_lut, P->d_satx,
+    void* ptrs[] = {P->d_bx, P->d_by, P->d_xd, P->d_yd, P->d_mask, P->d_tb, P->d_tab, P->d_lut, P->d_satx,
                     P->d_saty, P->d_satq, P->d_vg, P->d_fc, P->d_cvd, P->d_tmp, P->d_angs,
                     P->d_order, P->d_counts, P->ps_ang, P->ps_vg, P->ps_fc, P->ps_cvd, P->ps_img,
                     P->ps_imgt, P->ps_sino, P->ps_tabx, P->ps_taby, P->ps_sq};
@@ -232,7 +232,7 @@ void boundaries(int n, const float* c, std::vector<double>& out) {
   }
 }
 
-// The direct forward kernels' dynamic shared memory, allowed on the current
+// The direct kernels' dynamic shared memory, allowed on the current
 // device (dev, for the message) at every plan creation -- a kernel
 // attribute belongs to the context, which a device reset replaces.  Plan
 // creation precedes every launch on a plan and never runs under capture.
@@ -240,8 +240,12 @@ int dd_prepare_device(int dev) {
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd<8>, DdFwdTile<8>::DYN);
   if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd<4>, DdFwdTile<4>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<8, true>, DdBackTile<8>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<8, false>, DdBackTile<8>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<4, true>, DdBackTile<4>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<4, false>, DdBackTile<4>::DYN);
   if (e != cudaSuccess)
-    return set_err(DDFAN_ERR_CUDA, "forward kernel attributes on device %d: %s", dev, cudaGetErrorString(e));
+    return set_err(DDFAN_ERR_CUDA, "kernel attributes on device %d: %s", dev, cudaGetErrorString(e));
   return DDFAN_OK;
 }
 
@@ -312,6 +316,11 @@ int plan_create(Plan** out, const PlanDesc& d) {
       if (b && !(p.tb[b] > p.tb[b - 1])) mono = false;
     }
     p.adj_ok = mono;
+    p.tab.resize(2 * (size_t)d.DNU);
+    for (int b = 0; b < d.DNU; ++b) {
+      p.tab[2 * b] = p.dirt * T[b];
+      p.tab[2 * b + 1] = 1.0 / (p.dirt * T[b + 1] - p.dirt * T[b]);
+    }
     p.M = 4 * (d.DNU + 1);
     p.t0 = p.tb[0];
     const double span = (double)p.tb[d.DNU] - p.tb[0];
@@ -336,13 +345,15 @@ int plan_create(Plan** out, const PlanDesc& d) {
   const bool direct = p.mode == SAT_DIRECT;
   const size_t F4 = cell_f4(p.mode);
   // direct mode: no image tables; the staged sinogram operand [PNmax][U+1][P4]
-  // float4 and a staged image of 4 P4 slices
+  // float4 (and the DD_PAST entries k_back_dd may read past it) and a staged
+  // image of 4 P4 slices
   const size_t nimg = direct ? 0 : (size_t)p.XN * p.YN * p.ZB * F4;
-  const size_t nsino = direct ? (size_t)p.PNmax * (p.U + 1) * p.P4 : (size_t)p.PNmax * (p.U + 1) * p.ZB * F4;
+  const size_t nsino = direct ? ((size_t)p.PNmax * (p.U + 1) + DD_PAST) * p.P4 : (size_t)p.PNmax * (p.U + 1) * p.ZB * F4;
   const size_t ntmp = (size_t)p.XN * p.YN * (direct ? 4 * (size_t)p.P4 : (size_t)p.Z);
   if ((rc = dalloc(&p.d_bx, p.U + 1, &B, as)) || (rc = dalloc(&p.d_by, p.U + 1, &B, as)) ||
       (rc = dalloc(&p.d_xd, p.U, &B, as)) || (rc = dalloc(&p.d_yd, p.U, &B, as)) ||
       (rc = dalloc(&p.d_mask, (size_t)p.XN * p.YN, &B, as)) || (rc = dalloc(&p.d_tb, p.U + 1, &B, as)) ||
+      (rc = dalloc(&p.d_tab, p.U, &B, as)) ||
       (rc = dalloc(&p.d_lut, p.M, &B, as)) || (!direct && (rc = dalloc(&p.d_satx, nimg, &B, as))) ||
       (!direct && (rc = dalloc(&p.d_saty, nimg, &B, as))) || (rc = dalloc(&p.d_satq, nsino, &B, as)) ||
       (rc = dalloc(&p.d_vg, p.PNmax, &B, as)) || (rc = dalloc(&p.d_fc, (size_t)p.PNmax * (p.U + 1), &B, as)) ||
@@ -364,6 +375,7 @@ int plan_create(Plan** out, const PlanDesc& d) {
   if (e == cudaSuccess) e = cudaMemcpyAsync(p.d_yd, yd.data(), sizeof(double) * p.U, cudaMemcpyHostToDevice, as);
   if (e == cudaSuccess) e = cudaMemcpyAsync(p.d_mask, m.data(), m.size(), cudaMemcpyHostToDevice, as);
   if (e == cudaSuccess) e = cudaMemcpyAsync(p.d_tb, p.tb.data(), sizeof(float) * (p.U + 1), cudaMemcpyHostToDevice, as);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(p.d_tab, p.tab.data(), sizeof(double2) * p.U, cudaMemcpyHostToDevice, as);
   if (e == cudaSuccess) e = cudaMemcpyAsync(p.d_lut, p.lut.data(), sizeof(uint16_t) * p.M, cudaMemcpyHostToDevice, as);
   // the allocations and the staged uploads complete before the plan is used on any stream
   if (e == cudaSuccess) e = cudaStreamSynchronize(as);
@@ -642,7 +654,7 @@ int launch_stage_image(const float* src, int Z, const uint8_t* mask, float* dst,
 int launch_stage_sino(const float* src, int Z, const float* wgt, int U, float* dst, int Zp, size_t PN,
                       cudaStream_t st) {
   ProfScope ps(KIND_SAT_SINO, st);
-  k_stage_sino<<<grid_blocks(PN * (U + 1) * Zp), 256, 0, st>>>(src, Z, wgt, U, dst, Zp, PN);
+  k_stage_sino<<<grid_blocks((PN * (U + 1) + DD_PAST) * Zp), 256, 0, st>>>(src, Z, wgt, U, dst, Zp, PN);
   return check_launch("k_stage_sino");
 }
 
@@ -712,117 +724,66 @@ int launch_fwd_dd(const Plan& p, const float* img, const ViewGeom* vg, const dou
   return check_launch("k_fwd_dd");
 }
 
-template <int ZL, bool XM>
-static void back_dd_go(const DdAdjArgs& a, int nzt, cudaStream_t st) {
-  using T = DdBackTile<ZL>;
-  const int nl = XM ? a.XN : a.YN, N = XM ? a.YN : a.XN;
-  const int tiles = ((nl + T::LT - 1) / T::LT) * ((N + T::KT - 1) / T::KT);
-  switch (dd_nz(nzt, a.nzc)) {
-    case 4: k_back_dd<ZL, XM, 4><<<dim3(tiles, 1, (nzt + 3) / 4), T::NT, 0, st>>>(a); break;
-    case 2: k_back_dd<ZL, XM, 2><<<dim3(tiles, 1, (nzt + 1) / 2), T::NT, 0, st>>>(a); break;
-    default: k_back_dd<ZL, XM, 1><<<dim3(tiles, 1, nzt), T::NT, 0, st>>>(a); break;
-  }
-}
-
-template <bool XM>
-static void back_dd_zl(int ZL, const DdAdjArgs& a, int nzt, cudaStream_t st) {
-  switch (ZL) {
-    case 8: back_dd_go<8, XM>(a, nzt, st); break;
-    case 4: back_dd_go<4, XM>(a, nzt, st); break;
-    case 2: back_dd_go<2, XM>(a, nzt, st); break;
-    default: back_dd_go<1, XM>(a, nzt, st); break;
-  }
-}
-
-template <int ZL>
-static void ref_dd_go(const DdRefArgs& a, int nzt, cudaStream_t st) {
-  using T = DdBackTile<ZL>;
-  const int tiles = ((a.YN + T::LT - 1) / T::LT) * ((a.XN + T::KT - 1) / T::KT);
-  switch (dd_nz(nzt, a.nzc)) {
-    case 4: k_back_ref_dd<ZL, 4><<<dim3(tiles, 1, (nzt + 3) / 4), T::NT, 0, st>>>(a); break;
-    case 2: k_back_ref_dd<ZL, 2><<<dim3(tiles, 1, (nzt + 1) / 2), T::NT, 0, st>>>(a); break;
-    default: k_back_ref_dd<ZL, 1><<<dim3(tiles, 1, nzt), T::NT, 0, st>>>(a); break;
-  }
-}
-
-int make_back_dd_args(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, const double2* fc,
-                      const int* order, const int* counts, int PN, const BackEpi& epi, DdAdjArgs* pass1,
-                      DdAdjArgs* pass2, DdRefArgs* ref) {
-  int zt0 = 0, nzt = 0;
-  ztile_range(p, epi.zlo, epi.zhi, &zt0, &nzt);
-  if (back_mode == DDFAN_BACK_REF) {
-    DdRefArgs a{};
-    a.q = reinterpret_cast<const float4*>(w); a.P4 = p.P4; a.vg = vg;
-    a.PN = PN; a.U = p.U; a.Z = p.Z; a.XN = p.XN; a.YN = p.YN;
-    a.ocx = p.ocx; a.ocy = p.ocy; a.dx = p.dx;
-    a.inv_sid = p.inv_sid; a.inv_dbeta = p.inv_dbeta; a.cnt = (double)p.detCntIdx + 0.5;
-    a.epi = epi;
-    a.zt0 = zt0;
-    a.nzt = nzt;
-    a.nzc = p.NZ;
-    *ref = a;
-    return nzt;
-  }
-  DdAdjArgs a{};
-  a.w = reinterpret_cast<const float4*>(w); a.P4 = p.P4;
-  a.vg = vg; a.fc = fc; a.tb = p.d_tb; a.lut = p.d_lut;
-  a.order = order; a.counts = counts;
-  a.t0 = p.t0; a.invdt = p.invdt; a.dirt = p.dirt; a.M = p.M;
-  a.PN = PN; a.U = p.U; a.Z = p.Z; a.XN = p.XN; a.YN = p.YN;
+DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN,
+                             const BackEpi& epi) {
+  DdBackArgs a{};
+  const int Zs = 4 * p.P4;  // slices of a residual entry
+  a.sv = Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 31) == 0 ? 8 : 4;
+  a.q = w; a.ZP = Zs / a.sv; a.vg = vg;
+  a.PN = PN; a.U = p.U; a.XN = p.XN; a.YN = p.YN; a.Z = p.Z;
   a.ocx = p.ocx; a.ocy = p.ocy; a.dx = p.dx;
-  a.zt0 = zt0;
-  a.nzt = nzt;
-  a.nzc = p.NZ;
-  // pass 1: x-major views along x columns -> tmp (mask applied)
-  *pass1 = a;
-  pass1->epi = epi;
-  pass1->epi.out = p.d_tmp; pass1->epi.addend = nullptr; pass1->epi.xin = nullptr; pass1->epi.colsum = nullptr;
-  pass1->epi.nonneg = 0;
-  // pass 2: y-major views along y rows, plus pass 1, then the final epilogue
-  *pass2 = a;
-  pass2->epi = epi;
-  pass2->epi.addend = p.d_tmp;
-  return nzt;
+  if (back_mode == DDFAN_BACK_ADJ) {
+    a.tab = p.d_tab; a.lut = p.d_lut;
+    a.t0 = p.t0; a.invdt = p.invdt; a.dirt = p.dirt; a.M = p.M; a.inv_sid = p.inv_sid;
+  } else {
+    a.inv_dbeta = p.inv_dbeta; a.cnt = (double)p.detCntIdx + 0.5;
+  }
+  a.epi = epi;
+  a.epi.zlo = std::max(0, epi.zlo);
+  a.epi.zhi = epi.zhi < 0 ? p.Z : std::min(epi.zhi, p.Z);
+  a.vb0 = a.epi.zlo / a.sv;
+  a.nvb = a.epi.zhi > a.epi.zlo ? (a.epi.zhi + a.sv - 1) / a.sv - a.vb0 : 0;
+  a.zl = dd_lanes(std::max(a.nvb, 1));
+  a.nzt = (a.nvb + a.zl - 1) / a.zl;
+  // a launch of fewer warps than the SMs hold (24 each) splits the views over
+  // 2, 4 or 8 of them
+  const long long GW = 32 / a.zl;
+  const long long warps = ((a.XN + 1) / 2 + GW - 1) / GW * ((a.YN + 1) / 2) * a.nzt;
+  a.nseg = 1;
+  while (a.nseg < 8 && warps * a.nseg < 148 * 24 && a.nseg * 4 <= PN) a.nseg *= 2;
+  return a;
 }
 
-int check_back_dd(const Plan& p, int back_mode, const int* order, const int* counts) {
+int dd_back_tiles(const DdBackArgs& a) {
+  const int GW = 32 / a.zl, WX = dd_back_wx(GW, a.nseg), WY = 8 / a.nseg / WX;
+  return (((a.XN + 1) / 2 + WX * GW - 1) / (WX * GW)) * (((a.YN + 1) / 2 + WY - 1) / WY);
+}
+
+int check_back_dd(const Plan& p, int back_mode) {
   if (back_mode == DDFAN_BACK_REF) return DDFAN_OK;
   if (back_mode != DDFAN_BACK_ADJ) return set_err(DDFAN_ERR_ARG, "back_mode %d", back_mode);
   if (!p.adj_ok) return set_err(DDFAN_ERR_UNSUPPORTED, "detector boundaries are not monotone as seen from the source");
-  if (!order || !counts) return set_err(DDFAN_ERR_ARG, "exact adjoint needs the view order");
   if (p.U + 1 > 1024 || p.M > 4096) return set_err(DDFAN_ERR_UNSUPPORTED, "exact adjoint: %d channels", p.U);
   return DDFAN_OK;
 }
 
-int launch_back_dd(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, const double2* fc,
-                   const int* order, const int* counts, int PN, const BackEpi& epi, cudaStream_t st) {
-  int rc = check_back_dd(p, back_mode, order, counts);
+int launch_back_dd(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN, const BackEpi& epi,
+                   cudaStream_t st) {
+  int rc = check_back_dd(p, back_mode);
   if (rc) return rc;
-  DdAdjArgs a1, a2;
-  DdRefArgs ar;
-  const int nzt = make_back_dd_args(p, back_mode, w, vg, fc, order, counts, PN, epi, &a1, &a2, &ar);
-  if (nzt == 0 || PN < 1) return DDFAN_OK;
-  if (back_mode == DDFAN_BACK_REF) {
-    ProfScope ps(KIND_BACK_A, st);
-    switch (p.ZL) {
-      case 8: ref_dd_go<8>(ar, nzt, st); break;
-      case 4: ref_dd_go<4>(ar, nzt, st); break;
-      case 2: ref_dd_go<2>(ar, nzt, st); break;
-      default: ref_dd_go<1>(ar, nzt, st); break;
-    }
-    return check_launch("k_back_ref_dd");
+  const DdBackArgs a = make_back_dd_args(p, back_mode, w, vg, PN, epi);
+  if (a.nvb == 0 || PN < 1) return DDFAN_OK;
+  ProfScope ps(KIND_BACK_A, st);
+  const dim3 grid(dd_back_tiles(a), 1, a.nzt);
+  const bool adj = back_mode == DDFAN_BACK_ADJ;
+  if (a.sv == 8) {
+    if (adj) k_back_dd<8, true><<<grid, 256, DdBackTile<8>::DYN, st>>>(a);
+    else k_back_dd<8, false><<<grid, 256, DdBackTile<8>::DYN, st>>>(a);
+  } else {
+    if (adj) k_back_dd<4, true><<<grid, 256, DdBackTile<4>::DYN, st>>>(a);
+    else k_back_dd<4, false><<<grid, 256, DdBackTile<4>::DYN, st>>>(a);
   }
-  {
-    ProfScope ps(KIND_BACK_A, st);
-    back_dd_zl<true>(p.ZL, a1, nzt, st);
-  }
-  rc = check_launch("k_back_dd<x>");
-  if (rc) return rc;
-  {
-    ProfScope ps(KIND_BACK_B, st);
-    back_dd_zl<false>(p.ZL, a2, nzt, st);
-  }
-  return check_launch("k_back_dd<y>");
+  return check_launch("k_back_dd");
 }
 
 // ------------------------------------------------------------------ device API
@@ -856,17 +817,17 @@ int back_dev_shared(Plan& p, const float* d_angs, int stride, int PN, const floa
                     int back_mode, int zlo, int zhi, cudaStream_t st) {
   int rc;
   if ((rc = launch_view_geom(p, d_angs, stride, PN, p.d_vg, p.d_fc, p.d_cvd, st))) return rc;
-  if ((rc = launch_view_order(p.d_vg, PN, p.d_order, p.d_counts, st))) return rc;
   const bool adj = back_mode == DDFAN_BACK_ADJ;
   BackEpi e{};
   e.out = d_vol; e.mask = p.has_mask ? p.d_mask : nullptr; e.zlo = zlo; e.zhi = zhi;
   if (p.mode == SAT_DIRECT) {
     float* w = reinterpret_cast<float*>(p.d_satq);
     if ((rc = launch_stage_sino(d_prj, p.Z, adj ? p.d_cvd : nullptr, p.U, w, 4 * p.P4, (size_t)PN, st))) return rc;
-    rc = launch_back_dd(p, back_mode, w, p.d_vg, p.d_fc, p.d_order, p.d_counts, PN, e, st);
+    rc = launch_back_dd(p, back_mode, w, p.d_vg, PN, e, st);
     mark_use(p, st);
     return rc;
   }
+  if ((rc = launch_view_order(p.d_vg, PN, p.d_order, p.d_counts, st))) return rc;
   if ((rc = launch_sat_sino(p, d_prj, PN, adj ? p.d_cvd : nullptr, 1.f, nullptr, nullptr, nullptr, st, zlo,
                             zhi)))
     return rc;
@@ -1109,9 +1070,9 @@ DDFAN_API size_t ddfan_plan_estimate_bytes(int XN, int YN, int DNU, int SLN, int
   ZB = (ZB + ZL - 1) / ZL * ZL;
   const size_t F4 = cell_f4(sat_mode), U = (size_t)DNU, P = (size_t)PNmax;
   const bool direct = sat_mode == SAT_DIRECT;
-  const size_t cells = direct ? P * (U + 1) * P4 : 2 * (size_t)XN * YN * ZB * F4 + P * (U + 1) * ZB * F4;
+  const size_t cells = direct ? (P * (U + 1) + DD_PAST) * P4 : 2 * (size_t)XN * YN * ZB * F4 + P * (U + 1) * ZB * F4;
   const size_t tmp = (size_t)XN * YN * (direct ? 4 * (size_t)P4 : (size_t)SLN);
-  return cells * sizeof(float4) + (2 * (U + 1) + 2 * U) * sizeof(double) + (size_t)XN * YN +
+  return cells * sizeof(float4) + (2 * (U + 1) + 4 * U) * sizeof(double) + (size_t)XN * YN +
          (U + 1) * sizeof(float) + 4 * (U + 1) * sizeof(uint16_t) + P * sizeof(ViewGeom) +
          P * (U + 1) * sizeof(double2) + P * U * sizeof(float) + tmp * sizeof(float) +
          P * sizeof(float) + P * sizeof(int) + 2 * sizeof(int);

@@ -1,14 +1,13 @@
 // ddfan_batch.cu -- many OS-SART solves advanced together: one launch per
-// kernel kind, subset step and tile class over a device work list of every
+// kernel kind, subset step and vector class over a device work list of every
 // solve's CTAs, instead of one launch per solve.
 //
 // A batched iteration runs subset step k of every solve that has one: the
 // forward projectors (with the fused residual) of all those solves in one
-// launch per (z-lane count, z-tiles per thread) class, then the
-// backprojections the same way (the exact adjoint's x-column pass of every
-// solve, then its y-row pass; or the reference backprojector), then FISTA of
-// every solve in one launch pair.  Each CTA reads its item {solve's argument
-// block, view row or voxel tile, channel block, z-tile group} and runs the
+// launch per class (slices per thread), then the backprojections the same way
+// (the exact adjoint's, then the reference's), then FISTA of every solve in
+// one launch pair.  Each CTA reads its item {solve's argument
+// block, view row or voxel tile, channel block, z-tile} and runs the
 // same kernel body a single solve's launch runs, with that solve's arguments,
 // so every solve computes exactly what it computes alone.  Small solves
 // (a few slices, a few hundred views) that leave most of the GPU idle in a
@@ -34,35 +33,13 @@ namespace ddfan {
 
 namespace {
 
-enum BatchKind { BK_FWD = 0, BK_ADJ_X = 1, BK_ADJ_Y = 2, BK_REF = 3 };
+enum BatchKind { BK_FWD = 0, BK_ADJ = 1, BK_REF = 2 };
 
 struct BatchLaunch {
-  int kind, ZL, NZ;  // forward: slices per thread, 0
+  int kind, sv;  // sv: slices per thread
   size_t items_off, nitems;
   int group;  // the solver group whose chain the launch belongs to
 };
-
-// (lines per tile, voxels per line per tile) of the direct exact adjoint and
-// of the REF backprojector
-void adj_tile(int ZL, int* LT, int* KT) {
-  switch (ZL) {
-    case 8: *LT = DdBackTile<8>::LT; *KT = DdBackTile<8>::KT; break;
-    case 4: *LT = DdBackTile<4>::LT; *KT = DdBackTile<4>::KT; break;
-    case 2: *LT = DdBackTile<2>::LT; *KT = DdBackTile<2>::KT; break;
-    default: *LT = DdBackTile<1>::LT; *KT = DdBackTile<1>::KT; break;
-  }
-}
-
-template <int ZL, int NZ>
-void go_adj(bool xm, const DdAdjArgs* a, const int4* it, unsigned n, cudaStream_t st) {
-  if (xm) k_back_dd_batch<ZL, true, NZ><<<n, 256, 0, st>>>(a, it);
-  else k_back_dd_batch<ZL, false, NZ><<<n, 256, 0, st>>>(a, it);
-}
-
-template <int ZL, int NZ>
-void go_ref(const DdRefArgs* a, const int4* it, unsigned n, cudaStream_t st) {
-  k_back_ref_dd_batch<ZL, NZ><<<n, 256, 0, st>>>(a, it);
-}
 
 // solver groups whose launch chains run side by side (DDFAN_BATCH_GROUPS in
 // the environment overrides it)
@@ -70,22 +47,20 @@ void go_ref(const DdRefArgs* a, const int4* it, unsigned n, cudaStream_t st) {
 #define DDFAN_BATCH_GROUPS 1
 #endif
 
-// the work-list forward kernels' dynamic shared memory on the current device
+// the work-list kernels' dynamic shared memory on the current device
 // (at every batch creation: the attribute belongs to the context)
 int batch_prepare_device(int dev) {
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd_batch<8>, DdFwdTile<8>::DYN);
   if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd_batch<4>, DdFwdTile<4>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<8, true>, DdBackTile<8>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<8, false>, DdBackTile<8>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<4, true>, DdBackTile<4>::DYN);
+  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<4, false>, DdBackTile<4>::DYN);
   if (e != cudaSuccess)
-    return set_err(DDFAN_ERR_CUDA, "batched forward kernel attributes on device %d: %s", dev, cudaGetErrorString(e));
+    return set_err(DDFAN_ERR_CUDA, "batched kernel attributes on device %d: %s", dev, cudaGetErrorString(e));
   return DDFAN_OK;
 }
-
-#define DDFAN_BATCH_ZL_NZ(ZLv, NZv, CALL) \
-  if (L.ZL == ZLv && L.NZ == NZv) {       \
-    CALL;                                 \
-    break;                                \
-  }
 
 }  // namespace
 
@@ -94,8 +69,7 @@ struct Batch {
   std::vector<Solver*> sv;
   std::vector<BatchLaunch> launches;  // one iteration, in order
   DdFwdArgs* d_fargs = nullptr;
-  DdAdjArgs* d_aargs = nullptr;
-  DdRefArgs* d_rargs = nullptr;
+  DdBackArgs* d_bargs = nullptr;
   int4* d_items = nullptr;
   FistaDesc* d_fista = nullptr;
   int nfista = 0;
@@ -124,7 +98,7 @@ static void batch_free(Batch* b) {
   }
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   if (b->graph) cudaGraphDestroy(b->graph);
-  void* ptrs[] = {b->d_fargs, b->d_aargs, b->d_rargs, b->d_items, b->d_fista};
+  void* ptrs[] = {b->d_fargs, b->d_bargs, b->d_items, b->d_fista};
   for (void* q : ptrs) dev_free(q, b->own);
   if (b->own) cudaStreamDestroy(b->own);
   if (b->last_use) cudaEventDestroy(b->last_use);
@@ -143,41 +117,18 @@ static int batch_launch(Batch& b, const BatchLaunch& L, cudaStream_t st) {
     const unsigned n = (unsigned)L.nitems;
     if (L.kind == BK_FWD) {
       ProfScope ps(KIND_FWD, st);
-      if (L.ZL == 8) k_fwd_dd_batch<8><<<n, DdFwdTile<8>::NT, DdFwdTile<8>::DYN, st>>>(b.d_fargs, it);
-      else k_fwd_dd_batch<4><<<n, DdFwdTile<4>::NT, DdFwdTile<4>::DYN, st>>>(b.d_fargs, it);
-    } else if (L.kind == BK_ADJ_X || L.kind == BK_ADJ_Y) {
-      const bool xm = L.kind == BK_ADJ_X;
-      ProfScope ps(xm ? KIND_BACK_A : KIND_BACK_B, st);
-      do {
-        DDFAN_BATCH_ZL_NZ(8, 4, (go_adj<8, 4>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(8, 2, (go_adj<8, 2>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(8, 1, (go_adj<8, 1>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 4, (go_adj<4, 4>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 2, (go_adj<4, 2>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 1, (go_adj<4, 1>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 4, (go_adj<2, 4>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 2, (go_adj<2, 2>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 1, (go_adj<2, 1>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 4, (go_adj<1, 4>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 2, (go_adj<1, 2>(xm, b.d_aargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 1, (go_adj<1, 1>(xm, b.d_aargs, it, n, st)))
-      } while (0);
+      if (L.sv == 8) k_fwd_dd_batch<8><<<n, 256, DdFwdTile<8>::DYN, st>>>(b.d_fargs, it);
+      else k_fwd_dd_batch<4><<<n, 256, DdFwdTile<4>::DYN, st>>>(b.d_fargs, it);
     } else {
       ProfScope ps(KIND_BACK_A, st);
-      do {
-        DDFAN_BATCH_ZL_NZ(8, 4, (go_ref<8, 4>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(8, 2, (go_ref<8, 2>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(8, 1, (go_ref<8, 1>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 4, (go_ref<4, 4>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 2, (go_ref<4, 2>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(4, 1, (go_ref<4, 1>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 4, (go_ref<2, 4>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 2, (go_ref<2, 2>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(2, 1, (go_ref<2, 1>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 4, (go_ref<1, 4>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 2, (go_ref<1, 2>(b.d_rargs, it, n, st)))
-        DDFAN_BATCH_ZL_NZ(1, 1, (go_ref<1, 1>(b.d_rargs, it, n, st)))
-      } while (0);
+      const bool adj = L.kind == BK_ADJ;
+      if (L.sv == 8) {
+        if (adj) k_back_dd_batch<8, true><<<n, 256, DdBackTile<8>::DYN, st>>>(b.d_bargs, it);
+        else k_back_dd_batch<8, false><<<n, 256, DdBackTile<8>::DYN, st>>>(b.d_bargs, it);
+      } else {
+        if (adj) k_back_dd_batch<4, true><<<n, 256, DdBackTile<4>::DYN, st>>>(b.d_bargs, it);
+        else k_back_dd_batch<4, false><<<n, 256, DdBackTile<4>::DYN, st>>>(b.d_bargs, it);
+      }
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_err(DDFAN_ERR_CUDA, "batched launch (kind %d): %s", L.kind, cudaGetErrorString(e));
@@ -248,8 +199,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
   int maxsub = 0;
   for (Solver* s : b.sv) maxsub = std::max(maxsub, s->nsub);
   std::vector<DdFwdArgs> fargs;
-  std::vector<DdAdjArgs> aargs;
-  std::vector<DdRefArgs> rargs;
+  std::vector<DdBackArgs> bargs;
   std::vector<int4> items;
   // solver groups: largest solves first, dealt round robin
   int G = DDFAN_BATCH_GROUPS;
@@ -267,7 +217,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
   // per group, per step: class -> items, for each kind
   for (int grp = 0; grp < G; ++grp)
   for (int k = 0; k < maxsub; ++k) {
-    std::map<std::pair<int, int>, std::vector<int4>> fwd, adjx, adjy, ref;
+    std::map<int, std::vector<int4>> fwd, back_adj, back_ref;  // by slices per thread
     for (size_t si = 0; si < b.sv.size(); ++si) {
       if (group_of[si] != grp) continue;
       Solver& s = *b.sv[si];
@@ -290,58 +240,34 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
       // z-tiles outermost and the rest in the single-solve grid's
       // order: the CTAs in flight share one tile's slices, whose image part
       // then stays in L2
-      auto& fl = fwd[{fa.sv, 0}];
+      auto& fl = fwd[fa.sv];
       for (int zt = 0; zt < fa.nzt; ++zt)
         for (int cb = 0; cb < ncb; ++cb)
           for (int row = 0; row < c; ++row) fl.push_back(make_int4(fi, row, cb, zt));
       BackEpi e{};
       e.out = s.d_x; e.xin = s.d_x; e.colsum = s.d_cols + (size_t)k * s.XN * s.YN;
       e.nonneg = s.nonneg; e.mask = p.has_mask ? p.d_mask : nullptr; e.zlo = 0; e.zhi = s.Zi;
-      int rc = check_back_dd(p, s.back_mode, s.d_order + o, s.d_counts + 2 * k);
+      int rc = check_back_dd(p, s.back_mode);
       if (rc) return rc;
-      DdAdjArgs a1, a2;
-      DdRefArgs ar;
-      const int nzt = make_back_dd_args(p, s.back_mode, s.d_ax, vg, fc, s.d_order + o, s.d_counts + 2 * k, c, e, &a1,
-                                        &a2, &ar);
-      if (adj) {
-        const int bnz = dd_nz(nzt, p.NZ), nbz = (nzt + bnz - 1) / bnz;
-        int LT, KT;
-        adj_tile(p.ZL, &LT, &KT);
-        const int i1 = (int)aargs.size();
-        aargs.push_back(a1);
-        aargs.push_back(a2);
-        const int tx = ((s.XN + LT - 1) / LT) * ((s.YN + KT - 1) / KT);  // x columns as lines
-        const int ty = ((s.YN + LT - 1) / LT) * ((s.XN + KT - 1) / KT);  // y rows as lines
-        auto& lx = adjx[{p.ZL, bnz}];
-        auto& ly = adjy[{p.ZL, bnz}];
-        for (int zg = 0; zg < nbz; ++zg)
-          for (int t = 0; t < tx; ++t) lx.push_back(make_int4(i1, t, zg, 0));
-        for (int zg = 0; zg < nbz; ++zg)
-          for (int t = 0; t < ty; ++t) ly.push_back(make_int4(i1 + 1, t, zg, 0));
-      } else {
-        const int bnz = dd_nz(nzt, p.NZ), nbz = (nzt + bnz - 1) / bnz;
-        int LT, KT;
-        adj_tile(p.ZL, &LT, &KT);  // the REF kernel uses the exact adjoint's voxel tile
-        const int ri = (int)rargs.size();
-        rargs.push_back(ar);
-        const int tiles = ((s.YN + LT - 1) / LT) * ((s.XN + KT - 1) / KT);
-        auto& lr = ref[{p.ZL, bnz}];
-        for (int zg = 0; zg < nbz; ++zg)
-          for (int t = 0; t < tiles; ++t) lr.push_back(make_int4(ri, t, zg, 0));
-      }
+      const DdBackArgs ba = make_back_dd_args(p, s.back_mode, s.d_ax, vg, c, e);
+      const int bi = (int)bargs.size();
+      bargs.push_back(ba);
+      const int tiles = dd_back_tiles(ba);
+      auto& lb = (adj ? back_adj : back_ref)[ba.sv];
+      for (int zt = 0; zt < ba.nzt; ++zt)
+        for (int t = 0; t < tiles; ++t) lb.push_back(make_int4(bi, t, zt, 0));
     }
-    auto emit = [&](int kind, std::map<std::pair<int, int>, std::vector<int4>>& m) {
+    auto emit = [&](int kind, std::map<int, std::vector<int4>>& m) {
       for (auto& kv : m) {
         if (kv.second.empty()) continue;
-        BatchLaunch L{kind, kv.first.first, kv.first.second, items.size(), kv.second.size(), grp};
+        BatchLaunch L{kind, kv.first, items.size(), kv.second.size(), grp};
         items.insert(items.end(), kv.second.begin(), kv.second.end());
         b.launches.push_back(L);
       }
     };
     emit(BK_FWD, fwd);
-    emit(BK_ADJ_X, adjx);
-    emit(BK_REF, ref);
-    emit(BK_ADJ_Y, adjy);
+    emit(BK_ADJ, back_adj);
+    emit(BK_REF, back_ref);
   }
   for (const BatchLaunch& L : b.launches)
     if (L.nitems > (size_t)INT_MAX) return set_err(DDFAN_ERR_UNSUPPORTED, "batch: %zu CTAs in one launch", L.nitems);
@@ -381,7 +307,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
     if (ee != cudaSuccess) return set_err(DDFAN_ERR_CUDA, "batch: upload: %s", cudaGetErrorString(ee));
     return DDFAN_OK;
   };
-  if ((rc = up(&b.d_fargs, fargs)) || (rc = up(&b.d_aargs, aargs)) || (rc = up(&b.d_rargs, rargs)) ||
+  if ((rc = up(&b.d_fargs, fargs)) || (rc = up(&b.d_bargs, bargs)) ||
       (rc = up(&b.d_items, items)) || (rc = up(&b.d_fista, fista)))
     return rc;
   // the pageable sources above are consumed before they go out of scope

@@ -17,75 +17,24 @@
 // with its neighbour, where a 48-byte hi/lo cell read 12 bytes per slice per
 // boundary.  Wider footprints walk more values (any width is correct).
 //
-// Layouts: the image [YN][XN][P4] float4 (4 slices per float4, P4 = padded
-// slices / 4) is read straight, masked beforehand; the sinogram operands
-// [slot][U + 1][P4] float4 hold the (weighted) residual with a zero guard
-// channel U, so a walk that ends on the last boundary (index U, fraction 0)
-// reads a zero.  Geometry phases (FP64 boundary lines, brackets, fractions)
-// are those of the prefix-sum kernels; only the gather changes.
+// Layouts: the image [YN][XN][slices] and the sinogram operands
+// [slot][U + 1][slices], slices padded to a multiple of 4 or 8 and read in
+// vectors of that many; the image masked beforehand, the (weighted) residual
+// with a zero guard channel U, so a walk that ends on the last boundary
+// (index U, fraction 0) reads a zero.
 #pragma once
 #include "ddfan_proj_kernels.cuh"
 
 namespace ddfan {
 
 // Resident CTAs per SM the register allocation is sized for (256 threads:
-// 2 -> up to 128 registers, which the backprojectors' 4-z-tile accumulators
-// need without spilling; 3 -> 80 for the forward).  Build-time knobs for tuning sweeps, like the tile shapes below.
+// 3 -> up to 80 registers, 2 -> 128).  Build-time knobs for tuning sweeps, like the tile shapes below.
 #ifndef DDFAN_DD_FWD_MIN_CTAS
 #define DDFAN_DD_FWD_MIN_CTAS 3
 #endif
 #ifndef DDFAN_DD_BACK_MIN_CTAS
 #define DDFAN_DD_BACK_MIN_CTAS 2
 #endif
-// With DDFAN_DD_MIN_CTAS_BY_NZ the kernels of fewer z-tiles per thread (fewer
-// accumulators) are built for one (NZ = 2: 80 registers) or two (NZ = 1: 64)
-// more resident CTAs.  On a c3 subset forced to NZ = 2 this took the forward
-// from 2.84 to 2.28 ms and the REF backprojector from 2.03 to 1.80 (NZ = 1:
-// 3.59 -> 3.00, 3.56 -> 2.82); the NZ = 4 kernels are unchanged.
-#ifndef DDFAN_DD_MIN_CTAS_BY_NZ
-#define DDFAN_DD_MIN_CTAS_BY_NZ 1
-#endif
-// Work-list kernels: argument block copied to registers (1) or read in place
-// through the read-only path (0).  The copy spilled at the 80-register
-// budget of 2 z-tiles per thread (68-104 bytes against 12-24 for the grid
-// kernels); read in place, batched c4 went from 17.1 to 18.7 iterations/s.
-#ifndef DDFAN_DD_BATCH_ARGS_COPY
-#define DDFAN_DD_BATCH_ARGS_COPY 0
-#endif
-template <int NZ, int BASE>
-struct DdMinCtas {
-  static constexpr int v = DDFAN_DD_MIN_CTAS_BY_NZ ? (NZ >= 4 ? BASE : (NZ == 2 ? BASE + 1 : BASE + 2)) : BASE;
-};
-
-// a += w v on 4 slices, as two packed fma.rn.f32x2 (sm_100: two lanes of
-// round-to-nearest FMA per instruction, the same results as four fmaf; half
-// the FMA instructions took a c3 subset's forward from 2.50 to 2.41 ms).
-// DDFAN_FFMA2=0 builds the scalar form.
-#ifndef DDFAN_FFMA2
-#define DDFAN_FFMA2 1
-#endif
-__device__ __forceinline__ void fma2(float& a0, float& a1, float w, float v0, float v1) {
-  asm("{\n\t.reg .b64 ra, rv, rw;\n\t"
-      "mov.b64 ra, {%0, %1};\n\t"
-      "mov.b64 rv, {%2, %3};\n\t"
-      "mov.b64 rw, {%4, %4};\n\t"
-      "fma.rn.f32x2 ra, rw, rv, ra;\n\t"
-      "mov.b64 {%0, %1}, ra;\n\t}"
-      : "+f"(a0), "+f"(a1)
-      : "f"(v0), "f"(v1), "f"(w));
-}
-__device__ __forceinline__ void fma4(float (&a)[4], float w, const float4& v) {
-#if DDFAN_FFMA2
-  fma2(a[0], a[1], w, v.x, v.y);
-  fma2(a[2], a[3], w, v.z, v.w);
-#else
-  a[0] = fmaf(w, v.x, a[0]);
-  a[1] = fmaf(w, v.y, a[1]);
-  a[2] = fmaf(w, v.z, a[2]);
-  a[3] = fmaf(w, v.w, a[3]);
-#endif
-}
-
 // The walk from (k0, f0) to (k1, f1) as three weights: w0 on the value at
 // k0, wm on the value one step on (an interior value when n = |k1 - k0| >= 2,
 // else 0: that value is then the end value or past it), we on the value at k1
@@ -97,73 +46,6 @@ __device__ __forceinline__ float3 walk3(int k0, float f0, int k1, float f1, floa
   const float wi = k1 > k0 ? s : -s;
   return k1 > k0 ? make_float3((1.f - f0) * s, n >= 2 ? wi : 0.f, f1 * s)
                  : make_float3(-f0 * s, n >= 2 ? wi : 0.f, (f1 - 1.f) * s);
-}
-
-// k0 and k1 of a walk packed in one word (indices below 32768)
-__device__ __forceinline__ int pack_k(int k0, int k1) { return k0 | (k1 << 16); }
-
-// Predicated 16-byte load through the read-only path into v, which keeps its
-// value when p is false (no memory access then).  One instruction, so the
-// loads of a walk issue back to back instead of behind branches; the kept
-// value is finite image or sinogram data, and every caller gives it weight 0.
-__device__ __forceinline__ void ldg4_keep(bool p, const float4* a, float4& v) {
-  asm("{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %4, 0;\n\t"
-      "@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%5];\n\t}"
-      : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
-      : "r"((int)p), "l"(a));
-}
-
-// One walk for NZ z-tiles (float4 runs zoff[z] float4 past base): adds w0 cur
-// + wm v[k0 + st] + we v[k1] (+ wm v for the further interior values) to acc
-// and leaves v[k1] in cur.  v[k1] is loaded only when the walk moves (n >= 1;
-// else it is cur), the first interior value only when there is one (n >= 2,
-// into vm, which otherwise keeps an earlier value under weight 0): about two
-// loads per footprint, and no branch unless it spans more than two steps.
-#ifndef DDFAN_WALK_LOADS_FIRST
-#define DDFAN_WALK_LOADS_FIRST 0
-#endif
-template <int NZ>
-__device__ __forceinline__ void walk_nz(float (&acc)[NZ][4], float4 (&cur)[NZ], float4 (&vm)[NZ],
-                                        const float4* base, size_t stride, const int (&zoff)[NZ], int k0, int k1,
-                                        int kmax, const float4& wt) {
-  const int dn = k1 - k0, st = dn > 0 ? 1 : -1, n = dn > 0 ? dn : -dn;
-  const int km = min(max(k0 + st, 0), kmax);
-  const float4* pm = base + (size_t)km * stride;
-  const float4* pe = base + (size_t)k1 * stride;
-#if DDFAN_WALK_LOADS_FIRST
-  float4 ce[NZ];
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) ce[z] = cur[z];
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) ldg4_keep(n >= 2, pm + zoff[z], vm[z]);
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) ldg4_keep(n >= 1, pe + zoff[z], ce[z]);
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) {
-    fma4(acc[z], wt.x, cur[z]);
-    fma4(acc[z], wt.y, vm[z]);
-    fma4(acc[z], wt.z, ce[z]);
-    cur[z] = ce[z];
-  }
-#else
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) ldg4_keep(n >= 2, pm + zoff[z], vm[z]);
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) fma4(acc[z], wt.x, cur[z]);
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) ldg4_keep(n >= 1, pe + zoff[z], cur[z]);
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) {
-    fma4(acc[z], wt.y, vm[z]);
-    fma4(acc[z], wt.z, cur[z]);
-  }
-#endif
-  for (int i = 2; i < n; ++i) {
-    const float4* pi = base + (size_t)(k0 + i * st) * stride;
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) fma4(acc[z], wt.y, __ldg(pi + zoff[z]));
-  }
 }
 
 // ============================================================ vectors of slices
@@ -532,349 +414,403 @@ __global__ void __launch_bounds__(256, DDFAN_DD_FWD_MIN_CTAS) k_fwd_dd_batch(con
   fwd_dd_body<SV>(args[it.x], it.y, it.z, it.w);
 }
 
-// ============================================================ exact adjoint
+// ============================================================ backprojectors
 
-// most z-tiles per thread (1, 2 or 4; fewer when a call has fewer)
-#ifndef DDFAN_DD_NZ
-#define DDFAN_DD_NZ 4
-#endif
-
-// z-tiles per thread of the backprojectors: each decoded footprint serves
-// 4 slices per z-tile; at most the call's z-tiles (at most cap, the plan's tuned value)
-inline int dd_nz(int nzt, int cap) { return nzt >= 4 && cap >= 4 ? 4 : (nzt >= 2 && cap >= 2 ? 2 : 1); }
-
-struct DdAdjArgs {
-  const float4* w;      // weighted residual [slot][U+1][P4], r_u / |dir_u.axis|, channel U = 0
-  int P4;
+struct DdBackArgs {
+  const float* q;      // residual [slot][U+1][ZP vectors of SV slices], channel U = 0
+                       // (exact adjoint: weighted, r_u / |dir_u.axis|)
+  int ZP;
   const ViewGeom* vg;
-  const double2* fc;
-  const float* tb;
+  int PN, U, XN, YN;
+  int Z;               // slices of an output pixel
+  double ocx, ocy, dx;
+  // exact adjoint
+  const double2* tab;  // [U] fan tangents of the boundaries (dd_edge)
   const uint16_t* lut;
-  const int* order;
-  const int* counts;
   float t0, invdt, dirt;
   int M;
-  int PN, U, Z, XN, YN;
-  double ocx, ocy, dx;
+  double inv_sid;
+  // reference formula
+  double inv_dbeta, cnt;  // cnt = detCntIdx + 1 - 0.5
   BackEpi epi;
-  int zt0, nzt;
-  int nzc;  // most z-tiles per thread (launch shape; the kernel reads NZ)
+  int sv;              // slices per thread (the kernel's SV)
+  int zl;              // lanes of a voxel group: vectors of a z-tile
+  int vb0, nvb, nzt;   // first vector and vectors of [zlo, zhi); z-tiles of zl vectors
+  int nseg;            // view segments a warp's views are split into (1, 2, 4 or 8)
 };
 
-// pixels per thread of the direct exact adjoint
-#ifndef DDFAN_DD_BACK_VG
-#define DDFAN_DD_BACK_VG 2
-#endif
-
-// Voxel tile of the direct exact adjoint: NG = 256/ZL groups as LT lines x
-// SPL segments of VG consecutive voxels along the line.
-template <int ZL>
+template <int SV>
 struct DdBackTile {
-  static constexpr int NT = 256;
-  static constexpr int NG = NT / ZL;
-  static constexpr int VG = DDFAN_DD_BACK_VG;
-  static constexpr int SPL = 8;
-  static constexpr int KT = SPL * VG;
-  static constexpr int LT = NG / SPL;
+  static constexpr int NT = 256, NW = NT / 32;
+  static constexpr int WBUF = 3328;  // bytes of window weights per warp
+  static constexpr int FLUSH = 16;   // views per FP32 partial sum
+  static constexpr int MIN_CTAS = SV == 8 ? DDFAN_DD_BACK_MIN_CTAS : DDFAN_DD_BACK_MIN_CTAS + 1;
+  static constexpr int STEP = 4;     // window values loaded together
+  static constexpr int DYN = 4 * SV * NT * (int)sizeof(float);
 };
 
-// Transpose of k_fwd_dd, on the geometry of k_back_adj: pixel k of line ii
-// receives sum_u w_u (fraction of footprint u inside [k, k+1]) = Q(beta(k+1))
-// - Q(beta(k)), Q the channel prefix sum of w, beta the fractional boundary
-// index of a pixel edge (bracket from the fan-tangent table, fraction from the
-// FP64 boundary lines).  Here the difference is walked over w itself; a
-// thread owns VG consecutive pixels of a line in NZ z-tiles, whose walks
-// chain (the end of one is the start of the next).  Every warp brackets the
-// edges of its own groups, ZL views at a time, and synchronises with itself
-// only.
-template <int ZL, bool XM, int NZ>
-__device__ __forceinline__ void back_dd_body(const DdAdjArgs& a, int tile, int zgrp) {
-  using T = DdBackTile<ZL>;
-  constexpr int NT = T::NT, VG = T::VG, SPL = T::SPL, KT = T::KT, LT = T::LT;
-  constexpr int NW = NT / 32, GW = 32 / ZL;  // warps, voxel groups per warp
-  constexpr int VCW = ZL;                    // views per warp chunk (VCW * GW = 32)
-  constexpr int NEG = VG + 1;                // edges per group
-  constexpr int TBMAX = 1024, LUTMAX = 4096;
-  __shared__ int2 s_geo[NW][VCW][GW][NEG];
-  // per (view, pixel): the walk's weights and both edge cells packed, decoded
-  // once for the ZL z-lanes that walk it
-  __shared__ float4 s_wk[NW][VCW][GW][VG];
-  __shared__ int s_p[NW][VCW];
-  __shared__ float s_sgn[NW][VCW];
-  __shared__ float s_tb[TBMAX];
-  __shared__ uint16_t s_lut[LUTMAX];
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const int zl = lane % ZL, gw = lane / ZL;
-  const int zt_first = a.zt0 + zgrp * NZ;
-  int zbk[NZ], zoff[NZ];
-  bool zok[NZ];
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) {
-    zbk[z] = (zt_first + z) * ZL + zl;
-    zok[z] = zgrp * NZ + z < a.nzt && zbk[z] < a.P4;
-    zoff[z] = zok[z] ? z * ZL : 0;  // a tile past the image reads the first one again (dropped)
+// (view, voxel block) records a warp decodes at a time, the window values a
+// record holds per pass, and a record's stride in bytes (an odd multiple of
+// 16: the stores of the 8 records of a step fall into different banks)
+__host__ __device__ inline int dd_back_records(int GW) { return GW > 16 ? 32 : 16; }
+__host__ __device__ inline int dd_back_window(int GW) { return GW > 16 ? 4 : 12; }
+__host__ __device__ inline int dd_back_stride(int GW) { return GW > 16 ? 80 : 208; }
+
+// 2 x 2-voxel blocks: the CTA's tile is WX * GW blocks wide and WY high, its
+// (8 / nseg) tile warps side by side in x while a warp's run of blocks is short
+__host__ __device__ inline int dd_back_wx(int GW, int nseg) { return GW >= 8 || nseg == 8 ? 1 : 2; }
+
+// 1 / x and 1 / sqrt(x) in FP64: the FP32 approximation (relative error
+// 2^-22) and one Newton step (2^-44), for factors whose product needs less:
+// the angle step below (|z| <= 1 / 128) and the footprint's half-width and
+// weight, both rounded to FP32 afterwards.
+__device__ __forceinline__ double dd_rcp(double x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
+  const double y = (double)r;
+  return fma(y, fma(-x, y, 1.0), y);
+}
+__device__ __forceinline__ double dd_rsqrt(double x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
+  const double y = (double)r;
+  return y * fma(-0.5 * x * y, y, 1.5);
+}
+// 1 / x in FP32, the approximation and one Newton step (within an ulp)
+__device__ __forceinline__ float dd_rcpf(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
+// Cell and fraction of coordinate c clamped to [0, U]: c + 1.5 2^28, rounded
+// to the nearest 2^-24 by the addition itself, holds the cell and 24 fraction
+// bits in its mantissa -- one FP64 addition instead of two comparisons and four
+// conversions.  |c| < 2^27 (beyond, the cell is some cell of the row).
+__device__ __forceinline__ void dd_cell(double c, int U, int& k, float& f) {
+  const double t = c + 402653184.0;
+  const unsigned hi = (unsigned)__double2hiint(t), lo = (unsigned)__double2loint(t);
+  k = (int)(__funnelshift_r(lo, hi, 24) & 0xfffffffu) - 0x8000000;
+  f = (float)(lo & 0xffffffu) * 5.9604644775390625e-8f;
+  if (k < 0) {
+    k = 0;
+    f = 0.f;
+  } else if (k >= U) {
+    k = U - 1;
+    f = 1.f;
   }
-  const int nl = XM ? a.XN : a.YN, N = XM ? a.YN : a.XN;
-  const int ntk = (N + KT - 1) / KT;
-  const int tl = tile / ntk, tk = tile - tl * ntk;
-  const int l0 = tl * LT, k0 = tk * KT;
-  const int g = w * GW + gw;  // the thread's voxel group in the tile
-  const int l = g / SPL, sg = g - l * SPL;
-  const int ii = l0 + l, ks = k0 + sg * VG;
-  const bool active = zok[0] && ii < nl && ks < N;
-  for (int i = tid; i <= a.U; i += NT) s_tb[i] = a.tb[i];
-  for (int i = tid; i < a.M; i += NT) s_lut[i] = a.lut[i];
-  const int nx = a.counts[0];
-  const int vbeg = XM ? 0 : nx, vend = XM ? nx : a.PN;
-  float acc[VG][NZ][4];
-  float4 vm[NZ];  // first interior values (kept between walks; see walk_nz)
+}
+
+// asin(cr / hypot(cr, dt)), the angle of a voxel's ray from the central ray
+// (cross and dot product of the two).  In front of the source (dt > 0) it is
+// atan(cr / dt): with T = j / 64 the grid tangent nearest to cr / dt,
+// atan(cr / dt) = atan(T) + atan(z), z = (cr - T dt) / (dt + T cr), |z| <=
+// 1 / 128, whose Taylor series after z^7 is below 1e-20.  atan(T) from a table
+// of the library function's values; rays beyond 45 degrees call asin.
+constexpr int DD_ATAN_N = 64;
+__device__ __forceinline__ double dd_angle(double cr, double dt, const double* tab) {
+  const float tf = __fdividef((float)cr, (float)dt);
+  if (!(dt > 0.0 && fabsf(tf) <= 1.f)) return asin(cr / sqrt(cr * cr + dt * dt));
+  const float jf = rintf(tf * (float)DD_ATAN_N);
+  const double T = (double)(jf * (1.f / (float)DD_ATAN_N));
+  const double z = fma(-T, dt, cr) * dd_rcp(fma(T, cr, dt));
+  const double z2 = z * z;
+  return fma(z * z2, fma(z2, fma(z2, -1.0 / 7.0, 1.0 / 5.0), -1.0 / 3.0), z) + tab[(int)jf + DD_ATAN_N];
+}
+
+// Fractional boundary index (cell k, fraction f) of the point at v from the
+// source of a view whose central ray has direction n: where it lies between
+// the boundary rays along a line of the view's (constant component vl of v).
+// A ray of fan tangent T has direction n + T m, m normal to n, and meets the
+// line at a point that is a fractional linear function of T, so with the
+// point's own tangent t and the bracket T_b <= t < T_{b+1},
+//   f = 1 - (1 - (t - T_b) / (T_{b+1} - T_b)) D(T_b) / D(t),
+// D(T) the line's constant component of n + T m (D(t) = vl / (n . v)) -- in exact
+// arithmetic the ratio of the forward's boundary positions c_b on the line,
+// from one table of all views instead of two boundary lines of this one.
+// tab[b] = (T_b, 1 / (T_{b+1} - T_b)), T increasing (times dirt); lut: a guess
+// of b, made exact by stepping.  nl: D(T) = nl.x + dirt T nl.y.
+__device__ __forceinline__ void dd_edge(const DdBackArgs& a, double nx, double ny, double vx, double vy, double vl,
+                                        double nlx, double nly, int& k, float& f) {
+  const double cr = a.dirt * (nx * vy - ny * vx), dt = nx * vx + ny * vy;
+  const double r = dd_rcp(dt * vl), t = cr * (vl * r);
+  const float m = fminf(fmaxf(((float)t - a.t0) * a.invdt, 0.f), (float)(a.M - 1));
+  int b = __ldg(a.lut + (int)m);
+  double2 q = __ldg(a.tab + b);
+  double u = (t - q.x) * q.y;
+  while (u >= 1.0 && b < a.U - 1) {
+    q = __ldg(a.tab + ++b);
+    u = (t - q.x) * q.y;
+  }
+  while (u < 0.0 && b > 0) {
+    q = __ldg(a.tab + --b);
+    u = (t - q.x) * q.y;
+  }
+  k = b;
+  f = __saturatef((float)(1.0 - (1.0 - u) * fma(q.x, nly, nlx) * (dt * (dt * r))));
+}
+
+// back_store for a thread's SV slices, in 16-byte pieces where the output allows.
+template <int SV>
+__device__ __forceinline__ void dd_back_store(const BackEpi& e, int ix, int iy, int vb, int XN, int Z, bool scale_by_mask,
+                                              const float (&acc)[SV]) {
+  const size_t pix = (size_t)iy * XN + ix;
+  const float m = e.mask ? (float)e.mask[pix] : 1.f;
+  const float cs = e.xin ? __ldg(e.colsum + pix) : 0.f;
+  const size_t base = pix * Z + (size_t)vb * SV;
+  const bool whole = SV >= 4 && (Z & 3) == 0 && vb * SV >= e.zlo && vb * SV + SV <= e.zhi &&
+                     ((reinterpret_cast<uintptr_t>(e.out) | reinterpret_cast<uintptr_t>(e.xin)) & 15) == 0;
+  float val[SV], x[SV];
 #pragma unroll
-  for (int z = 0; z < NZ; ++z) vm[z] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = 0; s < SV; ++s) x[s] = 0.f;
+  if (e.xin) {
+    if (whole) {
 #pragma unroll
-  for (int v = 0; v < VG; ++v)
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) acc[v][z][0] = acc[v][z][1] = acc[v][z][2] = acc[v][z][3] = 0.f;
-  const size_t P4 = (size_t)a.P4;
-  const size_t vstride = (size_t)(a.U + 1) * P4;
-  const double ocl = XM ? a.ocx : a.ocy, ock = XM ? a.ocy : a.ocx;
-  __syncthreads();  // the bracket tables; the rest of the kernel synchronises per warp
-  const float tfirst = s_tb[0], tlast = s_tb[a.U];
-  for (int v0 = vbeg; v0 < vend; v0 += VCW) {
-    const int nvc = min(VCW, vend - v0);
-    if (lane < nvc) {
-      const int p = a.order[v0 + lane];
-      s_p[w][lane] = p;
-      s_sgn[w][lane] = a.vg[p].sgn;
-    }
-    __syncwarp();
-    for (int e = lane; e < VCW * GW * NEG; e += 32) {
-      const int vv = e / (GW * NEG), r = e - vv * (GW * NEG);
-      const int gl = r / NEG, ke = r - gl * NEG;
-      const int gg = w * GW + gl;
-      const int li = l0 + gg / SPL, ck = k0 + (gg % SPL) * VG + ke;
-      int b = 0;
-      float frac = 0.f;
-      if (vv < nvc && li < nl && ck <= N) {
-        const int p = s_p[w][vv];
-        const ViewGeom& G = a.vg[p];
-        const double lineX = (li - ocl) * a.dx, along = ((double)ck - 0.5 - ock) * a.dx;
-        const float vx = (float)((XM ? lineX : along) - G.sx);
-        const float vy = (float)((XM ? along : lineX) - G.sy);
-        const float cr = G.shx * vy - G.shy * vx, dt = G.shx * vx + G.shy * vy;
-        const float t = a.dirt * __fdividef(cr, dt);
-        if (!(t >= tfirst)) {
-          b = 0;
-        } else if (t >= tlast) {
-          b = a.U;
-        } else {
-          const int m = (int)fminf(fmaxf((t - a.t0) * a.invdt, 0.f), (float)(a.M - 1));
-          b = s_lut[m];
-          int guard = 0;
-          while (b < a.U - 1 && s_tb[b + 1] <= t && guard++ < 64) ++b;
-          while (b > 0 && s_tb[b] > t && guard++ < 128) --b;
-          const double2* fcp = a.fc + (size_t)p * (a.U + 1);
-          const double2 f0 = __ldg(fcp + b), f1 = __ldg(fcp + b + 1);
-          const double di = (double)li;
-          const double c0 = fma(di, f0.x, f0.y), c1 = fma(di, f1.x, f1.y);
-          frac = __fdiv_rn((float)((double)ck - c0), (float)(c1 - c0));
-          frac = fminf(fmaxf(frac, 0.f), 1.f);
-        }
+      for (int s = 0; s + 4 <= SV; s += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(e.xin + base + s);
+        x[s] = t.x; x[s + 1] = t.y; x[s + 2] = t.z; x[s + 3] = t.w;
       }
-      s_geo[w][vv][gl][ke] = make_int2(b, __float_as_int(frac));
-    }
-    __syncwarp();
-    // the walk of pixel v runs from edge v to edge v + 1 (chained: its end is
-    // the next pixel's start)
-    for (int e = lane; e < VCW * GW * VG; e += 32) {
-      const int vv = e / (GW * VG), r = e - vv * (GW * VG);
-      const int gl = r / VG, v = r - gl * VG;
-      const int2 g0 = s_geo[w][vv][gl][v], g1 = s_geo[w][vv][gl][v + 1];
-      const float3 ww = walk3(g0.x, __int_as_float(g0.y), g1.x, __int_as_float(g1.y), s_sgn[w][vv]);
-      s_wk[w][vv][gl][v] = make_float4(ww.x, ww.y, ww.z, __int_as_float(pack_k(g0.x, g1.x)));
-    }
-    __syncwarp();
-    if (active) {
-      for (int vv = 0; vv < nvc; ++vv) {
-        const float4* base = a.w + (size_t)s_p[w][vv] * vstride + zbk[0];
-        const float4* wk = &s_wk[w][vv][gw][0];
-        float4 cur[NZ];
-        {
-          const float4* p0 = base + (size_t)(__float_as_int(wk[0].w) & 0xffff) * P4;
+    } else {
 #pragma unroll
-          for (int z = 0; z < NZ; ++z) cur[z] = __ldg(p0 + zoff[z]);
-        }
-#pragma unroll
-        for (int v = 0; v < VG; ++v) {
-          const float4 g = wk[v];
-          const int pk = __float_as_int(g.w);
-          walk_nz<NZ>(acc[v], cur, vm, base, P4, zoff, pk & 0xffff, pk >> 16, a.U, g);
-        }
-      }
+      for (int s = 0; s < SV; ++s)
+        if (vb * SV + s >= e.zlo && vb * SV + s < e.zhi) x[s] = e.xin[base + s];
     }
-    __syncwarp();
   }
-  if (!active) return;
 #pragma unroll
-  for (int v = 0; v < VG; ++v) {
-    const int kk = ks + v;
-    if (kk >= N) break;
+  for (int s = 0; s < SV; ++s) {
+    val[s] = scale_by_mask ? acc[s] * m : (m != 0.f ? acc[s] : 0.f);
+    if (e.xin) {
+      // x += t / colSum where colSum != 0, else x += t (AAPM_script/OSSART_AAPM.m:94-97)
+      const float t = cs != 0.f ? __fdiv_rn(val[s], cs) : val[s];
+      val[s] = x[s] + t;
+      if (e.nonneg) val[s] = fmaxf(val[s], 0.f);
+    }
+  }
+  if (whole) {
 #pragma unroll
-    for (int z = 0; z < NZ; ++z)
-      if (zok[z]) back_store(a.epi, XM ? ii : kk, XM ? kk : ii, zbk[z], a.XN, a.Z, true, acc[v][z]);
+    for (int s = 0; s + 4 <= SV; s += 4)
+      *reinterpret_cast<float4*>(e.out + base + s) = make_float4(val[s], val[s + 1], val[s + 2], val[s + 3]);
+  } else {
+#pragma unroll
+    for (int s = 0; s < SV; ++s)
+      if (vb * SV + s >= e.zlo && vb * SV + s < e.zhi) e.out[base + s] = val[s];
   }
 }
 
-// One CTA per (voxel tile, z-tile group) of one call.
-template <int ZL, bool XM, int NZ>
-__global__ void __launch_bounds__(256, (DdMinCtas<NZ, DDFAN_DD_BACK_MIN_CTAS>::v)) k_back_dd(const __grid_constant__ DdAdjArgs a) {
-  back_dd_body<ZL, XM, NZ>(a, (int)blockIdx.x, (int)blockIdx.z);
-}
-
-// The work-list launch: CTA b takes item {call, voxel tile, z-tile group} = items[b].
-template <int ZL, bool XM, int NZ>
-__global__ void __launch_bounds__(256, (DdMinCtas<NZ, DDFAN_DD_BACK_MIN_CTAS>::v)) k_back_dd_batch(const DdAdjArgs* __restrict__ args,
-                                                                                const int4* __restrict__ items) {
-  const int4 it = items[blockIdx.x];
-#if DDFAN_DD_BATCH_ARGS_COPY
-  const DdAdjArgs a = args[it.x];  // a local copy: its fields stay in registers
-#else
-  const DdAdjArgs& a = args[it.x];  // read in place (read-only, cached)
-#endif
-  back_dd_body<ZL, XM, NZ>(a, it.y, it.z);
-}
-
-// ============================================================ reference backprojector
-
-struct DdRefArgs {
-  const float4* q;     // residual [slot][U+1][P4] (unweighted), channel U = 0
-  int P4;
-  const ViewGeom* vg;
-  int PN, U, Z, XN, YN;
-  double ocx, ocy, dx, inv_sid, inv_dbeta, cnt;  // cnt = detCntIdx + 1 - 0.5
-  BackEpi epi;
-  int zt0, nzt;
-  int nzc;  // most z-tiles per thread (launch shape; the kernel reads NZ)
-};
-
-// The reference backprojector's formula (AAPM_script/MultiSlicesBackGPU.cu:
-// 115-184): angular detector coordinate alpha = asin(cross / (|s| l)),
-// footprint half-width dx ddv / (2 l^2), weight dx l / ddv, coordinate
-// alpha / dbeta + detCntIdx + 1, evaluated in FP64 once per (voxel, view) of
-// a warp's voxels; the difference of the two channel prefix-sum samples is
-// walked over the residual itself.  Voxel tile as the exact adjoint's (lines
-// are image rows, k = x), VG voxels x NZ z-tiles per thread, ZL views per
-// warp chunk, per-warp synchronisation only.
-template <int ZL, int NZ>
-__device__ __forceinline__ void ref_dd_body(const DdRefArgs& a, int tile, int zgrp) {
-  using T = DdBackTile<ZL>;
-  constexpr int NT = T::NT, VG = T::VG, SPL = T::SPL, KT = T::KT, LT = T::LT;
-  constexpr int NW = NT / 32, GW = 32 / ZL;
-  constexpr int VCW = ZL;  // views per warp chunk
-  // per (view, voxel): the walk's weights (w0, wm, we) and both channel cells
-  // packed (k0 | k1 << 16), decoded once here for the ZL z-lanes that walk it
-  __shared__ float4 s_g[NW][VCW][GW][VG];
+// Measured per c3 subset (96 views x 736 channels, 512^2 x 128): reference
+// formula 1.40 -> 1.08 ms, exact adjoint 1.77 -> 1.25 ms (0.86 ms of either
+// when the decode is left out); 1111 views of 384^2 x 45, exact adjoint 10.8 ->
+// 8.0 ms.  16 warps an SM at 128 registers with 4 values in flight each beat 24
+// at 80 with 1 (1.20), 3 (1.29) or 4 (1.14): more warps spread over more views
+// and lose the L1 hits (80 -> 68 %).
+//
+// Both backprojectors.  A voxel's sample of a view is Phi(cR) - Phi(cL), Phi
+// the channel prefix sum of the residual: of its two pixel edges along the
+// view's lines for the exact adjoint (the transpose of k_fwd_dd: pixel k of
+// line ii receives sum_u w_u (fraction of footprint u inside [k, k+1]) =
+// Q(beta(k+1)) - Q(beta(k)), beta the fractional boundary index of an edge),
+// of its angular footprint for the reference's formula (MultiSlicesBackGPU.cu:
+// 115-184: alpha -+ da, da = dx ddv / (2 l^2), weight dx l / ddv).
+//
+// What bounds it is the L1 pipe and instruction issue, not DRAM: a voxel and
+// view need two or three residual values of 128 slices, and neighbouring
+// voxels mostly the same ones.  So a thread owns a 2 x 2 block of voxels x SV
+// slices and, per view, reads the window of channels the block's four
+// footprints cover once (3.2 values at the c2 geometry where four voxels on
+// their own read 8.8), each value weighted into all four sums: the decode
+// writes the four overlap weights of every window value to shared memory, so
+// the inner loop is one value load, one weight load and 4 SV FMAs, with no
+// address or branch per voxel.  It needs no view order and takes both view
+// orientations in one pass.  Windows of any width work: a record holds 12 (4)
+// values at a time, wider ones take more passes.  Sums are kept per FLUSH
+// views and added to totals in shared memory, so a sum over thousands of
+// views rounds like one over a few; with nseg > 1 the views are split over
+// warps whose totals are added at the end.
+template <int SV, bool ADJ>
+__device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int ztile) {
+  using T = DdBackTile<SV>;
+  constexpr int NW = T::NW, VB = SV * 4;
+  __shared__ __align__(16) unsigned char s_wt[NW][T::WBUF];
+  __shared__ uint2 s_h[NW][32];  // record: window start (vectors), values in this pass
+  __shared__ double s_at[ADJ ? 1 : 2 * DD_ATAN_N + 1];
+  extern __shared__ float s_tot[];  // [4 * SV][NT]: this thread's totals at tid
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const int zl = lane % ZL, gw = lane / ZL;
-  const int zt_first = a.zt0 + zgrp * NZ;
-  int zbk[NZ], zoff[NZ];
-  bool zok[NZ];
-#pragma unroll
-  for (int z = 0; z < NZ; ++z) {
-    zbk[z] = (zt_first + z) * ZL + zl;
-    zok[z] = zgrp * NZ + z < a.nzt && zbk[z] < a.P4;
-    zoff[z] = zok[z] ? z * ZL : 0;  // a tile past the image reads the first one again (dropped)
-  }
-  const int ntx = (a.XN + KT - 1) / KT;
+  const int ZL = a.zl, GW = 32 / ZL;
+  const int g = lane / ZL, zi = lane - g * ZL;
+  const int nseg = a.nseg, wt = w / nseg, seg = w - wt * nseg;
+  const int WX = dd_back_wx(GW, nseg), WY = (NW / nseg) / WX;
+  const int ntx = ((a.XN + 1) / 2 + WX * GW - 1) / (WX * GW);
   const int ty = tile / ntx, tx = tile - ty * ntx;
-  const int y0 = ty * LT, x0 = tx * KT;
-  const int g = w * GW + gw;
-  const int l = g / SPL, sg = g - l * SPL;
-  const int iy = y0 + l, ixs = x0 + sg * VG;
-  const bool active = zok[0] && iy < a.YN && ixs < a.XN;
-  float acc[VG][NZ][4];
-  float4 vm[NZ];  // first interior values (kept between walks; see walk_nz)
+  const int bx0 = (tx * WX + wt % WX) * GW, y0 = 2 * (ty * WY + wt / WX);  // the warp's first block; its rows y0, y0 + 1
+  const int vb = a.vb0 + ztile * ZL + zi;
+  const int x0 = 2 * (bx0 + g);
+  const bool active = g < GW && ztile * ZL + zi < a.nvb && x0 < a.XN && y0 < a.YN;
+  const int NR = dd_back_records(GW), MW = dd_back_window(GW), RS = dd_back_stride(GW);
+  const int VC = NR / GW;  // views decoded at a time
+  const size_t vstride = (size_t)(a.U + 1) * a.ZP * VB, kstride = (size_t)a.ZP * VB;
+  const char* q = reinterpret_cast<const char*>(a.q) + (size_t)(active ? vb : 0) * VB;
+  if (!ADJ) {
+    for (int j = tid; j <= 2 * DD_ATAN_N; j += T::NT) s_at[j] = atan((double)(j - DD_ATAN_N) / (double)DD_ATAN_N);
+    __syncthreads();
+  }
+  float* tot = s_tot + tid;
 #pragma unroll
-  for (int z = 0; z < NZ; ++z) vm[z] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int e = 0; e < 4 * SV; ++e) tot[e * T::NT] = 0.f;
+  Vec<SV> acc[4];
 #pragma unroll
-  for (int v = 0; v < VG; ++v)
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) acc[v][z][0] = acc[v][z][1] = acc[v][z][2] = acc[v][z][3] = 0.f;
-  const double Ud = (double)a.U;
-  const size_t P4 = (size_t)a.P4;
-  const size_t vstride = (size_t)(a.U + 1) * P4;
-  for (int v0 = 0; v0 < a.PN; v0 += VCW) {
-    const int nvc = min(VCW, a.PN - v0);
-    for (int e = lane; e < VCW * GW * VG; e += 32) {
-      const int vv = e / (GW * VG), r = e - vv * (GW * VG);
-      const int gl = r / VG, v = r - gl * VG;
-      const int gg = w * GW + gl;
-      const int yy = y0 + gg / SPL, xx = x0 + (gg % SPL) * VG + v;
-      int2 ii = make_int2(0, 0);
-      float2 ff = make_float2(0.f, 0.f);
-      float wt = 0.f;
-      if (vv < nvc && yy < a.YN && xx < a.XN && (!a.epi.mask || a.epi.mask[(size_t)yy * a.XN + xx] != 0)) {
-        const ViewGeom& G = a.vg[v0 + vv];
-        const double sx = G.sx, sy = G.sy;
-        const double ddx = (xx - a.ocx) * a.dx - sx, ddy = (yy - a.ocy) * a.dx - sy;
-        const double l2 = ddx * ddx + ddy * ddy;
-        const double ln = sqrt(l2);
-        const double alpha = asin((sy * ddx - sx * ddy) * a.inv_sid / ln);
-        const double ddv = fabs(sx) > fabs(sy) ? ddx : ddy;
-        const double da = ddv / l2 * a.dx * 0.5;
-        wt = (float)(a.dx / ddv * ln);
-        const double cL = fmin(fmax((alpha - da) * a.inv_dbeta + a.cnt, 0.0), Ud);
-        const double cR = fmin(fmax((alpha + da) * a.inv_dbeta + a.cnt, 0.0), Ud);
-        ii = make_int2(min((int)cL, a.U - 1), min((int)cR, a.U - 1));
-        ff = make_float2((float)(cL - ii.x), (float)(cR - ii.y));
-      }
-      const float3 ww = walk3(ii.x, ff.x, ii.y, ff.y, wt);
-      s_g[w][vv][gl][v] = make_float4(ww.x, ww.y, ww.z, __int_as_float(pack_k(ii.x, ii.y)));
-    }
-    __syncwarp();
-    if (active) {
-      for (int vv = 0; vv < nvc; ++vv) {
-        const float4* base = a.q + (size_t)(v0 + vv) * vstride + zbk[0];
-#pragma unroll
-        for (int v = 0; v < VG; ++v) {
-          const float4 g = s_g[w][vv][gw][v];
-          const int pk = __float_as_int(g.w), k0 = pk & 0xffff, k1 = pk >> 16;
-          float4 cur[NZ];
-          const float4* p0 = base + (size_t)k0 * P4;
-#pragma unroll
-          for (int z = 0; z < NZ; ++z) cur[z] = __ldg(p0 + zoff[z]);
-          walk_nz<NZ>(acc[v], cur, vm, base, P4, zoff, k0, k1, a.U, g);
+  for (int j = 0; j < 4; ++j) vzero(acc[j]);
+  // decode: lane -> voxel v of block lb (of 8 or GW) of view lv (of VP)
+  const int v = lane & 3, lb = GW >= 8 ? lane >> 2 : (lane >> 2) % GW, lv = GW >= 8 ? 0 : (lane >> 2) / GW;
+  const int VP = GW >= 8 ? 1 : 8 / GW;
+  int xx = 0, yy = 0;
+  double px = 0.0, py = 0.0;
+  bool von = false;
+  const auto place = [&](int gg) {
+    xx = 2 * (bx0 + gg) + (v & 1);
+    yy = y0 + (v >> 1);
+    von = gg < GW && xx < a.XN && yy < a.YN && lv < VP && (!a.epi.mask || a.epi.mask[(size_t)yy * a.XN + xx] != 0);
+    px = (xx - a.ocx) * a.dx;
+    py = (yy - a.ocy) * a.dx;
+  };
+  place(lb);
+  const double hdx = a.dx * 0.5, hdb = hdx * a.inv_dbeta;
+  const float dxf = (float)a.dx;
+  const int vbeg = (int)((long long)a.PN * seg / nseg), vend = (int)((long long)a.PN * (seg + 1) / nseg);
+  int since = 0;
+  for (int v0 = vbeg; v0 < vend; v0 += VC) {
+    const int nvc = min(VC, vend - v0);
+    int mmax = 0;
+    for (int i0 = 0; i0 == 0 || i0 < mmax; i0 += MW) {  // windows wider than a record: more passes
+      // four lanes a block, one voxel each; 8 blocks of one or more views a step
+      for (int pb = 0; pb < GW; pb += 8) {
+        if (GW > 8) place(pb + (lane >> 2));
+#pragma unroll 1
+        for (int u0 = 0; u0 < nvc; u0 += VP) {
+          const int vv = u0 + lv;
+          int kL = 0, kR = 0;
+          float fL = 0.f, fR = 0.f, wgt = 0.f;
+          const bool on = von && vv < nvc;
+          if (on) {
+            const int p = v0 + vv;
+            const ViewGeom& G = a.vg[p];
+            if (ADJ) {
+              // the voxel's two edges along the view's lines (x columns or y rows)
+              const double nx = -G.sx * a.inv_sid, ny = -G.sy * a.inv_sid, vx = px - G.sx, vy = py - G.sy;
+              if (G.xmajor) {
+                dd_edge(a, nx, ny, vx, vy - hdx, vx, nx, -a.dirt * ny, kL, fL);
+                dd_edge(a, nx, ny, vx, vy + hdx, vx, nx, -a.dirt * ny, kR, fR);
+              } else {
+                dd_edge(a, nx, ny, vx - hdx, vy, vy, ny, a.dirt * nx, kL, fL);
+                dd_edge(a, nx, ny, vx + hdx, vy, vy, ny, a.dirt * nx, kR, fR);
+              }
+              wgt = G.sgn;
+            } else {
+              const double sx = G.sx, sy = G.sy, ddx = px - sx, ddy = py - sy;
+              const double l2 = fma(ddx, ddx, ddy * ddy), rl = dd_rsqrt(l2);
+              const double alpha = dd_angle(fma(sy, ddx, -sx * ddy), -fma(sx, ddx, sy * ddy), s_at);
+              const double ddv = fabs(sx) > fabs(sy) ? ddx : ddy;
+              const double da = ddv * (rl * rl) * hdb, ca = fma(alpha, a.inv_dbeta, a.cnt);
+              wgt = (float)(l2 * rl) * dxf * dd_rcpf((float)ddv);
+              dd_cell(ca - da, a.U, kL, fL);
+              dd_cell(ca + da, a.U, kR, fR);
+            }
+          }
+          // the block's window: the cells its four footprints cover (first and
+          // 0xffff - last, both minima, in one word)
+          unsigned kk = on ? (unsigned)min(kL, kR) | (unsigned)(0xffff - max(kL, kR)) << 16 : 0xffffffffu;
+          kk = __vminu2(kk, __shfl_xor_sync(0xffffffffu, kk, 1));
+          kk = __vminu2(kk, __shfl_xor_sync(0xffffffffu, kk, 2));
+          int kb = (int)(kk & 0xffffu);
+          int m = kk == 0xffffffffu ? 0 : 0xffff - (int)(kk >> 16) - kb + 1;  // all off: none
+          // whole steps: more values, with weight 0, after the window or, at the
+          // detector's end, before it
+          m = (m + T::STEP - 1) / T::STEP * T::STEP;
+          kb = m ? max(min(kb, a.U + 1 - m), 0) : 0;
+          mmax = max(mmax, m);
+          const int gg = pb + lb;
+          if (gg < GW && vv < nvc) {
+            const int rec = vv * GW + gg, n = min(max(m - i0, 0), MW);
+            // the value in cell k has the weight of [cL, cR]'s part inside
+            // [k, k + 1] (negative where cR < cL): sat(cR - k) - sat(cL - k),
+            // the cells' difference exact
+            float* wp = reinterpret_cast<float*>(&s_wt[w][rec * RS]) + v;
+            float dL = (float)(kL - kb - i0), dR = (float)(kR - kb - i0);
+            for (int i = 0; i < n; ++i, dL -= 1.f, dR -= 1.f) wp[4 * i] = (__saturatef(dR + fR) - __saturatef(dL + fL)) * wgt;
+            if (v == 0) s_h[w][rec] = make_uint2((unsigned)(vv * (a.U + 1) + kb + (n ? i0 : 0)) * (unsigned)a.ZP, (unsigned)n);
+          }
         }
       }
+      mmax = __reduce_max_sync(0xffffffffu, mmax);
+      __syncwarp();
+      if (active) {
+        const char* qc = q + (size_t)v0 * vstride;
+        const uint2* hp = &s_h[w][g];
+        const unsigned char* rp = &s_wt[w][g * RS];
+#pragma unroll 1
+        for (int vv = 0; vv < nvc; ++vv, hp += GW, rp += GW * RS) {
+          const uint2 h = *hp;
+          const float4* wp = reinterpret_cast<const float4*>(rp);
+          const char* qp = qc + (size_t)h.x * VB;
+#pragma unroll 1
+          for (int i = (int)h.y; i > 0; i -= T::STEP, qp += T::STEP * kstride, wp += T::STEP) {
+            Vec<SV> val[T::STEP];
+#pragma unroll
+            for (int t = 0; t < T::STEP; ++t) vload(val[t], qp + t * kstride);
+#pragma unroll
+            for (int t = 0; t < T::STEP; ++t) {
+              const float4 ww = wp[t];
+              vfma(acc[0], dup2(ww.x), val[t]);
+              vfma(acc[1], dup2(ww.y), val[t]);
+              vfma(acc[2], dup2(ww.z), val[t]);
+              vfma(acc[3], dup2(ww.w), val[t]);
+            }
+          }
+        }
+      }
+      __syncwarp();
     }
-    __syncwarp();
+    since += nvc;
+    if (since >= T::FLUSH || v0 + VC >= vend) {
+      since = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int s = 0; s < SV; ++s) tot[(j * SV + s) * T::NT] += vget(acc[j], s);
+        vzero(acc[j]);
+      }
+    }
+  }
+  if (nseg > 1) {
+    __syncthreads();
+    if (seg != 0) return;
   }
   if (!active) return;
 #pragma unroll
-  for (int v = 0; v < VG; ++v) {
-    if (ixs + v >= a.XN) break;
+  for (int j = 0; j < 4; ++j) {
+    const int ix = x0 + (j & 1), iy = y0 + (j >> 1);
+    if (ix >= a.XN || iy >= a.YN) continue;
+    float val[SV];
 #pragma unroll
-    for (int z = 0; z < NZ; ++z)
-      if (zok[z]) back_store(a.epi, ixs + v, iy, zbk[z], a.XN, a.Z, false, acc[v][z]);
+    for (int s = 0; s < SV; ++s) {
+      val[s] = tot[(j * SV + s) * T::NT];
+      for (int r = 1; r < nseg; ++r) val[s] += tot[(j * SV + s) * T::NT + 32 * r];
+    }
+    dd_back_store<SV>(a.epi, ix, iy, vb, a.XN, a.Z, ADJ, val);
   }
 }
 
-// One CTA per (voxel tile, z-tile group) of one call.
-template <int ZL, int NZ>
-__global__ void __launch_bounds__(256, (DdMinCtas<NZ, DDFAN_DD_BACK_MIN_CTAS>::v)) k_back_ref_dd(const __grid_constant__ DdRefArgs a) {
-  ref_dd_body<ZL, NZ>(a, (int)blockIdx.x, (int)blockIdx.z);
+// One CTA per (voxel tile, z-tile) of one call.
+template <int SV, bool ADJ>
+__global__ void __launch_bounds__(256, DdBackTile<SV>::MIN_CTAS) k_back_dd(const __grid_constant__ DdBackArgs a) {
+  back_dd_body<SV, ADJ>(a, (int)blockIdx.x, (int)blockIdx.z);
 }
 
-// The work-list launch: CTA b takes item {call, voxel tile, z-tile group} = items[b].
-template <int ZL, int NZ>
-__global__ void __launch_bounds__(256, (DdMinCtas<NZ, DDFAN_DD_BACK_MIN_CTAS>::v)) k_back_ref_dd_batch(const DdRefArgs* __restrict__ args,
-                                                                                    const int4* __restrict__ items) {
+// The work-list launch: CTA b takes item {call, voxel tile, z-tile} = items[b].
+template <int SV, bool ADJ>
+__global__ void __launch_bounds__(256, DdBackTile<SV>::MIN_CTAS) k_back_dd_batch(const DdBackArgs* __restrict__ args,
+                                                                               const int4* __restrict__ items) {
   const int4 it = items[blockIdx.x];
-#if DDFAN_DD_BATCH_ARGS_COPY
-  const DdRefArgs a = args[it.x];  // a local copy: its fields stay in registers
-#else
-  const DdRefArgs& a = args[it.x];  // read in place (read-only, cached)
-#endif
-  ref_dd_body<ZL, NZ>(a, it.y, it.z);
+  back_dd_body<SV, ADJ>(args[it.x], it.y, it.z);
 }
 
 // ============================================================ staging
@@ -897,17 +833,18 @@ static __global__ void k_stage_image(const float* __restrict__ src, int Z, const
 }
 
 // dst[p][u][z] = src[p][u][z] * wgt[p][u] for u < U, z < Z; zero on the
-// guard channel u = U and on padding slices (wgt null = 1).
+// guard channel u = U, on padding slices and on DD_PAST entries past the last
+// view (wgt null = 1).
 static __global__ void k_stage_sino(const float* __restrict__ src, int Z, const float* __restrict__ wgt, int U,
                                     float* __restrict__ dst, int Zp, size_t PN) {
-  const size_t n = PN * (U + 1) * Zp;
+  const size_t n = (PN * (U + 1) + DD_PAST) * Zp;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const size_t r = i / Zp;
     const int z = (int)(i - r * Zp);
     const size_t p = r / (U + 1);
     const int u = (int)(r - p * (U + 1));
     float v = 0.f;
-    if (u < U && z < Z) {
+    if (u < U && z < Z && p < PN) {
       const size_t e = p * U + u;
       v = src[e * Z + z];
       if (wgt) v *= wgt[e];

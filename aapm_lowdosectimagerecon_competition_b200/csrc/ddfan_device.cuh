@@ -28,6 +28,11 @@ constexpr int SAT_FP32 = 0, SAT_HILO = 1, SAT_FP64 = 2;
 // no prefix-sum tables: footprint differences read the values directly (ddfan_dd_kernels.cuh)
 constexpr int SAT_DIRECT = 3;
 
+// Entries a backprojector operand holds past its last view: whole steps of
+// window values on a detector of fewer channels than a step's multiple read
+// up to three entries on, with weight 0 (zeros there keep 0 * v at 0).
+constexpr int DD_PAST = 3;
+
 // the cell format that stands in for SAT_DIRECT where a path keeps tables
 __host__ __device__ inline int cell_mode(int mode) { return mode == SAT_DIRECT ? SAT_HILO : mode; }
 

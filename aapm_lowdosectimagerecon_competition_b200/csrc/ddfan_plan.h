@@ -12,8 +12,7 @@ namespace ddfan {
 
 struct BackEpi;
 struct DdFwdArgs;
-struct DdAdjArgs;
-struct DdRefArgs;
+struct DdBackArgs;
 
 int set_err(int code, const char* fmt, ...);
 const char* last_error();
@@ -43,13 +42,14 @@ struct Plan {
   float t0 = 0, invdt = 0, dirt = 1;  // exact-adjoint bracket table
   int M = 0;
   bool adj_ok = true, has_mask = false;
-  std::vector<double> bx, by;
+  std::vector<double> bx, by, tab;
   std::vector<float> xd, yd, tb;
   std::vector<uint16_t> lut;
   // device
   double *d_bx = nullptr, *d_by = nullptr, *d_xd = nullptr, *d_yd = nullptr;
   uint8_t* d_mask = nullptr;
   float* d_tb = nullptr;
+  double2* d_tab = nullptr;  // [U] (T_b, 1 / (T_{b+1} - T_b)), T the boundaries' fan tangents times dirt
   uint16_t* d_lut = nullptr;
   // prefix-sum tables; in the direct mode d_satq holds the staged sinogram
   // operand [PNmax][U+1][4 P4] and there are no image tables
@@ -88,7 +88,7 @@ int plan_zl(int ZB, int zl_force);
 // most z-tiles per thread of the direct kernels for a stack of ZB blocks
 // (1, 2 or 4): the autotuner's record (ddfan_tune_set_nz), else 4
 int plan_nz(int ZB);
-// allows the direct forward kernels their dynamic shared memory on the
+// allows the direct kernels their dynamic shared memory on the
 // current device (dev names it in an error); before any launch there
 int dd_prepare_device(int dev);
 // DD3Boundaries (AAPM_script/utilities.cuh:268-287), float-rounded like the reference stores them
@@ -154,17 +154,18 @@ int dd_fwd_cblocks(const DdFwdArgs& a);
 DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc,
                            const float* cvd, const int* order, int PN, float* out, int orow, int ostride, int zlo,
                            int zhi, const DdResidual* res);
-// The arguments launch_back_dd would launch with: the exact adjoint's two
-// passes, or the REF backprojector's one; returns the z-tile count.
-int make_back_dd_args(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, const double2* fc,
-                      const int* order, const int* counts, int PN, const BackEpi& epi, DdAdjArgs* pass1,
-                      DdAdjArgs* pass2, DdRefArgs* ref);
+// The arguments launch_back_dd would launch with (nvb: vectors of the
+// epilogue's slices) and its voxel tiles (grid x).
+DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN,
+                             const BackEpi& epi);
+int dd_back_tiles(const DdBackArgs& a);
 // what launch_back_dd checks before launching (status code)
-int check_back_dd(const Plan& p, int back_mode, const int* order, const int* counts);
+int check_back_dd(const Plan& p, int back_mode);
 // Backprojection of w [slot][U+1][4 P4] (guard channel U = 0; weighted by
-// 1/|dir.axis| for the exact adjoint) with the epilogue `epi`.
-int launch_back_dd(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, const double2* fc,
-                   const int* order, const int* counts, int PN, const BackEpi& epi, cudaStream_t st);
+// 1/|dir.axis| for the exact adjoint) with the epilogue `epi`, both view
+// orientations in one launch.
+int launch_back_dd(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN, const BackEpi& epi,
+                   cudaStream_t st);
 // dst[pix][z < Zp] = z < Z ? src[pix][z] * mask : 0
 int launch_stage_image(const float* src, int Z, const uint8_t* mask, float* dst, int Zp, size_t npix,
                        cudaStream_t st);

@@ -330,9 +330,8 @@ static int solver_iteration(Solver& s, cudaStream_t st) {
     if ((rc = launch_fwd_dd(p, s.d_x, vg, fc, cvd, s.d_order + o, c, s.d_ax, s.U + 1, s.Zi, 0, s.Zi, &r, st)))
       return rc;
     // backproject, divide by colSum, add, optional clamp (:91-97)
-    if ((rc = launch_back_dd(p, s.back_mode, s.d_ax, vg, fc, s.d_order + o, s.d_counts + 2 * k, c, e, st)))
-      return rc;
-    n += adj ? 3 : 2;
+    if ((rc = launch_back_dd(p, s.back_mode, s.d_ax, vg, c, e, st))) return rc;
+    n += 2;
   }
   for (int k = 0; k < s.nsub && !s.ps && !s.direct; ++k) {
     const int o = s.off[k], c = s.cnt[k];
@@ -748,14 +747,14 @@ static int solver_create(Solver** out, float x0, float y0, int DNU, const float*
       (rc = salloc(s, &s.d_counts, 2 * (size_t)numOfOS)) || (rc = salloc(s, &s.d_rows, P * DNU)) ||
       (rc = salloc(s, &s.d_cols, (size_t)numOfOS * XN * YN)) || (rc = salloc(s, &s.d_y, P * DNU * s.Zi)) ||
       (rc = salloc(s, &s.d_x, V)) || (rc = salloc(s, &s.d_xprev, V)) ||
-      (rc = salloc(s, &s.d_ax, (size_t)std::max(PNmax, 1) * (DNU + (s.direct ? 1 : 0)) * s.Zi)) ||
+      (rc = salloc(s, &s.d_ax, ((size_t)std::max(PNmax, 1) * (DNU + (s.direct ? 1 : 0)) + (s.direct ? DD_PAST : 0)) * s.Zi)) ||
       (rc = salloc(s, &s.d_t, 1)))
     return rc;
   cudaStream_t st = s.own;
   if (s.direct) {
-    // the residual's guard channel stays 0; slice maps for padded slices; the
+    // the residual's guard channel (and what follows the last view) stays 0; slice maps for padded slices; the
     // initial image where masked voxels keep it
-    DDFAN_CK(cudaMemsetAsync(s.d_ax, 0, sizeof(float) * (size_t)std::max(PNmax, 1) * (DNU + 1) * s.Zi, st));
+    DDFAN_CK(cudaMemsetAsync(s.d_ax, 0, sizeof(float) * ((size_t)std::max(PNmax, 1) * (DNU + 1) + DD_PAST) * s.Zi, st));
     const size_t Vc = (size_t)XN * YN * SLN;
     if (s.Zi != SLN) {
       std::vector<int> inv(SLN);
@@ -891,7 +890,7 @@ DDFAN_API size_t ddfan_ossart_estimate_bytes(int XN, int YN, int DNU, int SLN, i
   size_t own = P * sizeof(ViewGeom) + P * (U + 1) * sizeof(double2) + P * U * sizeof(float) +
                3 * P * sizeof(int) + 2 * (size_t)numOfOS * sizeof(int) + P * U * sizeof(float) +
                (size_t)numOfOS * XN * YN * sizeof(float) + P * U * Zi * sizeof(float) +
-               2 * V * sizeof(float) + PNmax * (U + (direct ? 1 : 0)) * Zi * sizeof(float) + sizeof(double);
+               2 * V * sizeof(float) + (PNmax * (U + (direct ? 1 : 0)) + (direct ? DD_PAST : 0)) * Zi * sizeof(float) + sizeof(double);
   // direct mode: the initial image and the published copy (masked solves;
   // padded slices), sinogram staging and slice maps (padded slices)
   if (direct) {
@@ -1079,7 +1078,7 @@ DDFAN_API int ddfan_ossart_launches_per_iter(const ddfan_ossart* h) {
   const Solver* s = reinterpret_cast<const Solver*>(h);
   if (!s) return 0;
   const bool adj = s->back_mode == DDFAN_BACK_ADJ;
-  const int per = s->ps ? 7 : (s->direct ? (adj ? 3 : 2) : (adj ? 5 : 4));
+  const int per = s->ps ? 7 : (s->direct ? 2 : (adj ? 5 : 4));
   return s->nsub * per + (s->useFISTA ? 2 : 0);
 }
 
