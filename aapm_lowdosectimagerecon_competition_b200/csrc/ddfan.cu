@@ -71,7 +71,7 @@ LaunchProfiler::~LaunchProfiler() {
 // number of 4-slice blocks; consulted before the built-in cost model.
 static std::mutex g_tune_mutex;
 static std::map<int, int> g_tuned_zl;
-static std::map<int, int> g_tuned_nz;  // z-tiles per thread of the direct kernels
+static std::map<int, int> g_tuned_nz;  // ddfan_tune_set_nz
 
 static int tuned_zl(int ZB) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
@@ -101,14 +101,17 @@ int pow2_zl(int ZB) {
   return best;
 }
 
-int plan_nz(int ZB) {
-  if (const char* v = getenv("DDFAN_NZ")) {  // a fixed value for measurements, like DDFAN_ZL
-    const int nz = atoi(v);
-    if (nz == 1 || nz == 2 || nz == 4) return nz;
-  }
+// What ddfan_tune_set_nz recorded, or its default.  The direct kernels choose
+// their launch shape themselves (dd_lanes, nseg).
+static int recorded_nz(int ZB) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto it = g_tuned_nz.find(ZB);
   return it == g_tuned_nz.end() ? 4 : it->second;
+}
+
+int dd_pad(int Z) {
+  const int r = Z % 8;
+  return Z < 32 && r >= 1 && r <= 4 ? (Z + 3) / 4 * 4 : (Z + 7) / 8 * 8;
 }
 
 int plan_zl(int ZB, int zl_force) {
@@ -278,8 +281,9 @@ int plan_create(Plan** out, const PlanDesc& d) {
   Plan& p = *P;
   p.device = d.device;
   p.XN = d.XN; p.YN = d.YN; p.U = d.DNU; p.Z = d.SLN; p.ZB = (d.SLN + 3) / 4;
-  p.PNmax = d.PNmax; p.mode = d.sat_mode; p.ZL = plan_zl(p.ZB, d.zl_force); p.NZ = plan_nz(p.ZB);
-  p.P4 = p.ZB;
+  p.PNmax = d.PNmax; p.mode = d.sat_mode; p.ZL = plan_zl(p.ZB, d.zl_force);
+  p.dd = p.mode == SAT_DIRECT || (p.mode == SAT_HILO && !d.tables);
+  p.Zs = dd_pad(p.Z);
   // whole z-tiles: the padding blocks of the last tile are never written; the
   // projectors read them only for the slices past Z, whose results they drop
   p.ZB = (p.ZB + p.ZL - 1) / p.ZL * p.ZL;
@@ -342,14 +346,15 @@ int plan_create(Plan** out, const PlanDesc& d) {
     return set_err(DDFAN_ERR_CUDA, "plan: stream/event creation failed");
   }
   cudaStream_t as = p.alloc_stream;
-  const bool direct = p.mode == SAT_DIRECT;
+  const bool direct = p.dd;
   const size_t F4 = cell_f4(p.mode);
-  // direct mode: no image tables; the staged sinogram operand [PNmax][U+1][P4]
-  // float4 (and the DD_PAST entries k_back_dd may read past it) and a staged
-  // image of 4 P4 slices
+  // direct kernels: no image tables; the staged sinogram operand
+  // [PNmax][U+1][Zs] (and the DD_PAST entries k_back_dd may read past it) and a
+  // staged image
   const size_t nimg = direct ? 0 : (size_t)p.XN * p.YN * p.ZB * F4;
-  const size_t nsino = direct ? ((size_t)p.PNmax * (p.U + 1) + DD_PAST) * p.P4 : (size_t)p.PNmax * (p.U + 1) * p.ZB * F4;
-  const size_t ntmp = (size_t)p.XN * p.YN * (direct ? 4 * (size_t)p.P4 : (size_t)p.Z);
+  const size_t nsino = direct ? (((size_t)p.PNmax * (p.U + 1) + DD_PAST) * p.Zs + 3) / 4
+                              : (size_t)p.PNmax * (p.U + 1) * p.ZB * F4;
+  const size_t ntmp = (size_t)p.XN * p.YN * (direct ? p.Zs : p.Z);
   if ((rc = dalloc(&p.d_bx, p.U + 1, &B, as)) || (rc = dalloc(&p.d_by, p.U + 1, &B, as)) ||
       (rc = dalloc(&p.d_xd, p.U, &B, as)) || (rc = dalloc(&p.d_yd, p.U, &B, as)) ||
       (rc = dalloc(&p.d_mask, (size_t)p.XN * p.YN, &B, as)) || (rc = dalloc(&p.d_tb, p.U + 1, &B, as)) ||
@@ -684,9 +689,8 @@ DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, 
                            const float* cvd, const int* order, int PN, float* out, int orow, int ostride, int zlo,
                            int zhi, const DdResidual* res) {
   DdFwdArgs a{};
-  const int Zs = 4 * p.P4;  // slices of an image pixel
-  a.sv = Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(img) & 31) == 0 ? 8 : 4;
-  a.img = img; a.ZP = Zs / a.sv;
+  a.sv = p.Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(img) & 31) == 0 ? 8 : 4;
+  a.img = img; a.ZP = p.Zs / a.sv;
   a.vg = vg; a.fc = fc; a.cvd = cvd; a.order = order;
   a.out = out; a.orow = orow; a.ostride = ostride;
   a.PN = PN; a.U = p.U; a.XN = p.XN; a.YN = p.YN; a.dx = (float)p.dx;
@@ -727,9 +731,8 @@ int launch_fwd_dd(const Plan& p, const float* img, const ViewGeom* vg, const dou
 DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN,
                              const BackEpi& epi) {
   DdBackArgs a{};
-  const int Zs = 4 * p.P4;  // slices of a residual entry
-  a.sv = Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 31) == 0 ? 8 : 4;
-  a.q = w; a.ZP = Zs / a.sv; a.vg = vg;
+  a.sv = p.Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 31) == 0 ? 8 : 4;
+  a.q = w; a.ZP = p.Zs / a.sv; a.vg = vg;
   a.PN = PN; a.U = p.U; a.XN = p.XN; a.YN = p.YN; a.Z = p.Z;
   a.ocx = p.ocx; a.ocy = p.ocy; a.dx = p.dx;
   if (back_mode == DDFAN_BACK_ADJ) {
@@ -793,12 +796,12 @@ int proj_dev_shared(Plan& p, const float* d_angs, int stride, int PN, const floa
   int rc;
   if ((rc = launch_view_geom(p, d_angs, stride, PN, p.d_vg, p.d_fc, p.d_cvd, st))) return rc;
   if ((rc = launch_view_order(p.d_vg, PN, p.d_order, p.d_counts, st))) return rc;
-  if (p.mode == SAT_DIRECT) {
-    // the kernel reads 4-slice float4 runs of a masked image: stage the
-    // caller's image unless it already is one
+  if (p.dd) {
+    // the kernel reads vectors of slices of a masked image: stage the caller's
+    // image unless it already is one
     const float* img = d_vol;
-    if (p.has_mask || (p.Z & 3) || (reinterpret_cast<uintptr_t>(d_vol) & 15)) {
-      if ((rc = launch_stage_image(d_vol, p.Z, p.has_mask ? p.d_mask : nullptr, p.d_tmp, 4 * p.P4,
+    if (p.has_mask || p.Z != p.Zs || (reinterpret_cast<uintptr_t>(d_vol) & 15)) {
+      if ((rc = launch_stage_image(d_vol, p.Z, p.has_mask ? p.d_mask : nullptr, p.d_tmp, p.Zs,
                                    (size_t)p.XN * p.YN, st)))
         return rc;
       img = p.d_tmp;
@@ -820,9 +823,9 @@ int back_dev_shared(Plan& p, const float* d_angs, int stride, int PN, const floa
   const bool adj = back_mode == DDFAN_BACK_ADJ;
   BackEpi e{};
   e.out = d_vol; e.mask = p.has_mask ? p.d_mask : nullptr; e.zlo = zlo; e.zhi = zhi;
-  if (p.mode == SAT_DIRECT) {
+  if (p.dd) {
     float* w = reinterpret_cast<float*>(p.d_satq);
-    if ((rc = launch_stage_sino(d_prj, p.Z, adj ? p.d_cvd : nullptr, p.U, w, 4 * p.P4, (size_t)PN, st))) return rc;
+    if ((rc = launch_stage_sino(d_prj, p.Z, adj ? p.d_cvd : nullptr, p.U, w, p.Zs, (size_t)PN, st))) return rc;
     rc = launch_back_dd(p, back_mode, w, p.d_vg, PN, e, st);
     mark_use(p, st);
     return rc;
@@ -1060,18 +1063,18 @@ DDFAN_API int ddfan_tune_set_nz(int zblocks, int nz) {
   return DDFAN_OK;
 }
 
-DDFAN_API int ddfan_tune_get_nz(int zblocks) { return zblocks < 1 ? 0 : plan_nz(zblocks); }
+DDFAN_API int ddfan_tune_get_nz(int zblocks) { return zblocks < 1 ? 0 : recorded_nz(zblocks); }
 
 DDFAN_API size_t ddfan_plan_estimate_bytes(int XN, int YN, int DNU, int SLN, int PNmax, int sat_mode) {
   if (XN < 1 || YN < 1 || DNU < 2 || SLN < 1 || PNmax < 1 || sat_mode < 0 || sat_mode > SAT_DIRECT) return 0;
-  const int P4 = (SLN + 3) / 4;
-  int ZB = P4;
+  int ZB = (SLN + 3) / 4;
   const int ZL = pow2_zl(ZB);
   ZB = (ZB + ZL - 1) / ZL * ZL;
   const size_t F4 = cell_f4(sat_mode), U = (size_t)DNU, P = (size_t)PNmax;
-  const bool direct = sat_mode == SAT_DIRECT;
-  const size_t cells = direct ? (P * (U + 1) + DD_PAST) * P4 : 2 * (size_t)XN * YN * ZB * F4 + P * (U + 1) * ZB * F4;
-  const size_t tmp = (size_t)XN * YN * (direct ? 4 * (size_t)P4 : (size_t)SLN);
+  const bool direct = sat_mode == SAT_DIRECT || sat_mode == SAT_HILO;
+  const size_t Zs = (size_t)dd_pad(SLN);
+  const size_t cells = direct ? ((P * (U + 1) + DD_PAST) * Zs + 3) / 4 : 2 * (size_t)XN * YN * ZB * F4 + P * (U + 1) * ZB * F4;
+  const size_t tmp = (size_t)XN * YN * (direct ? Zs : (size_t)SLN);
   return cells * sizeof(float4) + (2 * (U + 1) + 4 * U) * sizeof(double) + (size_t)XN * YN +
          (U + 1) * sizeof(float) + 4 * (U + 1) * sizeof(uint16_t) + P * sizeof(ViewGeom) +
          P * (U + 1) * sizeof(double2) + P * U * sizeof(float) + tmp * sizeof(float) +

@@ -181,7 +181,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
   for (int i = 0; i < n; ++i) {
     Solver* s = solvers[i];
     if (!s) return set_err(DDFAN_ERR_ARG, "batch: solver %d is null", i);
-    if (!s->direct)
+    if (!s->batchable)
       return set_err(DDFAN_ERR_UNSUPPORTED,
                      "batch: solver %d is not a direct-mode solver with one angle list for all slices", i);
     if (i && s->device != solvers[0]->device)

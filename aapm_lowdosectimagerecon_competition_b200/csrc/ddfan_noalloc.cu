@@ -136,8 +136,8 @@ extern "C" DDFAN_API int ddfan_proj_noalloc(float x0, float y0, int DNU, const f
   p.device = dev;
   p.XN = XN; p.YN = YN; p.U = DNU; p.Z = SLN; p.ZB = (SLN + 3) / 4;
   p.PNmax = PN; p.mode = sat_mode; p.ZL = plan_zl(p.ZB, 0);  // the z-tile width a plan would take
-  p.NZ = plan_nz(p.ZB);
-  p.P4 = p.ZB;
+  p.dd = sat_mode == SAT_DIRECT || sat_mode == SAT_HILO;  // as a plan of that mode
+  p.Zs = (SLN + 3) / 4 * 4;  // the least padding: problems that fitted the scratch array still do
   p.ZB = (p.ZB + p.ZL - 1) / p.ZL * p.ZL;
   p.x0 = x0; p.y0 = y0; p.dx = dx;
   p.ocx = (XN - 1.0) * 0.5 - (double)imgXCenter / (double)dx;
@@ -150,16 +150,18 @@ extern "C" DDFAN_API int ddfan_proj_noalloc(float x0, float y0, int DNU, const f
   std::vector<uint8_t> hmask;
   if (mask) hmask.assign(mask, mask + (size_t)XN * YN);
   p.has_mask = mask != nullptr;
-  const bool direct = sat_mode == SAT_DIRECT;
-  // the direct kernels read 4-slice float4 runs of a masked image: staged
+  const bool direct = p.dd;
+  // the direct kernels read vectors of slices of a masked image: staged
   // unless the caller's image already is one
-  const bool stage = direct && (mask || (SLN & 3) || (reinterpret_cast<uintptr_t>(d_vol) & 15));
+  const bool stage = direct && (mask || SLN != p.Zs || (reinterpret_cast<uintptr_t>(d_vol) & 15));
   // Carve the scratch array.  Nothing in it needs to start at zero: each
   // region is written by this call before it is read, except the padding
   // z-blocks of the prefix-sum tables' last z-tile, which no kernel writes
   // and the forward projector reads only for slices past SLN, whose results
   // it drops -- a previous call's contents there are harmless.
-  const size_t cells = direct ? 0 : (size_t)XN * YN * p.ZB * cell_f4(sat_mode);
+  // What is refused does not depend on which kernels run: hi/lo calls count
+  // the tables of their cells, although the direct kernels need less.
+  const size_t cells = sat_mode == SAT_DIRECT ? 0 : (size_t)XN * YN * p.ZB * cell_f4(sat_mode);
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off += align256(bytes); return o; };
   const size_t o_bx = take(sizeof(double) * (DNU + 1)), o_by = take(sizeof(double) * (DNU + 1));
@@ -169,7 +171,7 @@ extern "C" DDFAN_API int ddfan_proj_noalloc(float x0, float y0, int DNU, const f
   const size_t o_cvd = take(sizeof(float) * PN * DNU), o_ord = take(sizeof(int) * PN);
   const size_t o_cnt = take(sizeof(int) * 2);
   const size_t o_satx = take(sizeof(float4) * cells), o_saty = take(sizeof(float4) * cells);
-  const size_t o_img = take(stage ? sizeof(float4) * (size_t)XN * YN * p.P4 : 0);
+  const size_t o_img = sat_mode == SAT_DIRECT ? take(stage ? sizeof(float) * (size_t)XN * YN * p.Zs : 0) : o_satx;
   if (off > DDFAN_NOALLOC_SCRATCH_BYTES)
     return set_err(DDFAN_ERR_UNSUPPORTED,
                    "proj_noalloc: this problem needs %zu bytes of scratch, the fixed scratch array holds %llu "
@@ -210,7 +212,7 @@ extern "C" DDFAN_API int ddfan_proj_noalloc(float x0, float y0, int DNU, const f
       const float* img = d_vol;
       if (stage) {
         float* si = reinterpret_cast<float*>(base + o_img);
-        rc = launch_stage_image(d_vol, SLN, p.d_mask, si, 4 * p.P4, (size_t)XN * YN, st);
+        rc = launch_stage_image(d_vol, SLN, p.d_mask, si, p.Zs, (size_t)XN * YN, st);
         img = si;
       }
       if (!rc) rc = launch_fwd_dd(p, img, p.d_vg, p.d_fc, p.d_cvd, p.d_order, PN, d_prj, DNU, SLN, 0, SLN, nullptr, st);

@@ -28,14 +28,18 @@ struct PlanDesc {
   const uint8_t* mask;
   int SLN, PNmax, sat_mode, device;
   int zl_force = 0;  // 1, 2, 4 or 8: exactly this many z-blocks per z-tile (else chosen by pow2_zl)
+  bool tables = false;  // hi/lo: keep prefix-sum tables (the windowed solver) instead of the direct kernels
 };
 
 // Geometry and device scratch for one (image, detector, slice count) shape.
 struct Plan {
   int device = 0;
   int XN = 0, YN = 0, U = 0, Z = 0, ZB = 0, PNmax = 0, mode = 0, ZL = 1;
-  int P4 = 0;  // 4-slice blocks of the direct mode's operands: ceil(Z / 4)
-  int NZ = 4;  // most z-tiles per thread of the direct kernels (1, 2 or 4)
+  // Calls with one angle list for all slices run the direct kernels (no
+  // tables): the direct mode, and the hi/lo mode, whose compensated sums they
+  // match in precision (both 1e-7 of the FP64 oracle) in half its time.
+  bool dd = false;
+  int Zs = 0;  // slices of the direct kernels' operands, padded (dd_pad)
   double x0 = 0, y0 = 0, dx = 1, ocx = 0, ocy = 0, detCntIdx = 0;
   double inv_dbeta = 0, inv_sid = 0;  // REF backprojector
   double sh0x = 0, sh0y = -1;         // unit vector source -> rotation centre, angle 0
@@ -51,13 +55,13 @@ struct Plan {
   float* d_tb = nullptr;
   double2* d_tab = nullptr;  // [U] (T_b, 1 / (T_{b+1} - T_b)), T the boundaries' fan tangents times dirt
   uint16_t* d_lut = nullptr;
-  // prefix-sum tables; in the direct mode d_satq holds the staged sinogram
-  // operand [PNmax][U+1][4 P4] and there are no image tables
+  // prefix-sum tables; with dd d_satq holds the staged sinogram operand
+  // [PNmax][U+1][Zs] and there are no image tables
   float4 *d_satx = nullptr, *d_saty = nullptr, *d_satq = nullptr;
   ViewGeom* d_vg = nullptr;
   double2* d_fc = nullptr;
   float* d_cvd = nullptr;
-  float* d_tmp = nullptr;   // one image of scratch (exact adjoint, pass 1; the direct mode's staged image)
+  float* d_tmp = nullptr;   // one image of scratch (exact adjoint, pass 1; with dd the staged image)
   float* d_angs = nullptr;  // PNmax angles (host-angle entry points)
   int* d_order = nullptr;   // PNmax views in dispatch order (x-major first)
   int* d_counts = nullptr;  // {x-major views, others}
@@ -85,9 +89,9 @@ int pow2_zl(int ZB);
 // the z-tile width a plan uses: pow2_zl, narrowed by the DDFAN_ZL environment
 // variable (1, 2, 4 or 8), or exactly zl_force when that is one of those
 int plan_zl(int ZB, int zl_force);
-// most z-tiles per thread of the direct kernels for a stack of ZB blocks
-// (1, 2 or 4): the autotuner's record (ddfan_tune_set_nz), else 4
-int plan_nz(int ZB);
+// Slices the direct kernels' operands hold for Z: a multiple of 8 (256-bit
+// loads), or of 4 where that would pad a short stack by half
+int dd_pad(int Z);
 // allows the direct kernels their dynamic shared memory on the
 // current device (dev names it in an error); before any launch there
 int dd_prepare_device(int dev);
@@ -141,7 +145,7 @@ struct DdResidual {
   const float* wgt = nullptr;     // [slot][U] or null
   int ystride = 0;
 };
-// Forward projection of the masked image img [YN][XN][4 P4] into
+// Forward projection of the masked image img [YN][XN][Zs] into
 // out[slot][orow][ostride] (slices [zlo, zhi) written).
 int launch_fwd_dd(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc, const float* cvd,
                   const int* order, int PN, float* out, int orow, int ostride, int zlo, int zhi,
@@ -161,7 +165,7 @@ DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const
 int dd_back_tiles(const DdBackArgs& a);
 // what launch_back_dd checks before launching (status code)
 int check_back_dd(const Plan& p, int back_mode);
-// Backprojection of w [slot][U+1][4 P4] (guard channel U = 0; weighted by
+// Backprojection of w [slot][U+1][Zs] (guard channel U = 0; weighted by
 // 1/|dir.axis| for the exact adjoint) with the epilogue `epi`, both view
 // orientations in one launch.
 int launch_back_dd(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN, const BackEpi& epi,

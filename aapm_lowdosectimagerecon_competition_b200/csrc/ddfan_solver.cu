@@ -520,6 +520,7 @@ static int solver_weights_cells(Solver& s, const PlanDesc& d, const std::vector<
   d1.PNmax = PNmax;
   d1.zl_force = 0;
   d1.sat_mode = cell_mode(d.sat_mode);
+  d1.tables = true;
   PlanPtr P1;
   int rc = plan_create(&P1.p, d1);
   if (rc) return rc;
@@ -712,14 +713,15 @@ static int solver_create(Solver** out, float x0, float y0, int DNU, const float*
     s.ps = want_ps || (s.win && !want_win && win_cost > threshold);
     if (s.ps) s.win = false;
   }
-  // the direct mode serves one angle list for all slices; the per-slice
-  // paths keep hi/lo tables
-  s.direct = sat_mode == SAT_DIRECT && !s.win && !s.ps;
+  // the direct kernels serve one angle list for all slices (direct and hi/lo
+  // modes); the per-slice paths keep hi/lo tables
+  s.direct = (sat_mode == SAT_DIRECT || sat_mode == SAT_HILO) && !s.win && !s.ps;
+  s.batchable = s.direct && sat_mode == SAT_DIRECT;
   if (sat_mode == SAT_DIRECT && !s.direct) sat_mode = cell_mode(sat_mode);
   if (s.win) {
     s.Zi = W.Zi; s.nzt = W.nzt; s.Mc = W.Mc; s.perm = W.perm; s.maxcnt = W.maxcnt;
   } else if (s.direct) {
-    s.Zi = (SLN + 3) / 4 * 4;
+    s.Zi = dd_pad(SLN);
     s.perm.assign(s.Zi, -1);
     for (int z = 0; z < SLN; ++z) s.perm[z] = z;
   } else {
@@ -728,7 +730,7 @@ static int solver_create(Solver** out, float x0, float y0, int DNU, const float*
   const int PNmax = s.win ? W.PNmax : PNsub;
   PlanDesc d{x0, y0, DNU, xds, yds, detCntIdx, imgXCenter, imgYCenter, XN, YN, dx, mask, s.Zi, std::max(PNmax, 1),
              sat_mode, device};
-  if (s.win) d.zl_force = W.ZL;
+  if (s.win) d.zl_force = W.ZL, d.tables = true;
   // the slice-major path uses the plan's geometry, mask and bracket tables only
   PlanDesc dp = d;
   if (s.ps) dp.SLN = dp.PNmax = 1;
@@ -881,9 +883,9 @@ DDFAN_API size_t ddfan_ossart_estimate_bytes(int XN, int YN, int DNU, int SLN, i
                                              int sat_mode) {
   if (numOfOS < 1 || PNall < numOfOS) return 0;
   const size_t PNmax = (size_t)(PNall + numOfOS - 1) / numOfOS;
-  const bool direct = sat_mode == SAT_DIRECT;
-  // the direct mode pads slices to a multiple of 4 and keeps a guard channel
-  const size_t Zi = direct ? (size_t)(SLN + 3) / 4 * 4 : (size_t)SLN;
+  const bool direct = sat_mode == SAT_DIRECT || sat_mode == SAT_HILO;
+  // the direct kernels pad slices and keep a guard channel
+  const size_t Zi = direct ? (size_t)dd_pad(SLN) : (size_t)SLN;
   const size_t U = (size_t)DNU, P = (size_t)PNall, V = (size_t)XN * YN * Zi;
   const size_t plan = ddfan_plan_estimate_bytes(XN, YN, DNU, (int)Zi, (int)PNmax, sat_mode);
   if (!plan) return 0;
@@ -891,7 +893,7 @@ DDFAN_API size_t ddfan_ossart_estimate_bytes(int XN, int YN, int DNU, int SLN, i
                3 * P * sizeof(int) + 2 * (size_t)numOfOS * sizeof(int) + P * U * sizeof(float) +
                (size_t)numOfOS * XN * YN * sizeof(float) + P * U * Zi * sizeof(float) +
                2 * V * sizeof(float) + (PNmax * (U + (direct ? 1 : 0)) + (direct ? DD_PAST : 0)) * Zi * sizeof(float) + sizeof(double);
-  // direct mode: the initial image and the published copy (masked solves;
+  // direct kernels: the initial image and the published copy (masked solves;
   // padded slices), sinogram staging and slice maps (padded slices)
   if (direct) {
     own += 2 * (size_t)XN * YN * SLN * sizeof(float);

@@ -61,13 +61,15 @@ struct Solver {
   float* d_tabx = nullptr;   // image rows table [Z][YN][XN] cells
   float* d_taby = nullptr;   // image columns table [Z][XN][YN] cells
   float* d_sq = nullptr;     // weighted residual table [Z][cstride][U+1] cells
-  // Direct mode (no prefix-sum tables; one angle list for all slices): the
-  // image d_x [YN][XN][Zi] has its slices padded to a multiple of 4 (Zi) and
+  // Direct kernels (no prefix-sum tables; one angle list for all slices; the
+  // direct and hi/lo modes): the image d_x [YN][XN][Zi] has its slices padded
+  // (Zi = dd_pad) and
   // its masked voxels kept at 0, so the projector reads it as it is; d_ax holds
   // the residual [PNmax][U+1][Zi] with a zero guard channel.  A masked voxel's
   // published value is its initial one (d_x0, the caller's layout), clamped
   // at 0 by the updates when they clamp -- what the table path computes there.
   bool direct = false;
+  bool batchable = false;    // created with DDFAN_SAT_DIRECT: what ddfan_batch_create takes
   float* d_x0 = nullptr;
   long long iters_done = 0;
   cudaStream_t own = nullptr;

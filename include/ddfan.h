@@ -40,12 +40,15 @@ extern "C" {
 
 /* precision of the prefix-sum (SAT) tables and of their differences */
 #define DDFAN_SAT_FP32 0 /* plain FP32 sums (the reference's precision class) */
-#define DDFAN_SAT_HILO 1 /* compensated hi/lo FP32 pairs */
+#define DDFAN_SAT_HILO 1 /* compensated: no cancellation between two prefix sums */
 #define DDFAN_SAT_FP64 2 /* FP64 sums */
 /* no tables: each difference of two interpolated prefix sums is evaluated as
  * the sum of the values it telescopes to (exact overlap weights, FP32, no
- * cancellation).  Used on the paths with one angle list for all slices; paths
- * that keep tables (per-slice angle lists) use hi/lo cells in this mode. */
+ * cancellation).  Used on the paths with one angle list for all slices, in the
+ * hi/lo mode too (its errors there are no larger than the hi/lo tables' and it
+ * takes half their time or less); paths that keep tables (per-slice angle
+ * lists) use hi/lo FP32 pairs in both modes.  Solvers of this mode can be
+ * batched. */
 #define DDFAN_SAT_DIRECT 3
 
 /* backprojector */
@@ -63,10 +66,10 @@ DDFAN_API int ddfan_version(void);
  * created afterwards. */
 DDFAN_API int ddfan_tune_set_zl(int zblocks, int zl);
 DDFAN_API int ddfan_tune_get_zl(int zblocks);
-/* the direct mode's (DDFAN_SAT_DIRECT) second tile dimension: each thread
- * walks the footprints it decodes for up to nz z-tiles (nz in {1, 2, 4};
- * default 4; nz = 0 forgets a record).  Results do not depend on it (every
- * slice sums the same terms in the same order); the launch shape does. */
+/* a second recorded dimension (nz in {1, 2, 4}; default 4; nz = 0 forgets a
+ * record), kept for autotuner caches: the kernels without tables choose their
+ * launch shape from the slice count themselves, so neither record changes
+ * them. */
 DDFAN_API int ddfan_tune_set_nz(int zblocks, int nz);
 DDFAN_API int ddfan_tune_get_nz(int zblocks);
 /* device bytes ddfan_plan_create / ddfan_ossart_create would allocate
