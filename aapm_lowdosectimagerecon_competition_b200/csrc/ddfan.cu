@@ -109,9 +109,12 @@ static int recorded_nz(int ZB) {
   return it == g_tuned_nz.end() ? 4 : it->second;
 }
 
-int dd_pad(int Z) {
-  const int r = Z % 8;
-  return Z < 32 && r >= 1 && r <= 4 ? (Z + 3) / 4 * 4 : (Z + 7) / 8 * 8;
+int dd_pad(int Z) { return Z == 1 ? 1 : (Z <= 4 ? 4 : (Z + 7) / 8 * 8); }
+
+// Slices per thread for operands of Zs slices at p
+static int dd_vector(int Zs, const void* p) {
+  if (Zs % 4) return 1;
+  return Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 31) == 0 ? 8 : 4;
 }
 
 int plan_zl(int ZB, int zl_force) {
@@ -241,12 +244,15 @@ void boundaries(int n, const float* c, std::vector<double>& out) {
 // creation precedes every launch on a plan and never runs under capture.
 int dd_prepare_device(int dev) {
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd<8>, DdFwdTile<8>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd<4>, DdFwdTile<4>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<8, true>, DdBackTile<8>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<8, false>, DdBackTile<8>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<4, true>, DdBackTile<4>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<4, false>, DdBackTile<4>::DYN);
+  for (const int sv : {8, 4, 1})
+    for (const int thin : {0, 1})
+      dd_dispatch(sv, thin, [&](auto SV, auto THIN) {
+        constexpr int v = decltype(SV)::value;
+        constexpr bool t = decltype(THIN)::value;
+        if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd<v, t>, DdFwdTile<v>::DYN);
+        if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<v, true, t>, DdBackTile<v>::DYN);
+        if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd<v, false, t>, DdBackTile<v>::DYN);
+      });
   if (e != cudaSuccess)
     return set_err(DDFAN_ERR_CUDA, "kernel attributes on device %d: %s", dev, cudaGetErrorString(e));
   return DDFAN_OK;
@@ -669,6 +675,11 @@ int launch_publish_masked(const float* x, int Zi, const float* x0, int Z, const 
   return check_launch("k_publish_masked");
 }
 
+// At most this many vectors of slices (1: up to 8 slices) run the thin kernels;
+// with two (256^2 x 16, 30 views) they took 78 us forward and 83 us back where
+// decoding once for both took 69 and 72
+constexpr int DD_THIN = 1;
+
 // Lanes per group (vectors per z-tile) of the direct kernels for nvb vectors
 // of slices: at most a warp's 32, and of the splits into z-tiles the one that
 // leaves the fewest lanes idle -- 32 / zl groups fill a warp only when zl
@@ -685,11 +696,14 @@ int dd_lanes(int nvb) {
   return best;
 }
 
+// Channels of a forward warp
+static int dd_fwd_channels(const DdFwdArgs& a) { return a.thin ? 64 : 32 / a.zl * DDFAN_DD_FWD_CG; }
+
 DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc,
                            const float* cvd, const int* order, int PN, float* out, int orow, int ostride, int zlo,
                            int zhi, const DdResidual* res) {
   DdFwdArgs a{};
-  a.sv = p.Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(img) & 31) == 0 ? 8 : 4;
+  a.sv = dd_vector(p.Zs, img);
   a.img = img; a.ZP = p.Zs / a.sv;
   a.vg = vg; a.fc = fc; a.cvd = cvd; a.order = order;
   a.out = out; a.orow = orow; a.ostride = ostride;
@@ -697,12 +711,12 @@ DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, 
   a.zlo = std::max(0, zlo); a.zhi = zhi < 0 ? p.Z : std::min(zhi, p.Z);
   a.vb0 = a.zlo / a.sv;
   a.nvb = a.zhi > a.zlo ? (a.zhi + a.sv - 1) / a.sv - a.vb0 : 0;
-  a.zl = dd_lanes(std::max(a.nvb, 1));
+  a.thin = a.sv == 1 || a.nvb <= DD_THIN;
+  a.zl = a.thin ? 1 : dd_lanes(a.nvb);
   a.nzt = (a.nvb + a.zl - 1) / a.zl;
   // a launch of fewer warps than the SMs hold (24 each) splits every ray's
   // lines over 2, 4 or 8 of them
-  const int cww = 32 / a.zl * DDFAN_DD_FWD_CG;
-  const long long warps = (long long)PN * ((p.U + cww - 1) / cww) * a.nzt;
+  const long long warps = (long long)PN * ((p.U + dd_fwd_channels(a) - 1) / dd_fwd_channels(a)) * a.nzt;
   a.nseg = 1;
   while (a.nseg < 8 && warps * a.nseg < 148 * 24) a.nseg *= 2;
   if (res) {
@@ -712,7 +726,7 @@ DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, 
 }
 
 int dd_fwd_cblocks(const DdFwdArgs& a) {
-  const int cw = 32 / a.zl * DDFAN_DD_FWD_CG * (8 / a.nseg);
+  const int cw = dd_fwd_channels(a) * (8 / a.nseg);
   return (a.U + cw - 1) / cw;
 }
 
@@ -723,21 +737,23 @@ int launch_fwd_dd(const Plan& p, const float* img, const ViewGeom* vg, const dou
   if (a.nvb == 0 || PN < 1) return DDFAN_OK;
   ProfScope ps(KIND_FWD, st);
   const dim3 grid(PN, dd_fwd_cblocks(a), a.nzt);
-  if (a.sv == 8) k_fwd_dd<8><<<grid, DdFwdTile<8>::NT, DdFwdTile<8>::DYN, st>>>(a);
-  else k_fwd_dd<4><<<grid, DdFwdTile<4>::NT, DdFwdTile<4>::DYN, st>>>(a);
+  dd_dispatch(a.sv, a.thin, [&](auto SV, auto THIN) {
+    constexpr int v = decltype(SV)::value;
+    k_fwd_dd<v, decltype(THIN)::value><<<grid, 256, DdFwdTile<v>::DYN, st>>>(a);
+  });
   return check_launch("k_fwd_dd");
 }
 
 DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN,
                              const BackEpi& epi) {
   DdBackArgs a{};
-  a.sv = p.Zs % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 31) == 0 ? 8 : 4;
+  a.sv = dd_vector(p.Zs, w);
   a.q = w; a.ZP = p.Zs / a.sv; a.vg = vg;
   a.PN = PN; a.U = p.U; a.XN = p.XN; a.YN = p.YN; a.Z = p.Z;
-  a.ocx = p.ocx; a.ocy = p.ocy; a.dx = p.dx;
+  a.ocx = p.ocx; a.ocy = p.ocy; a.dx = p.dx; a.sidf = (float)(1.0 / p.inv_sid);
   if (back_mode == DDFAN_BACK_ADJ) {
     a.tab = p.d_tab; a.lut = p.d_lut;
-    a.t0 = p.t0; a.invdt = p.invdt; a.dirt = p.dirt; a.M = p.M; a.inv_sid = p.inv_sid;
+    a.t0 = p.t0; a.invdt = p.invdt; a.dirtf = p.dirt; a.dirt = p.dirt; a.M = p.M; a.inv_sid = p.inv_sid;
   } else {
     a.inv_dbeta = p.inv_dbeta; a.cnt = (double)p.detCntIdx + 0.5;
   }
@@ -746,18 +762,23 @@ DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const
   a.epi.zhi = epi.zhi < 0 ? p.Z : std::min(epi.zhi, p.Z);
   a.vb0 = a.epi.zlo / a.sv;
   a.nvb = a.epi.zhi > a.epi.zlo ? (a.epi.zhi + a.sv - 1) / a.sv - a.vb0 : 0;
-  a.zl = dd_lanes(std::max(a.nvb, 1));
+  a.thin = a.sv == 1 || a.nvb <= DD_THIN;
+  a.zl = a.thin ? 1 : dd_lanes(a.nvb);
   a.nzt = (a.nvb + a.zl - 1) / a.zl;
   // a launch of fewer warps than the SMs hold (24 each) splits the views over
   // 2, 4 or 8 of them
-  const long long GW = 32 / a.zl;
-  const long long warps = ((a.XN + 1) / 2 + GW - 1) / GW * ((a.YN + 1) / 2) * a.nzt;
+  const long long GW = 32 / a.zl, nbx = (a.XN + 1) / 2, nby = (a.YN + 1) / 2;
+  const long long warps = (a.thin ? (nbx * nby + 31) / 32 : (nbx + GW - 1) / GW * nby) * a.nzt;
   a.nseg = 1;
   while (a.nseg < 8 && warps * a.nseg < 148 * 24 && a.nseg * 4 <= PN) a.nseg *= 2;
   return a;
 }
 
 int dd_back_tiles(const DdBackArgs& a) {
+  if (a.thin) {
+    const long long blocks = (long long)((a.XN + 1) / 2) * ((a.YN + 1) / 2), per = 32 * (8 / a.nseg);
+    return (int)((blocks + per - 1) / per);
+  }
   const int GW = 32 / a.zl, WX = dd_back_wx(GW, a.nseg), WY = 8 / a.nseg / WX;
   return (((a.XN + 1) / 2 + WX * GW - 1) / (WX * GW)) * (((a.YN + 1) / 2 + WY - 1) / WY);
 }
@@ -778,14 +799,12 @@ int launch_back_dd(const Plan& p, int back_mode, const float* w, const ViewGeom*
   if (a.nvb == 0 || PN < 1) return DDFAN_OK;
   ProfScope ps(KIND_BACK_A, st);
   const dim3 grid(dd_back_tiles(a), 1, a.nzt);
-  const bool adj = back_mode == DDFAN_BACK_ADJ;
-  if (a.sv == 8) {
-    if (adj) k_back_dd<8, true><<<grid, 256, DdBackTile<8>::DYN, st>>>(a);
-    else k_back_dd<8, false><<<grid, 256, DdBackTile<8>::DYN, st>>>(a);
-  } else {
-    if (adj) k_back_dd<4, true><<<grid, 256, DdBackTile<4>::DYN, st>>>(a);
-    else k_back_dd<4, false><<<grid, 256, DdBackTile<4>::DYN, st>>>(a);
-  }
+  dd_dispatch(a.sv, a.thin, [&](auto SV, auto THIN) {
+    constexpr int v = decltype(SV)::value;
+    constexpr bool t = decltype(THIN)::value;
+    if (back_mode == DDFAN_BACK_ADJ) k_back_dd<v, true, t><<<grid, 256, DdBackTile<v>::DYN, st>>>(a);
+    else k_back_dd<v, false, t><<<grid, 256, DdBackTile<v>::DYN, st>>>(a);
+  });
   return check_launch("k_back_dd");
 }
 
@@ -800,7 +819,7 @@ int proj_dev_shared(Plan& p, const float* d_angs, int stride, int PN, const floa
     // the kernel reads vectors of slices of a masked image: stage the caller's
     // image unless it already is one
     const float* img = d_vol;
-    if (p.has_mask || p.Z != p.Zs || (reinterpret_cast<uintptr_t>(d_vol) & 15)) {
+    if (p.has_mask || p.Z != p.Zs || (p.Zs % 4 == 0 && (reinterpret_cast<uintptr_t>(d_vol) & 15))) {
       if ((rc = launch_stage_image(d_vol, p.Z, p.has_mask ? p.d_mask : nullptr, p.d_tmp, p.Zs,
                                    (size_t)p.XN * p.YN, st)))
         return rc;

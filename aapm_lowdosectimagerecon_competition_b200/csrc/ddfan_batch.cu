@@ -4,7 +4,7 @@
 //
 // A batched iteration runs subset step k of every solve that has one: the
 // forward projectors (with the fused residual) of all those solves in one
-// launch per class (slices per thread), then the backprojections the same way
+// launch per class (slices per thread; thin or not), then the backprojections the same way
 // (the exact adjoint's, then the reference's), then FISTA of every solve in
 // one launch pair.  Each CTA reads its item {solve's argument
 // block, view row or voxel tile, channel block, z-tile} and runs the
@@ -36,7 +36,7 @@ namespace {
 enum BatchKind { BK_FWD = 0, BK_ADJ = 1, BK_REF = 2 };
 
 struct BatchLaunch {
-  int kind, sv;  // sv: slices per thread
+  int kind, sv, thin;  // the kernels' class (dd_dispatch)
   size_t items_off, nitems;
   int group;  // the solver group whose chain the launch belongs to
 };
@@ -51,12 +51,15 @@ struct BatchLaunch {
 // (at every batch creation: the attribute belongs to the context)
 int batch_prepare_device(int dev) {
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd_batch<8>, DdFwdTile<8>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd_batch<4>, DdFwdTile<4>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<8, true>, DdBackTile<8>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<8, false>, DdBackTile<8>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<4, true>, DdBackTile<4>::DYN);
-  if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<4, false>, DdBackTile<4>::DYN);
+  for (const int sv : {8, 4, 1})
+    for (const int thin : {0, 1})
+      dd_dispatch(sv, thin, [&](auto SV, auto THIN) {
+        constexpr int v = decltype(SV)::value;
+        constexpr bool t = decltype(THIN)::value;
+        if (e == cudaSuccess) e = dd_allow_dyn(k_fwd_dd_batch<v, t>, DdFwdTile<v>::DYN);
+        if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<v, true, t>, DdBackTile<v>::DYN);
+        if (e == cudaSuccess) e = dd_allow_dyn(k_back_dd_batch<v, false, t>, DdBackTile<v>::DYN);
+      });
   if (e != cudaSuccess)
     return set_err(DDFAN_ERR_CUDA, "batched kernel attributes on device %d: %s", dev, cudaGetErrorString(e));
   return DDFAN_OK;
@@ -117,18 +120,18 @@ static int batch_launch(Batch& b, const BatchLaunch& L, cudaStream_t st) {
     const unsigned n = (unsigned)L.nitems;
     if (L.kind == BK_FWD) {
       ProfScope ps(KIND_FWD, st);
-      if (L.sv == 8) k_fwd_dd_batch<8><<<n, 256, DdFwdTile<8>::DYN, st>>>(b.d_fargs, it);
-      else k_fwd_dd_batch<4><<<n, 256, DdFwdTile<4>::DYN, st>>>(b.d_fargs, it);
+      dd_dispatch(L.sv, L.thin, [&](auto SV, auto THIN) {
+        constexpr int v = decltype(SV)::value;
+        k_fwd_dd_batch<v, decltype(THIN)::value><<<n, 256, DdFwdTile<v>::DYN, st>>>(b.d_fargs, it);
+      });
     } else {
       ProfScope ps(KIND_BACK_A, st);
-      const bool adj = L.kind == BK_ADJ;
-      if (L.sv == 8) {
-        if (adj) k_back_dd_batch<8, true><<<n, 256, DdBackTile<8>::DYN, st>>>(b.d_bargs, it);
-        else k_back_dd_batch<8, false><<<n, 256, DdBackTile<8>::DYN, st>>>(b.d_bargs, it);
-      } else {
-        if (adj) k_back_dd_batch<4, true><<<n, 256, DdBackTile<4>::DYN, st>>>(b.d_bargs, it);
-        else k_back_dd_batch<4, false><<<n, 256, DdBackTile<4>::DYN, st>>>(b.d_bargs, it);
-      }
+      dd_dispatch(L.sv, L.thin, [&](auto SV, auto THIN) {
+        constexpr int v = decltype(SV)::value;
+        constexpr bool t = decltype(THIN)::value;
+        if (L.kind == BK_ADJ) k_back_dd_batch<v, true, t><<<n, 256, DdBackTile<v>::DYN, st>>>(b.d_bargs, it);
+        else k_back_dd_batch<v, false, t><<<n, 256, DdBackTile<v>::DYN, st>>>(b.d_bargs, it);
+      });
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_err(DDFAN_ERR_CUDA, "batched launch (kind %d): %s", L.kind, cudaGetErrorString(e));
@@ -217,7 +220,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
   // per group, per step: class -> items, for each kind
   for (int grp = 0; grp < G; ++grp)
   for (int k = 0; k < maxsub; ++k) {
-    std::map<int, std::vector<int4>> fwd, back_adj, back_ref;  // by slices per thread
+    std::map<std::pair<int, int>, std::vector<int4>> fwd, back_adj, back_ref;  // by class
     for (size_t si = 0; si < b.sv.size(); ++si) {
       if (group_of[si] != grp) continue;
       Solver& s = *b.sv[si];
@@ -240,7 +243,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
       // z-tiles outermost and the rest in the single-solve grid's
       // order: the CTAs in flight share one tile's slices, whose image part
       // then stays in L2
-      auto& fl = fwd[fa.sv];
+      auto& fl = fwd[{fa.sv, fa.thin}];
       for (int zt = 0; zt < fa.nzt; ++zt)
         for (int cb = 0; cb < ncb; ++cb)
           for (int row = 0; row < c; ++row) fl.push_back(make_int4(fi, row, cb, zt));
@@ -253,14 +256,14 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
       const int bi = (int)bargs.size();
       bargs.push_back(ba);
       const int tiles = dd_back_tiles(ba);
-      auto& lb = (adj ? back_adj : back_ref)[ba.sv];
+      auto& lb = (adj ? back_adj : back_ref)[{ba.sv, ba.thin}];
       for (int zt = 0; zt < ba.nzt; ++zt)
         for (int t = 0; t < tiles; ++t) lb.push_back(make_int4(bi, t, zt, 0));
     }
-    auto emit = [&](int kind, std::map<int, std::vector<int4>>& m) {
+    auto emit = [&](int kind, std::map<std::pair<int, int>, std::vector<int4>>& m) {
       for (auto& kv : m) {
         if (kv.second.empty()) continue;
-        BatchLaunch L{kind, kv.first, items.size(), kv.second.size(), grp};
+        BatchLaunch L{kind, kv.first.first, kv.first.second, items.size(), kv.second.size(), grp};
         items.insert(items.end(), kv.second.begin(), kv.second.end());
         b.launches.push_back(L);
       }

@@ -23,6 +23,8 @@
 // with a zero guard channel U, so a walk that ends on the last boundary
 // (index U, fraction 0) reads a zero.
 #pragma once
+#include <type_traits>
+
 #include "ddfan_proj_kernels.cuh"
 
 namespace ddfan {
@@ -35,17 +37,49 @@ namespace ddfan {
 #ifndef DDFAN_DD_BACK_MIN_CTAS
 #define DDFAN_DD_BACK_MIN_CTAS 2
 #endif
-// The walk from (k0, f0) to (k1, f1) as three weights: w0 on the value at
-// k0, wm on the value one step on (an interior value when n = |k1 - k0| >= 2,
-// else 0: that value is then the end value or past it), we on the value at k1
-// (0 when n = 0: it is the start value again); interior values beyond the
-// first (n > 2) take wm as well.  Scaled by s.
-__device__ __forceinline__ float3 walk3(int k0, float f0, int k1, float f1, float s) {
-  const int n = k1 > k0 ? k1 - k0 : k0 - k1;
-  if (n == 0) return make_float3((f1 - f0) * s, 0.f, 0.f);
-  const float wi = k1 > k0 ? s : -s;
-  return k1 > k0 ? make_float3((1.f - f0) * s, n >= 2 ? wi : 0.f, f1 * s)
-                 : make_float3(-f0 * s, n >= 2 ? wi : 0.f, (f1 - 1.f) * s);
+// ============================================================ decode arithmetic
+//
+// A warp decodes 32 positions at a time for its gathers, so with few slices
+// the decode is most of the work.  It keeps the FP64 formulas but none of
+// FP64's slow companions: comparisons, divisions and conversions (which share
+// a 4-lane unit) are replaced as below.
+
+// Position c, as t = c + DD_MAGIC: the cell (clamped so that 0 <= c <= N) and
+// the fraction.  The sum's low word holds 32 fraction bits, of which 24 are
+// kept (DD_MAGIC's 2^-25 rounds them), its high word the cell; a t outside
+// [2^20, 2^21) has a high word that clamps to the same end of the line as c.
+constexpr double DD_MAGIC = 1572864.0 + 2.98023223876953125e-8;
+__device__ __forceinline__ void dd_cell(double t, int N, int& k, float& f) {
+  k = max(__double2hiint(t), 0x41300000) - 0x41380000;
+  f = (float)((unsigned)__double2loint(t) >> 8) * 5.9604644775390625e-8f;
+  if ((unsigned)k >= (unsigned)N) {
+    f = k < 0 ? 0.f : 1.f;
+    k = k < 0 ? 0 : N - 1;
+  }
+}
+
+// The approximate reciprocal (relative error below 2^-22), and 1 / x within an
+// ulp: one Newton step on it
+__device__ __forceinline__ float dd_rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float dd_rcpf(float x) {
+  const float r = dd_rcp_approx(x);
+  return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
+// x as a double, exactly, for normal x, with integer instructions
+__device__ __forceinline__ double dd_widen(float x) {
+  const unsigned u = __float_as_uint(x);
+  return __hiloint2double((int)(((u & 0x7fffffffu) >> 3) + 0x38000000u | (u & 0x80000000u)), (int)(u << 29));
+}
+
+// 1 / x in FP64 from a float seed within 2^-20: one Newton step (2^-40)
+__device__ __forceinline__ double dd_newton(double x, float seed) {
+  const double y = dd_widen(seed);
+  return fma(y, fma(-x, y, 1.0), y);
 }
 
 // ============================================================ vectors of slices
@@ -123,6 +157,7 @@ struct DdFwdArgs {
   int zl;              // lanes of a channel group: vectors of a z-tile
   int vb0, nvb, nzt;   // first vector and vectors of [zlo, zhi); z-tiles of zl vectors
   int nseg;            // line segments a warp's lines are split into (1, 2, 4 or 8)
+  int thin;            // few slices: fwd_thin_body (zl = 1)
   // fused OS-SART residual (AAPM_script/OSSART_AAPM.m:86-88); y null = plain projection
   const float* y;      // measured [views][U][ystride]
   const int* yview;    // slot -> measured view
@@ -169,6 +204,67 @@ __device__ __forceinline__ void dd_line_range(double F, double C, double N, int 
   }
 }
 
+// The lines that any footprint of channels [wc0, wc0 + n) meets, and of those
+// the warp's segment.
+__device__ __forceinline__ void dd_warp_lines(const double2* fcp, int wc0, int n, int U, double N, int nl, int seg,
+                                              int nseg, int& lo, int& hi) {
+  lo = hi = 0;
+  if (wc0 >= U) return;
+  int pl = nl, ph = 0, ql = nl, qh = 0;
+  for (int b = threadIdx.x & 31; b <= n; b += 32) {
+    const double2 f = __ldg(fcp + min(wc0 + b, U));
+    int b0, b1, b2, b3;
+    dd_line_range(f.x, f.y, N, nl, b0, b1, b2, b3);
+    pl = min(pl, b0);
+    ph = max(ph, b1);
+    ql = min(ql, b2);
+    qh = max(qh, b3);
+  }
+  pl = __reduce_min_sync(0xffffffffu, pl);
+  ph = __reduce_max_sync(0xffffffffu, ph);
+  ql = __reduce_min_sync(0xffffffffu, ql);
+  qh = __reduce_max_sync(0xffffffffu, qh);
+  const int l0 = max(pl, ql), m = max(0, min(ph, qh) - l0);
+  lo = l0 + m * seg / nseg;
+  hi = l0 + m * (seg + 1) / nseg;
+}
+
+// Stores channel u of view p: the ray sums of slices [vb SV, vb SV + SV), or
+// the OS-SART residual made of them.
+template <int SV>
+__device__ __forceinline__ void dd_fwd_store(const DdFwdArgs& a, int p, int u, int vb, float (&val)[SV]) {
+  const size_t e = (size_t)p * a.U + u;
+  const float cv = __ldg(a.cvd + e) * a.dx;
+  float* oz = a.out + ((size_t)p * a.orow + u) * a.ostride + vb * SV;
+  const float* yv = nullptr;
+  float rs = 0.f, wt = 1.f;
+  if (a.y) {
+    rs = __ldg(a.rowsum + e);
+    if (a.wgt) wt = __ldg(a.wgt + e);
+    yv = a.y + ((size_t)__ldg(a.yview + p) * a.U + u) * a.ystride;
+  }
+#pragma unroll
+  for (int s = 0; s < SV; ++s) {
+    val[s] *= cv;
+    const int zs = vb * SV + s;
+    if (yv && zs >= a.zlo && zs < a.zhi) {
+      // (y - A x) / rowSum where rowSum != 0, else A x (AAPM_script/OSSART_AAPM.m:88)
+      val[s] = rs != 0.f ? __fdiv_rn(__fsub_rn(__ldg(yv + zs), val[s]), rs) : val[s];
+      val[s] *= wt;
+    }
+  }
+  if (SV >= 4 && (a.ostride & 3) == 0 && vb * SV >= a.zlo && vb * SV + SV <= a.zhi &&
+      (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) {
+#pragma unroll
+    for (int s = 0; s + 4 <= SV; s += 4)
+      *reinterpret_cast<float4*>(oz + s) = make_float4(val[s], val[s + 1], val[s + 2], val[s + 3]);
+  } else {
+#pragma unroll
+    for (int s = 0; s < SV; ++s)
+      if (vb * SV + s >= a.zlo && vb * SV + s < a.zhi) oz[s] = val[s];
+  }
+}
+
 // What bounds it (c3 subset, 96 views x 736 channels x 512^2 x 128): the loads'
 // latency, and behind it the L1 pipe -- 1.30 ms, of which 1.0 ms remain when
 // every load hits L1; 14.2 GB cross from L2 (every view reads the image once:
@@ -194,7 +290,7 @@ __device__ __forceinline__ void fwd_dd_body(const DdFwdArgs& a, int row, int cbl
   using T = DdFwdTile<SV>;
   constexpr int NW = T::NW, CG = T::CG, REC = T::REC, VB = SV * 4;
   static_assert(CG >= 1 && CG <= 3, "s_m holds a start and three interior offsets");
-  __shared__ float4 s_w[NW][REC];         // (w0, wm, we) / length, end offset (bits) of walk (line, j, group)
+  __shared__ float4 s_w[NW][REC];         // (w0, wm, we) / length, end offset (bits) of walk (line, group, j)
   __shared__ uint4 s_m[NW][REC / CG];     // (line, group): start offset, then each channel's interior one
   extern __shared__ float s_tot[];          // [CG * SV][NT]: this thread's totals at tid
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -220,57 +316,57 @@ __device__ __forceinline__ void fwd_dd_body(const DdFwdArgs& a, int row, int cbl
   Vec<SV> acc[CG];
 #pragma unroll
   for (int j = 0; j < CG; ++j) vzero(acc[j]);
-  // the lines that any of the warp's footprints meet
-  int lo = 0, hi = 0;
-  if (wc0 < a.U) {
-    int pl = nl, ph = 0, ql = nl, qh = 0;
-    for (int b = lane; b <= CWW; b += 32) {
-      const double2 f = __ldg(fcp + min(wc0 + b, a.U));
-      int b0, b1, b2, b3;
-      dd_line_range(f.x, f.y, Nd, nl, b0, b1, b2, b3);
-      pl = min(pl, b0);
-      ph = max(ph, b1);
-      ql = min(ql, b2);
-      qh = max(qh, b3);
-    }
-    pl = __reduce_min_sync(0xffffffffu, pl);
-    ph = __reduce_max_sync(0xffffffffu, ph);
-    ql = __reduce_min_sync(0xffffffffu, ql);
-    qh = __reduce_max_sync(0xffffffffu, qh);
-    lo = max(pl, ql);
-    hi = max(lo, min(ph, qh));
-  }
-  if (nseg > 1) {
-    const int n = hi - lo, l0 = lo;
-    lo = l0 + n * seg / nseg;
-    hi = l0 + n * (seg + 1) / nseg;
-  }
+  int lo, hi;
+  dd_warp_lines(fcp, wc0, CWW, a.U, Nd, nl, seg, nseg, lo, hi);
   const float dx = a.dx;
-  const float icww = 1.f / (float)CWW;
+  // decode: lane -> channel lr (of CWW, 32 at a time) on line lc of a step of LPS
+  const int LPS = CWW < 32 ? 32 / CWW : 1;
+  const int lc = CWW < 32 ? lane / CWW : 0, lr0 = CWW < 32 ? lane - lc * CWW : lane;
+  int rg = 0, rj = 0;
+  double2 fa = make_double2(0.0, 0.0), fb = fa;
+  bool uok = false;
+  const auto channel = [&](int r) {
+    rg = r / CG;
+    rj = r - rg * CG;
+    const int u = wc0 + r;
+    uok = u < a.U;
+    fa = __ldg(fcp + min(u, a.U));
+    fb = __ldg(fcp + min(u + 1, a.U));
+    fa.y += DD_MAGIC;
+    fb.y += DD_MAGIC;
+  };
+  if (wc0 < a.U) channel(lr0);
   int since = 0;
   for (int ii0 = lo; ii0 < hi; ii0 += CC) {
     const int ncol = min(CC, hi - ii0);
     bool wide = false;
+    for (int rb = 0; rb < CWW; rb += 32) {
+      if (CWW > 32) channel(rb + lane);
+      const bool ok = CWW > 32 ? rb + lane < CWW : lc < LPS;
 #pragma unroll 1
-    for (int e = lane; e < ncol * CWW; e += 32) {
-      const int col = (int)(((float)e + 0.5f) * icww), r = e - col * CWW;
-      const int gg = r / CG, j = r - gg * CG;
-      const int u = wc0 + gg * CG + j;
-      const double di = (double)(ii0 + col);
-      const double2 fa = __ldg(fcp + min(u, a.U)), fb = __ldg(fcp + min(u + 1, a.U));
-      const double c0 = fma(di, fa.x, fa.y), c1 = fma(di, fb.x, fb.y);
-      const double cc0 = fmin(fmax(c0, 0.0), Nd), cc1 = fmin(fmax(c1, 0.0), Nd);
-      const int k0 = min((int)cc0, N - 1), k1 = min((int)cc1, N - 1);
-      const float f0 = (float)(cc0 - (double)k0), f1 = (float)(cc1 - (double)k1);
-      const float inv = u < a.U ? __frcp_rn((float)(c1 - c0) * dx) : 0.f;
-      const float3 wt = walk3(k0, f0, k1, f1, inv);
-      const int n = k1 > k0 ? k1 - k0 : k0 - k1;
-      wide |= n > 2;
-      const unsigned oe = (unsigned)k1 * ks;
-      s_w[w][(col * GW + gg) * CG + j] = make_float4(wt.x, wt.y, wt.z, __uint_as_float(oe));
-      unsigned* m = reinterpret_cast<unsigned*>(&s_m[w][col * GW + gg]);
-      m[1 + j] = n >= 2 ? DD_INNER | (unsigned)(k1 > k0 ? k0 + 1 : k0 - 1) * ks : 0u;
-      if (j == 0) m[0] = (unsigned)k0 * ks;
+      for (int col = lc; col < ncol && ok; col += LPS) {
+        // cell and fraction of both boundaries on the line, footprint length
+        const double di = (double)(ii0 + col);
+        const double t0 = fma(di, fa.x, fa.y), t1 = fma(di, fb.x, fb.y);
+        int k0, k1;
+        float f0, f1;
+        dd_cell(t0, N, k0, f0);
+        dd_cell(t1, N, k1, f1);
+        const float inv = uok ? dd_rcpf((float)(t1 - t0) * dx) : 0.f;
+        // The walk from (k0, f0) to (k1, f1): w0 on the value at k0, we on the
+        // value at k1 (0 when the cells are the same: it is the start value
+        // again), wm on the interior values between, if any
+        const bool up = k1 > k0, same = k1 == k0;
+        const int n = up ? k1 - k0 : k0 - k1;
+        wide |= n > 2;
+        const float w0 = ((same ? f1 : (up ? 1.f : 0.f)) - f0) * inv;
+        const float we = same ? 0.f : (up ? f1 : f1 - 1.f) * inv;
+        const unsigned oe = (unsigned)k1 * ks;
+        s_w[w][(col * GW + rg) * CG + rj] = make_float4(w0, up ? inv : -inv, we, __uint_as_float(oe));
+        unsigned* m = reinterpret_cast<unsigned*>(&s_m[w][col * GW + rg]);
+        m[1 + rj] = n >= 2 ? DD_INNER | (unsigned)(up ? k0 + 1 : k0 - 1) * ks : 0u;
+        if (rj == 0) m[0] = (unsigned)k0 * ks;
+      }
     }
     wide = __any_sync(0xffffffffu, wide);
     __syncwarp();
@@ -351,39 +447,104 @@ __device__ __forceinline__ void fwd_dd_body(const DdFwdArgs& a, int row, int cbl
   for (int j = 0; j < CG; ++j) {
     const int u = wc0 + g * CG + j;
     if (u >= a.U) break;
-    const size_t e = (size_t)p * a.U + u;
-    const float cv = __ldg(a.cvd + e) * dx;
-    float* o = a.out + ((size_t)p * a.orow + u) * a.ostride;
-    float rs = 0.f, wt = 1.f;
-    const float* yv = nullptr;
-    if (a.y) {
-      rs = __ldg(a.rowsum + e);
-      if (a.wgt) wt = __ldg(a.wgt + e);
-      yv = a.y + ((size_t)__ldg(a.yview + p) * a.U + u) * a.ystride;
-    }
     float val[SV];
 #pragma unroll
     for (int s = 0; s < SV; ++s) {
-      float t = tot[(j * SV + s) * T::NT];
-      for (int q = 1; q < nseg; ++q) t += tot[(j * SV + s) * T::NT + 32 * q];
-      val[s] = t * cv;
-      const int zs = vb * SV + s;
-      if (yv && zs >= a.zlo && zs < a.zhi) {
-        // (y - A x) / rowSum where rowSum != 0, else A x (AAPM_script/OSSART_AAPM.m:88)
-        val[s] = rs != 0.f ? __fdiv_rn(__fsub_rn(__ldg(yv + zs), val[s]), rs) : val[s];
-        val[s] *= wt;
+      val[s] = tot[(j * SV + s) * T::NT];
+      for (int q = 1; q < nseg; ++q) val[s] += tot[(j * SV + s) * T::NT + 32 * q];
+    }
+    dd_fwd_store<SV>(a, p, u, vb, val);
+  }
+}
+
+// The same for at most 8 slices (one vector per lane and z-tile): no lanes
+// share a walk, so each decodes its own two channels' walks in registers --
+// three boundary cells and two footprint lengths a line -- instead of through
+// shared memory.  Warp = one view x 64 channels x SV slices.
+template <int SV>
+__device__ __forceinline__ void fwd_thin_body(const DdFwdArgs& a, int row, int cblk, int ztile) {
+  using T = DdFwdTile<SV>;
+  constexpr int NW = T::NW, VB = SV * 4;
+  extern __shared__ float s_tot[];  // [2 * SV][NT]: this thread's totals at tid
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int nseg = a.nseg, wch = w / nseg, seg = w - wch * nseg;
+  const int wc0 = (cblk * (NW / nseg) + wch) * 64;
+  const int p = a.order ? a.order[row] : row;
+  const int u0 = wc0 + 2 * lane, vb = a.vb0 + ztile;
+  const bool xm = a.vg[p].xmajor != 0;
+  const int nl = xm ? a.XN : a.YN, N = xm ? a.YN : a.XN;
+  const double2* fcp = a.fc + (size_t)p * (a.U + 1);
+  const size_t kstride = (size_t)(xm ? a.XN : 1) * a.ZP * VB, lstride = (size_t)(xm ? 1 : a.XN) * a.ZP * VB;
+  float* tot = s_tot + tid;
+#pragma unroll
+  for (int e = 0; e < 2 * SV; ++e) tot[e * T::NT] = 0.f;
+  Vec<SV> acc[2];
+  vzero(acc[0]);
+  vzero(acc[1]);
+  int lo, hi;
+  dd_warp_lines(fcp, wc0, 64, a.U, (double)N, nl, seg, nseg, lo, hi);
+  if (u0 < a.U) {
+    const float dx = a.dx;
+    double2 fl[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      fl[j] = __ldg(fcp + min(u0 + j, a.U));
+      fl[j].y += DD_MAGIC;
+    }
+    const bool two = u0 + 1 < a.U;
+    const char* lp = reinterpret_cast<const char*>(a.img) + (size_t)vb * VB + (size_t)lo * lstride;
+    int since = 0;
+#pragma unroll 2
+    for (int ii = lo; ii < hi; ++ii, lp += lstride) {
+      const double di = (double)ii;
+      double t[3];
+      int k[3];
+      float f[3];
+      Vec<SV> val[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        t[j] = fma(di, fl[j].x, fl[j].y);
+        dd_cell(t[j], N, k[j], f[j]);
+        vload(val[j], lp + (size_t)k[j] * kstride);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float inv = j == 0 || two ? dd_rcpf((float)(t[j + 1] - t[j]) * dx) : 0.f;
+        const bool up = k[j + 1] > k[j], same = k[j + 1] == k[j];
+        vfma(acc[j], dup2(((same ? f[j + 1] : (up ? 1.f : 0.f)) - f[j]) * inv), val[j]);
+        vfma(acc[j], dup2(same ? 0.f : (up ? f[j + 1] : f[j + 1] - 1.f) * inv), val[j + 1]);
+        const int st = up ? 1 : -1;
+        for (int q = k[j] + st; !same && q != k[j + 1]; q += st) {
+          Vec<SV> v;
+          vload(v, lp + (size_t)q * kstride);
+          vfma(acc[j], dup2(up ? inv : -inv), v);
+        }
+      }
+      if (++since == T::FLUSH || ii + 1 == hi) {
+        since = 0;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+          for (int s = 0; s < SV; ++s) tot[(j * SV + s) * T::NT] += vget(acc[j], s);
+          vzero(acc[j]);
+        }
       }
     }
-    float* oz = o + vb * SV;
-    if (SV >= 4 && (a.ostride & 3) == 0 && vb * SV >= a.zlo && vb * SV + SV <= a.zhi &&
-        (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) {
+  }
+  if (nseg > 1) {
+    __syncthreads();
+    if (seg != 0) return;
+  }
 #pragma unroll
-      for (int s = 0; s + 4 <= SV; s += 4) *reinterpret_cast<float4*>(oz + s) = make_float4(val[s], val[s + 1], val[s + 2], val[s + 3]);
-    } else {
+  for (int j = 0; j < 2; ++j) {
+    if (u0 + j >= a.U) break;
+    float val[SV];
 #pragma unroll
-      for (int s = 0; s < SV; ++s)
-        if (vb * SV + s >= a.zlo && vb * SV + s < a.zhi) oz[s] = val[s];
+    for (int s = 0; s < SV; ++s) {
+      val[s] = tot[(j * SV + s) * T::NT];
+      for (int q = 1; q < nseg; ++q) val[s] += tot[(j * SV + s) * T::NT + 32 * q];
     }
+    dd_fwd_store<SV>(a, p, u0 + j, vb, val);
   }
 }
 
@@ -400,18 +561,20 @@ inline cudaError_t dd_allow_dyn(K kernel, int bytes) {
 // a few channel blocks -- rays at one distance from the centre, which miss the
 // disk inside it -- instead of every channel block of a few views.  On a c3
 // subset this cut the DRAM reads of the image from 2.05 to 1.33 GB per launch.
-template <int SV>
+template <int SV, bool THIN>
 __global__ void __launch_bounds__(256, DDFAN_DD_FWD_MIN_CTAS) k_fwd_dd(const __grid_constant__ DdFwdArgs a) {
-  fwd_dd_body<SV>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z);
+  if constexpr (THIN) fwd_thin_body<SV>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z);
+  else fwd_dd_body<SV>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z);
 }
 
 // One launch over a work list of many calls (batched reconstructions): CTA
 // b takes item {call, view row, channel block, z-tile} = items[b].
-template <int SV>
+template <int SV, bool THIN>
 __global__ void __launch_bounds__(256, DDFAN_DD_FWD_MIN_CTAS) k_fwd_dd_batch(const DdFwdArgs* __restrict__ args,
                                                                              const int4* __restrict__ items) {
   const int4 it = items[blockIdx.x];
-  fwd_dd_body<SV>(args[it.x], it.y, it.z, it.w);
+  if constexpr (THIN) fwd_thin_body<SV>(args[it.x], it.y, it.z, it.w);
+  else fwd_dd_body<SV>(args[it.x], it.y, it.z, it.w);
 }
 
 // ============================================================ backprojectors
@@ -427,16 +590,18 @@ struct DdBackArgs {
   // exact adjoint
   const double2* tab;  // [U] fan tangents of the boundaries (dd_edge)
   const uint16_t* lut;
-  float t0, invdt, dirt;
+  float t0, invdt, dirtf;
   int M;
-  double inv_sid;
+  double dirt, inv_sid;
   // reference formula
   double inv_dbeta, cnt;  // cnt = detCntIdx + 1 - 0.5
+  float sidf;             // source distance
   BackEpi epi;
   int sv;              // slices per thread (the kernel's SV)
   int zl;              // lanes of a voxel group: vectors of a z-tile
   int vb0, nvb, nzt;   // first vector and vectors of [zlo, zhi); z-tiles of zl vectors
   int nseg;            // view segments a warp's views are split into (1, 2, 4 or 8)
+  int thin;            // few slices: back_thin_body (zl = 1)
 };
 
 template <int SV>
@@ -444,7 +609,7 @@ struct DdBackTile {
   static constexpr int NT = 256, NW = NT / 32;
   static constexpr int WBUF = 3328;  // bytes of window weights per warp
   static constexpr int FLUSH = 16;   // views per FP32 partial sum
-  static constexpr int MIN_CTAS = SV == 8 ? DDFAN_DD_BACK_MIN_CTAS : DDFAN_DD_BACK_MIN_CTAS + 1;
+  static constexpr int MIN_CTAS = SV == 4 ? DDFAN_DD_BACK_MIN_CTAS + 1 : DDFAN_DD_BACK_MIN_CTAS;
   static constexpr int STEP = 4;     // window values loaded together
   static constexpr int DYN = 4 * SV * NT * (int)sizeof(float);
 };
@@ -460,62 +625,32 @@ __host__ __device__ inline int dd_back_stride(int GW) { return GW > 16 ? 80 : 20
 // (8 / nseg) tile warps side by side in x while a warp's run of blocks is short
 __host__ __device__ inline int dd_back_wx(int GW, int nseg) { return GW >= 8 || nseg == 8 ? 1 : 2; }
 
-// 1 / x and 1 / sqrt(x) in FP64: the FP32 approximation (relative error
-// 2^-22) and one Newton step (2^-44), for factors whose product needs less:
-// the angle step below (|z| <= 1 / 128) and the footprint's half-width and
-// weight, both rounded to FP32 afterwards.
-__device__ __forceinline__ double dd_rcp(double x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
-  const double y = (double)r;
-  return fma(y, fma(-x, y, 1.0), y);
-}
-__device__ __forceinline__ double dd_rsqrt(double x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)x));
-  const double y = (double)r;
-  return y * fma(-0.5 * x * y, y, 1.5);
-}
-// 1 / x in FP32, the approximation and one Newton step (within an ulp)
-__device__ __forceinline__ float dd_rcpf(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(r, fmaf(-x, r, 1.f), r);
-}
+// A voxel's ray from the source, for the decode: the vector (FP64, FP32)
+struct DdRay {
+  double x, y;
+  float xf, yf;
+};
 
-// Cell and fraction of coordinate c clamped to [0, U]: c + 1.5 2^28, rounded
-// to the nearest 2^-24 by the addition itself, holds the cell and 24 fraction
-// bits in its mantissa -- one FP64 addition instead of two comparisons and four
-// conversions.  |c| < 2^27 (beyond, the cell is some cell of the row).
-__device__ __forceinline__ void dd_cell(double c, int U, int& k, float& f) {
-  const double t = c + 402653184.0;
-  const unsigned hi = (unsigned)__double2hiint(t), lo = (unsigned)__double2loint(t);
-  k = (int)(__funnelshift_r(lo, hi, 24) & 0xfffffffu) - 0x8000000;
-  f = (float)(lo & 0xffffffu) * 5.9604644775390625e-8f;
-  if (k < 0) {
-    k = 0;
-    f = 0.f;
-  } else if (k >= U) {
-    k = U - 1;
-    f = 1.f;
-  }
-}
-
-// asin(cr / hypot(cr, dt)), the angle of a voxel's ray from the central ray
-// (cross and dot product of the two).  In front of the source (dt > 0) it is
+// asin(cr / hypot(cr, dt)), the angle of a voxel's ray v from the central ray
+// (cross and dot product of -s and v).  In front of the source (dt > 0) it is
 // atan(cr / dt): with T = j / 64 the grid tangent nearest to cr / dt,
 // atan(cr / dt) = atan(T) + atan(z), z = (cr - T dt) / (dt + T cr), |z| <=
-// 1 / 128, whose Taylor series after z^7 is below 1e-20.  atan(T) from a table
-// of the library function's values; rays beyond 45 degrees call asin.
+// 1 / 128: z in FP64 and its Taylor series' next two terms, at most 1.6e-7, in
+// FP32.  tab: (T, atan(T) of the library function); rays beyond 45 degrees
+// call asin.
 constexpr int DD_ATAN_N = 64;
-__device__ __forceinline__ double dd_angle(double cr, double dt, const double* tab) {
-  const float tf = __fdividef((float)cr, (float)dt);
-  if (!(dt > 0.0 && fabsf(tf) <= 1.f)) return asin(cr / sqrt(cr * cr + dt * dt));
-  const float jf = rintf(tf * (float)DD_ATAN_N);
-  const double T = (double)(jf * (1.f / (float)DD_ATAN_N));
-  const double z = fma(-T, dt, cr) * dd_rcp(fma(T, cr, dt));
-  const double z2 = z * z;
-  return fma(z * z2, fma(z2, fma(z2, -1.0 / 7.0, 1.0 / 5.0), -1.0 / 3.0), z) + tab[(int)jf + DD_ATAN_N];
+__device__ __forceinline__ double dd_angle(const DdRay& v, double sx, double sy, float sxf, float syf, const double2* tab) {
+  const double cr = fma(sy, v.x, -sx * v.y), dt = -fma(sx, v.x, sy * v.y);
+  const float crf = fmaf(syf, v.xf, -sxf * v.yf), dtf = -fmaf(sxf, v.xf, syf * v.yf);
+  const float tf = crf * dd_rcp_approx(dtf);
+  if (!(dtf > 0.f && fabsf(tf) <= 1.f)) return asin(cr / sqrt(cr * cr + dt * dt));
+  const float jf = fmaf(tf, (float)DD_ATAN_N, 12582912.f);  // 1.5 2^23: rounds to an integer
+  const double2 q = tab[__float_as_int(jf) - 0x4b400000 + DD_ATAN_N];
+  const float Tf = (jf - 12582912.f) * (1.f / (float)DD_ATAN_N);
+  const float rf = dd_rcp_approx(fmaf(Tf, crf, dtf));
+  const double z = fma(-q.x, dt, cr) * dd_newton(fma(q.x, cr, dt), rf);
+  const float zf = fmaf(-Tf, dtf, crf) * rf, z2 = zf * zf;
+  return fma(-z, dd_widen(z2 * fmaf(z2, -0.2f, 1.f / 3.f)), z) + q.y;
 }
 
 // Fractional boundary index (cell k, fraction f) of the point at v from the
@@ -530,12 +665,15 @@ __device__ __forceinline__ double dd_angle(double cr, double dt, const double* t
 // from one table of all views instead of two boundary lines of this one.
 // tab[b] = (T_b, 1 / (T_{b+1} - T_b)), T increasing (times dirt); lut: a guess
 // of b, made exact by stepping.  nl: D(T) = nl.x + dirt T nl.y.
-__device__ __forceinline__ void dd_edge(const DdBackArgs& a, double nx, double ny, double vx, double vy, double vl,
-                                        double nlx, double nly, int& k, float& f) {
-  const double cr = a.dirt * (nx * vy - ny * vx), dt = nx * vx + ny * vy;
-  const double r = dd_rcp(dt * vl), t = cr * (vl * r);
-  const float m = fminf(fmaxf(((float)t - a.t0) * a.invdt, 0.f), (float)(a.M - 1));
-  int b = __ldg(a.lut + (int)m);
+__device__ __forceinline__ void dd_edge(const DdBackArgs& a, const DdRay& v, bool xm, double nx, double ny, float nxf,
+                                        float nyf, double nlx, double nly, int& k, float& f) {
+  const double cr = nx * v.y - ny * v.x, dt = fma(nx, v.x, ny * v.y), vl = xm ? v.x : v.y;
+  const float crf = nxf * v.yf - nyf * v.xf, dtf = fmaf(nxf, v.xf, nyf * v.yf), vlf = xm ? v.xf : v.yf;
+  const float rf = dd_rcp_approx(dtf * vlf);
+  const double r = dd_newton(dt * vl, rf), t = a.dirt * (cr * (vl * r));
+  const float tf = a.dirtf * crf * (vlf * rf);
+  const float m = fminf(fmaxf((tf - a.t0) * a.invdt, 0.f), (float)(a.M - 1));
+  int b = min((int)__ldg(a.lut + (__float_as_int(m + 8388608.f) & 0x7fffff)), a.U - 1);
   double2 q = __ldg(a.tab + b);
   double u = (t - q.x) * q.y;
   while (u >= 1.0 && b < a.U - 1) {
@@ -547,7 +685,7 @@ __device__ __forceinline__ void dd_edge(const DdBackArgs& a, double nx, double n
     u = (t - q.x) * q.y;
   }
   k = b;
-  f = __saturatef((float)(1.0 - (1.0 - u) * fma(q.x, nly, nlx) * (dt * (dt * r))));
+  f = __saturatef((float)fma(u - 1.0, fma(q.x, nly, nlx) * (dt * (dt * r)), 1.0));
 }
 
 // back_store for a thread's SV slices, in 16-byte pieces where the output allows.
@@ -597,6 +735,41 @@ __device__ __forceinline__ void dd_back_store(const BackEpi& e, int ix, int iy, 
   }
 }
 
+// Positions (cell, fraction) of the two ends of voxel (px, py)'s footprint in
+// view G and its weight.
+template <bool ADJ>
+__device__ __forceinline__ void dd_footprint(const DdBackArgs& a, const ViewGeom& G, double px, double py, float pxf,
+                                             float pyf, const double2* s_at, int& kL, float& fL, int& kR, float& fR,
+                                             float& wgt) {
+  const double sx = G.sx, sy = G.sy;
+  const float sxf = -a.sidf * G.shx, syf = -a.sidf * G.shy;
+  const DdRay v{px - sx, py - sy, pxf - sxf, pyf - syf};
+  if (ADJ) {
+    // the voxel's two edges along the view's lines (x columns or y rows)
+    const double nx = -sx * a.inv_sid, ny = -sy * a.inv_sid, hdx = 0.5 * a.dx;
+    const bool xm = G.xmajor != 0;
+    const double nlx = xm ? nx : ny, nly = xm ? -a.dirt * ny : a.dirt * nx;
+    const double ex = xm ? 0.0 : hdx, ey = xm ? hdx : 0.0;
+    const float exf = (float)ex, eyf = (float)ey;
+    dd_edge(a, DdRay{v.x - ex, v.y - ey, v.xf - exf, v.yf - eyf}, xm, nx, ny, G.shx, G.shy, nlx, nly, kL, fL);
+    dd_edge(a, DdRay{v.x + ex, v.y + ey, v.xf + exf, v.yf + eyf}, xm, nx, ny, G.shx, G.shy, nlx, nly, kR, fR);
+    wgt = G.sgn;
+  } else {
+    const float l2f = fmaf(v.xf, v.xf, v.yf * v.yf);
+    float rs;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(l2f));
+    const bool xdom = fabs(sx) > fabs(sy);
+    const double ca = fma(dd_angle(v, sx, sy, sxf, syf, s_at), a.inv_dbeta, a.cnt + DD_MAGIC);
+    const double l2 = fma(v.x, v.x, v.y * v.y);
+    const double da = (xdom ? v.x : v.y) * dd_newton(l2, rs * rs) * (0.5 * a.dx * a.inv_dbeta);
+    // dx l / ddv, l from the approximation and one Newton step
+    const float l = l2f * (rs * fmaf(-0.5f * l2f * rs, rs, 1.5f));
+    wgt = (float)a.dx * l * dd_rcpf(xdom ? v.xf : v.yf);
+    dd_cell(ca - da, a.U, kL, fL);
+    dd_cell(ca + da, a.U, kR, fR);
+  }
+}
+
 // Measured per c3 subset (96 views x 736 channels, 512^2 x 128): reference
 // formula 1.40 -> 1.08 ms, exact adjoint 1.77 -> 1.25 ms (0.86 ms of either
 // when the decode is left out); 1111 views of 384^2 x 45, exact adjoint 10.8 ->
@@ -632,7 +805,7 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
   constexpr int NW = T::NW, VB = SV * 4;
   __shared__ __align__(16) unsigned char s_wt[NW][T::WBUF];
   __shared__ uint2 s_h[NW][32];  // record: window start (vectors), values in this pass
-  __shared__ double s_at[ADJ ? 1 : 2 * DD_ATAN_N + 1];
+  __shared__ double2 s_at[ADJ ? 1 : 2 * DD_ATAN_N + 1];
   extern __shared__ float s_tot[];  // [4 * SV][NT]: this thread's totals at tid
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const int ZL = a.zl, GW = 32 / ZL;
@@ -650,7 +823,10 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
   const size_t vstride = (size_t)(a.U + 1) * a.ZP * VB, kstride = (size_t)a.ZP * VB;
   const char* q = reinterpret_cast<const char*>(a.q) + (size_t)(active ? vb : 0) * VB;
   if (!ADJ) {
-    for (int j = tid; j <= 2 * DD_ATAN_N; j += T::NT) s_at[j] = atan((double)(j - DD_ATAN_N) / (double)DD_ATAN_N);
+    for (int j = tid; j <= 2 * DD_ATAN_N; j += T::NT) {
+      const double tj = (double)(j - DD_ATAN_N) / (double)DD_ATAN_N;
+      s_at[j] = make_double2(tj, atan(tj));
+    }
     __syncthreads();
   }
   float* tot = s_tot + tid;
@@ -659,22 +835,23 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
   Vec<SV> acc[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) vzero(acc[j]);
-  // decode: lane -> voxel v of block lb (of 8 or GW) of view lv (of VP)
-  const int v = lane & 3, lb = GW >= 8 ? lane >> 2 : (lane >> 2) % GW, lv = GW >= 8 ? 0 : (lane >> 2) / GW;
+  // decode: lane -> voxel lvx of block lb (of 8 or GW) of view lv (of VP)
+  const int lvx = lane & 3, lb = GW >= 8 ? lane >> 2 : (lane >> 2) % GW, lv = GW >= 8 ? 0 : (lane >> 2) / GW;
   const int VP = GW >= 8 ? 1 : 8 / GW;
   int xx = 0, yy = 0;
   double px = 0.0, py = 0.0;
+  float pxf = 0.f, pyf = 0.f;
   bool von = false;
   const auto place = [&](int gg) {
-    xx = 2 * (bx0 + gg) + (v & 1);
-    yy = y0 + (v >> 1);
+    xx = 2 * (bx0 + gg) + (lvx & 1);
+    yy = y0 + (lvx >> 1);
     von = gg < GW && xx < a.XN && yy < a.YN && lv < VP && (!a.epi.mask || a.epi.mask[(size_t)yy * a.XN + xx] != 0);
     px = (xx - a.ocx) * a.dx;
     py = (yy - a.ocy) * a.dx;
+    pxf = (float)px;
+    pyf = (float)py;
   };
   place(lb);
-  const double hdx = a.dx * 0.5, hdb = hdx * a.inv_dbeta;
-  const float dxf = (float)a.dx;
   const int vbeg = (int)((long long)a.PN * seg / nseg), vend = (int)((long long)a.PN * (seg + 1) / nseg);
   int since = 0;
   for (int v0 = vbeg; v0 < vend; v0 += VC) {
@@ -691,29 +868,7 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
           float fL = 0.f, fR = 0.f, wgt = 0.f;
           const bool on = von && vv < nvc;
           if (on) {
-            const int p = v0 + vv;
-            const ViewGeom& G = a.vg[p];
-            if (ADJ) {
-              // the voxel's two edges along the view's lines (x columns or y rows)
-              const double nx = -G.sx * a.inv_sid, ny = -G.sy * a.inv_sid, vx = px - G.sx, vy = py - G.sy;
-              if (G.xmajor) {
-                dd_edge(a, nx, ny, vx, vy - hdx, vx, nx, -a.dirt * ny, kL, fL);
-                dd_edge(a, nx, ny, vx, vy + hdx, vx, nx, -a.dirt * ny, kR, fR);
-              } else {
-                dd_edge(a, nx, ny, vx - hdx, vy, vy, ny, a.dirt * nx, kL, fL);
-                dd_edge(a, nx, ny, vx + hdx, vy, vy, ny, a.dirt * nx, kR, fR);
-              }
-              wgt = G.sgn;
-            } else {
-              const double sx = G.sx, sy = G.sy, ddx = px - sx, ddy = py - sy;
-              const double l2 = fma(ddx, ddx, ddy * ddy), rl = dd_rsqrt(l2);
-              const double alpha = dd_angle(fma(sy, ddx, -sx * ddy), -fma(sx, ddx, sy * ddy), s_at);
-              const double ddv = fabs(sx) > fabs(sy) ? ddx : ddy;
-              const double da = ddv * (rl * rl) * hdb, ca = fma(alpha, a.inv_dbeta, a.cnt);
-              wgt = (float)(l2 * rl) * dxf * dd_rcpf((float)ddv);
-              dd_cell(ca - da, a.U, kL, fL);
-              dd_cell(ca + da, a.U, kR, fR);
-            }
+            dd_footprint<ADJ>(a, a.vg[v0 + vv], px, py, pxf, pyf, s_at, kL, fL, kR, fR, wgt);
           }
           // the block's window: the cells its four footprints cover (first and
           // 0xffff - last, both minima, in one word)
@@ -733,10 +888,10 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
             // the value in cell k has the weight of [cL, cR]'s part inside
             // [k, k + 1] (negative where cR < cL): sat(cR - k) - sat(cL - k),
             // the cells' difference exact
-            float* wp = reinterpret_cast<float*>(&s_wt[w][rec * RS]) + v;
+            float* wp = reinterpret_cast<float*>(&s_wt[w][rec * RS]) + lvx;
             float dL = (float)(kL - kb - i0), dR = (float)(kR - kb - i0);
             for (int i = 0; i < n; ++i, dL -= 1.f, dR -= 1.f) wp[4 * i] = (__saturatef(dR + fR) - __saturatef(dL + fL)) * wgt;
-            if (v == 0) s_h[w][rec] = make_uint2((unsigned)(vv * (a.U + 1) + kb + (n ? i0 : 0)) * (unsigned)a.ZP, (unsigned)n);
+            if (lvx == 0) s_h[w][rec] = make_uint2((unsigned)(vv * (a.U + 1) + kb + (n ? i0 : 0)) * (unsigned)a.ZP, (unsigned)n);
           }
         }
       }
@@ -799,18 +954,139 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
   }
 }
 
-// One CTA per (voxel tile, z-tile) of one call.
+// The same for at most 8 slices (one vector per lane and z-tile): no lanes
+// share a block, so each decodes its own four voxels in registers (four
+// independent chains of the decode's arithmetic) and weights the window values
+// as it loads them.
 template <int SV, bool ADJ>
+__device__ __forceinline__ void back_thin_body(const DdBackArgs& a, int tile, int ztile) {
+  using T = DdBackTile<SV>;
+  constexpr int NW = T::NW, VB = SV * 4;
+  __shared__ double2 s_at[ADJ ? 1 : 2 * DD_ATAN_N + 1];
+  extern __shared__ float s_tot[];  // [4 * SV][NT]: this thread's totals at tid
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int nseg = a.nseg, wt = w / nseg, seg = w - wt * nseg;
+  const int nbx = (a.XN + 1) / 2, nby = (a.YN + 1) / 2;
+  const int bi = (tile * (NW / nseg) + wt) * 32 + lane;  // the lane's block
+  const int by = bi / nbx, bx = bi - by * nbx;
+  const int vb = a.vb0 + ztile;
+  if (!ADJ) {
+    for (int j = tid; j <= 2 * DD_ATAN_N; j += T::NT) {
+      const double tj = (double)(j - DD_ATAN_N) / (double)DD_ATAN_N;
+      s_at[j] = make_double2(tj, atan(tj));
+    }
+    __syncthreads();
+  }
+  float* tot = s_tot + tid;
+#pragma unroll
+  for (int e = 0; e < 4 * SV; ++e) tot[e * T::NT] = 0.f;
+  Vec<SV> acc[4];
+  bool on[4], any = false;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    vzero(acc[j]);
+    const int ix = 2 * bx + (j & 1), iy = 2 * by + (j >> 1);
+    on[j] = by < nby && ix < a.XN && iy < a.YN && (!a.epi.mask || a.epi.mask[(size_t)iy * a.XN + ix] != 0);
+    any = any || on[j];
+  }
+  const double px = (2 * bx - a.ocx) * a.dx, py = (2 * by - a.ocy) * a.dx;
+  const float pxf = (float)px, pyf = (float)py, dxf = (float)a.dx;
+  const int vbeg = (int)((long long)a.PN * seg / nseg), vend = (int)((long long)a.PN * (seg + 1) / nseg);
+  const size_t kstride = (size_t)a.ZP * VB, vstride = (size_t)(a.U + 1) * kstride;
+  const char* q = reinterpret_cast<const char*>(a.q) + (size_t)vb * VB + (size_t)vbeg * vstride;
+  int since = 0;
+  for (int p = vbeg; any && p < vend; ++p, q += vstride) {
+    float fL[4], fR[4], wgt[4];
+    int kL[4], kR[4], kb = 0x7fffffff, ke = -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int ix = j & 1, iy = j >> 1;
+      dd_footprint<ADJ>(a, a.vg[p], px + ix * a.dx, py + iy * a.dx, pxf + ix * dxf, pyf + iy * dxf, s_at, kL[j], fL[j],
+                        kR[j], fR[j], wgt[j]);
+      if (on[j]) {
+        kb = min(kb, min(kL[j], kR[j]));
+        ke = max(ke, max(kL[j], kR[j]));
+      } else {
+        wgt[j] = 0.f;
+      }
+    }
+    // the value in cell k has the weight of [cL, cR]'s part inside [k, k + 1]:
+    // sat(cR - k) - sat(cL - k), the cells' difference exact
+    float dL[4], dR[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      dL[j] = (float)(kL[j] - kb);
+      dR[j] = (float)(kR[j] - kb);
+    }
+    const char* qp = q + (size_t)kb * kstride;
+#pragma unroll 2
+    for (int k = kb; k <= ke; ++k, qp += kstride) {
+      Vec<SV> v;
+      vload(v, qp);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        vfma(acc[j], dup2((__saturatef(dR[j] + fR[j]) - __saturatef(dL[j] + fL[j])) * wgt[j]), v);
+        dL[j] -= 1.f;
+        dR[j] -= 1.f;
+      }
+    }
+    if (++since == T::FLUSH || p + 1 == vend) {
+      since = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int s = 0; s < SV; ++s) tot[(j * SV + s) * T::NT] += vget(acc[j], s);
+        vzero(acc[j]);
+      }
+    }
+  }
+  if (nseg > 1) {
+    __syncthreads();
+    if (seg != 0) return;
+  }
+  if (by >= nby) return;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int ix = 2 * bx + (j & 1), iy = 2 * by + (j >> 1);
+    if (ix >= a.XN || iy >= a.YN) continue;
+    float val[SV];
+#pragma unroll
+    for (int s = 0; s < SV; ++s) {
+      val[s] = tot[(j * SV + s) * T::NT];
+      for (int r = 1; r < nseg; ++r) val[s] += tot[(j * SV + s) * T::NT + 32 * r];
+    }
+    dd_back_store<SV>(a.epi, ix, iy, vb, a.XN, a.Z, ADJ, val);
+  }
+}
+
+// One CTA per (voxel tile, z-tile) of one call.
+template <int SV, bool ADJ, bool THIN>
 __global__ void __launch_bounds__(256, DdBackTile<SV>::MIN_CTAS) k_back_dd(const __grid_constant__ DdBackArgs a) {
-  back_dd_body<SV, ADJ>(a, (int)blockIdx.x, (int)blockIdx.z);
+  if constexpr (THIN) back_thin_body<SV, ADJ>(a, (int)blockIdx.x, (int)blockIdx.z);
+  else back_dd_body<SV, ADJ>(a, (int)blockIdx.x, (int)blockIdx.z);
 }
 
 // The work-list launch: CTA b takes item {call, voxel tile, z-tile} = items[b].
-template <int SV, bool ADJ>
+template <int SV, bool ADJ, bool THIN>
 __global__ void __launch_bounds__(256, DdBackTile<SV>::MIN_CTAS) k_back_dd_batch(const DdBackArgs* __restrict__ args,
-                                                                               const int4* __restrict__ items) {
+                                                                                 const int4* __restrict__ items) {
   const int4 it = items[blockIdx.x];
-  back_dd_body<SV, ADJ>(args[it.x], it.y, it.z);
+  if constexpr (THIN) back_thin_body<SV, ADJ>(args[it.x], it.y, it.z);
+  else back_dd_body<SV, ADJ>(args[it.x], it.y, it.z);
+}
+
+// ============================================================ dispatch
+
+// go(SV, THIN) with the constants of a call: 8 or 4 slices per thread, and for
+// few slices the thin kernels (1 slice: thin only)
+template <class F>
+inline void dd_dispatch(int sv, int thin, F&& go) {
+  using I8 = std::integral_constant<int, 8>;
+  using I4 = std::integral_constant<int, 4>;
+  using I1 = std::integral_constant<int, 1>;
+  if (sv == 1) go(I1(), std::true_type());
+  else if (sv == 4) thin ? go(I4(), std::true_type()) : go(I4(), std::false_type());
+  else thin ? go(I8(), std::true_type()) : go(I8(), std::false_type());
 }
 
 // ============================================================ staging

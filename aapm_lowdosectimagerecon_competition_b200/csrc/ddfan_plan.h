@@ -89,8 +89,8 @@ int pow2_zl(int ZB);
 // the z-tile width a plan uses: pow2_zl, narrowed by the DDFAN_ZL environment
 // variable (1, 2, 4 or 8), or exactly zl_force when that is one of those
 int plan_zl(int ZB, int zl_force);
-// Slices the direct kernels' operands hold for Z: a multiple of 8 (256-bit
-// loads), or of 4 where that would pad a short stack by half
+// Slices the direct kernels' operands hold for Z: 1, 4, or a multiple of 8
+// (256-bit loads)
 int dd_pad(int Z);
 // allows the direct kernels their dynamic shared memory on the
 // current device (dev names it in an error); before any launch there
