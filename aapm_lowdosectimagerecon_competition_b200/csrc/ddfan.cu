@@ -111,6 +111,13 @@ static int recorded_nz(int ZB) {
 
 int dd_pad(int Z) { return Z == 1 ? 1 : (Z <= 4 ? 4 : (Z + 7) / 8 * 8); }
 
+bool dd_mode(int sat_mode, const uint8_t* mask, size_t npix) {
+  if (sat_mode != SAT_HILO) return sat_mode == SAT_DIRECT;
+  for (size_t i = 0; mask && i < npix; ++i)
+    if (mask[i] > 1) return false;
+  return true;
+}
+
 // Slices per thread for operands of Zs slices at p
 static int dd_vector(int Zs, const void* p) {
   if (Zs % 4) return 1;
@@ -288,7 +295,7 @@ int plan_create(Plan** out, const PlanDesc& d) {
   p.device = d.device;
   p.XN = d.XN; p.YN = d.YN; p.U = d.DNU; p.Z = d.SLN; p.ZB = (d.SLN + 3) / 4;
   p.PNmax = d.PNmax; p.mode = d.sat_mode; p.ZL = plan_zl(p.ZB, d.zl_force);
-  p.dd = p.mode == SAT_DIRECT || (p.mode == SAT_HILO && !d.tables);
+  p.dd = !d.tables && dd_mode(p.mode, d.mask, (size_t)d.XN * d.YN);
   p.Zs = dd_pad(p.Z);
   // whole z-tiles: the padding blocks of the last tile are never written; the
   // projectors read them only for the slices past Z, whose results they drop

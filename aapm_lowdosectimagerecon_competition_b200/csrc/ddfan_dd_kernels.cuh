@@ -181,29 +181,6 @@ struct DdFwdTile {
   static constexpr int DYN = CG * SV * NT * (int)sizeof(float);
 };
 
-// Lines on which a boundary ray c(ii) = ii F + C can lie above 0 and below N,
-// as [pl, ph) and [ql, qh) within [0, nl], rounded outwards.
-__device__ __forceinline__ void dd_line_range(double F, double C, double N, int nl, int& pl, int& ph, int& ql, int& qh) {
-  pl = ql = 0;
-  ph = qh = nl;
-  if (!isfinite(F) || !isfinite(C)) return;
-  if (F == 0.0) {
-    if (!(C > 0.0)) pl = nl, ph = 0;
-    if (!(C < N)) ql = nl, qh = 0;
-    return;
-  }
-  const double r = 1.0 / F, top = (double)nl;
-  const double z0 = fmin(fmax(-C * r, -2.0), top + 2.0), zN = fmin(fmax((N - C) * r, -2.0), top + 2.0);
-  const int a0 = (int)floor(z0), aN = (int)floor(zN);
-  if (F > 0.0) {
-    pl = min(max(a0 - 1, 0), nl);
-    qh = min(max(aN + 2, 0), nl);
-  } else {
-    ph = min(max(a0 + 2, 0), nl);
-    ql = min(max(aN - 1, 0), nl);
-  }
-}
-
 // The lines that any footprint of channels [wc0, wc0 + n) meets, and of those
 // the warp's segment.
 __device__ __forceinline__ void dd_warp_lines(const double2* fcp, int wc0, int n, int U, double N, int nl, int seg,
@@ -214,7 +191,7 @@ __device__ __forceinline__ void dd_warp_lines(const double2* fcp, int wc0, int n
   for (int b = threadIdx.x & 31; b <= n; b += 32) {
     const double2 f = __ldg(fcp + min(wc0 + b, U));
     int b0, b1, b2, b3;
-    dd_line_range(f.x, f.y, N, nl, b0, b1, b2, b3);
+    line_range(f.x, f.y, N, nl, b0, b1, b2, b3);
     pl = min(pl, b0);
     ph = max(ph, b1);
     ql = min(ql, b2);
@@ -1091,7 +1068,7 @@ inline void dd_dispatch(int sv, int thin, F&& go) {
 
 // ============================================================ staging
 
-// dst[pix][z] = z < Z ? src[pix][z] * mask[pix] : 0 for z < Zp (mask null = 1):
+// dst[pix][z] = z < Z ? src[pix][z] * mask[pix] : 0 for z < Zp (mask, src null = 1):
 // the masked image with its slices padded to a multiple of 4.
 static __global__ void k_stage_image(const float* __restrict__ src, int Z, const uint8_t* __restrict__ mask,
                                      float* __restrict__ dst, int Zp, size_t npix) {
@@ -1101,7 +1078,7 @@ static __global__ void k_stage_image(const float* __restrict__ src, int Z, const
     const int z = (int)(i - pix * Zp);
     float v = 0.f;
     if (z < Z) {
-      v = src[pix * Z + z];
+      v = src ? src[pix * Z + z] : 1.f;
       if (mask && mask[pix] == 0) v = 0.f;
     }
     dst[i] = v;
@@ -1110,7 +1087,7 @@ static __global__ void k_stage_image(const float* __restrict__ src, int Z, const
 
 // dst[p][u][z] = src[p][u][z] * wgt[p][u] for u < U, z < Z; zero on the
 // guard channel u = U, on padding slices and on DD_PAST entries past the last
-// view (wgt null = 1).
+// view (wgt, src null = 1).
 static __global__ void k_stage_sino(const float* __restrict__ src, int Z, const float* __restrict__ wgt, int U,
                                     float* __restrict__ dst, int Zp, size_t PN) {
   const size_t n = (PN * (U + 1) + DD_PAST) * Zp;
@@ -1122,7 +1099,7 @@ static __global__ void k_stage_sino(const float* __restrict__ src, int Z, const 
     float v = 0.f;
     if (u < U && z < Z && p < PN) {
       const size_t e = p * U + u;
-      v = src[e * Z + z];
+      v = src ? src[e * Z + z] : 1.f;
       if (wgt) v *= wgt[e];
     }
     dst[i] = v;

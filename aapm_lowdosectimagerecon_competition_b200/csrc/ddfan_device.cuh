@@ -207,6 +207,31 @@ template <> struct Phi4<SAT_FP64> {
   }
 };
 
+// ---------------------------------------------------------------- lines of a ray
+
+// Lines on which a boundary ray c(ii) = ii F + C can lie above 0 and below N,
+// as [pl, ph) and [ql, qh) within [0, nl], rounded outwards.
+__device__ __forceinline__ void line_range(double F, double C, double N, int nl, int& pl, int& ph, int& ql, int& qh) {
+  pl = ql = 0;
+  ph = qh = nl;
+  if (!isfinite(F) || !isfinite(C)) return;
+  if (F == 0.0) {
+    if (!(C > 0.0)) pl = nl, ph = 0;
+    if (!(C < N)) ql = nl, qh = 0;
+    return;
+  }
+  const double r = 1.0 / F, top = (double)nl;
+  const double z0 = fmin(fmax(-C * r, -2.0), top + 2.0), zN = fmin(fmax((N - C) * r, -2.0), top + 2.0);
+  const int a0 = (int)floor(z0), aN = (int)floor(zN);
+  if (F > 0.0) {
+    pl = min(max(a0 - 1, 0), nl);
+    qh = min(max(aN + 2, 0), nl);
+  } else {
+    ph = min(max(a0 + 2, 0), nl);
+    ql = min(max(aN - 1, 0), nl);
+  }
+}
+
 // ---------------------------------------------------------------- per-view geometry
 
 // Per-view constants written by k_view_geom (one entry per view of a call).

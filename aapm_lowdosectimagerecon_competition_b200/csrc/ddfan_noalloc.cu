@@ -136,7 +136,7 @@ extern "C" DDFAN_API int ddfan_proj_noalloc(float x0, float y0, int DNU, const f
   p.device = dev;
   p.XN = XN; p.YN = YN; p.U = DNU; p.Z = SLN; p.ZB = (SLN + 3) / 4;
   p.PNmax = PN; p.mode = sat_mode; p.ZL = plan_zl(p.ZB, 0);  // the z-tile width a plan would take
-  p.dd = sat_mode == SAT_DIRECT || sat_mode == SAT_HILO;  // as a plan of that mode
+  p.dd = dd_mode(sat_mode, mask, (size_t)XN * YN);  // as a plan of that mode
   p.Zs = (SLN + 3) / 4 * 4;  // the least padding: problems that fitted the scratch array still do
   p.ZB = (p.ZB + p.ZL - 1) / p.ZL * p.ZL;
   p.x0 = x0; p.y0 = y0; p.dx = dx;

@@ -92,6 +92,10 @@ int plan_zl(int ZB, int zl_force);
 // Slices the direct kernels' operands hold for Z: 1, 4, or a multiple of 8
 // (256-bit loads)
 int dd_pad(int Z);
+// Whether a plan of this mode and mask runs the direct kernels on shared angle
+// lists: the direct mode, and the hi/lo mode where every mask byte is 0 or 1
+// (its table kernels multiply by the byte, the direct ones only drop zeros).
+bool dd_mode(int sat_mode, const uint8_t* mask, size_t npix);
 // allows the direct kernels their dynamic shared memory on the
 // current device (dev names it in an error); before any launch there
 int dd_prepare_device(int dev);
@@ -170,10 +174,10 @@ int check_back_dd(const Plan& p, int back_mode);
 // orientations in one launch.
 int launch_back_dd(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN, const BackEpi& epi,
                    cudaStream_t st);
-// dst[pix][z < Zp] = z < Z ? src[pix][z] * mask : 0
+// dst[pix][z < Zp] = z < Z ? src[pix][z] * mask : 0 (src null = 1)
 int launch_stage_image(const float* src, int Z, const uint8_t* mask, float* dst, int Zp, size_t npix,
                        cudaStream_t st);
-// dst[p][u <= U][z < Zp] = u < U && z < Z ? src[p][u][z] * wgt[p][u] : 0
+// dst[p][u <= U][z < Zp] = u < U && z < Z ? src[p][u][z] * wgt[p][u] : 0 (src, wgt null = 1)
 int launch_stage_sino(const float* src, int Z, const float* wgt, int U, float* dst, int Zp, size_t PN,
                       cudaStream_t st);
 // out[pix][z] = mask ? x[pix][z] : (clamp0 ? max(x0, 0) : x0)

@@ -335,7 +335,8 @@ __global__ void __launch_bounds__(128) k_ps_scan(PsScanArgs a) {
 // line (error below 1e-7 cells over 1024 lines); the footprint length
 // (c_{b+1} - c_b) dx is linear in ii and runs in FP32.  Positions outside the
 // line clamp to its guard cells (prefix sum 0 before, the total after, value
-// 0), which reproduces k_fwd's clamp of c to [0, N].
+// 0), which reproduces k_fwd's clamp of c to [0, N].  Skipping the lines that
+// miss the image (a third of them at the c2 geometry) gives the same sums.
 template <int M>
 __global__ void __launch_bounds__(256) k_ps_fwd(PsFwdArgs a) {
   constexpr int CC = 16, CPW = 31;
@@ -357,9 +358,21 @@ __global__ void __launch_bounds__(256) k_ps_fwd(PsFwdArgs a) {
   long long cf = __double2ll_rn(f0.y * two32);
   const float dx = a.dx;
   const float lF = (float)((f1.x - f0.x) * (double)dx), lC = (float)((f1.y - f0.y) * (double)dx);
-  float fi = 0.f;
   float acc = 0.f;
-  for (int ii0 = 0; ii0 < nl; ii0 += CC) {
+  // lines on which none of the warp's boundaries lies inside [0, N] add exactly
+  // 0 (both samples in the same guard cell): only [lo, hi) is walked, from a
+  // multiple of CC so that the partial sums stay the same ones
+  int lo, hi;
+  {
+    int b0, b1, b2, b3;
+    line_range(f0.x, f0.y, (double)N, nl, b0, b1, b2, b3);
+    lo = max(__reduce_min_sync(0xffffffffu, b0), __reduce_min_sync(0xffffffffu, b2)) / CC * CC;
+    hi = min(__reduce_max_sync(0xffffffffu, b1), __reduce_max_sync(0xffffffffu, b3));
+  }
+  cf += dcf * lo;
+  float fi = (float)lo;
+  line += (size_t)lo * Nw;
+  for (int ii0 = lo; ii0 < hi; ii0 += CC) {
     const int ncol = min(CC, nl - ii0);
     float part = 0.f;
 #pragma unroll 4

@@ -561,12 +561,57 @@ static int solver_weights_cells(Solver& s, const PlanDesc& d, const std::vector<
 }
 
 // Row sums and column sums of every subset from slice 0's angles
+// (AAPM_script/OSSART_AAPM.m:57-66) on the direct kernels' one-slice form: the
+// row sums of all views in one forward launch of the masked image of ones, the
+// column sums one backprojection launch per subset over its rows of ones.  Both
+// backprojectors' geometry is FP64 there, so the REF weights need no other
+// kernels.  A whole c1 call (set-up, 40 subset steps, transfers) went from 18.1
+// to 9.2 ms with the set-up off the 4-slice cells.  Per-slice solvers keep
+// theirs (their residuals on rotated slices amplify any change of the sums).
+static int solver_weights_dd(Solver& s, const PlanDesc& d, const std::vector<float>& angs0, cudaStream_t st) {
+  const int XN = s.XN, YN = s.YN, U = s.U, P = s.PNall;
+  const bool adj = s.back_mode == DDFAN_BACK_ADJ;
+  PlanDesc d1 = d;
+  d1.SLN = 1;
+  d1.PNmax = 1;
+  d1.zl_force = 0;
+  d1.tables = false;
+  PlanPtr P1;
+  int rc = plan_create(&P1.p, d1);
+  if (rc) return rc;
+  const Plan& p = *P1.p;
+  DevBuf<float> ang(st), img(st), q(st), cvd(st);
+  DevBuf<ViewGeom> vg(st);
+  DevBuf<double2> fc(st);
+  if ((rc = ang.alloc(P)) || (rc = vg.alloc(P)) || (rc = fc.alloc((size_t)P * (U + 1))) ||
+      (rc = cvd.alloc((size_t)P * U)) || (rc = img.alloc((size_t)XN * YN)) ||
+      (rc = q.alloc((size_t)P * (U + 1) + DD_PAST)))
+    return rc;
+  DDFAN_CK(cudaMemcpyAsync(ang.p, angs0.data(), sizeof(float) * P, cudaMemcpyHostToDevice, st));
+  if ((rc = launch_view_geom(p, ang.p, 1, P, vg.p, fc.p, cvd.p, st))) return rc;
+  if ((rc = launch_stage_image(nullptr, 1, p.has_mask ? p.d_mask : nullptr, img.p, 1, (size_t)XN * YN, st))) return rc;
+  if ((rc = launch_fwd_dd(p, img.p, vg.p, fc.p, cvd.p, nullptr, P, s.d_rows, U, 1, 0, 1, nullptr, st))) return rc;
+  if ((rc = launch_stage_sino(nullptr, 1, adj ? cvd.p : nullptr, U, q.p, 1, (size_t)P, st))) return rc;
+  for (int k = 0; k < s.nsub; ++k) {
+    BackEpi e{};
+    e.out = s.d_cols + (size_t)k * XN * YN;
+    e.mask = p.has_mask ? p.d_mask : nullptr;
+    e.zlo = 0; e.zhi = 1;
+    if ((rc = launch_back_dd(p, s.back_mode, q.p + (size_t)s.off[k] * (U + 1), vg.p + s.off[k], s.cnt[k], e, st)))
+      return rc;
+  }
+  DDFAN_CK(cudaStreamSynchronize(st));
+  return DDFAN_OK;
+}
+
+// Row sums and column sums of every subset from slice 0's angles
 // (AAPM_script/OSSART_AAPM.m:57-66) on the slice-major kernels, which carry
 // one slice without the 4-slice cells' padding: the row sums of all views in
 // one forward launch, and the column sums of all subsets in one
 // backprojection launch, subset k standing in the place of slice k (its views
 // are rows k * cs + m; the pad rows of a short subset backproject zeros).
-// The exact adjoint only: the slice-major REF backprojector takes its
+// For the solvers that do not run the direct kernels, and the exact adjoint
+// only: the slice-major REF backprojector takes its
 // half-width and weight in FP32, and column sums divide every update, so the
 // REF weights stay on the cell kernels' FP64 formula.
 static int solver_weights(Solver& s, const PlanDesc& d, const std::vector<float>& angs0, int PNmax,
@@ -715,7 +760,7 @@ static int solver_create(Solver** out, float x0, float y0, int DNU, const float*
   }
   // the direct kernels serve one angle list for all slices (direct and hi/lo
   // modes); the per-slice paths keep hi/lo tables
-  s.direct = (sat_mode == SAT_DIRECT || sat_mode == SAT_HILO) && !s.win && !s.ps;
+  s.direct = dd_mode(sat_mode, mask, (size_t)XN * YN) && !s.win && !s.ps;
   s.batchable = s.direct && sat_mode == SAT_DIRECT;
   if (sat_mode == SAT_DIRECT && !s.direct) sat_mode = cell_mode(sat_mode);
   if (s.win) {
@@ -826,7 +871,10 @@ static int solver_create(Solver** out, float x0, float y0, int DNU, const float*
     DDFAN_CK(cudaMemsetAsync(s.d_xu, 0, sizeof(float) * XN * YN * SLN, st));
     DDFAN_CK(cudaStreamSynchronize(st));
   }
-  if ((rc = solver_weights(s, d, angs0, PNsub, st))) return rc;
+  rc = s.direct && dd_mode(SAT_HILO, mask, (size_t)XN * YN)
+           ? solver_weights_dd(s, d, angs0, st)
+           : solver_weights(s, d, angs0, PNsub, st);
+  if (rc) return rc;
   const double one = 1.0;
   DDFAN_CK(cudaMemcpyAsync(s.d_t, &one, sizeof(double), cudaMemcpyHostToDevice, st));
   DDFAN_CK(cudaMemsetAsync(s.d_x, 0, sizeof(float) * V, st));
@@ -899,9 +947,14 @@ DDFAN_API size_t ddfan_ossart_estimate_bytes(int XN, int YN, int DNU, int SLN, i
     own += 2 * (size_t)XN * YN * SLN * sizeof(float);
     if (Zi != (size_t)SLN) own += P * U * SLN * sizeof(float) + (Zi + SLN) * sizeof(int);
   }
-  sat_mode = cell_mode(sat_mode);  // the set-up's weight kernels keep tables
-  // transient at creation: the one-slice weight plan and the slice-major
-  // weight buffers (geometry, row sums, ones, tables) over nsub x PNmax rows
+  // transient at creation, direct kernels: the one-slice weight plan, the
+  // geometry of every view, the image and the rows of ones
+  if (direct)
+    return plan + own + ddfan_plan_estimate_bytes(XN, YN, DNU, 1, 1, sat_mode) +
+           P * (sizeof(ViewGeom) + (U + 1) * sizeof(double2) + (2 * U + 2) * sizeof(float)) +
+           ((size_t)XN * YN + DD_PAST) * sizeof(float);
+  // otherwise: the one-slice weight plan and the slice-major weight buffers
+  // (geometry, row sums, ones, tables) over nsub x PNmax rows
   const size_t R = (size_t)numOfOS * PNmax, CB = sat_mode == SAT_FP32 ? 8 : 16;
   const size_t weights = ddfan_plan_estimate_bytes(XN, YN, DNU, 1, 1, sat_mode) +
                          R * (sizeof(ViewGeom) + (U + 1) * sizeof(double2) + sizeof(float) + 3 * U * sizeof(float) +

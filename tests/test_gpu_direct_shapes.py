@@ -53,3 +53,29 @@ def test_direct_shapes_match_oracle(XN, YN, Z, PN, U, off, masked, sat):
         eb = O.back(x0, y0, U, xds, yds, s.detCntIdx, cx, cy, h, PN, XN, YN, Z, prj, s.dx, mask, mode=mode)
         assert rel(gb, eb) < 2e-6, back
     plan.close()
+
+
+@pytest.mark.parametrize("sat", ["hilo", "fp64"])
+def test_mask_bytes_above_one_scale_the_image(sat):
+    """A mask byte multiplies its voxel (MultiSlicesProjGPU.cu:202-209), also
+    in the hi/lo mode, whose direct kernels take 0/1 masks only: a plan with
+    other bytes keeps its tables, a solver its weights from them."""
+    import torch
+    from aapm_lowdosectimagerecon_competition_b200 import configs, dd2, device
+    from oracle import oracle as O
+    s = configs.scaled(configs.c2(SLN=9), XN=32, DNU=48, PN=24)
+    s.numOfOS = 4
+    x0, y0, xds, yds = dd2.fan_geometry(s.sid, s.sdd, s.DNU, s.detCellWidth, s.detCntIdx)
+    rng = np.random.default_rng(3)
+    vol = (rng.random((32, 32, 9)) * 0.04).astype(np.float32)
+    mask = rng.integers(0, 3, (32, 32)).astype(np.uint8)
+    rel = lambda g, e: float(np.linalg.norm((g - e).ravel()) / np.linalg.norm(e.ravel()))
+    plan = device.Plan(x0, y0, s.DNU, xds, yds, s.detCntIdx, 32, 32, 9, s.PN, s.dx, mask=mask, sat=sat)
+    y = plan.proj(torch.from_numpy(s.angles()).cuda(), torch.from_numpy(vol).cuda()).cpu().numpy()
+    assert rel(y, O.proj(x0, y0, s.DNU, xds, yds, 0, 0, s.hangs(), s.PN, 32, 32, 9, vol, s.dx, mask)) < 2e-6
+    plan.close()
+    init = np.zeros_like(vol)
+    xg = dd2.OSSART_AAPM(y, s.hangs(), init, s.conf(), 2, s.numOfOS, mask, 1, 1, sat=sat, back="ref")
+    xo = O.ossart(x0, y0, s.DNU, xds, yds, s.detCntIdx, 0, 0, s.hangs(), s.PN, 32, 32, 9, y, init, s.dx, mask, 2,
+                  s.numOfOS, 1, 1, O.REF)
+    assert rel(xg, xo) < 1e-5
