@@ -758,6 +758,13 @@ DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const
   a.q = w; a.ZP = p.Zs / a.sv; a.vg = vg;
   a.PN = PN; a.U = p.U; a.XN = p.XN; a.YN = p.YN; a.Z = p.Z;
   a.ocx = p.ocx; a.ocy = p.ocy; a.dx = p.dx; a.sidf = (float)(1.0 / p.inv_sid);
+  {
+    // a voxel's offset from its block's centre over the least distance from the source
+    const double rx = (0.5 * (p.XN - 1) + std::fabs(p.ocx - 0.5 * (p.XN - 1)) + 1.0) * p.dx;
+    const double ry = (0.5 * (p.YN - 1) + std::fabs(p.ocy - 0.5 * (p.YN - 1)) + 1.0) * p.dx;
+    const double near = 1.0 / p.inv_sid - std::hypot(rx, ry);
+    a.near = near > 0.0 && 1.5 * p.dx < 0.01 * near;
+  }
   if (back_mode == DDFAN_BACK_ADJ) {
     a.tab = p.d_tab; a.lut = p.d_lut;
     a.t0 = p.t0; a.invdt = p.invdt; a.dirtf = p.dirt; a.dirt = p.dirt; a.M = p.M; a.inv_sid = p.inv_sid;

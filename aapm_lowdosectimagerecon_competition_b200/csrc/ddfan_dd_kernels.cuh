@@ -573,6 +573,7 @@ struct DdBackArgs {
   // reference formula
   double inv_dbeta, cnt;  // cnt = detCntIdx + 1 - 0.5
   float sidf;             // source distance
+  int near;               // blocks seen under a small angle: dd_block's FP32 offsets (else FP64 per voxel)
   BackEpi epi;
   int sv;              // slices per thread (the kernel's SV)
   int zl;              // lanes of a voxel group: vectors of a z-tile
@@ -581,22 +582,20 @@ struct DdBackArgs {
   int thin;            // few slices: back_thin_body (zl = 1)
 };
 
+// (view, voxel block) records a warp decodes at a time (one per lane), the
+// window values a record holds per pass, and a record's stride in bytes (an odd
+// multiple of 16: the lanes' stores fall into different banks)
+constexpr int DD_BACK_MW = 8, DD_BACK_RS = 16 * (DD_BACK_MW + 1);
+
 template <int SV>
 struct DdBackTile {
   static constexpr int NT = 256, NW = NT / 32;
-  static constexpr int WBUF = 3328;  // bytes of window weights per warp
+  static constexpr int WBUF = 32 * DD_BACK_RS;  // bytes of window weights per warp
   static constexpr int FLUSH = 16;   // views per FP32 partial sum
   static constexpr int MIN_CTAS = SV == 4 ? DDFAN_DD_BACK_MIN_CTAS + 1 : DDFAN_DD_BACK_MIN_CTAS;
   static constexpr int STEP = 4;     // window values loaded together
   static constexpr int DYN = 4 * SV * NT * (int)sizeof(float);
 };
-
-// (view, voxel block) records a warp decodes at a time, the window values a
-// record holds per pass, and a record's stride in bytes (an odd multiple of
-// 16: the stores of the 8 records of a step fall into different banks)
-__host__ __device__ inline int dd_back_records(int GW) { return GW > 16 ? 32 : 16; }
-__host__ __device__ inline int dd_back_window(int GW) { return GW > 16 ? 4 : 12; }
-__host__ __device__ inline int dd_back_stride(int GW) { return GW > 16 ? 80 : 208; }
 
 // 2 x 2-voxel blocks: the CTA's tile is WX * GW blocks wide and WY high, its
 // (8 / nseg) tile warps side by side in x while a warp's run of blocks is short
@@ -747,6 +746,118 @@ __device__ __forceinline__ void dd_footprint(const DdBackArgs& a, const ViewGeom
   }
 }
 
+// The four footprints of a 2 x 2 block with centre (px, py).  The centre's
+// position is taken in FP64; the voxels' offsets from it, a channel or two, in
+// FP32 (angle between two rays from its tangent z, |z| <= 0.01: z - z^3 / 3;
+// error about 1e-7 channel, against the 3e-8 the positions' fractions round
+// by), which is a third of the work of four FP64 positions.  Blocks that the
+// source sees under a larger angle are decoded voxel by voxel.
+template <bool ADJ>
+__device__ __forceinline__ void dd_block(const DdBackArgs& a, const ViewGeom& G, double px, double py, float pxf, float pyf,
+                                         const double2* s_at, int (&kL)[4], float (&fL)[4], int (&kR)[4],
+                                         float (&fR)[4], float (&wgt)[4]) {
+  const float dxf = (float)a.dx, h = 0.5f * dxf;
+  if (!a.near) {
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      int k0, k1;
+      float f0, f1, w;
+      const double ex = ((j & 1) - 0.5) * a.dx, ey = ((j >> 1) - 0.5) * a.dx;
+      dd_footprint<ADJ>(a, G, px + ex, py + ey, pxf + (float)ex, pyf + (float)ey, s_at, k0, f0, k1, f1, w);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i == j) kL[i] = k0, fL[i] = f0, kR[i] = k1, fR[i] = f1, wgt[i] = w;
+    }
+    return;
+  }
+  const double sx = G.sx, sy = G.sy;
+  const float sxf = -a.sidf * G.shx, syf = -a.sidf * G.shy;
+  const DdRay v{px - sx, py - sy, pxf - sxf, pyf - syf};
+  if (ADJ) {
+    // six edge points: lines (columns or rows) -1/2, 1/2 and edges -1, 0, 1
+    // pixels from the centre.  A point's fan tangent is the centre's plus
+    // cross(v, e) / ((n . v) (n . w)), w = v + e
+    const bool xm = G.xmajor != 0;
+    const double nx = -sx * a.inv_sid, ny = -sy * a.inv_sid;
+    const double dt = fma(nx, v.x, ny * v.y);
+    const float dtf = fmaf(G.shx, v.xf, G.shy * v.yf);
+    const double tc = a.dirt * (nx * v.y - ny * v.x) * dd_newton(dt, dd_rcp_approx(dtf));
+    const float rdt = a.dirtf * dd_rcpf(dtf);
+    const float nly = xm ? -a.dirtf * G.shy : a.dirtf * G.shx;
+    int k[2][3];
+    float f[2][3];
+#pragma unroll
+    for (int l = 0; l < 2; ++l)
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        const float el = (l - 0.5f) * dxf, em = (m - 1) * dxf;
+        const float ex = xm ? el : em, ey = xm ? em : el;
+        const float wx = v.xf + ex, wy = v.yf + ey, dw = fmaf(G.shx, wx, G.shy * wy);
+        const float dlt = (v.xf * ey - v.yf * ex) * rdt * dd_rcpf(dw);
+        const double t = tc + (double)dlt;
+        const float i = fminf(fmaxf(((float)t - a.t0) * a.invdt, 0.f), (float)(a.M - 1));
+        int b = min((int)__ldg(a.lut + (__float_as_int(i + 8388608.f) & 0x7fffff)), a.U - 1);
+        double2 q = __ldg(a.tab + b);
+        float u = (float)((t - q.x) * q.y);
+        while (u >= 1.f && b < a.U - 1) {
+          q = __ldg(a.tab + ++b);
+          u = (float)((t - q.x) * q.y);
+        }
+        while (u < 0.f && b > 0) {
+          q = __ldg(a.tab + --b);
+          u = (float)((t - q.x) * q.y);
+        }
+        // f = 1 - (1 - u) D(T_b) / D(t) = u + (1 - u) u (T_{b+1} - T_b) nly / D(t),
+        // D(t) = vl / (n . v) of the point
+        const float e = u * dd_rcp_approx((float)q.y) * nly * dw * dd_rcp_approx(xm ? wx : wy);
+        k[l][m] = b;
+        f[l][m] = __saturatef(fmaf(1.f - u, e, u));
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int jx = j & 1, jy = j >> 1;  // x columns: line jx, edges jy, jy + 1; y rows: line jy, edges jx, jx + 1
+      kL[j] = xm ? k[jx][jy] : k[jy][jx];
+      fL[j] = xm ? f[jx][jy] : f[jy][jx];
+      kR[j] = xm ? k[jx][jy + 1] : k[jy][jx + 1];
+      fR[j] = xm ? f[jx][jy + 1] : f[jy][jx + 1];
+      wgt[j] = G.sgn;
+    }
+  } else {
+    const bool xdom = fabs(sx) > fabs(sy);
+    const double c = fma(dd_angle(v, sx, sy, sxf, syf, s_at), a.inv_dbeta, a.cnt + DD_MAGIC);
+    const int kc = max(__double2hiint(c), 0x41300000) - 0x41380000;
+    const float fc = (float)((unsigned)__double2loint(c) >> 8) * 5.9604644775390625e-8f;
+    const float idb = (float)a.inv_dbeta, hdb = h * idb;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float ex = (j & 1) ? h : -h, ey = (j >> 1) ? h : -h;
+      const float wx = v.xf + ex, wy = v.yf + ey;
+      const float z = (v.xf * ey - v.yf * ex) * dd_rcpf(fmaf(v.xf, wx, v.yf * wy));
+      const float dlt = fmaf(-z * (z * z), 1.f / 3.f, z) * idb;
+      const float l2 = fmaf(wx, wx, wy * wy), ddv = xdom ? wx : wy;
+      float rl;
+      asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rl) : "f"(l2));
+      rl *= fmaf(-0.5f * l2 * rl, rl, 1.5f);
+      const float da = ddv * (rl * rl) * hdb;
+      wgt[j] = dxf * (l2 * rl) * dd_rcpf(ddv);
+      // cell and fraction of centre + offset, clamped to [0, U]
+      const float r[2] = {(fc + dlt) - da, (fc + dlt) + da};
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float g = (r[e] - 0.5f) + 12582912.f;  // 1.5 2^23: rounds to the cell (a fraction of 1 may stay below)
+        int k = kc + (__float_as_int(g) - 0x4b400000);
+        float f = r[e] - (g - 12582912.f);
+        if ((unsigned)k >= (unsigned)a.U) {
+          f = k < 0 ? 0.f : 1.f;
+          k = k < 0 ? 0 : a.U - 1;
+        }
+        if (e) kR[j] = k, fR[j] = f;
+        else kL[j] = k, fL[j] = f;
+      }
+    }
+  }
+}
+
 // Measured per c3 subset (96 views x 736 channels, 512^2 x 128): reference
 // formula 1.40 -> 1.08 ms, exact adjoint 1.77 -> 1.25 ms (0.86 ms of either
 // when the decode is left out); 1111 views of 384^2 x 45, exact adjoint 10.8 ->
@@ -771,7 +882,7 @@ __device__ __forceinline__ void dd_footprint(const DdBackArgs& a, const ViewGeom
 // writes the four overlap weights of every window value to shared memory, so
 // the inner loop is one value load, one weight load and 4 SV FMAs, with no
 // address or branch per voxel.  It needs no view order and takes both view
-// orientations in one pass.  Windows of any width work: a record holds 12 (4)
+// orientations in one pass.  Windows of any width work: a record holds 8
 // values at a time, wider ones take more passes.  Sums are kept per FLUSH
 // views and added to totals in shared memory, so a sum over thousands of
 // views rounds like one over a few; with nseg > 1 the views are split over
@@ -795,8 +906,8 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
   const int vb = a.vb0 + ztile * ZL + zi;
   const int x0 = 2 * (bx0 + g);
   const bool active = g < GW && ztile * ZL + zi < a.nvb && x0 < a.XN && y0 < a.YN;
-  const int NR = dd_back_records(GW), MW = dd_back_window(GW), RS = dd_back_stride(GW);
-  const int VC = NR / GW;  // views decoded at a time
+  constexpr int MW = DD_BACK_MW, RS = DD_BACK_RS;
+  const int VC = 32 / GW;  // views decoded at a time
   const size_t vstride = (size_t)(a.U + 1) * a.ZP * VB, kstride = (size_t)a.ZP * VB;
   const char* q = reinterpret_cast<const char*>(a.q) + (size_t)(active ? vb : 0) * VB;
   if (!ADJ) {
@@ -812,65 +923,71 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
   Vec<SV> acc[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) vzero(acc[j]);
-  // decode: lane -> voxel lvx of block lb (of 8 or GW) of view lv (of VP)
-  const int lvx = lane & 3, lb = GW >= 8 ? lane >> 2 : (lane >> 2) % GW, lv = GW >= 8 ? 0 : (lane >> 2) / GW;
-  const int VP = GW >= 8 ? 1 : 8 / GW;
-  int xx = 0, yy = 0;
-  double px = 0.0, py = 0.0;
-  float pxf = 0.f, pyf = 0.f;
-  bool von = false;
-  const auto place = [&](int gg) {
-    xx = 2 * (bx0 + gg) + (lvx & 1);
-    yy = y0 + (lvx >> 1);
-    von = gg < GW && xx < a.XN && yy < a.YN && lv < VP && (!a.epi.mask || a.epi.mask[(size_t)yy * a.XN + xx] != 0);
-    px = (xx - a.ocx) * a.dx;
-    py = (yy - a.ocy) * a.dx;
-    pxf = (float)px;
-    pyf = (float)py;
-  };
-  place(lb);
+  // decode: lane -> block lb of view lv of VC
+  const int lv = lane / GW, lb = lane - lv * GW;
+  const double px = (2 * (bx0 + lb) + 0.5 - a.ocx) * a.dx, py = (y0 + 0.5 - a.ocy) * a.dx;
+  const float pxf = (float)px, pyf = (float)py;
+  bool on[4], von = false;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int xx = 2 * (bx0 + lb) + (j & 1), yy = y0 + (j >> 1);
+    on[j] = lv < VC && xx < a.XN && yy < a.YN && (!a.epi.mask || a.epi.mask[(size_t)yy * a.XN + xx] != 0);
+    von = von || on[j];
+  }
   const int vbeg = (int)((long long)a.PN * seg / nseg), vend = (int)((long long)a.PN * (seg + 1) / nseg);
   int since = 0;
   for (int v0 = vbeg; v0 < vend; v0 += VC) {
     const int nvc = min(VC, vend - v0);
     int mmax = 0;
     for (int i0 = 0; i0 == 0 || i0 < mmax; i0 += MW) {  // windows wider than a record: more passes
-      // four lanes a block, one voxel each; 8 blocks of one or more views a step
-      for (int pb = 0; pb < GW; pb += 8) {
-        if (GW > 8) place(pb + (lane >> 2));
-#pragma unroll 1
-        for (int u0 = 0; u0 < nvc; u0 += VP) {
-          const int vv = u0 + lv;
-          int kL = 0, kR = 0;
-          float fL = 0.f, fR = 0.f, wgt = 0.f;
-          const bool on = von && vv < nvc;
-          if (on) {
-            dd_footprint<ADJ>(a, a.vg[v0 + vv], px, py, pxf, pyf, s_at, kL, fL, kR, fR, wgt);
+      if (lv < nvc) {
+        int kL[4], kR[4], m = 0, kb = 0x7fffffff, ke = -1;
+        float fL[4], fR[4], wgt[4];
+        if (von) {
+          dd_block<ADJ>(a, a.vg[v0 + lv], px, py, pxf, pyf, s_at, kL, fL, kR, fR, wgt);
+          // the block's window: the cells its footprints cover
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (on[j]) {
+              kb = min(kb, min(kL[j], kR[j]));
+              ke = max(ke, max(kL[j], kR[j]));
+            } else {
+              wgt[j] = 0.f;
+            }
           }
-          // the block's window: the cells its four footprints cover (first and
-          // 0xffff - last, both minima, in one word)
-          unsigned kk = on ? (unsigned)min(kL, kR) | (unsigned)(0xffff - max(kL, kR)) << 16 : 0xffffffffu;
-          kk = __vminu2(kk, __shfl_xor_sync(0xffffffffu, kk, 1));
-          kk = __vminu2(kk, __shfl_xor_sync(0xffffffffu, kk, 2));
-          int kb = (int)(kk & 0xffffu);
-          int m = kk == 0xffffffffu ? 0 : 0xffff - (int)(kk >> 16) - kb + 1;  // all off: none
           // whole steps: more values, with weight 0, after the window or, at the
           // detector's end, before it
-          m = (m + T::STEP - 1) / T::STEP * T::STEP;
-          kb = m ? max(min(kb, a.U + 1 - m), 0) : 0;
-          mmax = max(mmax, m);
-          const int gg = pb + lb;
-          if (gg < GW && vv < nvc) {
-            const int rec = vv * GW + gg, n = min(max(m - i0, 0), MW);
-            // the value in cell k has the weight of [cL, cR]'s part inside
-            // [k, k + 1] (negative where cR < cL): sat(cR - k) - sat(cL - k),
-            // the cells' difference exact
-            float* wp = reinterpret_cast<float*>(&s_wt[w][rec * RS]) + lvx;
-            float dL = (float)(kL - kb - i0), dR = (float)(kR - kb - i0);
-            for (int i = 0; i < n; ++i, dL -= 1.f, dR -= 1.f) wp[4 * i] = (__saturatef(dR + fR) - __saturatef(dL + fL)) * wgt;
-            if (lvx == 0) s_h[w][rec] = make_uint2((unsigned)(vv * (a.U + 1) + kb + (n ? i0 : 0)) * (unsigned)a.ZP, (unsigned)n);
+          m = (ke - kb + T::STEP) / T::STEP * T::STEP;
+          kb = max(min(kb, a.U + 1 - m), 0);
+        } else {
+          kb = 0;
+        }
+        mmax = max(mmax, m);
+        const int n = min(max(m - i0, 0), MW);
+        if (n) {
+          // the value in cell k has the weight of [cL, cR]'s part inside
+          // [k, k + 1] (negative where cR < cL): sat(cR - k) - sat(cL - k), the
+          // cells' difference exact
+          float dL[4], dR[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            dL[j] = (float)(kL[j] - kb - i0);
+            dR[j] = (float)(kR[j] - kb - i0);
+          }
+          float4* wp = reinterpret_cast<float4*>(&s_wt[w][lane * RS]);
+#pragma unroll 1
+          for (int i = 0; i < n; ++i, ++wp) {
+            float x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              x[j] = (__saturatef(dR[j] + fR[j]) - __saturatef(dL[j] + fL[j])) * wgt[j];
+              dL[j] -= 1.f;
+              dR[j] -= 1.f;
+            }
+            *wp = make_float4(x[0], x[1], x[2], x[3]);
           }
         }
+        s_h[w][lane] = make_uint2((unsigned)(lv * (a.U + 1) + kb + (n ? i0 : 0)) * (unsigned)a.ZP, (unsigned)n);
       }
       mmax = __reduce_max_sync(0xffffffffu, mmax);
       __syncwarp();
@@ -932,9 +1049,8 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
 }
 
 // The same for at most 8 slices (one vector per lane and z-tile): no lanes
-// share a block, so each decodes its own four voxels in registers (four
-// independent chains of the decode's arithmetic) and weights the window values
-// as it loads them.
+// share a block, so each decodes its own in registers and weights the window
+// values as it loads them.
 template <int SV, bool ADJ>
 __device__ __forceinline__ void back_thin_body(const DdBackArgs& a, int tile, int ztile) {
   using T = DdBackTile<SV>;
@@ -966,8 +1082,8 @@ __device__ __forceinline__ void back_thin_body(const DdBackArgs& a, int tile, in
     on[j] = by < nby && ix < a.XN && iy < a.YN && (!a.epi.mask || a.epi.mask[(size_t)iy * a.XN + ix] != 0);
     any = any || on[j];
   }
-  const double px = (2 * bx - a.ocx) * a.dx, py = (2 * by - a.ocy) * a.dx;
-  const float pxf = (float)px, pyf = (float)py, dxf = (float)a.dx;
+  const double px = (2 * bx + 0.5 - a.ocx) * a.dx, py = (2 * by + 0.5 - a.ocy) * a.dx;
+  const float pxf = (float)px, pyf = (float)py;
   const int vbeg = (int)((long long)a.PN * seg / nseg), vend = (int)((long long)a.PN * (seg + 1) / nseg);
   const size_t kstride = (size_t)a.ZP * VB, vstride = (size_t)(a.U + 1) * kstride;
   const char* q = reinterpret_cast<const char*>(a.q) + (size_t)vb * VB + (size_t)vbeg * vstride;
@@ -975,11 +1091,9 @@ __device__ __forceinline__ void back_thin_body(const DdBackArgs& a, int tile, in
   for (int p = vbeg; any && p < vend; ++p, q += vstride) {
     float fL[4], fR[4], wgt[4];
     int kL[4], kR[4], kb = 0x7fffffff, ke = -1;
+    dd_block<ADJ>(a, a.vg[p], px, py, pxf, pyf, s_at, kL, fL, kR, fR, wgt);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int ix = j & 1, iy = j >> 1;
-      dd_footprint<ADJ>(a, a.vg[p], px + ix * a.dx, py + iy * a.dx, pxf + ix * dxf, pyf + iy * dxf, s_at, kL[j], fL[j],
-                        kR[j], fR[j], wgt[j]);
       if (on[j]) {
         kb = min(kb, min(kL[j], kR[j]));
         ke = max(ke, max(kL[j], kR[j]));

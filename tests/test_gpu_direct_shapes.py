@@ -23,6 +23,8 @@ CASES = [
     (12, 12, 16, 20, 240, False, False),   # 20 channels a pixel: narrow footprints, wide voxels
     (48, 40, 24, 700, 64, False, True),    # enough warps that lines are not split
     (3, 5, 9, 7, 2, False, False),         # fewer pixels and channels than any tile
+    (160, 150, 9, 6, 900, True, True),     # windows of more values than a record holds
+    (161, 160, 2, 6, 900, False, False),   # the same for one vector of slices
 ]
 
 
