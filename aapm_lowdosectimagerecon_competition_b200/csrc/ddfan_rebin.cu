@@ -44,6 +44,8 @@ struct RebinParams {
   const int* sslice;   // [nsorted] their slices
   int nsorted, chunks; // chunks: warps per raw view (32 slices each) to cover its slices
   int SLN, T, W, H;    // T = DefTimes
+  int stride;          // k_rebin_routine: typical raw views between two slices' starts
+  int cblocks;         // k_rebin_routine: channel blocks the launch is split into
   float SD, SD2, PH, DCH, deltaZ, delta, BV, twopi, sm_lo, sm_hi;
 };
 
@@ -195,14 +197,33 @@ __global__ void __launch_bounds__(256) k_rebin_unvisited(RebinParams p) {
 
 // Routine layout (after HelicalToFan_routine.m:44-45 permutes, the solver's
 // sinogram layout): out[ib][j][s], views[ib][s].  A CTA owns 32 slices of one
-// view; warps compute rows (lanes over 32 channels) into a shared tile, then
-// store it transposed with lanes over slices (128-byte rows).
+// view and a block of channels; warps compute rows (lanes over 32 channels)
+// into a shared tile, then store it transposed with lanes over slices
+// (128-byte rows).
+//
+// What bounds it is DRAM: a raw view serves one row of every slice within a
+// detector's height of it (27 slices at the AAPM spacing), each of those rows
+// at another view index ib = i - start, and taking the views in order read the
+// raw data again for each (14 GB, 6.6 TB/s, for 2.6 GB of raw views and output).
+// So the launch takes the views with stride "stride", the typical distance of
+// two starts: rows (ib + m stride, slice - m) share a raw view, and one pass over
+// m and the slices reads some 120 raw views several times each.  Channels are
+// taken a block at a time to keep the passes in flight within L2.
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_rebin_routine(RebinParams p) {
   __shared__ float tile[32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ib = blockIdx.x;
-  const int s0 = blockIdx.y * 32;
+  // grid x: the slice blocks of a view, the views in strided order
+  const int nsb = (p.SLN + 31) / 32, nv = blockIdx.x / nsb;
+  const int s0 = (blockIdx.x - nv * nsb) * 32;
+  // view nv of the order 0, stride, 2 stride, ..., 1, 1 + stride, ...
+  const int full = p.T / p.stride, rem = p.T - full * p.stride;  // rem phases have one view more
+  const int long_views = rem * (full + 1);
+  const int phase = nv < long_views ? nv / (full + 1) : rem + (nv - long_views) / full;
+  const int m = nv < long_views ? nv - phase * (full + 1) : (nv - long_views) - (phase - rem) * full;
+  const int ib = phase + m * p.stride;
+  const int cw = ((p.W + 31) / 32 + p.cblocks - 1) / p.cblocks * 32;  // channels of a block
+  const int jbeg = blockIdx.y * cw, jend = min(p.W, jbeg + cw);
   RebinRow rows[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -215,10 +236,10 @@ __global__ void __launch_bounds__(256) k_rebin_routine(RebinParams p) {
       rows[q].n = 0.f;
     }
   }
-  if (warp == 0 && s0 + lane < p.SLN)
+  if (blockIdx.y == 0 && warp == 0 && s0 + lane < p.SLN)
     p.views[(size_t)ib * p.SLN + s0 + lane] = rebin_view_angle(p, s0 + lane, ib);
   const int ns = min(32, p.SLN - s0);
-  for (int j0 = 0; j0 < p.W; j0 += 32) {
+  for (int j0 = jbeg; j0 < jend; j0 += 32) {
     const int j = j0 + lane;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -345,8 +366,22 @@ int rebin_prepare(RebinHost& h, long long nViews, const float* zPos, int SLN, fl
   p.SD = SD; p.SD2 = SD * SD; p.PH = PerDetH; p.DCH = DetCenterHreal;
   p.deltaZ = deltaZ; p.delta = delta; p.BV = BVAngle; p.twopi = (float)(2 * M_PI);
   p.sm_lo = lo; p.sm_hi = hi;
+  // the mean distance of two starts, when a view range holds several of them
+  p.stride = 1;
+  if (idx.size() > 1) {
+    const long long d = ((long long)h.sstart.back() - h.sstart.front() + (long long)(idx.size() - 1) / 2) / (long long)(idx.size() - 1);
+    if (d > 1 && d < DefTimes) p.stride = (int)d;
+  }
   return DDFAN_OK;
 }
+
+// channel blocks of k_rebin_routine: 96 slices of a 736 x 64 scan took 0.98 ms
+// with 4, 1.00 with 1, 1.05 with 8, 1.24 with 16 (2.22 in view order); three
+// other scans 4 too
+#ifndef DDFAN_REBIN_CBLOCKS
+#define DDFAN_REBIN_CBLOCKS 4
+#endif
+constexpr int kRebinChannelBlocks = DDFAN_REBIN_CBLOCKS;
 
 // layout 0 (mex layouts): raw-view-order traversal, plus the rows it never
 // visits; layout 1 (slices last): one CTA per (32 slices, view).
@@ -365,9 +400,13 @@ int rebin_launch(const RebinHost& h, int layout, cudaStream_t st) {
       else k_rebin_diag<false><<<(unsigned)ctas, 256, 0, st>>>(p, h.lo, h.hi);
     }
   } else {
-    dim3 grid(p.T, (p.SLN + 31) / 32);
-    if (vec) k_rebin_routine<true><<<grid, 256, 0, st>>>(p);
-    else k_rebin_routine<false><<<grid, 256, 0, st>>>(p);
+    const long long ctas = (long long)p.T * ((p.SLN + 31) / 32);
+    if (ctas > 0x7fffffffLL) return set_err(DDFAN_ERR_UNSUPPORTED, "HelicalToFan: %d views x %d slices", p.T, p.SLN);
+    RebinParams p2 = p;
+    p2.cblocks = std::min((p.W + 31) / 32, kRebinChannelBlocks);
+    dim3 grid((unsigned)ctas, p2.cblocks);
+    if (vec) k_rebin_routine<true><<<grid, 256, 0, st>>>(p2);
+    else k_rebin_routine<false><<<grid, 256, 0, st>>>(p2);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(DDFAN_ERR_CUDA, "HelicalToFan launch: %s", cudaGetErrorString(e));
