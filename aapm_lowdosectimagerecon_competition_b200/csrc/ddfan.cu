@@ -67,6 +67,12 @@ LaunchProfiler::~LaunchProfiler() {
 
 // ------------------------------------------------------------------ plan
 
+static int check_launch(const char* what) {
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return set_err(DDFAN_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
+  return DDFAN_OK;
+}
+
 // Tile widths chosen by the autotuner (ddfan_tune_set_zl), keyed by the
 // number of 4-slice blocks; consulted before the built-in cost model.
 static std::mutex g_tune_mutex;
@@ -116,6 +122,15 @@ bool dd_mode(int sat_mode, const uint8_t* mask, size_t npix) {
   for (size_t i = 0; mask && i < npix; ++i)
     if (mask[i] > 1) return false;
   return true;
+}
+
+bool dd_wants_columns(int Zs) { return Zs <= 8; }
+
+int launch_columns(const float* img, float* imgT, int XN, int YN, int Zs, cudaStream_t st) {
+  if (Zs == 1) return ps_transpose(img, imgT, 1, YN, XN, st);
+  k_columns<<<dim3((XN + 31) / 32, (YN + 31) / 32), 256, 0, st>>>(reinterpret_cast<const float4*>(img),
+                                                                  reinterpret_cast<float4*>(imgT), XN, YN, Zs / 4);
+  return check_launch("k_columns");
 }
 
 // Slices per thread for operands of Zs slices at p
@@ -367,7 +382,7 @@ int plan_create(Plan** out, const PlanDesc& d) {
   const size_t nimg = direct ? 0 : (size_t)p.XN * p.YN * p.ZB * F4;
   const size_t nsino = direct ? (((size_t)p.PNmax * (p.U + 1) + DD_PAST) * p.Zs + 3) / 4
                               : (size_t)p.PNmax * (p.U + 1) * p.ZB * F4;
-  const size_t ntmp = (size_t)p.XN * p.YN * (direct ? p.Zs : p.Z);
+  const size_t ntmp = (size_t)p.XN * p.YN * (direct ? (dd_wants_columns(p.Zs) ? 2 : 1) * p.Zs : p.Z);
   if ((rc = dalloc(&p.d_bx, p.U + 1, &B, as)) || (rc = dalloc(&p.d_by, p.U + 1, &B, as)) ||
       (rc = dalloc(&p.d_xd, p.U, &B, as)) || (rc = dalloc(&p.d_yd, p.U, &B, as)) ||
       (rc = dalloc(&p.d_mask, (size_t)p.XN * p.YN, &B, as)) || (rc = dalloc(&p.d_tb, p.U + 1, &B, as)) ||
@@ -405,11 +420,6 @@ int plan_create(Plan** out, const PlanDesc& d) {
 
 // ------------------------------------------------------------------ launches
 
-static int check_launch(const char* what) {
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return set_err(DDFAN_ERR_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
-  return DDFAN_OK;
-}
 
 static GeomConsts geom_consts(const Plan& p) {
   GeomConsts g;
@@ -424,7 +434,9 @@ int launch_view_geom(const Plan& p, const float* d_angs, int stride, int PN, Vie
                      double2* fc, float* cvd, cudaStream_t st) {
   if (PN < 1) return set_err(DDFAN_ERR_ARG, "PN must be >= 1");
   ProfScope ps(KIND_VIEW_GEOM, st);
-  k_view_geom<<<PN, 128, 0, st>>>(geom_consts(p), d_angs, stride, PN, vg, fc, cvd);
+  // one view of 736 channels took a CTA 13 us, six boundaries a thread
+  const int per_view = PN >= 1024 ? 1 : std::min(8, (p.U + 128) / 128);
+  k_view_geom<<<dim3(PN, per_view), 128, 0, st>>>(geom_consts(p), d_angs, stride, PN, vg, fc, cvd);
   return check_launch("k_view_geom");
 }
 
@@ -688,14 +700,14 @@ int launch_publish_masked(const float* x, int Zi, const float* x0, int Z, const 
 constexpr int DD_THIN = 1;
 
 // Lanes per group (vectors per z-tile) of the direct kernels for nvb vectors
-// of slices: at most a warp's 32, and of the splits into z-tiles the one that
+// of slices: at most "most", and of the splits into z-tiles the one that
 // leaves the fewest lanes idle -- 32 / zl groups fill a warp only when zl
 // divides it well, and the last tile may be short.  Every extra tile decodes
 // the walks again (a third of a walk's own cost at 4 lanes), hence the 10 %.
-int dd_lanes(int nvb) {
+int dd_lanes(int nvb, int most) {
   int best = 1;
   double bc = 1e300;
-  for (int nt = (nvb + 31) / 32; nt <= std::max(1, (nvb + 3) / 4); ++nt) {
+  for (int nt = (nvb + most - 1) / most; nt <= std::max(1, (nvb + 3) / 4); ++nt) {
     const int zl = (nvb + nt - 1) / nt;
     const double c = (double)nt / (32 / zl) * (1.0 + 0.1 * (nt - 1));
     if (c < bc - 1e-9) { bc = c; best = zl; }
@@ -706,12 +718,12 @@ int dd_lanes(int nvb) {
 // Channels of a forward warp
 static int dd_fwd_channels(const DdFwdArgs& a) { return a.thin ? 64 : 32 / a.zl * DDFAN_DD_FWD_CG; }
 
-DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc,
+DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const float* imgT, const ViewGeom* vg, const double2* fc,
                            const float* cvd, const int* order, int PN, float* out, int orow, int ostride, int zlo,
                            int zhi, const DdResidual* res) {
   DdFwdArgs a{};
   a.sv = dd_vector(p.Zs, img);
-  a.img = img; a.ZP = p.Zs / a.sv;
+  a.img = img; a.imgT = imgT; a.ZP = p.Zs / a.sv;
   a.vg = vg; a.fc = fc; a.cvd = cvd; a.order = order;
   a.out = out; a.orow = orow; a.ostride = ostride;
   a.PN = PN; a.U = p.U; a.XN = p.XN; a.YN = p.YN; a.dx = (float)p.dx;
@@ -719,7 +731,10 @@ DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, 
   a.vb0 = a.zlo / a.sv;
   a.nvb = a.zhi > a.zlo ? (a.zhi + a.sv - 1) / a.sv - a.vb0 : 0;
   a.thin = a.sv == 1 || a.nvb <= DD_THIN;
-  a.zl = a.thin ? 1 : dd_lanes(a.nvb);
+  // 64 slices a tile: the image part that the views in flight share then stays
+  // below half of L2 (128 slices, 512^2, 96 views: 1.31 ms in one tile, 1.28 in
+  // two, 1.47 in four)
+  a.zl = a.thin ? 1 : dd_lanes(a.nvb, 8);
   a.nzt = (a.nvb + a.zl - 1) / a.zl;
   // a launch of fewer warps than the SMs hold (24 each) splits every ray's
   // lines over 2, 4 or 8 of them
@@ -737,10 +752,10 @@ int dd_fwd_cblocks(const DdFwdArgs& a) {
   return (a.U + cw - 1) / cw;
 }
 
-int launch_fwd_dd(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc, const float* cvd,
+int launch_fwd_dd(const Plan& p, const float* img, const float* imgT, const ViewGeom* vg, const double2* fc, const float* cvd,
                   const int* order, int PN, float* out, int orow, int ostride, int zlo, int zhi,
                   const DdResidual* res, cudaStream_t st) {
-  const DdFwdArgs a = make_fwd_dd_args(p, img, vg, fc, cvd, order, PN, out, orow, ostride, zlo, zhi, res);
+  const DdFwdArgs a = make_fwd_dd_args(p, img, imgT, vg, fc, cvd, order, PN, out, orow, ostride, zlo, zhi, res);
   if (a.nvb == 0 || PN < 1) return DDFAN_OK;
   ProfScope ps(KIND_FWD, st);
   const dim3 grid(PN, dd_fwd_cblocks(a), a.nzt);
@@ -777,7 +792,7 @@ DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const
   a.vb0 = a.epi.zlo / a.sv;
   a.nvb = a.epi.zhi > a.epi.zlo ? (a.epi.zhi + a.sv - 1) / a.sv - a.vb0 : 0;
   a.thin = a.sv == 1 || a.nvb <= DD_THIN;
-  a.zl = a.thin ? 1 : dd_lanes(a.nvb);
+  a.zl = a.thin ? 1 : dd_lanes(a.nvb, 32);
   a.nzt = (a.nvb + a.zl - 1) / a.zl;
   // a launch of fewer warps than the SMs hold (24 each) splits the views over
   // 2, 4 or 8 of them
@@ -839,7 +854,12 @@ int proj_dev_shared(Plan& p, const float* d_angs, int stride, int PN, const floa
         return rc;
       img = p.d_tmp;
     }
-    rc = launch_fwd_dd(p, img, p.d_vg, p.d_fc, p.d_cvd, p.d_order, PN, d_prj, p.U, p.Z, zlo, zhi, nullptr, st);
+    float* imgT = nullptr;
+    if (dd_wants_columns(p.Zs)) {
+      imgT = p.d_tmp + (size_t)p.XN * p.YN * p.Zs;
+      if ((rc = launch_columns(img, imgT, p.XN, p.YN, p.Zs, st))) return rc;
+    }
+    rc = launch_fwd_dd(p, img, imgT, p.d_vg, p.d_fc, p.d_cvd, p.d_order, PN, d_prj, p.U, p.Z, zlo, zhi, nullptr, st);
     mark_use(p, st);
     return rc;
   }
@@ -1107,7 +1127,7 @@ DDFAN_API size_t ddfan_plan_estimate_bytes(int XN, int YN, int DNU, int SLN, int
   const bool direct = sat_mode == SAT_DIRECT || sat_mode == SAT_HILO;
   const size_t Zs = (size_t)dd_pad(SLN);
   const size_t cells = direct ? ((P * (U + 1) + DD_PAST) * Zs + 3) / 4 : 2 * (size_t)XN * YN * ZB * F4 + P * (U + 1) * ZB * F4;
-  const size_t tmp = (size_t)XN * YN * (direct ? Zs : (size_t)SLN);
+  const size_t tmp = (size_t)XN * YN * (direct ? (dd_wants_columns((int)Zs) ? 2 : 1) * Zs : (size_t)SLN);
   return cells * sizeof(float4) + (2 * (U + 1) + 4 * U) * sizeof(double) + (size_t)XN * YN +
          (U + 1) * sizeof(float) + 4 * (U + 1) * sizeof(uint16_t) + P * sizeof(ViewGeom) +
          P * (U + 1) * sizeof(double2) + P * U * sizeof(float) + tmp * sizeof(float) +

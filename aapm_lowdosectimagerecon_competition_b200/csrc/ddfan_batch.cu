@@ -235,7 +235,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
       DdResidual r;
       r.y = s.d_y; r.yview = s.d_yview + o; r.rowsum = s.d_rows + (size_t)o * s.U; r.wgt = adj ? cvd : nullptr;
       r.ystride = s.Zi;
-      const DdFwdArgs fa = make_fwd_dd_args(p, s.d_x, vg, fc, cvd, s.d_order + o, c, s.d_ax, s.U + 1, s.Zi, 0, s.Zi, &r);
+      const DdFwdArgs fa = make_fwd_dd_args(p, s.d_x, nullptr, vg, fc, cvd, s.d_order + o, c, s.d_ax, s.U + 1, s.Zi, 0, s.Zi, &r);
       if (fa.nvb < 1) continue;
       const int fi = (int)fargs.size();
       fargs.push_back(fa);

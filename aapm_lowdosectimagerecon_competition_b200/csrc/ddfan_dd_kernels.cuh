@@ -143,6 +143,7 @@ __device__ __forceinline__ float vget(const Vec<1>& a, int) { return a.f; }
 
 struct DdFwdArgs {
   const float* img;    // masked image [YN][XN][ZP vectors of SV slices]
+  const float* imgT;   // its columns [XN][YN][ZP vectors] or null (fwd_thin_body)
   int ZP;
   const ViewGeom* vg;
   const double2* fc;   // [PN][U+1] boundary lines
@@ -451,7 +452,10 @@ __device__ __forceinline__ void fwd_thin_body(const DdFwdArgs& a, int row, int c
   const bool xm = a.vg[p].xmajor != 0;
   const int nl = xm ? a.XN : a.YN, N = xm ? a.YN : a.XN;
   const double2* fcp = a.fc + (size_t)p * (a.U + 1);
-  const size_t kstride = (size_t)(xm ? a.XN : 1) * a.ZP * VB, lstride = (size_t)(xm ? 1 : a.XN) * a.ZP * VB;
+  // neighbouring lanes read neighbouring k: x-major views from the columns
+  const bool cols = xm && a.imgT;
+  const size_t kstride = (size_t)(xm && !cols ? a.XN : 1) * a.ZP * VB;
+  const size_t lstride = (size_t)(cols ? a.YN : (xm ? 1 : a.XN)) * a.ZP * VB;
   float* tot = s_tot + tid;
 #pragma unroll
   for (int e = 0; e < 2 * SV; ++e) tot[e * T::NT] = 0.f;
@@ -469,7 +473,7 @@ __device__ __forceinline__ void fwd_thin_body(const DdFwdArgs& a, int row, int c
       fl[j].y += DD_MAGIC;
     }
     const bool two = u0 + 1 < a.U;
-    const char* lp = reinterpret_cast<const char*>(a.img) + (size_t)vb * VB + (size_t)lo * lstride;
+    const char* lp = reinterpret_cast<const char*>(cols ? a.imgT : a.img) + (size_t)vb * VB + (size_t)lo * lstride;
     int since = 0;
 #pragma unroll 2
     for (int ii = lo; ii < hi; ++ii, lp += lstride) {
@@ -1196,6 +1200,16 @@ static __global__ void k_stage_image(const float* __restrict__ src, int Z, const
       if (mask && mask[pix] == 0) v = 0.f;
     }
     dst[i] = v;
+  }
+}
+
+// out[x][y][z] = in[y][x][z] for pixels of P float4: 32 x 32 pixels a CTA
+static __global__ void __launch_bounds__(256) k_columns(const float4* __restrict__ in, float4* __restrict__ out, int XN,
+                                                        int YN, int P) {
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
+  for (int e = threadIdx.x; e < 32 * 32 * P; e += 256) {
+    const int z = e % P, i = e / P, y = y0 + (i & 31), x = x0 + (i >> 5);
+    if (x < XN && y < YN) out[((size_t)x * YN + y) * P + z] = __ldg(in + ((size_t)y * XN + x) * P + z);
   }
 }
 

@@ -32,7 +32,8 @@ __device__ inline double wrap_angle(double c) {
   return c;
 }
 
-// One CTA per view.  Writes, in double, the boundary lines of the forward
+// gridDim.y CTAs per view (few views: more of them, so that a thread takes
+// one or two boundaries).  Writes, in double, the boundary lines of the forward
 // kernel (AAPM_script/MultiSlicesProjGPU.cu:120-168) in texel-sample
 // coordinates: along line ii the boundary ray b crosses the prefix-sum axis at
 // c_b(ii) = ii * F_b + C_b (c = texture coordinate - 0.5), and the per-channel
@@ -60,18 +61,19 @@ static __global__ void k_view_geom(GeomConsts g, const float* __restrict__ angs,
       C = ((-g.ocy * g.dx - By) * f + Bx) / g.dx + g.ocx + 0.5;
     }
   };
-  for (int b = threadIdx.x; b <= U; b += blockDim.x) {
+  const int t0 = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
+  for (int b = t0; b <= U; b += step) {
     double F, C;
     line_of(b, F, C);
     fc[(size_t)p * (U + 1) + b] = make_double2(F, C);
   }
-  for (int u = threadIdx.x; u < U; u += blockDim.x) {
+  for (int u = t0; u < U; u += step) {
     const double Dx = g.xd[u] * cs - g.yd[u] * sn, Dy = g.xd[u] * sn + g.yd[u] * cs;
     const double ddx = Dx - sx, ddy = Dy - sy;
     const double nrm = sqrt(ddx * ddx + ddy * ddy);
     cvd[(size_t)p * U + u] = (float)(nrm / fabs(xm ? ddx : ddy));
   }
-  if (threadIdx.x == 0) {
+  if (t0 == 0) {
     double F0, C0, F1, C1;
     line_of(0, F0, C0);
     line_of(U, F1, C1);

@@ -215,7 +215,7 @@ extern "C" DDFAN_API int ddfan_proj_noalloc(float x0, float y0, int DNU, const f
         rc = launch_stage_image(d_vol, SLN, p.d_mask, si, p.Zs, (size_t)XN * YN, st);
         img = si;
       }
-      if (!rc) rc = launch_fwd_dd(p, img, p.d_vg, p.d_fc, p.d_cvd, p.d_order, PN, d_prj, DNU, SLN, 0, SLN, nullptr, st);
+      if (!rc) rc = launch_fwd_dd(p, img, nullptr, p.d_vg, p.d_fc, p.d_cvd, p.d_order, PN, d_prj, DNU, SLN, 0, SLN, nullptr, st);
     } else if (!(rc = launch_sat_image(p, d_vol, st))) {
       rc = launch_fwd(p, p.d_vg, p.d_fc, p.d_cvd, p.d_order, PN, d_prj, 0, SLN, st);
     }

@@ -149,17 +149,23 @@ struct DdResidual {
   const float* wgt = nullptr;     // [slot][U] or null
   int ystride = 0;
 };
-// Forward projection of the masked image img [YN][XN][Zs] into
+// The image's columns [XN][YN][Zs] from its rows, for a forward launch that
+// wants them (dd_wants_columns: the thin kernels, whose lanes walk neighbouring
+// channels and read x-major views' columns along y).
+bool dd_wants_columns(int Zs);
+int launch_columns(const float* img, float* imgT, int XN, int YN, int Zs, cudaStream_t st);
+// Forward projection of the masked image img [YN][XN][Zs] (and its columns, or
+// null) into
 // out[slot][orow][ostride] (slices [zlo, zhi) written).
-int launch_fwd_dd(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc, const float* cvd,
+int launch_fwd_dd(const Plan& p, const float* img, const float* imgT, const ViewGeom* vg, const double2* fc, const float* cvd,
                   const int* order, int PN, float* out, int orow, int ostride, int zlo, int zhi,
                   const DdResidual* res, cudaStream_t st);
-// Lanes per group of the direct kernels for nvb vectors of slices.
-int dd_lanes(int nvb);
+// Lanes per group of the direct kernels for nvb vectors of slices, at most "most".
+int dd_lanes(int nvb, int most);
 // Channel blocks (grid y) of a forward launch.
 int dd_fwd_cblocks(const DdFwdArgs& a);
 // The arguments launch_fwd_dd would launch with (nvb: vectors of [zlo, zhi)).
-DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const ViewGeom* vg, const double2* fc,
+DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const float* imgT, const ViewGeom* vg, const double2* fc,
                            const float* cvd, const int* order, int PN, float* out, int orow, int ostride, int zlo,
                            int zhi, const DdResidual* res);
 // The arguments launch_back_dd would launch with (nvb: vectors of the

@@ -327,11 +327,12 @@ static int solver_iteration(Solver& s, cudaStream_t st) {
     DdResidual r;
     r.y = s.d_y; r.yview = s.d_yview + o; r.rowsum = s.d_rows + (size_t)o * s.U; r.wgt = adj ? cvd : nullptr;
     r.ystride = s.Zi;
-    if ((rc = launch_fwd_dd(p, s.d_x, vg, fc, cvd, s.d_order + o, c, s.d_ax, s.U + 1, s.Zi, 0, s.Zi, &r, st)))
+    if (s.d_xt && (rc = launch_columns(s.d_x, s.d_xt, s.XN, s.YN, s.Zi, st))) return rc;
+    if ((rc = launch_fwd_dd(p, s.d_x, s.d_xt, vg, fc, cvd, s.d_order + o, c, s.d_ax, s.U + 1, s.Zi, 0, s.Zi, &r, st)))
       return rc;
     // backproject, divide by colSum, add, optional clamp (:91-97)
     if ((rc = launch_back_dd(p, s.back_mode, s.d_ax, vg, c, e, st))) return rc;
-    n += 2;
+    n += s.d_xt ? 3 : 2;
   }
   for (int k = 0; k < s.nsub && !s.ps && !s.direct; ++k) {
     const int o = s.off[k], c = s.cnt[k];
@@ -580,17 +581,18 @@ static int solver_weights_dd(Solver& s, const PlanDesc& d, const std::vector<flo
   int rc = plan_create(&P1.p, d1);
   if (rc) return rc;
   const Plan& p = *P1.p;
-  DevBuf<float> ang(st), img(st), q(st), cvd(st);
+  DevBuf<float> ang(st), img(st), imgT(st), q(st), cvd(st);
   DevBuf<ViewGeom> vg(st);
   DevBuf<double2> fc(st);
   if ((rc = ang.alloc(P)) || (rc = vg.alloc(P)) || (rc = fc.alloc((size_t)P * (U + 1))) ||
       (rc = cvd.alloc((size_t)P * U)) || (rc = img.alloc((size_t)XN * YN)) ||
-      (rc = q.alloc((size_t)P * (U + 1) + DD_PAST)))
+      (rc = imgT.alloc((size_t)XN * YN)) || (rc = q.alloc((size_t)P * (U + 1) + DD_PAST)))
     return rc;
   DDFAN_CK(cudaMemcpyAsync(ang.p, angs0.data(), sizeof(float) * P, cudaMemcpyHostToDevice, st));
   if ((rc = launch_view_geom(p, ang.p, 1, P, vg.p, fc.p, cvd.p, st))) return rc;
   if ((rc = launch_stage_image(nullptr, 1, p.has_mask ? p.d_mask : nullptr, img.p, 1, (size_t)XN * YN, st))) return rc;
-  if ((rc = launch_fwd_dd(p, img.p, vg.p, fc.p, cvd.p, nullptr, P, s.d_rows, U, 1, 0, 1, nullptr, st))) return rc;
+  if ((rc = launch_columns(img.p, imgT.p, XN, YN, 1, st))) return rc;
+  if ((rc = launch_fwd_dd(p, img.p, imgT.p, vg.p, fc.p, cvd.p, nullptr, P, s.d_rows, U, 1, 0, 1, nullptr, st))) return rc;
   if ((rc = launch_stage_sino(nullptr, 1, adj ? cvd.p : nullptr, U, q.p, 1, (size_t)P, st))) return rc;
   for (int k = 0; k < s.nsub; ++k) {
     BackEpi e{};
@@ -812,6 +814,7 @@ static int solver_create(Solver** out, float x0, float y0, int DNU, const float*
       DDFAN_CK(cudaMemcpyAsync(s.d_perm, s.perm.data(), sizeof(int) * s.Zi, cudaMemcpyHostToDevice, st));
       DDFAN_CK(cudaMemcpyAsync(s.d_inv, inv.data(), sizeof(int) * SLN, cudaMemcpyHostToDevice, st));
     }
+    if (dd_wants_columns(s.Zi) && (rc = salloc(s, &s.d_xt, V))) return rc;
     if (s.P->has_mask && (rc = salloc(s, &s.d_x0, Vc))) return rc;
     if (published_copy(s) && (rc = salloc(s, &s.d_xu, Vc))) return rc;
     DDFAN_CK(cudaStreamSynchronize(st));
@@ -946,13 +949,14 @@ DDFAN_API size_t ddfan_ossart_estimate_bytes(int XN, int YN, int DNU, int SLN, i
   if (direct) {
     own += 2 * (size_t)XN * YN * SLN * sizeof(float);
     if (Zi != (size_t)SLN) own += P * U * SLN * sizeof(float) + (Zi + SLN) * sizeof(int);
+    if (dd_wants_columns((int)Zi)) own += V * sizeof(float);
   }
   // transient at creation, direct kernels: the one-slice weight plan, the
   // geometry of every view, the image and the rows of ones
   if (direct)
     return plan + own + ddfan_plan_estimate_bytes(XN, YN, DNU, 1, 1, sat_mode) +
            P * (sizeof(ViewGeom) + (U + 1) * sizeof(double2) + (2 * U + 2) * sizeof(float)) +
-           ((size_t)XN * YN + DD_PAST) * sizeof(float);
+           (2 * (size_t)XN * YN + DD_PAST) * sizeof(float);
   // otherwise: the one-slice weight plan and the slice-major weight buffers
   // (geometry, row sums, ones, tables) over nsub x PNmax rows
   const size_t R = (size_t)numOfOS * PNmax, CB = sat_mode == SAT_FP32 ? 8 : 16;
@@ -1133,7 +1137,7 @@ DDFAN_API int ddfan_ossart_launches_per_iter(const ddfan_ossart* h) {
   const Solver* s = reinterpret_cast<const Solver*>(h);
   if (!s) return 0;
   const bool adj = s->back_mode == DDFAN_BACK_ADJ;
-  const int per = s->ps ? 7 : (s->direct ? 2 : (adj ? 5 : 4));
+  const int per = s->ps ? 7 : (s->direct ? (s->d_xt ? 3 : 2) : (adj ? 5 : 4));
   return s->nsub * per + (s->useFISTA ? 2 : 0);
 }
 

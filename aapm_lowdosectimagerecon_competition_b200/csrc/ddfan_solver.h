@@ -57,7 +57,7 @@ struct Solver {
   bool ps = false;
   int cstride = 0;
   float* d_pang = nullptr;   // [nsub][Z][cstride] angles of each slice's views per subset
-  float* d_xt = nullptr;     // [Z][XN][YN] image columns
+  float* d_xt = nullptr;     // [Z][XN][YN] image columns (slice-major), [XN][YN][Zi] (direct, few slices)
   float* d_tabx = nullptr;   // image rows table [Z][YN][XN] cells
   float* d_taby = nullptr;   // image columns table [Z][XN][YN] cells
   float* d_sq = nullptr;     // weighted residual table [Z][cstride][U+1] cells
