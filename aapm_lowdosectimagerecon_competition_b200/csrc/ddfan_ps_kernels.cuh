@@ -21,6 +21,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "ddfan_decode.cuh"
 #include "ddfan_device.cuh"
 #include "ddfan_ps.h"
 
@@ -189,21 +190,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-
-// The REF backprojector's angle step with a Newton reciprocal in place of
-// the FP64 division (1: per-slice c3 iteration 365 -> 355 ms of REF
-// backprojection) or the division (0)
-#ifndef DDFAN_PS_REF_NEWTON
-#define DDFAN_PS_REF_NEWTON 1
-#endif
-
-// The REF backprojector's channel coordinates in 32.32 fixed point (1: two
-// conversions per pixel and view instead of six, which took the per-slice c3
-// iteration's REF backprojection from 355 to 314 ms) or FP64 with float
-// conversions (0)
-#ifndef DDFAN_PS_REF_FIXED
-#define DDFAN_PS_REF_FIXED 1
-#endif
 
 // ---------------------------------------------------------------- transposes
 
@@ -533,103 +519,102 @@ __global__ void __launch_bounds__(256) k_ps_back_adj(PsBackArgs a) {
 
 // The reference backprojector's formula (AAPM_script/MultiSlicesBackGPU.cu:115-184,
 // as k_back_ref) per slice: voxel-driven, angular detector coordinate
-// alpha = asin(cross / (|s| l)) (here as the equal atan(cross / dot), in
-// FP64), footprint half-width dx ddv / (2 l^2) and weight dx l / ddv (FP32,
-// relative terms), coordinate alpha / dbeta + detCntIdx + 1 in FP64 per
-// (voxel, view), then the two samples of the channel prefix sums in table
-// precision.  Warp = 32 consecutive pixels of a row x R rows of one slice;
-// the OS-SART update (or the plain backprojection) is fused as in
+// alpha = asin(cross / (|s| l)), footprint half-width dx ddv / (2 l^2) and weight
+// dx l / ddv (FP32, relative terms), then the two samples of the channel prefix
+// sums in table precision.  Warp = 32 consecutive pixels of a row x R rows of
+// one slice; the OS-SART update (or the plain backprojection) is fused as in
 // k_ps_back_adj, with k_back_ref's mask rule (masked voxels get 0).
+//
+// alpha is the angle from -s to the voxel's ray d.  On a view's first row it is
+// dd_angle's; down the column it moves by the angle between consecutive rows'
+// rays, whose tangent t = d_x dx / (d_{i-1} . d_i) is exact and small: t in FP64,
+// the next terms of its series (t^3 / 3 - t^5 / 5 + t^7 / 7, below 5e-5 for |t|
+// <= 0.05) in FP32.  The centre's channel coordinate is a cell and a fraction
+// from one FP64 addition's bits; the half-width, below a few channels, is added
+// to the fraction in FP32.  What bounds it is instruction issue: conversions to
+// and from FP64 and 64-bit integers, which share a slow unit, made up most of
+// the 141 instructions a pixel and view took before: 384^2 x 24 slices, 720
+// views of 736 channels, hi/lo cells: 11.1 -> 8.9 ms, error of a solve against
+// 64 bits 1.8 .. 5.5e-7 -> 1.9 .. 3.2e-7 over seven sizes.  16 rows a warp: the same.
 template <int M>
 __global__ void __launch_bounds__(256) k_ps_back_ref(PsBackArgs a) {
   constexpr int R = kPsRefRows, PX = 32;
   using Cell = typename PsCell<M>::T;
+  __shared__ double2 s_at[2 * DD_ATAN_N + 1];
+  for (int j = threadIdx.x; j <= 2 * DD_ATAN_N; j += 256) s_at[j] = dd_atan_entry(j);
+  __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int z = blockIdx.z;
   const int x0 = (blockIdx.x * 2 + (w & 1)) * PX, y0 = (blockIdx.y * 4 + (w >> 1)) * R;
-  if (x0 >= a.XN || y0 >= a.YN) return;  // uniform per warp
+  if (x0 >= a.XN || y0 >= a.YN) return;  // uniform per warp; no barrier below
   const int ix = x0 + lane;
   const int U = a.U;
-  const double Ud = (double)U;
   const size_t rowQ = (size_t)(U + 1);
-  const float dxf = (float)a.dx, hdx = (float)(a.dx * 0.5);
-#if DDFAN_PS_REF_FIXED
-  const double two32 = 4294967296.0;
-  const double K32 = a.inv_dbeta * two32, C32 = a.cnt_ref * two32;  // coordinate per radian, offset; x 2^32
-  const float hdxK = (float)(a.dx * 0.5 * a.inv_dbeta * two32);
-  const long long cmax = (long long)U << 32;
-#endif
+  const float dxf = (float)a.dx, hdb = (float)(a.dx * 0.5 * a.inv_dbeta);
+  // what the two constants' rounding, which every sample shares, takes off
+  const float corr = (float)((a.dx * (a.dx * 0.5 * a.inv_dbeta)) / ((double)dxf * (double)hdb) - 1.0);
+  const double px = ((double)ix - a.ocx) * a.dx, py = ((double)y0 - a.ocy) * a.dx, cnt = a.cnt_ref + DD_MAGIC;
   float acc[R];
 #pragma unroll
   for (int i = 0; i < R; ++i) acc[i] = 0.f;
   for (int m = 0; m < a.cnt; ++m) {
     const size_t r = (size_t)z * a.cstride + m;
-    const double sx = a.vg[r].sx, sy = a.vg[r].sy;
+    const ViewGeom& G = a.vg[r];
+    const double sx = G.sx, sy = G.sy;
+    const float sxf = (float)sx, syf = (float)sy;
     const bool xdom = fabs(sx) > fabs(sy);
     const Cell* qrow = reinterpret_cast<const Cell*>(a.sq) + r * rowQ;
-    const double ddx = ((double)ix - a.ocx) * a.dx - sx;
-    double alpha = 0.0, ddy_prev = 0.0;
+    DdRay v{px - sx, py - sy, (float)(px - sx), (float)(py - sy)};
+    const float yf0 = v.yf;
+    const double dx2 = v.x * v.x, step = v.x * a.dx;
+    const float dx2f = v.xf * v.xf, stepf = v.xf * dxf;
+    double alpha = 0.0;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const double ddy = ((double)(y0 + i) - a.ocy) * a.dx - sy;
-      // alpha = asin((s_y d_x - s_x d_y) / (|s| l)) is the signed angle from
-      // -s to d: atan of the cross over the dot product (dot > 0 for voxels in
-      // front of the source), which needs no square root in FP64.  Down the
-      // column the angle moves by the angle from the previous row's d to this
-      // one, whose tangent t = d_x (dy_i - dy_{i-1}) / (d_{i-1} . d_i) is exact
-      // and small; for |t| <= 0.05 the series t - t^3/3 + t^5/5 - t^7/7 is
-      // exact to FP64 rounding (next term below 2e-13 t), otherwise the full
-      // atan.  The half-width and the weight only need FP32.
       bool full = i == 0;
-      if (!full) {
-#if DDFAN_PS_REF_NEWTON
-        // 1 / (d_{i-1} . d_i) from the FP32 approximate reciprocal (relative
-        // error below 2^-22) and one FP64 Newton step (error squared: ~1e-13)
-        const double den = fma(ddy_prev, ddy, ddx * ddx);
-        const double r0 = (double)rcp_approx((float)den);
-        const double rr = r0 * fma(-den, r0, 2.0);
-        const double t = ddx * (ddy - ddy_prev) * rr;
-#else
-        const double t = ddx * (ddy - ddy_prev) / fma(ddy_prev, ddy, ddx * ddx);
-#endif
-        if (fabs(t) <= 0.05) {
-          const double t2 = t * t;
-          alpha += t * fma(t2, fma(t2, fma(t2, -1.0 / 7.0, 1.0 / 5.0), -1.0 / 3.0), 1.0);
+      if (i) {
+        const double yprev = v.y;
+        const float yprevf = v.yf;
+        v.y += a.dx;
+        v.yf = fmaf((float)i, dxf, yf0);
+        const float rf = dd_rcp_approx(fmaf(yprevf, v.yf, dx2f));
+        const double t = step * dd_newton(fma(yprev, v.y, dx2), rf);
+        const float tf = stepf * rf, t2 = tf * tf;
+        if (fabsf(tf) <= 0.05f) {
+          const float q = t2 * fmaf(t2, fmaf(t2, 1.f / 7.f, -0.2f), 1.f / 3.f);
+          alpha += fma(-t, dd_widen(q), t);
         } else {
           full = true;
         }
       }
-      if (full) alpha = atan((sy * ddx - sx * ddy) / -(sx * ddx + sy * ddy));
-      ddy_prev = ddy;
-      const float fx = (float)ddx, fy = (float)ddy, fdv = xdom ? fx : fy;
-      const float l2 = fmaf(fx, fx, fy * fy);
-      const double da = (double)(__fdividef(fdv, l2) * hdx);
-      const float wt = __fdividef(dxf, fdv) * sqrtf(l2);
-#if DDFAN_PS_REF_FIXED
-      // both channel coordinates in 32.32 fixed point: the centre from FP64,
-      // the half-width from FP32 (below a few channels, so its FP32 rounding
-      // is ~1e-7 channel), clamped to [0, U] as integers; the fraction comes
-      // from the low word (cell U holds the total with value 0, so a
-      // coordinate of U samples it with fraction 0)
-      (void)da;
-      (void)Ud;
-      const long long cc = __double2ll_rn(fma(alpha, K32, C32));
-      // (bounded before the sums: a conversion out of range saturates)
-      const long long hw = min(max(__float2ll_rn(__fdividef(fdv, l2) * hdxK), -(1LL << 50)), 1LL << 50);
-      const long long cl = min(max(cc - hw, 0LL), cmax), cr = min(max(cc + hw, 0LL), cmax);
-      const int iL = (int)(cl >> 32), iR = (int)(cr >> 32);
-      PhiS<M> pL, pR;
-      pL.load(qrow + iL, __int_as_float(0x3f800000 | ((unsigned)cl >> 9)) - 1.f);
-      pR.load(qrow + iR, __int_as_float(0x3f800000 | ((unsigned)cr >> 9)) - 1.f);
-#else
-      const double cL = fmin(fmax((alpha - da) * a.inv_dbeta + a.cnt_ref, 0.0), Ud);
-      const double cR = fmin(fmax((alpha + da) * a.inv_dbeta + a.cnt_ref, 0.0), Ud);
-      const int iL = min((int)cL, U - 1), iR = min((int)cR, U - 1);
-      PhiS<M> pL, pR;
-      pL.load(qrow + iL, (float)(cL - iL));
-      pR.load(qrow + iR, (float)(cR - iR));
-#endif
-      acc[i] = fmaf(pR.diff(pL), wt, acc[i]);
+      if (full) alpha = dd_angle(v, sx, sy, sxf, syf, s_at);
+      const double c = fma(alpha, a.inv_dbeta, cnt);
+      const int kc = max(__double2hiint(c), 0x41300000) - 0x41380000;
+      const float fc = (float)((unsigned)__double2loint(c) >> 8) * 5.9604644775390625e-8f;
+      const float l2 = fmaf(v.yf, v.yf, dx2f), ddv = xdom ? v.xf : v.yf;
+      float rl;
+      asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rl) : "f"(l2));
+      // 1 / l and l: one Newton step as a correction, so that the
+      // approximation's bias does not survive in the step's rounding
+      const float h = l2 * rl, er = 0.5f * fmaf(-h, rl, 1.f);
+      rl = fmaf(rl, er, rl);
+      const float da = ddv * (rl * rl) * hdb, wt = dxf * fmaf(h, er, h) * dd_rcpf(ddv);
+      // both samples: cell and fraction of centre -+ half-width, clamped to
+      // [0, U] (cell U holds the total with value 0)
+      const float p[2] = {fc - da, fc + da};
+      PhiS<M> phi[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float g = (p[e] - 0.5f) + 12582912.f;  // 1.5 2^23: rounds to the cell (a fraction of 1 may stay below)
+        int k = kc + (__float_as_int(g) - 0x4b400000);
+        float f = p[e] - (g - 12582912.f);
+        if ((unsigned)k >= (unsigned)U) {
+          k = k < 0 ? 0 : U;
+          f = 0.f;
+        }
+        phi[e].load(qrow + k, f);
+      }
+      acc[i] = fmaf(phi[1].diff(phi[0]), wt, acc[i]);
     }
   }
   if (ix >= a.XN) return;
@@ -637,6 +622,7 @@ __global__ void __launch_bounds__(256) k_ps_back_ref(PsBackArgs a) {
   for (int i = 0; i < R; ++i) {
     const int iy = y0 + i;
     if (iy >= a.YN) break;
+    acc[i] = fmaf(acc[i], corr, acc[i]);
     const size_t pix = (size_t)iy * a.XN + ix;
     const size_t idx = (size_t)z * a.XN * a.YN + pix;
     float val = (!a.mask || a.mask[pix] != 0) ? acc[i] : 0.f;

@@ -81,3 +81,32 @@ def test_mask_bytes_above_one_scale_the_image(sat):
     xo = O.ossart(x0, y0, s.DNU, xds, yds, s.detCntIdx, 0, 0, s.hangs(), s.PN, 32, 32, 9, y, init, s.dx, mask, 2,
                   s.numOfOS, 1, 1, O.REF)
     assert rel(xg, xo) < 1e-5
+
+
+# (XN, YN, slices, views, channels, image centre in mm)
+REF_ROWS = [
+    (40, 40, 3, 24, 72, 0.0),    # a warp's and a row group's remainders
+    (33, 27, 2, 17, 41, 3.0),
+    (3, 5, 4, 7, 12, 0.0),
+    (12, 13, 2, 30, 48, 0.0),    # 30 mm pixels: angle steps beyond the series
+    (64, 65, 2, 12, 900, 300.0),  # rays far off the fan, beyond 45 degrees
+    (160, 9, 2, 12, 60, 0.0),
+]
+
+
+@pytest.mark.parametrize("XN,YN,Z,PN,U,cx", REF_ROWS)
+@pytest.mark.parametrize("sat", ["hilo", "fp64"])
+def test_per_slice_ref_backprojection_matches_oracle(XN, YN, Z, PN, U, cx, sat):
+    """The slice-major REF backprojector (per-slice angle lists) at the edges
+    of its row groups and of its angle steps, within the compensated modes'
+    2e-6 of the FP64 oracle."""
+    from aapm_lowdosectimagerecon_competition_b200 import configs, dd2
+    from oracle import oracle as O
+    s = configs.scaled(configs.c2(SLN=Z), XN=XN, DNU=U, PN=PN)
+    x0, y0, xds, yds = dd2.fan_geometry(s.sid, s.sdd, U, s.detCellWidth, s.detCntIdx)
+    a = s.angles()
+    h = np.stack([(a + 0.37 * z).astype(np.float32) for z in range(Z)], 1)
+    prj = np.random.default_rng(XN + PN).random((PN, U, Z)).astype(np.float32)
+    args = (x0, y0, U, xds, yds, s.detCntIdx, np.float32(cx), np.float32(0), h, PN, XN, YN, Z, prj, s.dx)
+    got, exp = dd2.MultiSlicesBackGPU(*args, sat=sat, back="ref"), O.back(*args, mode=O.REF)
+    assert np.linalg.norm((got - exp).ravel()) < 2e-6 * np.linalg.norm(exp.ravel())
