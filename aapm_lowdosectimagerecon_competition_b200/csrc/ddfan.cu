@@ -961,10 +961,13 @@ static long long grouped_slices(const Plan& p, const std::vector<std::vector<int
   return n;
 }
 
-// Time per slice of the slice-major kernels over the shared-list ones,
-// measured at 512 x 512, 96 views: forward 1.45x, exact adjoint 2.7x, REF
-// backprojector 4.4x (its FP64 geometry per sample is no longer shared by 32
-// slices).  The grouped path costs its computed slices over Z times the
+// Time per slice of the slice-major kernels over the shared-list table
+// kernels, measured at 512 x 512, 96 views: forward 1.45x, exact adjoint 2.7x,
+// REF backprojector 4.4x (its FP64 geometry per sample is no longer shared by
+// 32 slices).  The direct kernels are two to three times faster than the
+// table kernels, so calls of hi/lo or direct plans that lie between these
+// ratios and that multiple of them would be faster grouped; the lines have not
+// been moved for them.  The grouped path costs its computed slices over Z times the
 // shared-list time.
 static bool use_slice_major(const Plan& p, const std::vector<std::vector<int>>& groups, int PN, double ratio) {
   return groups.size() > 1 && PN <= 65535 && (double)grouped_slices(p, groups) > ratio * p.Z;

@@ -200,11 +200,11 @@ __device__ __forceinline__ void dd_fwd_store(const DdFwdArgs& a, int p, int u, i
 }
 
 // What bounds it (c3 subset, 96 views x 736 channels x 512^2 x 128): the loads'
-// latency, and behind it the L1 pipe -- 1.30 ms, of which 1.0 ms remain when
-// every load hits L1; 14.2 GB cross from L2 (every view reads the image once:
-// 12.9 GB) at 11 TB/s, half of what L2 gives a 64 MB working set.  24 warps an
-// SM at 80 registers and 2 channels a thread beat 16 warps at 128 with 3
-// channels (1.34 ms) or 2 (1.41).  Before: 1.90 ms (4 z-tiles of 4 slices a
+// latency, and behind it the L1 pipe -- 1.28 ms (1.30 in one tile of 128
+// slices), of which 1.0 ms remain when every load hits L1; 14.2 GB cross from
+// L2 (every view reads the image once: 12.9 GB) at 11 TB/s; 60 % of L1's
+// wavefronts, 95 % L2 hits.  24 warps an SM at 80 registers and 2 channels a
+// thread beat 16 warps at 128 with 3 channels (1.34 ms) or 2 (1.41).  Before: 1.90 ms (4 z-tiles of 4 slices a
 // thread, no lines skipped).
 //
 // Warp = one view x (32 / zl) groups of CG consecutive channels x zl vectors
@@ -791,9 +791,9 @@ __device__ __forceinline__ void dd_block(const DdBackArgs& a, const ViewGeom& G,
 }
 
 // Measured per c3 subset (96 views x 736 channels, 512^2 x 128): reference
-// formula 1.40 -> 1.08 ms, exact adjoint 1.77 -> 1.25 ms (0.86 ms of either
+// formula 1.40 -> 0.94 ms, exact adjoint 1.77 -> 1.10 ms (0.86 ms of either
 // when the decode is left out); 1111 views of 384^2 x 45, exact adjoint 10.8 ->
-// 8.0 ms.  16 warps an SM at 128 registers with 4 values in flight each beat 24
+// 5.2 ms.  With each voxel decoded by itself (1.08 and 1.25 ms), 16 warps an SM at 128 registers with 4 values in flight each beat 24
 // at 80 with 1 (1.20), 3 (1.29) or 4 (1.14): more warps spread over more views
 // and lose the L1 hits (80 -> 68 %).
 //

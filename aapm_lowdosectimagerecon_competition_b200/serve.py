@@ -1,9 +1,9 @@
 """Batched and served OS-SART reconstructions on one GPU.
 
 * `TileTuner` -- the autotuner: times the projector kernels for each
-  candidate tile shape (z-tile width; in the direct mode also the z-tiles a
-  thread walks) on a bucket's shape and records the fastest in the library
-  (ddfan_tune_set_zl, ddfan_tune_set_nz) and in a JSON cache.
+  candidate tile shape of the table kernels (z-tile width) on a bucket's
+  shape and records the fastest in the library (ddfan_tune_set_zl,
+  ddfan_tune_set_nz) and in a JSON cache.
 * `Engine` -- continuous batching: requests of uneven sizes are admitted, in
   arrival order with back-fill, while the HBM budget (exact per-request
   estimates from ddfan_ossart_estimate_bytes) and the slot count allow; every
@@ -106,8 +106,9 @@ def make_instance(N, Z, P, seed, device, iters=5, numOfOS=24, I0=1.5e5):
 class TileTuner:
     """Measures every valid tile shape for a slice count (4-slice blocks) on
     a representative shape and keeps the fastest: the z-tile width (z-lanes
-    per channel or voxel group, 1-8 blocks) and, in the direct mode, how many
-    z-tiles each thread walks per decoded footprint (1, 2 or 4)."""
+    per channel or voxel group, 1-8 blocks) and, in the direct mode, a z-tiles
+    count per thread.  The table kernels follow them; the direct kernels take
+    their tiles from the slice count and the launch's size instead."""
 
     def __init__(self, cache_path=None, sat="hilo", back="adj"):
         self.cache_path = cache_path

@@ -6,7 +6,8 @@ sid 595 mm, sdd 1085.6 mm, 24 ordered subsets, FISTA momentum and
 non-negativity, the reference's backprojector (the one OSSART_AAPM.m
 drives; --back adj selects the exact adjoint), the direct mode (every
 prefix-sum difference summed from the values it telescopes to; --sat fp32 /
-hilo / fp64 selects prefix-sum tables instead);
+fp64 selects prefix-sum tables instead, hilo the direct kernels or, for
+per-slice lists, tables);
 the sinogram is the log of seeded Poisson counts at I0 = 1.5e5 photons/ray of
 a seeded ellipsoid phantom (synthetic stand-in for the AAPM projections).
 A step is one OS-SART iteration (one CUDA graph replay, 24 subsets).
@@ -539,7 +540,7 @@ def config_dict(s, args, n):
                             "rebinned-irregular": "per-slice lists as helical rebinning makes them, slices 86.07 "
                                                   "raw views apart"}[getattr(args, "views", "shared")],
             "l2": "inputs larger than L2 (sinogram 868 MB, image 134 MB%s)" % (
-                "" if args.sat == "direct" else ", prefix-sum tables 0.8 GB"),
+                "" if on_direct_kernels(args.sat, getattr(args, "views", "shared")) else ", prefix-sum tables 0.8 GB"),
             "parallelism": "one independent reconstruction per GPU (slices/requests shard with no exchange)"}
 
 
@@ -642,21 +643,26 @@ class ClockSampler:
                 "samples": len(sm), "reasons": sorted(reasons)}
 
 
-# ncu summaries in profiles/ by (direct mode?, backprojector) and kernel slot
+def on_direct_kernels(sat, views="shared"):
+    """With one angle list for all slices and the workloads' 0/1 mask, the
+    direct kernels run the direct and the hi/lo mode."""
+    return sat in ("direct", "hilo") and views == "shared"
+
+
+# ncu summaries in profiles/ by (direct kernels?, backprojector) and kernel slot
 PROFILE_OF = {
     (False, "adj"): {"fwd": "k_fwd_c3_subset.md", "back_a": "k_back_adj_c3_subset.md",
                      "back_b": "k_back_adj_c3_subset.md"},
     (False, "ref"): {"fwd": "k_fwd_c3_subset.md"},
-    (True, "adj"): {"fwd": "k_fwd_dd_c3_subset.md", "back_a": "k_back_dd_c3_subset.md",
-                    "back_b": "k_back_dd_c3_subset.md"},
+    (True, "adj"): {"fwd": "k_fwd_dd_c3_subset.md", "back_a": "k_back_dd_c3_subset.md"},
     (True, "ref"): {"fwd": "k_fwd_dd_c3_subset.md", "back_a": "k_back_ref_dd_c3_subset.md"},
 }
 
 
-def profiled_traffic(kernel, sat="hilo", back="adj"):
+def profiled_traffic(kernel, sat="hilo", back="adj", views="shared"):
     """DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum)
     recorded from an ncu capture of this kernel in profiles/, or None."""
-    name = PROFILE_OF[(sat == "direct", back)].get(kernel)
+    name = PROFILE_OF[(on_direct_kernels(sat), back)].get(kernel) if views == "shared" else None
     if not name:
         return None
     try:
@@ -758,7 +764,7 @@ def run_ours(args):
     # backprojection 4S + 4V (read the subset residual table once, write the image)
     alg = {"fwd": 4.0 * (V + S_sub), "back_a": 4.0 * (V + S_sub), "back_b": 4.0 * (V + S_sub),
            "sat_image": 4.0 * V + 2 * 12.0 * V, "sat_sino": 4.0 * S_sub + 12.0 * S_sub}
-    if args.sat == "direct":
+    if on_direct_kernels(args.sat, args.views):
         # the forward also reads the measured sinogram and writes the residual
         # (the prefix-sum kernels it replaces did that)
         alg["fwd"] = 4.0 * V + 8.0 * S_sub
@@ -767,12 +773,12 @@ def run_ours(args):
     achieved = alg[top] / (top_ms / 1e3) / 1e9
     roofline = {"bound": "hbm", "kernel": top, "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind,
-                "traffic": profiled_traffic(top, args.sat, args.back), "algorithmic_bytes": alg[top],
+                "traffic": profiled_traffic(top, args.sat, args.back, args.views), "algorithmic_bytes": alg[top],
                 "launch_ms": top_ms,
                 "kernel_ms_per_iter": {k: round(v[0], 3) for k, v in prof.items()},
                 "note": "achieved = algorithmic bytes per launch / CUDA-event launch time; the "
                         "path is gather/issue bound, not HBM bound"}
-    if top == "fwd" and args.views == "shared" and args.sat != "direct":
+    if top == "fwd" and args.views == "shared" and not on_direct_kernels(args.sat):
         # the bound that applies: L1 gathers of prefix-sum cells -- per line of
         # each ray group one cell per boundary (CG channels share CG + 1
         # boundaries), a cell holding 4 slices (32 B FP32, 48 B hi/lo or FP64)
@@ -840,7 +846,7 @@ def run_ours(args):
                 modes["%s/%s" % (sat, back)] = mode_rate(s, (x0, y0, xds, yds), y, mask, hangs, sat, back, local)
         line["other_modes"] = {"iters_per_s": modes,
                                "how": "the same workload and sinogram, 2 warm-up and 5 timed graph replays "
-                                      "per mode (sat/back); hilo = compensated prefix-sum tables"}
+                                      "per mode (sat/back); hilo runs on the direct kernels with shared lists"}
 
     # ---- final-image parity at this configuration, and the CPU baseline
     parity_failed = False

@@ -220,7 +220,8 @@ DDFAN_API float* ddfan_ossart_image_ptr(ddfan_ossart* s);
  * CUDA events on `stream`; returns per kind the summed device milliseconds
  * and launch counts.  Kinds: 0 view geometry, 1 image prefix sums,
  * 2 forward projection, 3 sinogram prefix sums (+ residual), 4 backprojection
- * (REF, or exact-adjoint column pass), 5 exact-adjoint row pass, 6 FISTA.
+ * (with tables and the exact adjoint: its column pass), 5 the exact adjoint's
+ * row pass with tables, 6 FISTA.
  * Arrays must hold 7 entries.  (Diagnostics; no counterpart in the reference.) */
 DDFAN_API int ddfan_ossart_profile(ddfan_ossart* s, int numOfIter, void* stream, float* ms_by_kind,
                                    int* launches_by_kind);
