@@ -664,14 +664,12 @@ __device__ __forceinline__ void dd_footprint(const DdBackArgs& a, const ViewGeom
     wgt = G.sgn;
   } else {
     const float l2f = fmaf(v.xf, v.xf, v.yf * v.yf);
-    float rs;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(l2f));
+    float l, rs;
+    dd_length(l2f, l, rs);
     const bool xdom = fabs(sx) > fabs(sy);
     const double ca = fma(dd_angle(v, sx, sy, sxf, syf, s_at), a.inv_dbeta, a.cnt + DD_MAGIC);
     const double l2 = fma(v.x, v.x, v.y * v.y);
     const double da = (xdom ? v.x : v.y) * dd_newton(l2, rs * rs) * (0.5 * a.dx * a.inv_dbeta);
-    // dx l / ddv, l from the approximation and one Newton step
-    const float l = l2f * (rs * fmaf(-0.5f * l2f * rs, rs, 1.5f));
     wgt = (float)a.dx * l * dd_rcpf(xdom ? v.xf : v.yf);
     dd_cell(ca - da, a.U, kL, fL);
     dd_cell(ca + da, a.U, kR, fR);
@@ -767,11 +765,10 @@ __device__ __forceinline__ void dd_block(const DdBackArgs& a, const ViewGeom& G,
       const float z = (v.xf * ey - v.yf * ex) * dd_rcpf(fmaf(v.xf, wx, v.yf * wy));
       const float dlt = fmaf(-z * (z * z), 1.f / 3.f, z) * idb;
       const float l2 = fmaf(wx, wx, wy * wy), ddv = xdom ? wx : wy;
-      float rl;
-      asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rl) : "f"(l2));
-      rl *= fmaf(-0.5f * l2 * rl, rl, 1.5f);
+      float l, rl;
+      dd_length(l2, l, rl);
       const float da = ddv * (rl * rl) * hdb;
-      wgt[j] = dxf * (l2 * rl) * dd_rcpf(ddv);
+      wgt[j] = dxf * l * dd_rcpf(ddv);
       // cell and fraction of centre + offset, clamped to [0, U]
       const float r[2] = {(fc + dlt) - da, (fc + dlt) + da};
 #pragma unroll

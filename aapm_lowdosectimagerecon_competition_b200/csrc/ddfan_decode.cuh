@@ -38,6 +38,18 @@ __device__ __forceinline__ float dd_rcpf(float x) {
   return fmaf(r, fmaf(-x, r, 1.f), r);
 }
 
+// l = sqrt(l2) and 1 / l, for normal l2: the approximate reciprocal square root
+// and one Newton step.  The step is added as a correction: as the factor
+// 1.5 - l2 r r / 2, which rounds near 1, it would leave the approximation's bias
+// in the result, and every sample of a voxel has the same one.
+__device__ __forceinline__ void dd_length(float l2, float& l, float& rl) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(l2));
+  const float h = l2 * r, e = 0.5f * fmaf(-h, r, 1.f);
+  rl = fmaf(r, e, r);
+  l = fmaf(h, e, h);
+}
+
 // x as a double, exactly, for normal x, with integer instructions
 __device__ __forceinline__ double dd_widen(float x) {
   const unsigned u = __float_as_uint(x);

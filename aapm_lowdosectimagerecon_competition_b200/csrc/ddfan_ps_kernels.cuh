@@ -592,13 +592,9 @@ __global__ void __launch_bounds__(256) k_ps_back_ref(PsBackArgs a) {
       const int kc = max(__double2hiint(c), 0x41300000) - 0x41380000;
       const float fc = (float)((unsigned)__double2loint(c) >> 8) * 5.9604644775390625e-8f;
       const float l2 = fmaf(v.yf, v.yf, dx2f), ddv = xdom ? v.xf : v.yf;
-      float rl;
-      asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rl) : "f"(l2));
-      // 1 / l and l: one Newton step as a correction, so that the
-      // approximation's bias does not survive in the step's rounding
-      const float h = l2 * rl, er = 0.5f * fmaf(-h, rl, 1.f);
-      rl = fmaf(rl, er, rl);
-      const float da = ddv * (rl * rl) * hdb, wt = dxf * fmaf(h, er, h) * dd_rcpf(ddv);
+      float l, rl;
+      dd_length(l2, l, rl);
+      const float da = ddv * (rl * rl) * hdb, wt = dxf * l * dd_rcpf(ddv);
       // both samples: cell and fraction of centre -+ half-width, clamped to
       // [0, U] (cell U holds the total with value 0)
       const float p[2] = {fc - da, fc + da};
