@@ -282,21 +282,16 @@ __device__ __forceinline__ void fwd_dd_body(const DdFwdArgs& a, int row, int cbl
         // cell and fraction of both boundaries on the line, footprint length
         const double di = (double)(ii0 + col);
         const double t0 = fma(di, fa.x, fa.y), t1 = fma(di, fb.x, fb.y);
-        int k0, k1;
-        float f0, f1;
-        dd_cell(t0, N, k0, f0);
-        dd_cell(t1, N, k1, f1);
+        const DdPos p0 = dd_pos(t0, N), p1 = dd_pos(t1, N);
         const float inv = uok ? dd_rcpf((float)(t1 - t0) * dx) : 0.f;
-        // The walk from (k0, f0) to (k1, f1): w0 on the value at k0, we on the
-        // value at k1 (0 when the cells are the same: it is the start value
-        // again), wm on the interior values between, if any
-        const bool up = k1 > k0, same = k1 == k0;
+        float w0, wm, we;
+        dd_walk(p0, p1, inv, w0, wm, we);
+        const int k0 = p0.k, k1 = p1.k;
+        const bool up = k1 > k0;
         const int n = up ? k1 - k0 : k0 - k1;
         wide |= n > 2;
-        const float w0 = ((same ? f1 : (up ? 1.f : 0.f)) - f0) * inv;
-        const float we = same ? 0.f : (up ? f1 : f1 - 1.f) * inv;
         const unsigned oe = (unsigned)k1 * ks;
-        s_w[w][(col * GW + rg) * CG + rj] = make_float4(w0, up ? inv : -inv, we, __uint_as_float(oe));
+        s_w[w][(col * GW + rg) * CG + rj] = make_float4(w0, wm, we, __uint_as_float(oe));
         unsigned* m = reinterpret_cast<unsigned*>(&s_m[w][col * GW + rg]);
         m[1 + rj] = n >= 2 ? DD_INNER | (unsigned)(up ? k0 + 1 : k0 - 1) * ks : 0u;
         if (rj == 0) m[0] = (unsigned)k0 * ks;
@@ -435,26 +430,26 @@ __device__ __forceinline__ void fwd_thin_body(const DdFwdArgs& a, int row, int c
     for (int ii = lo; ii < hi; ++ii, lp += lstride) {
       const double di = (double)ii;
       double t[3];
-      int k[3];
-      float f[3];
+      DdPos pos[3];
       Vec<SV> val[3];
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         t[j] = fma(di, fl[j].x, fl[j].y);
-        dd_cell(t[j], N, k[j], f[j]);
-        vload(val[j], lp + (size_t)k[j] * kstride);
+        pos[j] = dd_pos(t[j], N);
+        vload(val[j], lp + (size_t)pos[j].k * kstride);
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const float inv = j == 0 || two ? dd_rcpf((float)(t[j + 1] - t[j]) * dx) : 0.f;
-        const bool up = k[j + 1] > k[j], same = k[j + 1] == k[j];
-        vfma(acc[j], dup2(((same ? f[j + 1] : (up ? 1.f : 0.f)) - f[j]) * inv), val[j]);
-        vfma(acc[j], dup2(same ? 0.f : (up ? f[j + 1] : f[j + 1] - 1.f) * inv), val[j + 1]);
-        const int st = up ? 1 : -1;
-        for (int q = k[j] + st; !same && q != k[j + 1]; q += st) {
+        float w0, wm, we;
+        dd_walk(pos[j], pos[j + 1], inv, w0, wm, we);
+        vfma(acc[j], dup2(w0), val[j]);
+        vfma(acc[j], dup2(we), val[j + 1]);
+        const int k0 = pos[j].k, k1 = pos[j + 1].k, st = k1 > k0 ? 1 : -1;
+        for (int q = k0 + st; k1 != k0 && q != k1; q += st) {
           Vec<SV> v;
           vload(v, lp + (size_t)q * kstride);
-          vfma(acc[j], dup2(up ? inv : -inv), v);
+          vfma(acc[j], dup2(wm), v);
         }
       }
       if (++since == T::FLUSH || ii + 1 == hi) {
@@ -754,9 +749,9 @@ __device__ __forceinline__ void dd_block(const DdBackArgs& a, const ViewGeom& G,
     }
   } else {
     const bool xdom = fabs(sx) > fabs(sy);
-    const double c = fma(dd_angle(v, sx, sy, sxf, syf, s_at), a.inv_dbeta, a.cnt + DD_MAGIC);
+    const double c = fma(dd_angle(v, sx, sy, sxf, syf, s_at), a.inv_dbeta, a.cnt + DD_MAGIC24);
     const int kc = max(__double2hiint(c), 0x41300000) - 0x41380000;
-    const float fc = (float)((unsigned)__double2loint(c) >> 8) * 5.9604644775390625e-8f;
+    const float fc = dd_fraction24(c);
     const float idb = (float)a.inv_dbeta, hdb = h * idb;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(256) k_ps_back_ref(PsBackArgs a) {
   const float dxf = (float)a.dx, hdb = (float)(a.dx * 0.5 * a.inv_dbeta);
   // what the two constants' rounding, which every sample shares, takes off
   const float corr = (float)((a.dx * (a.dx * 0.5 * a.inv_dbeta)) / ((double)dxf * (double)hdb) - 1.0);
-  const double px = ((double)ix - a.ocx) * a.dx, py = ((double)y0 - a.ocy) * a.dx, cnt = a.cnt_ref + DD_MAGIC;
+  const double px = ((double)ix - a.ocx) * a.dx, py = ((double)y0 - a.ocy) * a.dx, cnt = a.cnt_ref + DD_MAGIC24;
   float acc[R];
 #pragma unroll
   for (int i = 0; i < R; ++i) acc[i] = 0.f;
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(256) k_ps_back_ref(PsBackArgs a) {
       if (full) alpha = dd_angle(v, sx, sy, sxf, syf, s_at);
       const double c = fma(alpha, a.inv_dbeta, cnt);
       const int kc = max(__double2hiint(c), 0x41300000) - 0x41380000;
-      const float fc = (float)((unsigned)__double2loint(c) >> 8) * 5.9604644775390625e-8f;
+      const float fc = dd_fraction24(c);
       const float l2 = fmaf(v.yf, v.yf, dx2f), ddv = xdom ? v.xf : v.yf;
       float l, rl;
       dd_length(l2, l, rl);
