@@ -1,9 +1,9 @@
 """Batched and served OS-SART reconstructions on one GPU.
 
-* `TileTuner` -- the autotuner: times the projector kernels for each
-  candidate tile shape of the table kernels (z-tile width) on a bucket's
-  shape and records the fastest in the library (ddfan_tune_set_zl,
-  ddfan_tune_set_nz) and in a JSON cache.
+* `TileTuner` -- the autotuner: times the table kernels for each candidate
+  tile shape (z-tile width) on a bucket's shape and records the fastest in
+  the library (ddfan_tune_set_zl) and in a JSON cache; modes without tables
+  have nothing to choose.
 * `Engine` -- continuous batching: requests of uneven sizes are admitted, in
   arrival order with back-fill, while the HBM budget (exact per-request
   estimates from ddfan_ossart_estimate_bytes) and the slot count allow; every
@@ -104,11 +104,13 @@ def make_instance(N, Z, P, seed, device, iters=5, numOfOS=24, I0=1.5e5):
 # ---------------------------------------------------------------- autotuner
 
 class TileTuner:
-    """Measures every valid tile shape for a slice count (4-slice blocks) on
-    a representative shape and keeps the fastest: the z-tile width (z-lanes
-    per channel or voxel group, 1-8 blocks) and, in the direct mode, a z-tiles
-    count per thread.  The table kernels follow them; the direct kernels take
-    their tiles from the slice count and the launch's size instead."""
+    """Measures every valid tile shape of the table kernels for a slice count
+    (4-slice blocks) on a representative shape and keeps the fastest: the z-tile
+    width (z-lanes per channel or voxel group, 1-8 blocks).  The hi/lo and direct
+    modes run kernels without tables, which take their tiles from the slice count
+    and the launch's size: for them a shape is timed once and nothing is
+    recorded (a choice among equal launches would be noise, and FP32 and FP64
+    plans of the same slice count would follow it)."""
 
     def __init__(self, cache_path=None, sat="hilo", back="adj"):
         self.cache_path = cache_path
@@ -134,8 +136,8 @@ class TileTuner:
                 json.dump({str(k): v for k, v in sorted(self.table.items())}, f, indent=1)
 
     def candidates(self, zb):
-        """(zl, nz) pairs worth timing for zb blocks: every width that fits,
-        and in the direct mode every z-tiles-per-thread count its tiles allow."""
+        """(zl, nz) pairs for zb blocks: every width that fits, and in the
+        direct mode every z-tiles-per-thread count its tiles allow."""
         out = []
         for zl in (8, 4, 2, 1):
             if zl > zb:
@@ -153,31 +155,21 @@ class TileTuner:
         zb = (Z + 3) // 4
         if zb in self.table:
             return self.table[zb]
-        s = configs.c2(SLN=Z)
-        x0, y0, xds, yds = dd2.fan_geometry(s.sid, s.sdd, s.DNU, s.detCellWidth, s.detCntIdx)
-        dx = 0.7 * 512 / N
-        angs = torch.from_numpy(s.angles(P)).to(device)
-        vol = torch.rand((N, N, Z), device=device) * 0.02
+        cands = self.candidates(zb)
+        if self.sat in ("hilo", "direct"):
+            # the kernels without tables take their tiles from the slice count
+            # whatever is recorded: one measurement stands for every candidate,
+            # and the record keeps what it holds
+            ms = self._time(N, Z, P, device, reps)
+            self.timings[zb] = {"%d,%d" % c: round(ms, 4) for c in cands}
+            self.table[zb] = [lib.ddfan_tune_get_zl(zb), lib.ddfan_tune_get_nz(zb) if self.sat == "direct" else 0]
+            return self.table[zb]
         best, best_ms, timings = None, float("inf"), {}
-        for zl, nz in self.candidates(zb):
+        for zl, nz in cands:
             lib.ddfan_tune_set_zl(zb, zl)
             lib.ddfan_tune_set_nz(zb, nz)
-            pl = Plan(x0, y0, s.DNU, xds, yds, s.detCntIdx, N, N, Z, P, dx, sat=self.sat,
-                      device=device.index)
-            prj = pl.proj(angs, vol)
-            out = torch.empty_like(vol)
-            pl.back(angs, prj, out=out, mode=self.back)
-            torch.cuda.synchronize(device)
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            for _ in range(reps):
-                pl.proj(angs, vol, out=prj)
-                pl.back(angs, prj, out=out, mode=self.back)
-            e1.record()
-            torch.cuda.synchronize(device)
-            ms = e0.elapsed_time(e1) / reps
+            ms = self._time(N, Z, P, device, reps)
             timings["%d,%d" % (zl, nz)] = round(ms, 4)
-            pl.close()
             if ms < best_ms:
                 best, best_ms = [zl, nz], ms
         lib.ddfan_tune_set_zl(zb, best[0])
@@ -185,6 +177,27 @@ class TileTuner:
         self.table[zb] = best
         self.timings[zb] = timings
         return best
+
+    def _time(self, N, Z, P, device, reps):
+        """Milliseconds of a forward + backprojection on a plan made now."""
+        s = configs.c2(SLN=Z)
+        x0, y0, xds, yds = dd2.fan_geometry(s.sid, s.sdd, s.DNU, s.detCellWidth, s.detCntIdx)
+        angs = torch.from_numpy(s.angles(P)).to(device)
+        vol = torch.rand((N, N, Z), device=device) * 0.02
+        pl = Plan(x0, y0, s.DNU, xds, yds, s.detCntIdx, N, N, Z, P, 0.7 * 512 / N, sat=self.sat, device=device.index)
+        prj = pl.proj(angs, vol)
+        out = torch.empty_like(vol)
+        pl.back(angs, prj, out=out, mode=self.back)
+        torch.cuda.synchronize(device)
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        for _ in range(reps):
+            pl.proj(angs, vol, out=prj)
+            pl.back(angs, prj, out=out, mode=self.back)
+        e1.record()
+        torch.cuda.synchronize(device)
+        pl.close()
+        return e0.elapsed_time(e1) / reps
 
 
 # ---------------------------------------------------------------- engine
