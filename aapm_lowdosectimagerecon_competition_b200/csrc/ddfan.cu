@@ -117,6 +117,14 @@ static int recorded_nz(int ZB) {
 
 int dd_pad(int Z) { return Z == 1 ? 1 : (Z <= 4 ? 4 : (Z + 7) / 8 * 8); }
 
+// The slices the direct kernels read for results in [r.lo, r.hi) of Z: whole
+// vectors of the padded operand
+static DdSlices dd_slices(DdSlices r, int Z, int Zs) {
+  const int v = Zs % 8 == 0 ? 8 : (Zs % 4 == 0 ? 4 : 1);
+  const int lo = std::max(0, r.lo), hi = r.hi < 0 ? Z : std::min(r.hi, Z);
+  return lo < hi ? DdSlices{lo / v * v, (hi + v - 1) / v * v} : DdSlices{0, 0};
+}
+
 bool dd_mode(int sat_mode, const uint8_t* mask, size_t npix) {
   if (sat_mode != SAT_HILO) return sat_mode == SAT_DIRECT;
   for (size_t i = 0; mask && i < npix; ++i)
@@ -676,15 +684,20 @@ int launch_back(const Plan& p, int back_mode, const ViewGeom* vg, const double2*
 static int grid_blocks(size_t n) { return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 148 * 16)); }
 
 int launch_stage_image(const float* src, int Z, const uint8_t* mask, float* dst, int Zp, size_t npix,
-                       cudaStream_t st) {
-  k_stage_image<<<grid_blocks(npix * Zp), 256, 0, st>>>(src, Z, mask, dst, Zp, npix);
+                       cudaStream_t st, DdSlices r) {
+  r = dd_slices(r, Z, Zp);
+  if (r.lo >= r.hi) return DDFAN_OK;
+  k_stage_image<<<grid_blocks(npix * (r.hi - r.lo)), 256, 0, st>>>(src, Z, mask, dst, Zp, npix, r.lo, r.hi);
   return check_launch("k_stage_image");
 }
 
 int launch_stage_sino(const float* src, int Z, const float* wgt, int U, float* dst, int Zp, size_t PN,
-                      cudaStream_t st) {
+                      cudaStream_t st, DdSlices r) {
+  r = dd_slices(r, Z, Zp);
+  if (r.lo >= r.hi) return DDFAN_OK;
   ProfScope ps(KIND_SAT_SINO, st);
-  k_stage_sino<<<grid_blocks((PN * (U + 1) + DD_PAST) * Zp), 256, 0, st>>>(src, Z, wgt, U, dst, Zp, PN);
+  k_stage_sino<<<grid_blocks((PN * (U + 1) + DD_PAST) * (r.hi - r.lo)), 256, 0, st>>>(src, Z, wgt, U, dst, Zp, PN, r.lo,
+                                                                                    r.hi);
   return check_launch("k_stage_sino");
 }
 
@@ -850,7 +863,7 @@ int proj_dev_shared(Plan& p, const float* d_angs, int stride, int PN, const floa
     const float* img = d_vol;
     if (p.has_mask || p.Z != p.Zs || (p.Zs % 4 == 0 && (reinterpret_cast<uintptr_t>(d_vol) & 15))) {
       if ((rc = launch_stage_image(d_vol, p.Z, p.has_mask ? p.d_mask : nullptr, p.d_tmp, p.Zs,
-                                   (size_t)p.XN * p.YN, st)))
+                                   (size_t)p.XN * p.YN, st, {zlo, zhi})))
         return rc;
       img = p.d_tmp;
     }
@@ -878,7 +891,9 @@ int back_dev_shared(Plan& p, const float* d_angs, int stride, int PN, const floa
   e.out = d_vol; e.mask = p.has_mask ? p.d_mask : nullptr; e.zlo = zlo; e.zhi = zhi;
   if (p.dd) {
     float* w = reinterpret_cast<float*>(p.d_satq);
-    if ((rc = launch_stage_sino(d_prj, p.Z, adj ? p.d_cvd : nullptr, p.U, w, p.Zs, (size_t)PN, st))) return rc;
+    if ((rc = launch_stage_sino(d_prj, p.Z, adj ? p.d_cvd : nullptr, p.U, w, p.Zs, (size_t)PN, st,
+                                {zlo, zhi})))
+      return rc;
     rc = launch_back_dd(p, back_mode, w, p.d_vg, PN, e, st);
     mark_use(p, st);
     return rc;

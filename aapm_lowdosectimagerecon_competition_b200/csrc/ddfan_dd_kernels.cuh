@@ -1100,20 +1100,22 @@ inline void dd_dispatch(int sv, int thin, F&& go) {
 
 // ============================================================ staging
 
-// dst[pix][z] = z < Z ? src[pix][z] * mask[pix] : 0 for z < Zp (mask, src null = 1):
-// the masked image with its slices padded to a multiple of 4.
+// dst[pix][z] = z < Z ? src[pix][z] * mask[pix] : 0 for za <= z < zb of Zp
+// slices (mask, src null = 1): the masked image with its slices padded, or the
+// vectors of a slice range of it.
 static __global__ void k_stage_image(const float* __restrict__ src, int Z, const uint8_t* __restrict__ mask,
-                                     float* __restrict__ dst, int Zp, size_t npix) {
-  const size_t n = npix * Zp;
+                                     float* __restrict__ dst, int Zp, size_t npix, int za, int zb) {
+  const int nz = zb - za;
+  const size_t n = npix * nz;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t pix = i / Zp;
-    const int z = (int)(i - pix * Zp);
+    const size_t pix = i / nz;
+    const int z = za + (int)(i - pix * nz);
     float v = 0.f;
     if (z < Z) {
       v = src ? src[pix * Z + z] : 1.f;
       if (mask && mask[pix] == 0) v = 0.f;
     }
-    dst[i] = v;
+    dst[pix * Zp + z] = v;
   }
 }
 
@@ -1129,13 +1131,14 @@ static __global__ void __launch_bounds__(256) k_columns(const float4* __restrict
 
 // dst[p][u][z] = src[p][u][z] * wgt[p][u] for u < U, z < Z; zero on the
 // guard channel u = U, on padding slices and on DD_PAST entries past the last
-// view (wgt, src null = 1).
+// view (wgt, src null = 1); za <= z < zb of Zp slices.
 static __global__ void k_stage_sino(const float* __restrict__ src, int Z, const float* __restrict__ wgt, int U,
-                                    float* __restrict__ dst, int Zp, size_t PN) {
-  const size_t n = (PN * (U + 1) + DD_PAST) * Zp;
+                                    float* __restrict__ dst, int Zp, size_t PN, int za, int zb) {
+  const int nz = zb - za;
+  const size_t n = (PN * (U + 1) + DD_PAST) * nz;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = i / Zp;
-    const int z = (int)(i - r * Zp);
+    const size_t r = i / nz;
+    const int z = za + (int)(i - r * nz);
     const size_t p = r / (U + 1);
     const int u = (int)(r - p * (U + 1));
     float v = 0.f;
@@ -1144,7 +1147,7 @@ static __global__ void k_stage_sino(const float* __restrict__ src, int Z, const 
       v = src ? src[e * Z + z] : 1.f;
       if (wgt) v *= wgt[e];
     }
-    dst[i] = v;
+    dst[r * Zp + z] = v;
   }
 }
 

@@ -180,12 +180,18 @@ int check_back_dd(const Plan& p, int back_mode);
 // orientations in one launch.
 int launch_back_dd(const Plan& p, int back_mode, const float* w, const ViewGeom* vg, int PN, const BackEpi& epi,
                    cudaStream_t st);
+// Slices [lo, hi) of a call's results (hi < 0: all of them).  The operands of
+// the direct kernels are staged for these only: a call of many slice groups,
+// each with its own angles, stages every slice about once.
+struct DdSlices {
+  int lo = 0, hi = -1;
+};
 // dst[pix][z < Zp] = z < Z ? src[pix][z] * mask : 0 (src null = 1)
 int launch_stage_image(const float* src, int Z, const uint8_t* mask, float* dst, int Zp, size_t npix,
-                       cudaStream_t st);
+                       cudaStream_t st, DdSlices r = {});
 // dst[p][u <= U][z < Zp] = u < U && z < Z ? src[p][u][z] * wgt[p][u] : 0 (src, wgt null = 1)
 int launch_stage_sino(const float* src, int Z, const float* wgt, int U, float* dst, int Zp, size_t PN,
-                      cudaStream_t st);
+                      cudaStream_t st, DdSlices r = {});
 // out[pix][z] = mask ? x[pix][z] : (clamp0 ? max(x0, 0) : x0)
 int launch_publish_masked(const float* x, int Zi, const float* x0, int Z, const uint8_t* mask, int clamp0,
                           float* out, size_t npix, cudaStream_t st);

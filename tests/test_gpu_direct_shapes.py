@@ -111,3 +111,41 @@ def test_per_slice_ref_backprojection_matches_oracle(XN, YN, Z, PN, U, cx, sat):
     args = (x0, y0, U, xds, yds, s.detCntIdx, np.float32(cx), np.float32(0), h, PN, XN, YN, Z, prj, s.dx)
     got, exp = dd2.MultiSlicesBackGPU(*args, sat=sat, back="ref"), O.back(*args, mode=O.REF)
     assert np.linalg.norm((got - exp).ravel()) < 2e-6 * np.linalg.norm(exp.ravel())
+
+
+# runs of slices with one angle list each; few enough that the calls stay
+# grouped (z-tiles of 8 or 32 slices against 1.45, 2.7 and 4.4 times the slices)
+GROUPS = [(96, (31, 96)), (96, (3, 61, 96)), (26, (13, 26)), (8, (5, 8)), (7, (2, 7))]
+
+
+@pytest.mark.parametrize("Z,ends", GROUPS)
+@pytest.mark.parametrize("sat", ["direct", "hilo"])
+def test_slice_groups_stage_their_own_slices(Z, ends, sat):
+    """Calls whose slices fall into runs with different angle lists stage each
+    run's vectors of slices only; runs that share a vector, begin or end inside
+    one, and few slices, against the oracle.  A second call on other inputs
+    meets what the first left in the staging buffers."""
+    import torch
+    from aapm_lowdosectimagerecon_competition_b200 import configs, dd2, device
+    from oracle import oracle as O
+    XN, YN, PN, U = 30, 26, 11, 40
+    s = configs.scaled(configs.c2(SLN=Z), XN=XN, DNU=U, PN=PN)
+    x0, y0, xds, yds = dd2.fan_geometry(s.sid, s.sdd, U, s.detCellWidth, s.detCntIdx)
+    a = s.angles()
+    h = np.stack([(a + 0.21 * sum(z >= e for e in ends)).astype(np.float32) for z in range(Z)], 1)
+    mask = np.ones((YN, XN), np.uint8)
+    mask[:, :2] = 0
+    plan = device.Plan(x0, y0, U, xds, yds, s.detCntIdx, XN, YN, Z, PN, s.dx, mask=mask, sat=sat)
+    hd = torch.from_numpy(np.ascontiguousarray(h)).cuda()
+    rel = lambda g, e: float(np.linalg.norm((g - e).ravel()) / np.linalg.norm(e.ravel()))
+    for seed in (1, 2):
+        rng = np.random.default_rng(seed)
+        vol = (rng.random((YN, XN, Z)) * 0.04).astype(np.float32)
+        prj = (rng.random((PN, U, Z)) - 0.3).astype(np.float32)
+        got = plan.proj(hd, torch.from_numpy(vol).cuda()).cpu().numpy()
+        assert rel(got, O.proj(x0, y0, U, xds, yds, 0, 0, h, PN, XN, YN, Z, vol, s.dx, mask)) < 2e-6
+        for back, mode in (("adj", O.ADJ), ("ref", O.REF)):
+            gb = plan.back(hd, torch.from_numpy(prj).cuda(), mode=back).cpu().numpy()
+            eb = O.back(x0, y0, U, xds, yds, s.detCntIdx, 0, 0, h, PN, XN, YN, Z, prj, s.dx, mask, mode=mode)
+            assert rel(gb, eb) < 2e-6, back
+    plan.close()
