@@ -782,10 +782,32 @@ __device__ __forceinline__ void dd_block(const DdBackArgs& a, const ViewGeom& G,
   }
 }
 
+// A thread's totals (4 voxels x SV slices), cleared; whether any is infinite or
+// NaN.  Where one is, the views are summed again value by value ("careful"): a
+// window value outside a voxel's footprint has weight 0 for that voxel, and 0
+// times an infinite or NaN value is NaN.  So such a value reaches the voxels
+// whose footprints hold it and no others, and finite data are summed once.  The
+// wide kernel takes its loop again, with the decode's one copy of the code: a
+// function of its own, called at the end, cost the REF kernel 5 % (0.93 -> 0.98
+// ms per c3 subset).  The thin one has the loop twice: the branch in it cost 2 %
+// (one slice of 256^2, 123 views, exact adjoint: 113 -> 115 us).
+template <int SV>
+__device__ __forceinline__ void back_dd_clear(float* tot) {
+#pragma unroll
+  for (int e = 0; e < 4 * SV; ++e) tot[e * DdBackTile<SV>::NT] = 0.f;
+}
+template <int SV>
+__device__ __forceinline__ bool back_dd_nonfinite(const float* tot) {
+  bool bad = false;
+#pragma unroll
+  for (int e = 0; e < 4 * SV; ++e) bad = bad || !(fabsf(tot[e * DdBackTile<SV>::NT]) <= 3.402823466e38f);
+  return bad;
+}
+
 // Measured per c3 subset (96 views x 736 channels, 512^2 x 128): reference
-// formula 1.40 -> 0.94 ms, exact adjoint 1.77 -> 1.10 ms (0.86 ms of either
+// formula 1.40 -> 0.91 ms, exact adjoint 1.77 -> 1.05 ms (0.86 ms of either
 // when the decode is left out); 1111 views of 384^2 x 45, exact adjoint 10.8 ->
-// 5.2 ms.  With each voxel decoded by itself (1.08 and 1.25 ms), 16 warps an SM at 128 registers with 4 values in flight each beat 24
+// 5.0 ms.  With each voxel decoded by itself (1.08 and 1.25 ms), 16 warps an SM at 128 registers with 4 values in flight each beat 24
 // at 80 with 1 (1.20), 3 (1.29) or 4 (1.14): more warps spread over more views
 // and lose the L1 hits (80 -> 68 %).
 //
@@ -839,8 +861,6 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
     __syncthreads();
   }
   float* tot = s_tot + tid;
-#pragma unroll
-  for (int e = 0; e < 4 * SV; ++e) tot[e * T::NT] = 0.f;
   Vec<SV> acc[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) vzero(acc[j]);
@@ -856,99 +876,115 @@ __device__ __forceinline__ void back_dd_body(const DdBackArgs& a, int tile, int 
     von = von || on[j];
   }
   const int vbeg = (int)((long long)a.PN * seg / nseg), vend = (int)((long long)a.PN * (seg + 1) / nseg);
-  int since = 0;
-  for (int v0 = vbeg; v0 < vend; v0 += VC) {
-    const int nvc = min(VC, vend - v0);
-    int mmax = 0;
-    for (int i0 = 0; i0 == 0 || i0 < mmax; i0 += MW) {  // windows wider than a record: more passes
-      if (lv < nvc) {
-        int kL[4], kR[4], m = 0, kb = 0x7fffffff, ke = -1;
-        float fL[4], fR[4], wgt[4];
-        if (von) {
-          dd_block<ADJ>(a, a.vg[v0 + lv], px, py, pxf, pyf, s_at, kL, fL, kR, fR, wgt);
-          // the block's window: the cells its footprints cover
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (on[j]) {
-              kb = min(kb, min(kL[j], kR[j]));
-              ke = max(ke, max(kL[j], kR[j]));
-            } else {
-              wgt[j] = 0.f;
-            }
-          }
-          // whole steps: more values, with weight 0, after the window or, at the
-          // detector's end, before it
-          m = (ke - kb + T::STEP) / T::STEP * T::STEP;
-          kb = max(min(kb, a.U + 1 - m), 0);
-        } else {
-          kb = 0;
-        }
-        mmax = max(mmax, m);
-        const int n = min(max(m - i0, 0), MW);
-        if (n) {
-          // the value in cell k has the weight of [cL, cR]'s part inside
-          // [k, k + 1] (negative where cR < cL): sat(cR - k) - sat(cL - k), the
-          // cells' difference exact
-          float dL[4], dR[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            dL[j] = (float)(kL[j] - kb - i0);
-            dR[j] = (float)(kR[j] - kb - i0);
-          }
-          float4* wp = reinterpret_cast<float4*>(&s_wt[w][lane * RS]);
-#pragma unroll 1
-          for (int i = 0; i < n; ++i, ++wp) {
-            float x[4];
+  for (bool careful = false;; careful = true) {
+    back_dd_clear<SV>(tot);
+    int since = 0;
+    for (int v0 = vbeg; v0 < vend; v0 += VC) {
+      const int nvc = min(VC, vend - v0);
+      int mmax = 0;
+      for (int i0 = 0; i0 == 0 || i0 < mmax; i0 += MW) {  // windows wider than a record: more passes
+        if (lv < nvc) {
+          int kL[4], kR[4], m = 0, kb = 0x7fffffff, ke = -1;
+          float fL[4], fR[4], wgt[4];
+          if (von) {
+            dd_block<ADJ>(a, a.vg[v0 + lv], px, py, pxf, pyf, s_at, kL, fL, kR, fR, wgt);
+            // the block's window: the cells its footprints cover
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              x[j] = (__saturatef(dR[j] + fR[j]) - __saturatef(dL[j] + fL[j])) * wgt[j];
-              dL[j] -= 1.f;
-              dR[j] -= 1.f;
+              if (on[j]) {
+                kb = min(kb, min(kL[j], kR[j]));
+                ke = max(ke, max(kL[j], kR[j]));
+              } else {
+                wgt[j] = 0.f;
+              }
             }
-            *wp = make_float4(x[0], x[1], x[2], x[3]);
+            // whole steps: more values, with weight 0, after the window or, at the
+            // detector's end, before it
+            m = (ke - kb + T::STEP) / T::STEP * T::STEP;
+            kb = max(min(kb, a.U + 1 - m), 0);
+          } else {
+            kb = 0;
+          }
+          mmax = max(mmax, m);
+          const int n = min(max(m - i0, 0), MW);
+          if (n) {
+            // the value in cell k has the weight of [cL, cR]'s part inside
+            // [k, k + 1] (negative where cR < cL): sat(cR - k) - sat(cL - k), the
+            // cells' difference exact
+            float dL[4], dR[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              dL[j] = (float)(kL[j] - kb - i0);
+              dR[j] = (float)(kR[j] - kb - i0);
+            }
+            float4* wp = reinterpret_cast<float4*>(&s_wt[w][lane * RS]);
+#pragma unroll 1
+            for (int i = 0; i < n; ++i, ++wp) {
+              float x[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                x[j] = (__saturatef(dR[j] + fR[j]) - __saturatef(dL[j] + fL[j])) * wgt[j];
+                dL[j] -= 1.f;
+                dR[j] -= 1.f;
+              }
+              *wp = make_float4(x[0], x[1], x[2], x[3]);
+            }
+          }
+          s_h[w][lane] = make_uint2((unsigned)(lv * (a.U + 1) + kb + (n ? i0 : 0)) * (unsigned)a.ZP, (unsigned)n);
+        }
+        mmax = __reduce_max_sync(0xffffffffu, mmax);
+        __syncwarp();
+        if (active) {
+          const char* qc = q + (size_t)v0 * vstride;
+          const uint2* hp = &s_h[w][g];
+          const unsigned char* rp = &s_wt[w][g * RS];
+#pragma unroll 1
+          for (int vv = 0; vv < nvc; ++vv, hp += GW, rp += GW * RS) {
+            const uint2 h = *hp;
+            const float4* wp = reinterpret_cast<const float4*>(rp);
+            const char* qp = qc + (size_t)h.x * VB;
+            if (careful) {
+#pragma unroll 1
+              for (int i = (int)h.y; i > 0; --i, qp += kstride, ++wp) {
+                Vec<SV> val;
+                vload(val, qp);
+                if (wp->x != 0.f) vfma(acc[0], dup2(wp->x), val);
+                if (wp->y != 0.f) vfma(acc[1], dup2(wp->y), val);
+                if (wp->z != 0.f) vfma(acc[2], dup2(wp->z), val);
+                if (wp->w != 0.f) vfma(acc[3], dup2(wp->w), val);
+              }
+              continue;
+            }
+#pragma unroll 1
+            for (int i = (int)h.y; i > 0; i -= T::STEP, qp += T::STEP * kstride, wp += T::STEP) {
+              Vec<SV> val[T::STEP];
+#pragma unroll
+              for (int t = 0; t < T::STEP; ++t) vload(val[t], qp + t * kstride);
+#pragma unroll
+              for (int t = 0; t < T::STEP; ++t) {
+                const float4 ww = wp[t];
+                vfma(acc[0], dup2(ww.x), val[t]);
+                vfma(acc[1], dup2(ww.y), val[t]);
+                vfma(acc[2], dup2(ww.z), val[t]);
+                vfma(acc[3], dup2(ww.w), val[t]);
+              }
+            }
           }
         }
-        s_h[w][lane] = make_uint2((unsigned)(lv * (a.U + 1) + kb + (n ? i0 : 0)) * (unsigned)a.ZP, (unsigned)n);
+        __syncwarp();
       }
-      mmax = __reduce_max_sync(0xffffffffu, mmax);
-      __syncwarp();
-      if (active) {
-        const char* qc = q + (size_t)v0 * vstride;
-        const uint2* hp = &s_h[w][g];
-        const unsigned char* rp = &s_wt[w][g * RS];
-#pragma unroll 1
-        for (int vv = 0; vv < nvc; ++vv, hp += GW, rp += GW * RS) {
-          const uint2 h = *hp;
-          const float4* wp = reinterpret_cast<const float4*>(rp);
-          const char* qp = qc + (size_t)h.x * VB;
-#pragma unroll 1
-          for (int i = (int)h.y; i > 0; i -= T::STEP, qp += T::STEP * kstride, wp += T::STEP) {
-            Vec<SV> val[T::STEP];
+      since += nvc;
+      if (since >= T::FLUSH || v0 + VC >= vend) {
+        since = 0;
 #pragma unroll
-            for (int t = 0; t < T::STEP; ++t) vload(val[t], qp + t * kstride);
+        for (int j = 0; j < 4; ++j) {
 #pragma unroll
-            for (int t = 0; t < T::STEP; ++t) {
-              const float4 ww = wp[t];
-              vfma(acc[0], dup2(ww.x), val[t]);
-              vfma(acc[1], dup2(ww.y), val[t]);
-              vfma(acc[2], dup2(ww.z), val[t]);
-              vfma(acc[3], dup2(ww.w), val[t]);
-            }
-          }
+          for (int s = 0; s < SV; ++s) tot[(j * SV + s) * T::NT] += vget(acc[j], s);
+          vzero(acc[j]);
         }
       }
-      __syncwarp();
     }
-    since += nvc;
-    if (since >= T::FLUSH || v0 + VC >= vend) {
-      since = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int s = 0; s < SV; ++s) tot[(j * SV + s) * T::NT] += vget(acc[j], s);
-        vzero(acc[j]);
-      }
-    }
+    if (careful || !__any_sync(0xffffffffu, back_dd_nonfinite<SV>(tot))) break;
   }
   if (nseg > 1) {
     __syncthreads();
@@ -989,8 +1025,6 @@ __device__ __forceinline__ void back_thin_body(const DdBackArgs& a, int tile, in
     __syncthreads();
   }
   float* tot = s_tot + tid;
-#pragma unroll
-  for (int e = 0; e < 4 * SV; ++e) tot[e * T::NT] = 0.f;
   Vec<SV> acc[4];
   bool on[4], any = false;
 #pragma unroll
@@ -1004,51 +1038,58 @@ __device__ __forceinline__ void back_thin_body(const DdBackArgs& a, int tile, in
   const float pxf = (float)px, pyf = (float)py;
   const int vbeg = (int)((long long)a.PN * seg / nseg), vend = (int)((long long)a.PN * (seg + 1) / nseg);
   const size_t kstride = (size_t)a.ZP * VB, vstride = (size_t)(a.U + 1) * kstride;
-  const char* q = reinterpret_cast<const char*>(a.q) + (size_t)vb * VB + (size_t)vbeg * vstride;
-  int since = 0;
-  for (int p = vbeg; any && p < vend; ++p, q += vstride) {
-    float fL[4], fR[4], wgt[4];
-    int kL[4], kR[4], kb = 0x7fffffff, ke = -1;
-    dd_block<ADJ>(a, a.vg[p], px, py, pxf, pyf, s_at, kL, fL, kR, fR, wgt);
+  const char* q0 = reinterpret_cast<const char*>(a.q) + (size_t)vb * VB + (size_t)vbeg * vstride;
+  const auto views = [&](auto careful) {
+    back_dd_clear<SV>(tot);
+    const char* q = q0;
+    int since = 0;
+    for (int p = vbeg; any && p < vend; ++p, q += vstride) {
+      float fL[4], fR[4], wgt[4];
+      int kL[4], kR[4], kb = 0x7fffffff, ke = -1;
+      dd_block<ADJ>(a, a.vg[p], px, py, pxf, pyf, s_at, kL, fL, kR, fR, wgt);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (on[j]) {
-        kb = min(kb, min(kL[j], kR[j]));
-        ke = max(ke, max(kL[j], kR[j]));
-      } else {
-        wgt[j] = 0.f;
+      for (int j = 0; j < 4; ++j) {
+        if (on[j]) {
+          kb = min(kb, min(kL[j], kR[j]));
+          ke = max(ke, max(kL[j], kR[j]));
+        } else {
+          wgt[j] = 0.f;
+        }
       }
-    }
-    // the value in cell k has the weight of [cL, cR]'s part inside [k, k + 1]:
-    // sat(cR - k) - sat(cL - k), the cells' difference exact
-    float dL[4], dR[4];
+      // the value in cell k has the weight of [cL, cR]'s part inside [k, k + 1]:
+      // sat(cR - k) - sat(cL - k), the cells' difference exact
+      float dL[4], dR[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      dL[j] = (float)(kL[j] - kb);
-      dR[j] = (float)(kR[j] - kb);
-    }
-    const char* qp = q + (size_t)kb * kstride;
+      for (int j = 0; j < 4; ++j) {
+        dL[j] = (float)(kL[j] - kb);
+        dR[j] = (float)(kR[j] - kb);
+      }
+      const char* qp = q + (size_t)kb * kstride;
 #pragma unroll 2
-    for (int k = kb; k <= ke; ++k, qp += kstride) {
-      Vec<SV> v;
-      vload(v, qp);
+      for (int k = kb; k <= ke; ++k, qp += kstride) {
+        Vec<SV> v;
+        vload(v, qp);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        vfma(acc[j], dup2((__saturatef(dR[j] + fR[j]) - __saturatef(dL[j] + fL[j])) * wgt[j]), v);
-        dL[j] -= 1.f;
-        dR[j] -= 1.f;
+        for (int j = 0; j < 4; ++j) {
+          const float x = (__saturatef(dR[j] + fR[j]) - __saturatef(dL[j] + fL[j])) * wgt[j];
+          if (!decltype(careful)::value || x != 0.f) vfma(acc[j], dup2(x), v);
+          dL[j] -= 1.f;
+          dR[j] -= 1.f;
+        }
+      }
+      if (++since == T::FLUSH || p + 1 == vend) {
+        since = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+          for (int s = 0; s < SV; ++s) tot[(j * SV + s) * T::NT] += vget(acc[j], s);
+          vzero(acc[j]);
+        }
       }
     }
-    if (++since == T::FLUSH || p + 1 == vend) {
-      since = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int s = 0; s < SV; ++s) tot[(j * SV + s) * T::NT] += vget(acc[j], s);
-        vzero(acc[j]);
-      }
-    }
-  }
+  };
+  views(std::false_type());
+  if (back_dd_nonfinite<SV>(tot)) views(std::true_type());
   if (nseg > 1) {
     __syncthreads();
     if (seg != 0) return;
