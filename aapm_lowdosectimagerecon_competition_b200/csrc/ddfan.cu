@@ -1103,6 +1103,21 @@ int back_dev_per_slice(Plan& p, const float* d_angs, const float* h_angs, int PN
   }, st);
 }
 
+// Device bytes of a plan that runs the direct kernels (dd) or keeps tables.
+size_t plan_bytes(int XN, int YN, int DNU, int SLN, int PNmax, int sat_mode, bool dd) {
+  int ZB = (SLN + 3) / 4;
+  const int ZL = pow2_zl(ZB);
+  ZB = (ZB + ZL - 1) / ZL * ZL;
+  const size_t F4 = cell_f4(sat_mode), U = (size_t)DNU, P = (size_t)PNmax;
+  const size_t Zs = (size_t)dd_pad(SLN);
+  const size_t cells = dd ? ((P * (U + 1) + DD_PAST) * Zs + 3) / 4 : 2 * (size_t)XN * YN * ZB * F4 + P * (U + 1) * ZB * F4;
+  const size_t tmp = (size_t)XN * YN * (dd ? (dd_wants_columns((int)Zs) ? 2 : 1) * Zs : (size_t)SLN);
+  return cells * sizeof(float4) + (2 * (U + 1) + 4 * U) * sizeof(double) + (size_t)XN * YN +
+         (U + 1) * sizeof(float) + 4 * (U + 1) * sizeof(uint16_t) + P * sizeof(ViewGeom) +
+         P * (U + 1) * sizeof(double2) + P * U * sizeof(float) + tmp * sizeof(float) +
+         P * sizeof(float) + P * sizeof(int) + 2 * sizeof(int);
+}
+
 }  // namespace ddfan
 
 // ====================================================================== C ABI
@@ -1138,18 +1153,8 @@ DDFAN_API int ddfan_tune_get_nz(int zblocks) { return zblocks < 1 ? 0 : recorded
 
 DDFAN_API size_t ddfan_plan_estimate_bytes(int XN, int YN, int DNU, int SLN, int PNmax, int sat_mode) {
   if (XN < 1 || YN < 1 || DNU < 2 || SLN < 1 || PNmax < 1 || sat_mode < 0 || sat_mode > SAT_DIRECT) return 0;
-  int ZB = (SLN + 3) / 4;
-  const int ZL = pow2_zl(ZB);
-  ZB = (ZB + ZL - 1) / ZL * ZL;
-  const size_t F4 = cell_f4(sat_mode), U = (size_t)DNU, P = (size_t)PNmax;
-  const bool direct = sat_mode == SAT_DIRECT || sat_mode == SAT_HILO;
-  const size_t Zs = (size_t)dd_pad(SLN);
-  const size_t cells = direct ? ((P * (U + 1) + DD_PAST) * Zs + 3) / 4 : 2 * (size_t)XN * YN * ZB * F4 + P * (U + 1) * ZB * F4;
-  const size_t tmp = (size_t)XN * YN * (direct ? (dd_wants_columns((int)Zs) ? 2 : 1) * Zs : (size_t)SLN);
-  return cells * sizeof(float4) + (2 * (U + 1) + 4 * U) * sizeof(double) + (size_t)XN * YN +
-         (U + 1) * sizeof(float) + 4 * (U + 1) * sizeof(uint16_t) + P * sizeof(ViewGeom) +
-         P * (U + 1) * sizeof(double2) + P * U * sizeof(float) + tmp * sizeof(float) +
-         P * sizeof(float) + P * sizeof(int) + 2 * sizeof(int);
+  const size_t dd = sat_mode >= SAT_HILO && sat_mode != SAT_FP64 ? plan_bytes(XN, YN, DNU, SLN, PNmax, sat_mode, true) : 0;
+  return sat_mode == SAT_DIRECT ? dd : std::max(dd, plan_bytes(XN, YN, DNU, SLN, PNmax, sat_mode, false));
 }
 
 DDFAN_API int ddfan_fan_geometry(float sid, float sdd, int DNU, float detCellWidth, float detCntIdx,

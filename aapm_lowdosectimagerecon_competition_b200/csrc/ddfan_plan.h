@@ -96,6 +96,8 @@ int dd_pad(int Z);
 // lists: the direct mode, and the hi/lo mode where every mask byte is 0 or 1
 // (its table kernels multiply by the byte, the direct ones only drop zeros).
 bool dd_mode(int sat_mode, const uint8_t* mask, size_t npix);
+// device bytes of a plan that runs the direct kernels (dd) or keeps tables
+size_t plan_bytes(int XN, int YN, int DNU, int SLN, int PNmax, int sat_mode, bool dd);
 // allows the direct kernels their dynamic shared memory on the
 // current device (dev names it in an error); before any launch there
 int dd_prepare_device(int dev);

@@ -932,39 +932,45 @@ DDFAN_API void ddfan_ossart_destroy(ddfan_ossart* s) { solver_free(reinterpret_c
 
 DDFAN_API size_t ddfan_ossart_estimate_bytes(int XN, int YN, int DNU, int SLN, int PNall, int numOfOS,
                                              int sat_mode) {
+  if (XN < 1 || YN < 1 || DNU < 2 || SLN < 1 || sat_mode < 0 || sat_mode > SAT_DIRECT) return 0;
   if (numOfOS < 1 || PNall < numOfOS) return 0;
   const size_t PNmax = (size_t)(PNall + numOfOS - 1) / numOfOS;
-  const bool direct = sat_mode == SAT_DIRECT || sat_mode == SAT_HILO;
-  // the direct kernels pad slices and keep a guard channel
-  const size_t Zi = direct ? (size_t)dd_pad(SLN) : (size_t)SLN;
-  const size_t U = (size_t)DNU, P = (size_t)PNall, V = (size_t)XN * YN * Zi;
-  const size_t plan = ddfan_plan_estimate_bytes(XN, YN, DNU, (int)Zi, (int)PNmax, sat_mode);
-  if (!plan) return 0;
-  size_t own = P * sizeof(ViewGeom) + P * (U + 1) * sizeof(double2) + P * U * sizeof(float) +
-               3 * P * sizeof(int) + 2 * (size_t)numOfOS * sizeof(int) + P * U * sizeof(float) +
-               (size_t)numOfOS * XN * YN * sizeof(float) + P * U * Zi * sizeof(float) +
-               2 * V * sizeof(float) + (PNmax * (U + (direct ? 1 : 0)) + (direct ? DD_PAST : 0)) * Zi * sizeof(float) + sizeof(double);
-  // direct kernels: the initial image and the published copy (masked solves;
-  // padded slices), sinogram staging and slice maps (padded slices)
-  if (direct) {
-    own += 2 * (size_t)XN * YN * SLN * sizeof(float);
-    if (Zi != (size_t)SLN) own += P * U * SLN * sizeof(float) + (Zi + SLN) * sizeof(int);
-    if (dd_wants_columns((int)Zi)) own += V * sizeof(float);
-  }
-  // transient at creation, direct kernels: the one-slice weight plan, the
-  // geometry of every view, the image and the rows of ones
-  if (direct)
-    return plan + own + ddfan_plan_estimate_bytes(XN, YN, DNU, 1, 1, sat_mode) +
-           P * (sizeof(ViewGeom) + (U + 1) * sizeof(double2) + (2 * U + 2) * sizeof(float)) +
-           (2 * (size_t)XN * YN + DD_PAST) * sizeof(float);
-  // otherwise: the one-slice weight plan and the slice-major weight buffers
-  // (geometry, row sums, ones, tables) over nsub x PNmax rows
-  const size_t R = (size_t)numOfOS * PNmax, CB = sat_mode == SAT_FP32 ? 8 : 16;
-  const size_t weights = ddfan_plan_estimate_bytes(XN, YN, DNU, 1, 1, sat_mode) +
-                         R * (sizeof(ViewGeom) + (U + 1) * sizeof(double2) + sizeof(float) + 3 * U * sizeof(float) +
-                              (U + 1) * CB) +
-                         (size_t)XN * YN * sizeof(float) + ((size_t)(XN + 2) * YN + (size_t)(YN + 2) * XN) * CB;
-  return plan + own + weights;
+  const size_t U = (size_t)DNU, P = (size_t)PNall, pix = (size_t)XN * YN;
+  const auto held = [&](bool dd) {
+    // the direct kernels pad slices and keep a guard channel
+    const size_t Zi = dd ? (size_t)dd_pad(SLN) : (size_t)SLN, V = pix * Zi;
+    size_t own = P * sizeof(ViewGeom) + P * (U + 1) * sizeof(double2) + P * U * sizeof(float) + 3 * P * sizeof(int) +
+                 2 * (size_t)numOfOS * sizeof(int) + P * U * sizeof(float) + (size_t)numOfOS * pix * sizeof(float) +
+                 P * U * Zi * sizeof(float) + 2 * V * sizeof(float) +
+                 (PNmax * (U + (dd ? 1 : 0)) + (dd ? DD_PAST : 0)) * Zi * sizeof(float) + sizeof(double);
+    // direct kernels: the initial image and the published copy (masked solves;
+    // padded slices), sinogram staging and slice maps (padded slices)
+    if (dd) {
+      own += 2 * pix * SLN * sizeof(float);
+      if (Zi != (size_t)SLN) own += P * U * SLN * sizeof(float) + (Zi + SLN) * sizeof(int);
+      if (dd_wants_columns((int)Zi)) own += V * sizeof(float);
+    }
+    return own + plan_bytes(XN, YN, DNU, (int)Zi, (int)PNmax, sat_mode, dd);
+  };
+  // transient at creation: the one-slice weight plan and, on the direct
+  // kernels, the geometry of every view, the image and the rows of ones ...
+  const auto weights_dd = [&] {
+    return plan_bytes(XN, YN, DNU, 1, 1, sat_mode, true) +
+           P * (sizeof(ViewGeom) + (U + 1) * sizeof(double2) + (2 * U + 2) * sizeof(float)) + (2 * pix + DD_PAST) * sizeof(float);
+  };
+  // ... otherwise the slice-major weight buffers (geometry, row sums, ones,
+  // tables) over nsub x PNmax rows
+  const auto weights_tables = [&] {
+    const size_t R = (size_t)numOfOS * PNmax, CB = sat_mode == SAT_FP32 ? 8 : 16;
+    return plan_bytes(XN, YN, DNU, 1, 1, cell_mode(sat_mode), false) +
+           R * (sizeof(ViewGeom) + (U + 1) * sizeof(double2) + sizeof(float) + 3 * U * sizeof(float) + (U + 1) * CB) +
+           pix * sizeof(float) + ((size_t)(XN + 2) * YN + (size_t)(YN + 2) * XN) * CB;
+  };
+  // a mask with bytes above 1 takes its weights from tables in every mode, and
+  // keeps tables for the hi/lo mode's iterations
+  if (sat_mode == SAT_DIRECT) return held(true) + std::max(weights_dd(), weights_tables());
+  const size_t tables = held(false) + weights_tables();
+  return sat_mode == SAT_HILO ? std::max(tables, held(true) + weights_dd()) : tables;
 }
 
 DDFAN_API size_t ddfan_ossart_device_bytes(const ddfan_ossart* s) {

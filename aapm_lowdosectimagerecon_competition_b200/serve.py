@@ -237,8 +237,13 @@ class Engine:
 
     def estimate(self, inst):
         s = inst.scan
-        return float(load().ddfan_ossart_estimate_bytes(s.XN, s.YN, s.DNU, s.SLN, s.PN, s.numOfOS,
-                                                        SAT_MODES[self.sat]))
+        mode = self.sat
+        if mode == "hilo":
+            # without tables unless the mask scales voxels or slices have lists of their own
+            h = s.hangs()
+            if (inst.mask is None or np.max(inst.mask) <= 1) and np.array_equal(h, np.broadcast_to(h[:, :1], h.shape)):
+                mode = "direct"
+        return float(load().ddfan_ossart_estimate_bytes(s.XN, s.YN, s.DNU, s.SLN, s.PN, s.numOfOS, SAT_MODES[mode]))
 
     def submit(self, inst, t_arrival=None):
         req = {"inst": inst, "t_arrival": time.perf_counter() if t_arrival is None else t_arrival,

@@ -72,8 +72,11 @@ DDFAN_API int ddfan_tune_get_zl(int zblocks);
  * them. */
 DDFAN_API int ddfan_tune_set_nz(int zblocks, int nz);
 DDFAN_API int ddfan_tune_get_nz(int zblocks);
-/* device bytes ddfan_plan_create / ddfan_ossart_create would allocate
+/* device bytes ddfan_plan_create / ddfan_ossart_create would allocate at most
  * (the solver figure includes its transient set-up buffers); 0 = bad sizes.
+ * DDFAN_SAT_HILO: the larger of what it takes with tables (a mask with bytes
+ * above 1; the windowed solver) and without; with one angle list for all slices
+ * and mask bytes 0 and 1 it allocates what the DDFAN_SAT_DIRECT figure says.
  * Both are for one angle list shared by all slices.  Per-slice lists take
  * more: a solver on the slice-major path about 16 B x (XN+2) x (YN+2) x SLN
  * x 2 for its tables plus 2 x 4 B x PNall x DNU x SLN for the sinogram and
