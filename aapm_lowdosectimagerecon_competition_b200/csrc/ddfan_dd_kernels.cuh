@@ -134,8 +134,9 @@ struct DdFwdTile {
   static constexpr int CG = DDFAN_DD_FWD_CG;
   static constexpr int REC = 128;      // (line, channel) walks a warp decodes at a time
   static constexpr int FLUSH = 32;     // lines per FP32 partial sum
-  // dynamic shared memory of the ray totals
-  static constexpr int DYN = CG * SV * NT * (int)sizeof(float);
+  static constexpr int THIN_CG = 2;    // channels per thread of fwd_thin_body
+  // dynamic shared memory of the ray totals, of either body
+  static constexpr int DYN = (CG > THIN_CG ? CG : THIN_CG) * SV * NT * (int)sizeof(float);
 };
 
 // The lines that any footprint of channels [wc0, wc0 + n) meets, and of those
@@ -394,6 +395,7 @@ template <int SV>
 __device__ __forceinline__ void fwd_thin_body(const DdFwdArgs& a, int row, int cblk, int ztile) {
   using T = DdFwdTile<SV>;
   constexpr int NW = T::NW, VB = SV * 4;
+  static_assert(T::THIN_CG == 2, "the body's two channels");
   extern __shared__ float s_tot[];  // [2 * SV][NT]: this thread's totals at tid
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const int nseg = a.nseg, wch = w / nseg, seg = w - wch * nseg;
