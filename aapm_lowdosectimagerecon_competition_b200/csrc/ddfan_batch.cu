@@ -2,14 +2,15 @@
 // kernel kind, subset step and vector class over a device work list of every
 // solve's CTAs, instead of one launch per solve.
 //
-// A batched iteration runs subset step k of every solve that has one: the
-// forward projectors (with the fused residual) of all those solves in one
-// launch per class (slices per thread; thin or not), then the backprojections the same way
-// (the exact adjoint's, then the reference's), then FISTA of every solve in
-// one launch pair.  Each CTA reads its item {solve's argument
-// block, view row or voxel tile, channel block, z-tile} and runs the
-// same kernel body a single solve's launch runs, with that solve's arguments,
-// so every solve computes exactly what it computes alone.  Small solves
+// A batched iteration runs subset step k of every solve that has one: the image
+// columns of the solves of few slices, the forward projectors (with the fused
+// residual) of all those solves in one launch per class (slices per thread;
+// thin or not), then the backprojections the same way (the exact adjoint's,
+// then the reference's), then FISTA of every solve in one launch pair.  Each
+// CTA reads its item {solve's argument block, view row or voxel tile, channel
+// block, z-tile} and runs the same kernel body a single solve's launch runs,
+// with that solve's arguments, so every solve computes exactly what it computes
+// alone.  Small solves
 // (a few slices, a few hundred views) that leave most of the GPU idle in a
 // launch of their own fill it together.  The iteration is captured as one
 // CUDA graph.  No counterpart in the reference, which runs one
@@ -33,7 +34,7 @@ namespace ddfan {
 
 namespace {
 
-enum BatchKind { BK_FWD = 0, BK_ADJ = 1, BK_REF = 2 };
+enum BatchKind { BK_FWD = 0, BK_ADJ = 1, BK_REF = 2, BK_COL = 3 };
 
 struct BatchLaunch {
   int kind, sv, thin;  // the kernels' class (dd_dispatch)
@@ -73,6 +74,7 @@ struct Batch {
   std::vector<BatchLaunch> launches;  // one iteration, in order
   DdFwdArgs* d_fargs = nullptr;
   DdBackArgs* d_bargs = nullptr;
+  ColArgs* d_cargs = nullptr;
   int4* d_items = nullptr;
   FistaDesc* d_fista = nullptr;
   int nfista = 0;
@@ -101,7 +103,7 @@ static void batch_free(Batch* b) {
   }
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   if (b->graph) cudaGraphDestroy(b->graph);
-  void* ptrs[] = {b->d_fargs, b->d_bargs, b->d_items, b->d_fista};
+  void* ptrs[] = {b->d_fargs, b->d_bargs, b->d_cargs, b->d_items, b->d_fista};
   for (void* q : ptrs) dev_free(q, b->own);
   if (b->own) cudaStreamDestroy(b->own);
   if (b->last_use) cudaEventDestroy(b->last_use);
@@ -118,7 +120,10 @@ static int batch_launch(Batch& b, const BatchLaunch& L, cudaStream_t st) {
   {
     const int4* it = b.d_items + L.items_off;
     const unsigned n = (unsigned)L.nitems;
-    if (L.kind == BK_FWD) {
+    if (L.kind == BK_COL) {
+      ProfScope ps(KIND_FWD, st);
+      k_columns_batch<<<n, 256, 0, st>>>(b.d_cargs, it);
+    } else if (L.kind == BK_FWD) {
       ProfScope ps(KIND_FWD, st);
       dd_dispatch(L.sv, L.thin, [&](auto SV, auto THIN) {
         constexpr int v = decltype(SV)::value;
@@ -203,6 +208,8 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
   for (Solver* s : b.sv) maxsub = std::max(maxsub, s->nsub);
   std::vector<DdFwdArgs> fargs;
   std::vector<DdBackArgs> bargs;
+  std::vector<ColArgs> cargs;
+  std::vector<int> col_of(b.sv.size(), -1);  // each solver's entry in cargs
   std::vector<int4> items;
   // solver groups: largest solves first, dealt round robin
   int G = DDFAN_BATCH_GROUPS;
@@ -220,7 +227,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
   // per group, per step: class -> items, for each kind
   for (int grp = 0; grp < G; ++grp)
   for (int k = 0; k < maxsub; ++k) {
-    std::map<std::pair<int, int>, std::vector<int4>> fwd, back_adj, back_ref;  // by class
+    std::map<std::pair<int, int>, std::vector<int4>> cols, fwd, back_adj, back_ref;  // by class
     for (size_t si = 0; si < b.sv.size(); ++si) {
       if (group_of[si] != grp) continue;
       Solver& s = *b.sv[si];
@@ -235,8 +242,16 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
       DdResidual r;
       r.y = s.d_y; r.yview = s.d_yview + o; r.rowsum = s.d_rows + (size_t)o * s.U; r.wgt = adj ? cvd : nullptr;
       r.ystride = s.Zi;
-      const DdFwdArgs fa = make_fwd_dd_args(p, s.d_x, nullptr, vg, fc, cvd, s.d_order + o, c, s.d_ax, s.U + 1, s.Zi, 0, s.Zi, &r);
+      const DdFwdArgs fa = make_fwd_dd_args(p, s.d_x, s.d_xt, vg, fc, cvd, s.d_order + o, c, s.d_ax, s.U + 1, s.Zi, 0, s.Zi, &r);
       if (fa.nvb < 1) continue;
+      if (s.d_xt) {
+        if (col_of[si] < 0) {
+          col_of[si] = (int)cargs.size();
+          cargs.push_back(ColArgs{s.d_x, s.d_xt, s.XN, s.YN, s.Zi});
+        }
+        for (int y = 0; y < (s.YN + 31) / 32; ++y)
+          for (int x = 0; x < (s.XN + 31) / 32; ++x) cols[{0, 0}].push_back(make_int4(col_of[si], x, y, 0));
+      }
       const int fi = (int)fargs.size();
       fargs.push_back(fa);
       const int ncb = dd_fwd_cblocks(fa);
@@ -268,6 +283,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
         b.launches.push_back(L);
       }
     };
+    emit(BK_COL, cols);
     emit(BK_FWD, fwd);
     emit(BK_ADJ, back_adj);
     emit(BK_REF, back_ref);
@@ -310,7 +326,7 @@ static int batch_create(Batch** out, Solver* const* solvers, int n) {
     if (ee != cudaSuccess) return set_err(DDFAN_ERR_CUDA, "batch: upload: %s", cudaGetErrorString(ee));
     return DDFAN_OK;
   };
-  if ((rc = up(&b.d_fargs, fargs)) || (rc = up(&b.d_bargs, bargs)) ||
+  if ((rc = up(&b.d_fargs, fargs)) || (rc = up(&b.d_bargs, bargs)) || (rc = up(&b.d_cargs, cargs)) ||
       (rc = up(&b.d_items, items)) || (rc = up(&b.d_fista, fista)))
     return rc;
   // the pageable sources above are consumed before they go out of scope

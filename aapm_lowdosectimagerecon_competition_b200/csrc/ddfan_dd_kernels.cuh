@@ -1172,6 +1172,36 @@ static __global__ void __launch_bounds__(256) k_columns(const float4* __restrict
   }
 }
 
+// The same for many images in one launch (batched reconstructions): CTA b takes
+// item {image, 32-pixel column block, row block} = items[b].
+struct ColArgs {
+  const float* in;
+  float* out;
+  int XN, YN, Zs;  // Zs = 1, or a multiple of 4
+};
+static __global__ void __launch_bounds__(256) k_columns_batch(const ColArgs* __restrict__ args, const int4* __restrict__ items) {
+  __shared__ float t[32][33];
+  const int4 it = items[blockIdx.x];
+  const ColArgs a = args[it.x];
+  const int x0 = it.y * 32, y0 = it.z * 32;
+  if (a.Zs == 1) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = w; i < 32; i += 8)
+      if (y0 + i < a.YN && x0 + lane < a.XN) t[i][lane] = a.in[(size_t)(y0 + i) * a.XN + x0 + lane];
+    __syncthreads();
+    for (int i = w; i < 32; i += 8)
+      if (x0 + i < a.XN && y0 + lane < a.YN) a.out[(size_t)(x0 + i) * a.YN + y0 + lane] = t[lane][i];
+    return;
+  }
+  const int P = a.Zs / 4;
+  const float4* in = reinterpret_cast<const float4*>(a.in);
+  float4* out = reinterpret_cast<float4*>(a.out);
+  for (int e = threadIdx.x; e < 32 * 32 * P; e += 256) {
+    const int z = e % P, i = e / P, y = y0 + (i & 31), x = x0 + (i >> 5);
+    if (x < a.XN && y < a.YN) out[((size_t)x * a.YN + y) * P + z] = in[((size_t)y * a.XN + x) * P + z];
+  }
+}
+
 // dst[p][u][z] = src[p][u][z] * wgt[p][u] for u < U, z < Z; zero on the
 // guard channel u = U, on padding slices and on DD_PAST entries past the last
 // view (wgt, src null = 1); za <= z < zb of Zp slices.

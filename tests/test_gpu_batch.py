@@ -84,3 +84,32 @@ def test_batch_refuses_table_mode_solvers():
     with pytest.raises(DdfanError):
         device.OSSARTBatch([sv])
     sv.close()
+
+
+def test_batched_solves_of_few_slices_run_the_solo_kernels():
+    """Solves of up to 8 slices read x-major views from the image's columns, in
+    a batch as alone: as many launches a step as one solve of their class, and
+    the same bits.  Odd sizes; 1, 2, 5 and 8 slices."""
+    import torch
+    from aapm_lowdosectimagerecon_competition_b200 import configs, dd2, device
+    from oracle import oracle as O
+    for sizes in ([(45, 1, 60), (33, 1, 40), (64, 1, 41)], [(31, 2, 40), (40, 5, 48), (65, 8, 52)]):
+        svs, solo = [], []
+        for i, (N, Z, P) in enumerate(sizes):
+            s, (x0, y0, xds, yds), mask, y = _case(configs, dd2, O, N, Z, P, 4, i % 2 == 0, 40 + i)
+            for keep in (solo, svs):
+                sv = device.OSSART(x0, y0, s.DNU, xds, yds, s.detCntIdx, s.hangs(), s.XN, s.YN, s.SLN, s.dx, mask=mask,
+                                   numOfOS=4, useFISTA=1, nonneg=1, sat="direct", back="ref")
+                sv.set_sinogram(torch.from_numpy(y).cuda())
+                sv.set_image(torch.zeros((s.YN, s.XN, s.SLN), device="cuda"))
+                keep.append(sv)
+        batch = device.OSSARTBatch(svs)
+        if sizes[0][1] == 1:  # one class of kernels
+            assert batch.launches_per_iter == solo[0].launches_per_iter
+        batch.iterate(2)
+        for sv, alone in zip(svs, solo):
+            alone.iterate(2)
+            np.testing.assert_array_equal(sv.image().cpu().numpy(), alone.image().cpu().numpy())
+        batch.close()
+        for sv in svs + solo:
+            sv.close()
