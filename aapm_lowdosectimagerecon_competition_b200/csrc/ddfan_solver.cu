@@ -564,11 +564,12 @@ static int solver_weights_cells(Solver& s, const PlanDesc& d, const std::vector<
 // Row sums and column sums of every subset from slice 0's angles
 // (AAPM_script/OSSART_AAPM.m:57-66) on the direct kernels' one-slice form: the
 // row sums of all views in one forward launch of the masked image of ones, the
-// column sums one backprojection launch per subset over its rows of ones.  Both
-// backprojectors' geometry is FP64 there, so the REF weights need no other
-// kernels.  A whole c1 call (set-up, 40 subset steps, transfers) went from 18.1
-// to 9.2 ms with the set-up off the 4-slice cells.  Per-slice solvers keep
-// theirs (their residuals on rotated slices amplify any change of the sums).
+// column sums one backprojection launch per subset over its rows of ones.  The
+// column sums come from the arithmetic that the direct solvers backproject with
+// (a block's centre in FP64, its voxels' offsets, half-widths and weights in
+// FP32), so a voxel that a subset barely sees is divided by the sum of the very
+// parts it was given.  A whole c1 call (set-up, 40 subset steps, transfers) went
+// from 18.1 to 9.2 ms with the set-up off the 4-slice cells.
 static int solver_weights_dd(Solver& s, const PlanDesc& d, const std::vector<float>& angs0, cudaStream_t st) {
   const int XN = s.XN, YN = s.YN, U = s.U, P = s.PNall;
   const bool adj = s.back_mode == DDFAN_BACK_ADJ;
@@ -612,10 +613,9 @@ static int solver_weights_dd(Solver& s, const PlanDesc& d, const std::vector<flo
 // one forward launch, and the column sums of all subsets in one
 // backprojection launch, subset k standing in the place of slice k (its views
 // are rows k * cs + m; the pad rows of a short subset backproject zeros).
-// For the solvers that do not run the direct kernels, and the exact adjoint
-// only: the slice-major REF backprojector takes its
-// half-width and weight in FP32, and column sums divide every update, so the
-// REF weights stay on the cell kernels' FP64 formula.
+// For the solvers with tables (FP32 and FP64 modes, the windowed solver, masks
+// with bytes above 1), and the exact adjoint only: the REF weights of these stay
+// on the cell kernels, whose half-width and weight are FP64.
 static int solver_weights(Solver& s, const PlanDesc& d, const std::vector<float>& angs0, int PNmax,
                           cudaStream_t st) {
   const int XN = s.XN, YN = s.YN, DNU = s.U, nsub = s.nsub, cs = PNmax;
@@ -874,7 +874,11 @@ static int solver_create(Solver** out, float x0, float y0, int DNU, const float*
     DDFAN_CK(cudaMemsetAsync(s.d_xu, 0, sizeof(float) * XN * YN * SLN, st));
     DDFAN_CK(cudaStreamSynchronize(st));
   }
-  rc = s.direct && dd_mode(SAT_HILO, mask, (size_t)XN * YN)
+  // the direct kernels' weights for the solvers that run them, and for the
+  // slice-major ones of the same modes: row sums of grazing rays right relative to
+  // themselves (error of a solve of 384^2 x 24, 720 views, a list per slice: REF
+  // 3.0e-7 -> 2.0e-7, exact adjoint 6.2e-7 -> 2.0e-7 against tables' row sums)
+  rc = (s.direct || (s.ps && sat_mode == SAT_HILO)) && dd_mode(SAT_HILO, mask, (size_t)XN * YN)
            ? solver_weights_dd(s, d, angs0, st)
            : solver_weights(s, d, angs0, PNsub, st);
   if (rc) return rc;
