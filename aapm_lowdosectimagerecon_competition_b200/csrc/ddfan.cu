@@ -744,13 +744,14 @@ DdFwdArgs make_fwd_dd_args(const Plan& p, const float* img, const float* imgT, c
   a.vb0 = a.zlo / a.sv;
   a.nvb = a.zhi > a.zlo ? (a.zhi + a.sv - 1) / a.sv - a.vb0 : 0;
   a.thin = a.sv == 1 || a.nvb <= DD_THIN;
-  // 64 slices a tile: the image part that the views in flight share then stays
-  // below half of L2 (128 slices, 512^2, 96 views: 1.31 ms in one tile, 1.28 in
-  // two, 1.47 in four)
-  a.zl = a.thin ? 1 : dd_lanes(a.nvb, 8);
+  // One tile of 128 slices while all views' part of the image stays within three
+  // quarters of L2, else 64: 512^2 (134 MB), 96 views, 1.29 ms in one tile, 1.27 in
+  // two, 1.47 in four; 768^2 3.03 and 3.00; 384^2 (75 MB) 0.82 and 0.87; 256^2 0.53
+  // and 0.56.
+  a.zl = a.thin ? 1 : dd_lanes(a.nvb, (size_t)p.XN * p.YN * std::min(a.nvb * a.sv, 128) * 4 <= (size_t)96 << 20 ? 16 : 8);
   a.nzt = (a.nvb + a.zl - 1) / a.zl;
-  // a launch of fewer warps than the SMs hold (24 each) splits every ray's
-  // lines over 2, 4 or 8 of them
+  // a launch of fewer warps than the SMs hold (24 each, three CTAs) splits every
+  // ray's lines over 2, 4 or 8 of them
   const long long warps = (long long)PN * ((p.U + dd_fwd_channels(a) - 1) / dd_fwd_channels(a)) * a.nzt;
   a.nseg = 1;
   while (a.nseg < 8 && warps * a.nseg < 148 * 24) a.nseg *= 2;
@@ -807,8 +808,9 @@ DdBackArgs make_back_dd_args(const Plan& p, int back_mode, const float* w, const
   a.thin = a.sv == 1 || a.nvb <= DD_THIN;
   a.zl = a.thin ? 1 : dd_lanes(a.nvb, 32);
   a.nzt = (a.nvb + a.zl - 1) / a.zl;
-  // a launch of fewer warps than the SMs hold (24 each) splits the views over
-  // 2, 4 or 8 of them
+  // a launch of few warps splits the views over 2, 4 or 8 of them, up to 24 warps
+  // an SM: what the 4-slice kernels hold; the 8-slice and one-slice ones hold 16,
+  // and other lines have not been measured for them
   const long long GW = 32 / a.zl, nbx = (a.XN + 1) / 2, nby = (a.YN + 1) / 2;
   const long long warps = (a.thin ? (nbx * nby + 31) / 32 : (nbx + GW - 1) / GW * nby) * a.nzt;
   a.nseg = 1;

@@ -149,3 +149,44 @@ def test_slice_groups_stage_their_own_slices(Z, ends, sat):
             eb = O.back(x0, y0, U, xds, yds, s.detCntIdx, 0, 0, h, PN, XN, YN, Z, prj, s.dx, mask, mode=mode)
             assert rel(gb, eb) < 2e-6, back
     plan.close()
+
+
+@pytest.mark.parametrize("offset", [0, 4, 1])
+def test_image_alignment(offset):
+    """An image 16 but not 32 bytes aligned is read in vectors of 4 slices
+    instead of 8, one that is neither is staged first; 16 and 72 slices (one
+    z-tile and two), against the oracle."""
+    import torch
+    from aapm_lowdosectimagerecon_competition_b200 import configs, dd2, device
+    from oracle import oracle as O
+    for Z in (16, 72):
+        XN, YN, PN, U = 30, 26, 13, 40
+        s = configs.scaled(configs.c2(SLN=Z), XN=XN, DNU=U, PN=PN)
+        x0, y0, xds, yds = dd2.fan_geometry(s.sid, s.sdd, U, s.detCellWidth, s.detCntIdx)
+        vol = (np.random.default_rng(Z).random((YN, XN, Z)) * 0.04).astype(np.float32)
+        buf = torch.zeros(vol.size + 8, device="cuda")
+        img = buf[offset:offset + vol.size].view(YN, XN, Z)
+        img.copy_(torch.from_numpy(vol))
+        assert img.data_ptr() % 32 == 4 * offset
+        plan = device.Plan(x0, y0, U, xds, yds, s.detCntIdx, XN, YN, Z, PN, s.dx, sat="direct")
+        got = plan.proj(torch.from_numpy(s.angles()).cuda(), img).cpu().numpy()
+        plan.close()
+        exp = O.proj(x0, y0, U, xds, yds, 0, 0, s.hangs(), PN, XN, YN, Z, vol, s.dx)
+        assert np.linalg.norm((got - exp).ravel()) < 2e-6 * np.linalg.norm(exp.ravel())
+
+
+# one z-tile of 16 vectors, and two of 8 for an image that L2 does not hold
+@pytest.mark.parametrize("N,PN,U", [(96, 9, 64), (512, 5, 48)])
+def test_many_slices_in_one_tile_or_two(N, PN, U):
+    import torch
+    from aapm_lowdosectimagerecon_competition_b200 import configs, dd2, device
+    from oracle import oracle as O
+    Z = 128
+    s = configs.scaled(configs.c2(SLN=Z), XN=N, DNU=U, PN=PN)
+    x0, y0, xds, yds = dd2.fan_geometry(s.sid, s.sdd, U, s.detCellWidth, s.detCntIdx)
+    vol = (np.random.default_rng(N).random((N, N, Z), dtype=np.float32) * np.float32(0.04))
+    plan = device.Plan(x0, y0, U, xds, yds, s.detCntIdx, N, N, Z, PN, s.dx, sat="direct")
+    got = plan.proj(torch.from_numpy(s.angles()).cuda(), torch.from_numpy(vol).cuda()).cpu().numpy()
+    plan.close()
+    exp = O.proj(x0, y0, U, xds, yds, 0, 0, s.hangs(), PN, N, N, Z, vol, s.dx)
+    assert np.linalg.norm((got - exp).ravel()) < 2e-6 * np.linalg.norm(exp.ravel())
