@@ -201,7 +201,7 @@ __device__ __forceinline__ void dd_fwd_store(const DdFwdArgs& a, int p, int u, i
 }
 
 // What bounds it (c3 subset, 96 views x 736 channels x 512^2 x 128): the loads'
-// latency, and behind it the L1 pipe -- 1.28 ms (1.30 in one tile of 128
+// latency, and behind it the L1 pipe -- 1.26 ms (1.29 in one tile of 128
 // slices), of which 1.0 ms remain when every load hits L1; 14.2 GB cross from
 // L2 (every view reads the image once: 12.9 GB) at 11 TB/s; 60 % of L1's
 // wavefronts, 95 % L2 hits.  24 warps an SM at 80 registers and 2 channels a

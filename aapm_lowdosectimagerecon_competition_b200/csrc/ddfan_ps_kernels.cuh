@@ -534,8 +534,12 @@ __global__ void __launch_bounds__(256) k_ps_back_adj(PsBackArgs a) {
 // to the fraction in FP32.  What bounds it is instruction issue: conversions to
 // and from FP64 and 64-bit integers, which share a slow unit, made up most of
 // the 141 instructions a pixel and view took before: 384^2 x 24 slices, 720
-// views of 736 channels, hi/lo cells: 11.1 -> 8.9 ms, error of a solve against
-// 64 bits 1.8 .. 5.5e-7 -> 1.9 .. 3.2e-7 over seven sizes.  16 rows a warp: the same.
+// views of 736 channels, hi/lo cells: 11.1 -> 8.9 ms; error of one channel's
+// backprojection against 64 bits 1.0e-7 -> 0.8e-7, of a channel at the disk's edge
+// 2.4e-6 -> 3e-7.  Of eight solves it made four better and four worse, all within
+// 1.9 .. 4.7e-7, as long as their row sums came from tables (the old truncation
+// offset part of theirs); with the direct kernels' row sums they are at 2.0 ..
+// 3.6e-7.  16 rows a warp: the same.
 template <int M>
 __global__ void __launch_bounds__(256) k_ps_back_ref(PsBackArgs a) {
   constexpr int R = kPsRefRows, PX = 32;
