@@ -376,8 +376,8 @@ int rebin_prepare(RebinHost& h, long long nViews, const float* zPos, int SLN, fl
 }
 
 // channel blocks of k_rebin_routine: 96 slices of a 736 x 64 scan took 0.98 ms
-// (up to 1.02 on other boxes) with 4, 1.00 with 1, 1.05 with 8, 1.24 with 16 (2.22 in view order); three
-// other scans 4 too
+// with 4 (0.98 to 1.02 in later runs), 1.00 with 1, 1.05 with 8, 1.24 with 16
+// (2.22 in view order); three other scans 4 too
 #ifndef DDFAN_REBIN_CBLOCKS
 #define DDFAN_REBIN_CBLOCKS 4
 #endif

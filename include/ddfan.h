@@ -45,8 +45,9 @@ extern "C" {
 /* no tables: each difference of two interpolated prefix sums is evaluated as
  * the sum of the values it telescopes to (exact overlap weights, FP32, no
  * cancellation).  Used on the paths with one angle list for all slices, in the
- * hi/lo mode too (its errors there are no larger than the hi/lo tables' and it
- * takes half their time or less); paths that keep tables (per-slice angle
+ * hi/lo mode too (its errors there are the hi/lo tables' or smaller --
+ * projections at 24 sizes 7.3e-8 to 8.6e-8 against 7.9e-8 to 1.3e-7, at one of
+ * them 3 % above the tables' -- and it takes half their time or less); paths that keep tables (per-slice angle
  * lists) use hi/lo FP32 pairs in both modes.  Solvers of this mode can be
  * batched. */
 #define DDFAN_SAT_DIRECT 3
